@@ -31,11 +31,12 @@ struct Blocking {
     }
     // Monarch position of natural token n.
     __host__ __device__ __forceinline__ int nat2mon(int n) const {
-        int j = n % ww; int t = n / ww;
-        int e = t % w_reduce; t /= w_reduce;
-        int i = t % hh; t /= hh;
-        int c = t % h_reduce; t /= h_reduce;
-        int f = t % f_tied; int a = t / f_tied;
+        // bands of one (no reduction) and groups of one frame are common: their divisions are skipped
+        const int frow = n / w, col = n - frow * w;                 // row of the whole token grid, column
+        const int frame = frow / h, row = frow - frame * h;
+        const int e = w_reduce == 1 ? 0 : col / ww, j = col - e * ww;
+        const int c = h_reduce == 1 ? 0 : row / hh, i = row - c * hh;
+        const int a = f_tied == 1 ? frame : frame / f_tied, f = frame - a * f_tied;
         return ((((a * h_reduce + c) * w_reduce + e) * f_tied + f) * hh + i) * ww + j;
     }
 };

@@ -6,11 +6,15 @@
 
 namespace sfm {
 
-// One CTA moves one token: all heads x 16 vectors of 16 bytes (8 bf16 = 4 rotary pairs) of q, k and
-// v.  The token's position arithmetic (grid coordinates, Monarch slot) is done once per CTA and its
-// 64 (cos, sin) pairs are staged in shared memory for all heads.  Reads and writes are 16-byte
-// vectors; consecutive threads cover consecutive 256-byte rows.  The kernel is HBM bound: it reads
-// 3 tensors and writes 3 (2 when q is absent).
+// An item is one token of one of the tensors k, v and q (grid y; grid z = batch): all heads x 16 vectors of 16 bytes (8 bf16 = 4 rotary pairs),
+// moved by W warps (W = 1, 2 or 4, a launch constant).  A lane's vectors lie 32 * W apart, so they all carry the same four
+// rotary pairs: the token's position arithmetic and its (cos, sin) pairs cost each lane one 32-byte read, and the row stays
+// in registers between the sum of squares and the rotation (at most kMaxVec vectors per lane: 12 heads on one warp, 48
+// on four; wider tokens take the looping form, which reads them twice).  The kernel is HBM bound: it reads 3 tensors and
+// writes 3 (2 when q is absent); beside that, its instructions count: with 64-bit index divisions and separately rounded
+// conversions the 4680 tokens of a 12-head chunk, normalised and rotated, took 26 us (0.63 of the issue slots busy),
+// now 21 (cold caches, 86 MB moved).  One warp per tensor row instead of one CTA per token keeps 24 warps per SM
+// resident, each with its whole row in flight, and lets the eviction's chains of k and v run beside each other.
 //
 // Sources may be sharded by token over up to kMaxPeers GPUs of one box (head-sharded attention): token n
 // then lives in buffer n / src_tokens, a [B, src_tokens, src_heads, 128] tensor of which this GPU takes
@@ -30,7 +34,43 @@ struct PeerSrc {
     const uint4* v[kMaxPeers];
 };
 
-__global__ void __launch_bounds__(256)
+constexpr int kLayoutThreads = 128;
+constexpr int kMaxVec = 6;                 // vectors per lane and tensor held in registers
+
+__device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); }
+__device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+__device__ __forceinline__ float sum_squares(const uint4& v, float acc) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const float a = lo_f(w[p]), c = hi_f(w[p]);
+        acc = fmaf(a, a, fmaf(c, c, acc));
+    }
+    return acc;
+}
+// y = bf16(bf16(x * rs) * weight): the two roundings of the reference (the bf16 product rounds the exact one, once)
+__device__ __forceinline__ void norm_vec(uint4& v, const uint4& weight, float rs) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+    const uint32_t* g = reinterpret_cast<const uint32_t*>(&weight);
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+        w[p] = as_u32(__hmul2(__floats2bfloat162_rn(lo_f(w[p]) * rs, hi_f(w[p]) * rs), as_bf162(g[p])));
+}
+__device__ __forceinline__ void rotate_vec(uint4& v, const float2 (&cs)[4]) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const float re = lo_f(w[p]), im = hi_f(w[p]);
+        w[p] = pack_bf16(re * cs[p].x - im * cs[p].y, re * cs[p].y + im * cs[p].x);
+    }
+}
+
+// kWarps warps per item.  kRegs: the item's vectors stay in registers between the two passes.
+template <int kWarps, bool kRegs>
+__global__ void __launch_bounds__(kLayoutThreads, 6)
 rope_cache_write_kernel(const __grid_constant__ PeerSrc src, int src_tokens, int src_heads, int head0,
                         uint4* __restrict__ q_out, uint4* k_cache, uint4* v_cache,
                         long long cache_batch_stride_vec, const float2* __restrict__ rope,
@@ -39,142 +79,101 @@ rope_cache_write_kernel(const __grid_constant__ PeerSrc src, int src_tokens, int
                         const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk, float eps,
                         int roll_dst, int roll_shift, int rope_tok0) {
     constexpr int kVecPerRow = kHeadDim / 8;  // 16
-    __shared__ float2 cs_s[kHeadDim / 2];
-    __shared__ float red_s[2][8];
-    __shared__ float rs_s[2];                  // 1/rms of the token's q and k rows (full width)
-    const int frame_tokens = blk.h * blk.w;
-    for (long long bn = blockIdx.x; bn < (long long)B * n_new; bn += gridDim.x) {
-        const int n = (int)(bn % n_new);
-        const int b = (int)(bn / n_new);
-        if (rope) {
-            __syncthreads();                                    // previous token's table no longer in use
-            for (int m = threadIdx.x; m < kHeadDim / 2; m += blockDim.x) {   // m: rotary pair index within the head
-                const int np = n + rope_tok0;                   // position in the chunk's token grid (token slices)
-                const int fr = np / frame_tokens, rem = np - fr * frame_tokens;
-                const int rw = rem / blk.w, cl = rem - rw * blk.w;
-                const int pos = m < p0 ? start_frame + fr : (m < p0 + p1 ? rw : cl);
-                cs_s[m] = rope[pos * (kHeadDim / 2) + m];
+    constexpr int kLanes = 32 * kWarps;       // lanes per item
+    __shared__ float red_s[kLayoutThreads / 32];
+    const int warp = threadIdx.x >> 5;
+    const int l = threadIdx.x & (kLanes - 1);                   // lane within the item's group
+    const int n_all = (int)blockIdx.x * (kLayoutThreads / kLanes) + (int)threadIdx.x / kLanes;
+    const bool live = n_all < n_new;                            // groups past the end only take part in the barriers
+    const int n = live ? n_all : 0, which = blockIdx.y, b = blockIdx.z;     // which = 0: k, 1: v, 2: q
+    const int vecs = H * kVecPerRow;
+
+    const int peer = src_tokens == n_new ? 0 : n / src_tokens;
+    const uint4* __restrict__ x = (which == 0 ? src.k[peer] : (which == 1 ? src.v[peer] : src.q[peer])) +
+                                  (((long long)b * src_tokens + (n - peer * src_tokens)) * src_heads + head0) * kVecPerRow;
+    uint4 r[kMaxVec];
+    if constexpr (kRegs) {
+#pragma unroll
+        for (int i = 0; i < kMaxVec; ++i)
+            if (live && l + i * kLanes < vecs) r[i] = x[l + i * kLanes];
+    }
+    const bool rotate = rope && which != 1;
+    float2 cs[4];
+    if (rotate) {
+        const int frame_tokens = blk.h * blk.w;
+        const int np = n + rope_tok0;                           // position in the chunk's token grid (token slices)
+        const int fr = np / frame_tokens, rem = np - fr * frame_tokens;
+        const int rw = rem / blk.w, cl = rem - rw * blk.w;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int m = (l & (kVecPerRow - 1)) * 4 + p;       // rotary pair within the head: the same for all of a lane's vectors
+            const int pos = m < p0 ? start_frame + fr : (m < p0 + p1 ? rw : cl);
+            cs[p] = rope[pos * (kHeadDim / 2) + m];
+        }
+    }
+    const int dst_tok = start_idx + (monarch_order && which != 2 ? blk.nat2mon(n) : n);
+    const long long base = (long long)b * cache_batch_stride_vec;
+    uint4* const cache = which == 1 ? v_cache : k_cache;
+    uint4* const dst = which == 2 ? q_out + ((long long)b * n_new + n) * vecs : cache + base + (long long)dst_tok * vecs;
+
+    if (live && which != 2 && roll_shift > 0 && dst_tok - start_idx < roll_shift) {
+        // this token's slot ends a chain of the eviction shift: walk it (same lane-to-vector mapping as the write below, so
+        // the last source element is read by the lane that then overwrites it), one chain element ahead
+        const long long step = (long long)roll_shift * vecs;
+        const int first = roll_dst + (dst_tok - roll_dst) % roll_shift;
+        if (first < dst_tok) {
+            for (int t0 = l; t0 < vecs; t0 += kMaxVec * kLanes) {
+                uint4 c[kMaxVec];
+                uint4* d = cache + base + (long long)first * vecs + t0;
+                for (int pos = first; pos < dst_tok; pos += roll_shift, d += step) {
+#pragma unroll
+                    for (int i = 0; i < kMaxVec; ++i)
+                        if (t0 + i * kLanes < vecs) c[i] = d[step + i * kLanes];
+#pragma unroll
+                    for (int i = 0; i < kMaxVec; ++i)
+                        if (t0 + i * kLanes < vecs) d[i * kLanes] = c[i];
+                }
             }
+        }
+    }
+
+    const __nv_bfloat16* const weight = which == 1 ? nullptr : (which == 0 ? wk : wq);
+    float rs = 1.f;
+    if (wk) {
+        // RMS normalisation over the token's full width (all heads)
+        float sq = 0.f;
+        if constexpr (kRegs) {
+#pragma unroll
+            for (int i = 0; i < kMaxVec; ++i)
+                if (live && l + i * kLanes < vecs) sq = sum_squares(r[i], sq);
+        } else if (live && weight) {
+            for (int t = l; t < vecs; t += kLanes) sq = sum_squares(x[t], sq);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if constexpr (kWarps > 1) {
+            if ((threadIdx.x & 31) == 0) red_s[warp] = sq;
             __syncthreads();
+            const int w0 = warp & ~(kWarps - 1);
+            sq = 0.f;
+#pragma unroll
+            for (int i = 0; i < kWarps; ++i) sq += red_s[w0 + i];
         }
-        const int dst_tok = start_idx + (monarch_order ? blk.nat2mon(n) : n);
-        const int peer = n / src_tokens;
-        const uint4* __restrict__ q = src.q[peer];
-        const uint4* __restrict__ k = src.k[peer];
-        const uint4* __restrict__ v = src.v[peer];
-        const long long src_vec0 = (((long long)b * src_tokens + (n - peer * src_tokens)) * src_heads + head0) * kVecPerRow;
-        const long long out_vec0 = bn * H * kVecPerRow;
-        if (wk) {
-            // RMS normalisation over the token's full width (all heads), q and k separately
-            float sq = 0.f, sk = 0.f;
-            for (int t = threadIdx.x; t < H * kVecPerRow; t += blockDim.x) {
-                const uint4 kv = k[src_vec0 + t];
-                const uint32_t* kw = reinterpret_cast<const uint32_t*>(&kv);
+        rs = rsqrtf(sq / (float)(H * kHeadDim) + eps);
+    }
+    if (!live) return;
+
+    auto finish = [&](int t, uint4 v) {
+        if (weight) norm_vec(v, reinterpret_cast<const uint4*>(weight)[t], rs);
+        if (rotate) rotate_vec(v, cs);
+        dst[t] = v;
+    };
+    if constexpr (kRegs) {
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&kw[p]);
-                    const float a = __low2float(x), c = __high2float(x);
-                    sk = fmaf(a, a, fmaf(c, c, sk));
-                }
-                if (q) {
-                    const uint4 qv = q[src_vec0 + t];
-                    const uint32_t* qw = reinterpret_cast<const uint32_t*>(&qv);
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&qw[p]);
-                        const float a = __low2float(x), c = __high2float(x);
-                        sq = fmaf(a, a, fmaf(c, c, sq));
-                    }
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                sq += __shfl_xor_sync(0xffffffffu, sq, o);
-                sk += __shfl_xor_sync(0xffffffffu, sk, o);
-            }
-            __syncthreads();                                    // previous token's factors no longer in use
-            if ((threadIdx.x & 31) == 0) { red_s[0][threadIdx.x >> 5] = sq; red_s[1][threadIdx.x >> 5] = sk; }
-            __syncthreads();
-            if (threadIdx.x < 2) {
-                float tot = 0.f;
-                for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red_s[threadIdx.x][i];
-                rs_s[threadIdx.x] = rsqrtf(tot / (float)(H * kHeadDim) + eps);
-            }
-            __syncthreads();
-        }
-        const long long dst_row = (long long)b * cache_batch_stride_vec + (long long)dst_tok * H * kVecPerRow;
-        if (roll_shift > 0 && dst_tok - start_idx < roll_shift) {
-            // this token's slot ends a chain of the eviction shift: walk it (same thread-to-vector mapping as
-            // the write below, so the last source element is read by the thread that then overwrites it)
-            const long long tok_vecs = (long long)H * kVecPerRow;
-            const long long base = (long long)b * cache_batch_stride_vec;
-            const int first = roll_dst + (dst_tok - roll_dst) % roll_shift;
-            for (int pos = first; pos < dst_tok; pos += roll_shift) {
-                for (int t = threadIdx.x; t < H * kVecPerRow; t += blockDim.x) {
-                    const long long d = base + pos * tok_vecs + t, sidx = d + roll_shift * tok_vecs;
-                    const uint4 kk = k_cache[sidx];
-                    const uint4 vv = v_cache[sidx];
-                    k_cache[d] = kk;
-                    v_cache[d] = vv;
-                }
-            }
-        }
-        for (int t = threadIdx.x; t < H * kVecPerRow; t += blockDim.x) {
-            const int vec = t & (kVecPerRow - 1);
-            const long long idx = src_vec0 + t;
-            uint4 kv = k[idx];
-            uint4 vv = v[idx];
-            uint4 qv = make_uint4(0, 0, 0, 0);
-            if (q) qv = q[idx];
-            if (wk) {
-                // y = bf16(bf16(x * rsqrt(mean x^2 + eps)) * weight): the two roundings of the reference
-                const uint4 wkv = reinterpret_cast<const uint4*>(wk)[t];
-                const uint32_t* wkw = reinterpret_cast<const uint32_t*>(&wkv);
-                uint32_t* kw = reinterpret_cast<uint32_t*>(&kv);
-                const float rk = rs_s[1];
-#pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&kw[p]);
-                    const __nv_bfloat162 wv = *reinterpret_cast<const __nv_bfloat162*>(&wkw[p]);
-                    const __nv_bfloat162 y = __floats2bfloat162_rn(__low2float(x) * rk, __high2float(x) * rk);
-                    kw[p] = pack_bf16(__low2float(y) * __low2float(wv), __high2float(y) * __high2float(wv));
-                }
-                if (q) {
-                    const uint4 wqv = reinterpret_cast<const uint4*>(wq)[t];
-                    const uint32_t* wqw = reinterpret_cast<const uint32_t*>(&wqv);
-                    uint32_t* qw = reinterpret_cast<uint32_t*>(&qv);
-                    const float rq = rs_s[0];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        const __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&qw[p]);
-                        const __nv_bfloat162 wv = *reinterpret_cast<const __nv_bfloat162*>(&wqw[p]);
-                        const __nv_bfloat162 y = __floats2bfloat162_rn(__low2float(x) * rq, __high2float(x) * rq);
-                        qw[p] = pack_bf16(__low2float(y) * __low2float(wv), __high2float(y) * __high2float(wv));
-                    }
-                }
-            }
-            if (rope) {
-                uint32_t* kw = reinterpret_cast<uint32_t*>(&kv);
-                uint32_t* qw = reinterpret_cast<uint32_t*>(&qv);
-#pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const float2 cs = cs_s[vec * 4 + p];
-                    {
-                        __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&kw[p]);
-                        float re = __low2float(x), im = __high2float(x);
-                        kw[p] = pack_bf16(re * cs.x - im * cs.y, re * cs.y + im * cs.x);
-                    }
-                    if (q) {
-                        __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&qw[p]);
-                        float re = __low2float(x), im = __high2float(x);
-                        qw[p] = pack_bf16(re * cs.x - im * cs.y, re * cs.y + im * cs.x);
-                    }
-                }
-            }
-            if (q) q_out[out_vec0 + t] = qv;
-            k_cache[dst_row + t] = kv;
-            v_cache[dst_row + t] = vv;
-        }
+        for (int i = 0; i < kMaxVec; ++i)
+            if (l + i * kLanes < vecs) finish(l + i * kLanes, r[i]);
+    } else {
+        for (int t = l; t < vecs; t += kLanes) finish(t, x[t]);
     }
 }
 
@@ -245,15 +244,24 @@ int rope_cache_write_impl(const PeerSrc& src, bool have_q, int src_tokens, int s
     if (roll_shift < 0 || (roll_shift > 0 && (roll_dst > start_idx || roll_shift > n_new))) return SFM_ERR_BAD_SHAPE;
     int c = D / 2;
     int p0 = c - 2 * (c / 3), p1 = c / 3;
-    int threads = H * (D / 8);
-    threads = threads > 256 ? 256 : ((threads + 31) & ~31);
-    long long want = (long long)B * n_new;                       // one token per CTA pass
-    int blocks = (int)(want < 148LL * 32 ? want : 148LL * 32);  // grid-stride over tokens
+    // the narrowest group of warps whose lanes hold a token's row in registers; wider tokens are walked by four warps
+    const int vecs = H * (D / 8);
+    const int warps = vecs <= 32 * kMaxVec ? 1 : (vecs <= 64 * kMaxVec ? 2 : 4);
+    const bool in_regs = vecs <= 32 * warps * kMaxVec;
+    const int per_cta = kLayoutThreads / 32 / warps, tensors = have_q ? 3 : 2;
+    const dim3 grid((n_new + per_cta - 1) / per_cta, tensors, B);
+    if (B > 65535) return SFM_ERR_BAD_SHAPE;
     LaunchScope scope(kClsLayout, (cudaStream_t)stream);
-    rope_cache_write_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(
-        src, src_tokens, src_heads, head0, (uint4*)q_out, (uint4*)k_cache, (uint4*)v_cache, cache_batch_stride / 8,
-        (const float2*)rope, B, n_new, H, start_idx, blk, start_frame, monarch_order, p0, p1,
-        (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, eps, roll_dst, roll_shift, rope_tok0 < 0 ? 0 : rope_tok0);
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kLayoutThreads, 0, (cudaStream_t)stream>>>(
+            src, src_tokens, src_heads, head0, (uint4*)q_out, (uint4*)k_cache, (uint4*)v_cache, cache_batch_stride / 8,
+            (const float2*)rope, B, n_new, H, start_idx, blk, start_frame, monarch_order, p0, p1,
+            (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, eps, roll_dst, roll_shift, rope_tok0 < 0 ? 0 : rope_tok0);
+    };
+    if (!in_regs) go(rope_cache_write_kernel<4, false>);
+    else if (warps == 1) go(rope_cache_write_kernel<1, true>);
+    else if (warps == 2) go(rope_cache_write_kernel<2, true>);
+    else go(rope_cache_write_kernel<4, true>);
     return (int)cudaGetLastError();
 }
 }  // namespace
