@@ -8,12 +8,9 @@
 using namespace sfm;
 
 namespace sfm {
-int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps, int rows_per_group, int n_s, int* status,
-                     int num_sms, cudaStream_t s);
-int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* maps, int* status, int num_sms, cudaStream_t s,
-                     int write_lse = 0);
-int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_al, const CUtensorMap* map_qrows, int* status,
-                     int num_sms, cudaStream_t s);
+int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps, int n_s, int* status, int num_sms, cudaStream_t s);
+int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s, int write_lse);
+int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s);
 }
 
 namespace {
@@ -151,8 +148,7 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     }
     int* status = reinterpret_cast<int*>(base + pl.off_status);
-    CUtensorMap maps[7];
-    const int rows_per_group = (pl.blk.b2 + 7) & ~7;
+    CUtensorMap maps[5];     // q, K, V, query rows, iteration state
     const int n_s = (pl.blk.b2 + 15) & ~15;
     {
         // Every path starts from a clear status word: the workspace may be recycled memory, and the kernels
@@ -161,33 +157,21 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         if (e != cudaSuccess) return (int)e;
     }
     if (use_tc) {
-        cudaError_t e;
-        // cL rows are padded to 16 bytes; the pad floats travel with the column step's bulk copies and
-        // must act as "key masked": fill the buffer with a huge positive bias (0x7f7f7f7f = 3.4e38).
-        e = cudaMemsetAsync(p.cL, 0x7f, (size_t)pl.nbh_chunk * pl.na_chunk * pl.blk.b2 * p.n_keys_c * sizeof(float), stream);
-        if (e != cudaSuccess) return (int)e;
         const uint64_t row = (uint64_t)kHeadDim * 2, tok = (uint64_t)H * row;
         uint64_t dq[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_q, (uint64_t)B};
         uint64_t sq[3] = {row, tok, (uint64_t)q_bs * 2};
-        uint32_t bq[4] = {64, 1, (uint32_t)rows_per_group, 1};
+        uint32_t bq[4] = {64, 1, (uint32_t)pl.blk.b2, 1};
         uint64_t dk[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_kv, (uint64_t)B};
         uint64_t sk[3] = {row, tok, (uint64_t)c_bs * 2};
         uint32_t bk[4] = {64, 1, (uint32_t)n_s, 1};
-        const uint64_t n_aj = (uint64_t)pl.nbh_chunk * pl.na_chunk * pl.blk.b2;
-        uint64_t db[3] = {(uint64_t)kHeadDim, (uint64_t)pl.n_keys, n_aj};
-        uint64_t sb[2] = {row, (uint64_t)pl.n_keys * row};
-        uint32_t bb[3] = {64, 128, 1};   // column step: 128 keys of one (query group, column) per load
         if ((rc = make_tmap_bf16(&maps[0], q, 4, dq, sq, bq))) return rc;
         if ((rc = make_tmap_bf16(&maps[1], kc, 4, dk, sk, bk))) return rc;
         if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
-        if ((rc = make_tmap_bf16(&maps[3], p.aL, 3, db, sb, bb))) return rc;
-        if ((rc = make_tmap_bf16(&maps[4], p.Y, 3, db, sb, bb))) return rc;
         // queries of one (query group, column): rows of the token grid at a fixed column
-        const int rows_per_quadrant = (pl.blk.b1 + 3) / 4;
         uint64_t dqr[5] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)w, (uint64_t)(n_q / w), (uint64_t)B};
         uint64_t sqr[4] = {row, tok, (uint64_t)w * tok, (uint64_t)q_bs * 2};
-        uint32_t bqr[5] = {64, 1, 1, (uint32_t)rows_per_quadrant, 1};
-        if ((rc = make_tmap_bf16(&maps[5], q, 5, dqr, sqr, bqr))) return rc;
+        uint32_t bqr[5] = {64, 1, 1, (uint32_t)pl.blk.b1, 1};
+        if (pl.blk.b1 <= 128 && (rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
     }
 
     const int BH = B * H;
@@ -195,48 +179,21 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         p.bh0 = bh0; p.nbh = std::min(pl.nbh_chunk, BH - bh0);
         for (int a0 = 0; a0 < pl.A; a0 += pl.na_chunk) {
             p.a0 = a0; p.na = std::min(pl.na_chunk, pl.A - a0);
-            if (use_tc && causal_groups > 0) {
-                // Block-causal: the row step skips the (query group, f) pairs no query may see, so the
-                // column step finds bridge rows nobody wrote.  Give them defined contents: zero keys /
-                // values and the "masked" bias.
-                const size_t rows = (size_t)p.nbh * p.na * pl.blk.b2;
-                cudaError_t e = cudaMemsetAsync(p.aL, 0, rows * pl.n_keys * kHeadDim * 2, stream);
-                if (e == cudaSuccess) e = cudaMemsetAsync(p.Y, 0, rows * pl.n_keys * kHeadDim * 2, stream);
-                if (e == cudaSuccess) e = cudaMemsetAsync(p.cL, 0x7f, rows * p.n_keys_c * sizeof(float), stream);
-                if (e != cudaSuccess) return (int)e;
+            if (!use_tc) {
+                // enough row-step CTAs to fill the GPU about twice over (the tensor-core launcher plans its own units)
+                const int base_ctas = pl.blk.b1 * ((p.na + p.na_cta - 1) / p.na_cta) * p.nbh;
+                const int fsplit = std::max(1, std::min(pl.F, (2 * num_sms + base_ctas - 1) / base_ctas));
+                p.f_per = (pl.F + fsplit - 1) / fsplit;
+                p.fsplit = (pl.F + p.f_per - 1) / p.f_per;
             }
-            // enough row-step CTAs to fill the GPU about twice over
-            int asubs = use_tc ? (p.na + (128 / rows_per_group) - 1) / (128 / rows_per_group)
-                               : (p.na + p.na_cta - 1) / p.na_cta;
-            int base_ctas = pl.blk.b1 * asubs * p.nbh;
-            int fsplit;
-            if (use_tc) {
-                // Persistent CTAs take whole units round-robin, so the launch lasts (units per CTA, rounded
-                // up) x (steps per unit).  Pick the split of the F loop that makes that smallest, with at
-                // least three steps per unit (every unit reloads its query tile) and an extra step's worth
-                // charged per unit for that reload.
-                fsplit = 1;
-                long long best = -1;
-                for (int fs = 1; fs <= std::max(1, pl.F / 3); ++fs) {
-                    const int per = (pl.F + fs - 1) / fs;
-                    const int splits = (pl.F + per - 1) / per;
-                    const long long units = (long long)base_ctas * splits;
-                    const long long cost = ((units + num_sms - 1) / num_sms) * (per + 1);
-                    if (best < 0 || cost < best) { best = cost; fsplit = fs; }
-                }
-            } else {
-                fsplit = std::max(1, std::min(pl.F, (2 * num_sms + base_ctas - 1) / base_ctas));
-            }
-            p.f_per = (pl.F + fsplit - 1) / fsplit;
-            p.fsplit = (pl.F + p.f_per - 1) / p.f_per;
             if (iter_tc) {
                 // iteration state aR of this chunk as [nbh * F * b1][na * b2][128]: one (f, k) block of stacked
                 // (query group, column) rows per index of the slowest dimension
                 const uint64_t row = (uint64_t)kHeadDim * 2;
                 uint64_t dar[3] = {(uint64_t)kHeadDim, (uint64_t)p.na * pl.blk.b2, (uint64_t)p.nbh * pl.F * pl.blk.b1};
                 uint64_t sar[2] = {row, (uint64_t)p.na * pl.blk.b2 * row};
-                uint32_t bar[3] = {64, (uint32_t)rows_per_group, 1};
-                if ((rc = make_tmap_bf16(&maps[6], p.aR, 3, dar, sar, bar))) return rc;
+                uint32_t bar[3] = {64, (uint32_t)pl.blk.b2, 1};
+                if ((rc = make_tmap_bf16(&maps[4], p.aR, 3, dar, sar, bar))) return rc;
             }
 
             for (int it = 0; it < num_iters; ++it) {
@@ -246,20 +203,20 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
                 p.mult0 = num_iters > 1 ? sm_scale * (1.0f / (1.0f + 1e-6f)) : sm_scale;
                 if (use_tc) {
                     // later passes of the iterative variant read their query operand from the state aR
-                    CUtensorMap rmaps[3] = {p.use_aR ? maps[6] : maps[0], maps[1], maps[2]};
-                    if ((rc = launch_r_step_tc(p, rmaps, rows_per_group, n_s, status, num_sms, stream))) return rc;
+                    CUtensorMap rmaps[3] = {p.use_aR ? maps[4] : maps[0], maps[1], maps[2]};
+                    if ((rc = launch_r_step_tc(p, rmaps, n_s, status, num_sms, stream))) return rc;
                 } else {
                     if ((rc = launch_r_step(p, stream))) return rc;
                 }
                 if (last) {
                     if (use_tc && pl.blk.b1 <= 128) {
-                        if ((rc = launch_l_step_tc(p, maps + 3, status, num_sms, stream))) return rc;
+                        if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 0))) return rc;
                     } else if ((rc = launch_l_step(p, 0, stream))) return rc;
                 } else if (iter_tc) {
                     // the column step's softmax statistics (its output row is overwritten by the last pass), then
                     // the update of the state
-                    if ((rc = launch_l_step_tc(p, maps + 3, status, num_sms, stream, 2))) return rc;
-                    if ((rc = launch_l_iter_tc(p, &maps[3], &maps[5], status, num_sms, stream))) return rc;
+                    if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 2))) return rc;
+                    if ((rc = launch_l_iter_tc(p, &maps[3], status, num_sms, stream))) return rc;
                 } else {
                     if ((rc = launch_l_step(p, 1, stream))) return rc;
                     if ((rc = launch_l_iter(p, stream))) return rc;
@@ -274,10 +231,10 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
 
 namespace sfm {
 // Single-pass forward on the tensor-core kernels for the (batch, head) pairs [bh0, bh0 + nbh) with all query
-// groups at once, into caller-given bridge buffers (aL, Y: bf16 [slab][n_keys][128], cL: fp32 [slab][n_keys_c],
+// groups at once, into caller-given bridge buffers (aL, Y: bf16 [bh_local * A + a][n_keys][b2][128], cL: fp32 [slab][n_keys_c],
 // slab = (bh_local * A + a) * b2 + j) and, optionally, the column step's log-sum-exp per query row
 // (lse: fp32 [slab][b1]).  The backward uses it to recompute what the forward did not keep.  Returns the launch
-// parameters and the six tensor maps (q, K, V, aL bridge, Y bridge, query rows) for the kernels that follow.
+// parameters and the tensor maps of q, K, V and the query rows for the kernels that follow.
 int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out,
                      __nv_bfloat16* aL, __nv_bfloat16* Y, float* cL, float* lse, int* status, int B, int H, int n_q,
                      int n_kv, const Blocking& blk, float scale, int bh0, int nbh, MonarchParams* p_out,
@@ -305,49 +262,25 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
         int dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     }
-    const int rows_per_group = (blk.b2 + 7) & ~7;
     const int n_s = (blk.b2 + 15) & ~15;
     const size_t slabs = (size_t)nbh * p.A * blk.b2;
-    // the caller owns the status word (set once per call, shared by its slices)
-    cudaError_t e = cudaMemsetAsync(cL, 0x7f, slabs * p.n_keys_c * sizeof(float), stream);
-    if (e != cudaSuccess) return (int)e;
     int rc;
     const uint64_t row = (uint64_t)kHeadDim * 2, tok = (uint64_t)H * row;
     uint64_t dq[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_q, (uint64_t)B};
     uint64_t sq[3] = {row, tok, (uint64_t)q_bs * 2};
-    uint32_t bq[4] = {64, 1, (uint32_t)rows_per_group, 1};
+    uint32_t bq[4] = {64, 1, (uint32_t)blk.b2, 1};
     uint64_t dk[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_kv, (uint64_t)B};
     uint64_t sk[3] = {row, tok, (uint64_t)c_bs * 2};
     uint32_t bk[4] = {64, 1, (uint32_t)n_s, 1};
-    uint64_t db[3] = {(uint64_t)kHeadDim, (uint64_t)p.n_keys, (uint64_t)slabs};
-    uint64_t sb[2] = {row, (uint64_t)p.n_keys * row};
-    uint32_t bb[3] = {64, 128, 1};
-    const int rows_per_quadrant = (blk.b1 + 3) / 4;
     uint64_t dqr[5] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)blk.w, (uint64_t)(n_q / blk.w), (uint64_t)B};
     uint64_t sqr[4] = {row, tok, (uint64_t)blk.w * tok, (uint64_t)q_bs * 2};
-    uint32_t bqr[5] = {64, 1, 1, (uint32_t)rows_per_quadrant, 1};
+    uint32_t bqr[5] = {64, 1, 1, (uint32_t)blk.b1, 1};
     if ((rc = make_tmap_bf16(&maps[0], q, 4, dq, sq, bq))) return rc;
     if ((rc = make_tmap_bf16(&maps[1], kc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
-    if ((rc = make_tmap_bf16(&maps[3], aL, 3, db, sb, bb))) return rc;
-    if ((rc = make_tmap_bf16(&maps[4], Y, 3, db, sb, bb))) return rc;
-    if ((rc = make_tmap_bf16(&maps[5], q, 5, dqr, sqr, bqr))) return rc;
-    // split of the F loop over persistent CTAs, as in the forward proper
-    const int asubs = (p.na + (128 / rows_per_group) - 1) / (128 / rows_per_group);
-    const int base_ctas = blk.b1 * asubs * nbh;
-    int fsplit = 1;
-    long long best = -1;
-    for (int fs = 1; fs <= std::max(1, p.F / 3); ++fs) {
-        const int per = (p.F + fs - 1) / fs;
-        const int splits = (p.F + per - 1) / per;
-        const long long units = (long long)base_ctas * splits;
-        const long long cost = ((units + num_sms - 1) / num_sms) * (per + 1);
-        if (best < 0 || cost < best) { best = cost; fsplit = fs; }
-    }
-    p.f_per = (p.F + fsplit - 1) / fsplit;
-    p.fsplit = (p.F + p.f_per - 1) / p.f_per;
-    if ((rc = launch_r_step_tc(p, maps, rows_per_group, n_s, status, num_sms, stream))) return rc;
-    if ((rc = launch_l_step_tc(p, maps + 3, status, num_sms, stream, lse ? 1 : 0))) return rc;
+    if ((rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
+    if ((rc = launch_r_step_tc(p, maps, n_s, status, num_sms, stream))) return rc;
+    if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
     *p_out = p;
     return SFM_OK;
 }

@@ -1,7 +1,5 @@
 // Dense softmax attention without a mask over the whole key range: the dense-init chunk and the
-// "regular" configuration.  Runs on the tensor-core flash kernel of monarch_lstep_tc.cu (dense
-// instantiation): one unit = 128 consecutive queries of one (batch, head), keys and values stream
-// from the cache view in 128-token tiles by TMA.
+// "regular" configuration.  Host side of the tensor-core kernel in dense_tc.cu.
 //
 // Stands in for flash_attention / attention (wan/modules/attention.py:34-187).
 #include "common.cuh"

@@ -487,10 +487,11 @@ __global__ void __launch_bounds__(512) bwd_row_kernel(const BwdParams p) {
                     float4 a4 = zero4, y4 = zero4;
                     if (seen) {
                         if (p.aLb) {            // bf16 gradients of the unscaled aL: daL of the scaled one = that / sqrt(scale)
-                            const float4 t4 = ld4(p.aLb + o + lane * 4);
+                            const int64_t ob = ((((int64_t)bhl * p.A + a) * p.n_keys + n) * b2 + j) * kD;
+                            const float4 t4 = ld4(p.aLb + ob + lane * 4);
                             const float ir = 1.0f / p.rs;
                             a4 = make_float4(t4.x * ir, t4.y * ir, t4.z * ir, t4.w * ir);
-                            y4 = ld4(p.Yb + o + lane * 4);
+                            y4 = ld4(p.Yb + ob + lane * 4);
                         } else {
                             a4 = *reinterpret_cast<const float4*>(p.aL + o + lane * 4);
                             y4 = *reinterpret_cast<const float4*>(p.Y + o + lane * 4);
@@ -840,11 +841,10 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
                 uint64_t sq_[4] = {row, tok, (uint64_t)blk.w * tok, (uint64_t)q_batch_stride * 2};
                 uint64_t sdo[4] = {row, tok, (uint64_t)blk.w * tok, (uint64_t)n_q * tok};
                 uint32_t bqr[5] = {64, 1, 1, box_rows, 1};
-                if ((rc = make_tmap_bf16(&maps[5], q, 5, dqr, sq_, bqr))) return rc;
-                if ((rc = make_tmap_bf16(&maps[6], dout, 5, dqr, sdo, bqr))) return rc;
+                if ((rc = make_tmap_bf16(&maps[4], q, 5, dqr, sq_, bqr))) return rc;
+                if ((rc = make_tmap_bf16(&maps[5], dout, 5, dqr, sdo, bqr))) return rc;
             }
-            CUtensorMap cmaps[4] = {maps[3], maps[4], maps[5], maps[6]};
-            if ((rc = launch_bwd_col_tc(mp, cmaps, delta, dcL, p.dq, status, num_sms, s))) return rc;
+            if ((rc = launch_bwd_col_tc(mp, maps + 4, delta, dcL, p.dq, status, num_sms, s))) return rc;
             p.aLb = aLb; p.Yb = Yb; p.dcL = dcL; p.dcl_pitch = n_keys_c;
             // Row-step backward on tcgen05 when its per-tile dK / dV partials fit what is left of the workspace;
             // SFM_BWD_ROW_FP32=1 keeps the fp32 row kernel.
@@ -853,14 +853,7 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
             if (!(row_fp32 && row_fp32[0] == '1') && o + 2 * part <= workspace_bytes) {
                 float* part_k = (float*)(ws + o);
                 float* part_v = (float*)(ws + o + part);
-                const int rows_per_group = (blk.b2 + 7) & ~7;
-                uint64_t db[3] = {(uint64_t)kHeadDim, (uint64_t)pl.n_keys, (uint64_t)slabs};
-                uint64_t sb[2] = {(uint64_t)kHeadDim * 2, (uint64_t)pl.n_keys * kHeadDim * 2};
-                uint32_t bb[3] = {64, 1, (uint32_t)rows_per_group};
-                CUtensorMap rmaps[5] = {maps[0], maps[1], maps[2]};
-                if ((rc = make_tmap_bf16(&rmaps[3], aLb, 3, db, sb, bb))) return rc;
-                if ((rc = make_tmap_bf16(&rmaps[4], Yb, 3, db, sb, bb))) return rc;
-                if ((rc = launch_bwd_row_tc(mp, rmaps, dcL, p.dq, part_k, part_v, p.dk, p.dv, p.g0, p.g1, status, num_sms, s)))
+                if ((rc = launch_bwd_row_tc(mp, maps, dcL, p.dq, part_k, part_v, p.dk, p.dv, p.g0, p.g1, status, num_sms, s)))
                     return rc;
                 continue;
             }

@@ -2,7 +2,7 @@
 //
 // Forward row step, per (batch*head, block row k, cached group f) and stacked query row r = (query group a, column j):
 //   z_l = scale * q[r] . K[f,k,l],  R = softmax_l z,  aL[r] = sum_l R_l K_l,  Y[r] = sum_l R_l V_l,  cL[r] = sum_l R_l ln R_l
-// Given daL[r], dY[r] (bf16, in the bridge layout [slab][key][128], left there by the column step's backward) and dcL[r]:
+// Given daL[r], dY[r] (bf16, in the bridge layout [query group][key][column][128], left there by the column step's backward) and dcL[r]:
 //   dR_l = daL[r] . K_l + dY[r] . V_l + dcL[r] (ln R_l + 1)          dz_l = R_l (dR_l - sum_m R_m dR_m)
 //   dQ[r] += scale * sum_l dz_l K_l
 //   dK_l  += sum_r (R_l daL[r] + scale dz_l q[r])                      dV_l += sum_r R_l dY[r]
@@ -73,7 +73,7 @@ __device__ __forceinline__ RBUnit rb_decode(const BwdRowParams& rp, int u) {
     return r;
 }
 
-// tq, tk, tv: the forward's maps of q, K, V; tda, tdy: bridge maps of daL / dY with a (64, 1 key, rows_per_group) box.
+// tq, tk, tv: the forward's maps of q, K, V; tda, tdy: bridge maps of daL / dY (box 64 x rows_per_group columns x 1 key).
 template <int N_S>
 __global__ void __launch_bounds__(kThreadsRB, 1)
 monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
@@ -137,7 +137,7 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 const int g_first = un.tile * rp.groups_per_tile;
                 const int ng = min(rp.groups_per_tile, p.na - g_first);
                 if (uc > 0 && !mbar_wait(&bars->q_empty, (uc - 1) & 1)) { fail(10); break; }
-                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(ng * RG * 256));
+                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(ng * b2 * 256));           // the padding rows stay zero
                 for (int gi = 0; gi < ng; ++gi) {
                     const int tok = blk.row_token(p.a0 + g_first + gi, un.k);
                     tma_load_4d(q_s + gi * RG * 128, &tq, &bars->q_full, 0, hd, tok, b);
@@ -157,11 +157,11 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                     const int key = f * b1 + un.k;
                     mbar_arrive_expect_tx(&bars->da_full, (uint32_t)(2 * ng * RG * 256));
                     for (int gi = 0; gi < ng; ++gi) {
-                        const int slab = (un.bhl * p.na + g_first + gi) * b2;
-                        tma_load_3d(da_s + gi * RG * 128, &tda, &bars->da_full, 0, key, slab);
-                        tma_load_3d(da_s + kRows * 128 + gi * RG * 128, &tda, &bars->da_full, 64, key, slab);
-                        tma_load_3d(dy_s + gi * RG * 128, &tdy, &bars->da_full, 0, key, slab);
-                        tma_load_3d(dy_s + kRows * 128 + gi * RG * 128, &tdy, &bars->da_full, 64, key, slab);
+                        const int grp = un.bhl * p.na + g_first + gi;
+                        tma_load_4d(da_s + gi * RG * 128, &tda, &bars->da_full, 0, 0, key, grp);
+                        tma_load_4d(da_s + kRows * 128 + gi * RG * 128, &tda, &bars->da_full, 64, 0, key, grp);
+                        tma_load_4d(dy_s + gi * RG * 128, &tdy, &bars->da_full, 0, 0, key, grp);
+                        tma_load_4d(dy_s + kRows * 128 + gi * RG * 128, &tdy, &bars->da_full, 64, 0, key, grp);
                     }
                 }
             }
@@ -471,7 +471,7 @@ size_t bwd_row_tc_partial_bytes(const MonarchParams& mp, int g0, int g1) {
     return (size_t)tiles * mp.nbh * (size_t)(g1 - g0) * mp.blk.b1 * mp.blk.b2 * kHeadDim * sizeof(float);
 }
 
-// Row-step backward for one slice.  maps = {q, K, V (the forward's), daL bridge, dY bridge (box 64 x 1 x rows_per_group)}.
+// Row-step backward for one slice.  maps = {q, K, V} (the forward's).
 int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* dcL, float* dq, float* part_k,
                       float* part_v, __nv_bfloat16* dk, __nv_bfloat16* dv, int g0, int g1, int* status, int num_sms,
                       cudaStream_t s) {
@@ -487,10 +487,13 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     rp.status = status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
     const int n_s = (mp.blk.b2 + 15) & ~15;
+    CUtensorMap bridge[2];
+    if (int rc = make_bridge_tmap(&bridge[0], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, rp.rows_per_group, 1)) return rc;
+    if (int rc = make_bridge_tmap(&bridge[1], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, rp.rows_per_group, 1)) return rc;
     auto go = [&](auto kernel) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRBSmem);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<grid, kThreadsRB, kRBSmem, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], rp);
+        kernel<<<grid, kThreadsRB, kRBSmem, s>>>(maps[0], maps[1], maps[2], bridge[0], bridge[1], rp);
         return 0;
     };
     int rc;

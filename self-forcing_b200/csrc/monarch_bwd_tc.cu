@@ -3,7 +3,7 @@
 // Forward column step, per slab (batch*head, query group a, column j), query row i, key n = (f, k):
 //   s[i,n] = scale * q[a,i,j] . aL[n] - cL[n],   P = softmax_n s,   out[a,i,j] = sum_n P[i,n] Y[n]
 // with aL[n] = sum_l R_l K_l and Y[n] = sum_l R_l V_l the row step's results (bf16, in the bridge layout
-// [slab][key][128]).  Given dOut, lse[i] = log sum_n exp s[i,n] (from a forward column step run just before)
+// [query group][key][column][128]).  Given dOut, lse[i] = log sum_n exp s[i,n] (from a forward column step run just before)
 // and delta[i] = dOut[i] . out[i], one sweep over the slab's keys in tiles of 128 gives every gradient:
 //   dP[i,n] = dOut[i] . Y[n]                      dS = P (dP - delta)
 //   dY[n]  = sum_i P[i,n] dOut[i]                 daL[n] = scale * sum_i dS[i,n] q[i]        dcL[n] = -sum_i dS[i,n]
@@ -53,7 +53,7 @@ struct BwdColParams {
     long long q_bs;
     const float* delta;            // [B, n_q, H]: dOut . out per token and head
     const float* lse;              // [slab][b1]
-    __nv_bfloat16* aL;             // bridge [slab][n_keys][128]: aL in, daL out
+    __nv_bfloat16* aL;             // bridge [group][n_keys][column][128]: aL in, daL out
     __nv_bfloat16* Y;              // bridge: Y in, dY out
     const float* cL;               // [slab][n_keys_c]
     float* dcL;                    // [slab][n_keys_c]
@@ -108,7 +108,7 @@ __device__ __forceinline__ BUnit b_decode(const BwdColParams& p, int u) {
     return r;
 }
 
-// tal / ty = bridge maps (box 64 x 128 keys x 1); tqr / tdo = query rows of q / dOut (5-D, box of 32 rows).
+// tal / ty = bridge maps (box 64 x 1 column x 128 keys); tqr / tdo = query rows of q / dOut (5-D, box of 32 rows).
 template <int NC>
 __global__ void __launch_bounds__(kThreadsB, 1)
 monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap ty,
@@ -165,6 +165,7 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
         for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u, ++uc) {
             const BUnit un = b_decode(p, u);
             const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+            const int grp = un.bhl * p.A + un.a;
             const int qb = kQBufs == 2 ? (uc & 1) : 0;
             unsigned char* qt = qd_s + qb * kQdBuf;
             auto load_tiles = [&](int t_begin, int t_end) {      // lane 0 only
@@ -173,10 +174,10 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                     if (g >= kStgB && !mbar_wait(&bars->a_empty[s], ((g / kStgB) - 1) & 1)) { fail(11); ok = false; break; }
                     unsigned char* st = a_s + s * kBStage;
                     mbar_arrive_expect_tx(&bars->a_full[s], (uint32_t)kBStage);
-                    tma_load_3d(st, &tal, &bars->a_full[s], 0, t * kKB, u);
-                    tma_load_3d(st + kKB * 128, &tal, &bars->a_full[s], 64, t * kKB, u);
-                    tma_load_3d(st + kBTile, &ty, &bars->a_full[s], 0, t * kKB, u);
-                    tma_load_3d(st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, t * kKB, u);
+                    tma_load_4d(st, &tal, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                    tma_load_4d(st + kKB * 128, &tal, &bars->a_full[s], 64, un.j, t * kKB, grp);
+                    tma_load_4d(st + kBTile, &ty, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                    tma_load_4d(st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, un.j, t * kKB, grp);
                 }
             };
             // the slab's first tile does not wait for the query-side buffer
@@ -360,7 +361,8 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 for (int cc = 0; cc < NC; ++cc) acc += bars->dsum[gt & 1][cc][row];
                 p.dcL[(long long)u * p.n_keys_c + key] = -acc;
             }
-            const long long ro = ((long long)u * n_keys + key) * kHeadDim;
+            const BUnit un = b_decode(p, u);
+            const long long ro = ((((long long)un.bhl * p.A + un.a) * n_keys + key) * blk.b2 + un.j) * kHeadDim;
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 __nv_bfloat16* dst = (half ? p.Y : p.aL) + ro;
@@ -396,7 +398,6 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 tmem_wait_ld();
                 tc_fence_before();
                 mbar_arrive(&bars->dq_free);
-                const BUnit un = b_decode(p, u);
                 const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
 #pragma unroll
                 for (int cc = 0; cc < NC; ++cc) {
@@ -444,8 +445,7 @@ int launch_bwd_delta(const void* dout, const void* out, float* delta, long long 
     return (int)cudaGetLastError();
 }
 
-// Column-step backward for one slice of (batch, head) pairs.  maps = {aL bridge, Y bridge, q rows, dOut rows}; the
-// two row maps are 5-D (d, head, column, row of the token grid, batch) with boxes of 32 rows.
+// Column-step backward for one slice of (batch, head) pairs.  maps = {q rows, dOut rows}, 5-D (d, head, column, row of the token grid, batch) with boxes of 32 rows.
 int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* delta, float* dcL, float* dq,
                       int* status, int num_sms, cudaStream_t s) {
     if (mp.blk.b1 > kMaxNC * kNI) return SFM_ERR_UNSUPPORTED;
@@ -464,10 +464,13 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     p.status = status;
     dim3 grid(p.n_units < num_sms ? p.n_units : num_sms);
     const int nc = (mp.blk.b1 + kNI - 1) / kNI;
+    CUtensorMap bridge[2];
+    if (int rc = make_bridge_tmap(&bridge[0], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
+    if (int rc = make_bridge_tmap(&bridge[1], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
     auto go = [&](auto kernel, int smem) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<grid, kThreadsB, smem, s>>>(maps[0], maps[1], maps[2], maps[3], p);
+        kernel<<<grid, kThreadsB, smem, s>>>(bridge[0], bridge[1], maps[0], maps[1], p);
         return 0;
     };
     int rc = nc == 1 ? go(monarch_bwd_col_tc_kernel<1>, b_smem_bytes(1))

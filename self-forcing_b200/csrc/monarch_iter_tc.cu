@@ -35,7 +35,6 @@ __host__ __device__ constexpr uint32_t it_col_o(int w) { return 256u + (uint32_t
 struct ItParams {
     MonarchParams mp;
     int n_units;       // nbh * na * b2
-    int R4;            // query rows per TMA box (ceil(b1 / 4))
     int q_rows_tma;    // query rows of a unit are consecutive rows of the token grid
     int* status;
 };
@@ -73,7 +72,7 @@ __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
     return r;
 }
 
-// tal = bridge aL map (box 64 x 128 keys x 1), tqr = query rows (5-D, box rows = R4).
+// tal = bridge aL map (box 64 x 1 column x 128 keys), tqr = query rows (5-D, box of b1 rows).
 template <int N_I>
 __global__ void __launch_bounds__(kThreadsIt, 1)
 monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap tqr, ItParams ip) {
@@ -89,7 +88,6 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
     const int b1 = blk.b1, b2 = blk.b2;
     const int n_keys = p.n_keys;
     const int n_tiles = (n_keys + kKTile - 1) / kKTile;
-    const int R4 = ip.R4;
     const long long tok_pitch = (long long)p.H * kHeadDim;
     const int u_begin = (int)((long long)ip.n_units * blockIdx.x / gridDim.x);
     const int u_end = (int)((long long)ip.n_units * (blockIdx.x + 1) / gridDim.x);
@@ -138,15 +136,11 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             if (ip.q_rows_tma) {
                 __syncwarp();
                 if (lane == 0) {
-                    const int nq = (b1 + R4 - 1) / R4;
-                    mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(nq * R4 * 256));
+                    mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(b1 * 256));
                     const int tok0 = blk.row_token(p.a0 + un.al, 0);
                     const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
-                    for (int qd = 0; qd < nq; ++qd) {
-                        unsigned char* dst = qd_s + (qd * R4) * 128;
-                        tma_load_5d(dst, &tqr, &bars->q_full[qb], 0, hd, col, frow0 + qd * R4, b);
-                        tma_load_5d(dst + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0 + qd * R4, b);
-                    }
+                    tma_load_5d(qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
+                    tma_load_5d(qd_s + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
                 }
             } else {
                 const __nv_bfloat16* qg = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
@@ -166,8 +160,8 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                     if (g >= kAStg && !mbar_wait(&bars->a_empty[s], ((g / kAStg) - 1) & 1)) { fail(11); ok = false; break; }
                     unsigned char* st = a_s + s * kItTileBytes;
                     mbar_arrive_expect_tx(&bars->a_full[s], (uint32_t)kItTileBytes);
-                    tma_load_3d(st, &tal, &bars->a_full[s], 0, t * kKTile, u);
-                    tma_load_3d(st + kKTile * 128, &tal, &bars->a_full[s], 64, t * kKTile, u);
+                    tma_load_4d(st, &tal, &bars->a_full[s], 0, un.j, t * kKTile, un.bhl * p.na + un.al);
+                    tma_load_4d(st + kKTile * 128, &tal, &bars->a_full[s], 64, un.j, t * kKTile, un.bhl * p.na + un.al);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -294,22 +288,22 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
 
 }  // namespace
 
-// Launches the tensor-core iteration update for one chunk.  maps = {aL (box 64 x 128 keys x 1), query rows (5-D)}.
-int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_al, const CUtensorMap* map_qrows, int* status,
-                     int num_sms, cudaStream_t s) {
+// Launches the tensor-core iteration update for one chunk.  map_qrows = query rows, 5-D, box of b1 rows.
+int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s) {
     if (p.blk.b1 > 128) return SFM_ERR_UNSUPPORTED;
     LaunchScope scope(kClsLIter, s);
     ItParams ip;
     ip.mp = p;
     ip.n_units = p.nbh * p.na * p.blk.b2;
-    ip.R4 = (p.blk.b1 + 3) / 4;
+    CUtensorMap map_al;
+    if (int rc = make_bridge_tmap(&map_al, p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, 1, kKTile)) return rc;
     ip.q_rows_tma = (p.blk.f_tied == 1 || p.blk.h_reduce == 1) ? 1 : 0;
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kItSmemBytes);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<grid, kThreadsIt, kItSmemBytes, s>>>(*map_al, *map_qrows, ip);
+        kernel<<<grid, kThreadsIt, kItSmemBytes, s>>>(map_al, *map_qrows, ip);
         return 0;
     };
     int rc;

@@ -45,8 +45,10 @@ __global__ void __launch_bounds__(kLWarps * 32, 1) monarch_l_kernel(MonarchParam
     const int ntiles = (nkeys + kLTileKeys - 1) / kLTileKeys;
     const long long tok_pitch = (long long)p.H * kHeadDim;
 
-    const __nv_bfloat16* a_src = p.aL + aj * p.n_keys * kHeadDim;
-    const __nv_bfloat16* y_src = kLseOnly ? nullptr : p.Y + aj * p.n_keys * kHeadDim;
+    // bridge rows [group][key][column]: this unit's keys lie b2 rows apart
+    const long long src0 = (((long long)bhl * p.na + al) * p.n_keys * b2 + j) * kHeadDim;
+    const __nv_bfloat16* a_src = p.aL + src0;
+    const __nv_bfloat16* y_src = kLseOnly ? nullptr : p.Y + src0;
     const float* c_src = p.cL + aj * p.n_keys_c;
 
     {   // queries Q[a, i0.., j]: rows of 256 bytes gathered from natural order
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(kLWarps * 32, 1) monarch_l_kernel(MonarchParam
         for (int idx = tid; idx < kLTileKeys * 16; idx += kLWarps * 32) {
             int r = idx >> 4, vec = idx & 15;
             bool ok = key0 + r < nkeys;
-            long long off = ok ? (long long)(key0 + r) * kHeadDim + vec * 8 : 0;
+            long long off = ok ? (long long)(key0 + r) * b2 * kHeadDim + vec * 8 : 0;
             cp_async16(Ad + r * kLds + vec * 8, a_src + off, ok ? 16 : 0);
             if (!kLseOnly) cp_async16(Yd + r * kLds + vec * 8, y_src + off, ok ? 16 : 0);
         }
@@ -294,11 +296,11 @@ __global__ void __launch_bounds__(128, 2) monarch_l_iter_kernel(MonarchParams p)
         long long off = ok ? (blk.row_token(a_abs, r) + j) * tok_pitch + vec * 8 : 0;
         cp_async16(Qs + r * kLds + vec * 8, qb + off, ok ? 16 : 0);
     }
-    const __nv_bfloat16* a_src = p.aL + aj * nkeys * kHeadDim;
+    const __nv_bfloat16* a_src = p.aL + (((long long)bhl * p.na + al) * nkeys * b2 + j) * kHeadDim;
     for (int idx = tid; idx < 64 * 16; idx += 128) {
         int r = idx >> 4, vec = idx & 15;
         bool ok = key0 + r < nkeys;
-        long long off = ok ? (long long)(key0 + r) * kHeadDim + vec * 8 : 0;
+        long long off = ok ? (long long)(key0 + r) * b2 * kHeadDim + vec * 8 : 0;
         cp_async16(As + r * kLds + vec * 8, a_src + off, ok ? 16 : 0);
     }
     cp_async_commit();

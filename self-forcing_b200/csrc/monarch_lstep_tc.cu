@@ -1,28 +1,36 @@
-// Monarch column step, and dense attention, on the 5th-generation tensor cores (tcgen05 + TMEM).
+// Monarch column step on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
-// Column step.  One unit = (batch*head, query group a, column j): the b1 queries Q[a,:,j] attend the
-// n_keys = F*b1 summary keys aL[a,f,j,k] (bias -cL, values Y) produced by the row step.  The MMA tile
-// is 128 rows tall but a unit has only b1 queries (30 at 480p framewise), so a CTA works on a GROUP
-// of U = floor(32 / ceil(b1/4)) consecutive units at once: query i of unit slot u sits on tile row
-// (i / R4)*32 + u*R4 + i % R4 with R4 = ceil(b1/4), i.e. every TMEM lane quadrant carries R4 rows of
-// every unit.  Keys stream through shared memory in tiles of 128 per unit:
+// One unit = (batch*head, query group a, column j): the b1 queries Q[a,:,j] attend the n_keys = F*b1 summary keys
+// aL[a,f,j,k] (bias -cL, values Y) produced by the row step.  The MMA tile is 128 rows tall but a unit has only b1
+// queries (30 at 480p framewise), so a CTA works on a GROUP of U = min(8, 128 / b1) consecutive units at once: query i of
+// unit slot u sits on tile row u*R + i with R = 128 / U.  Keys stream through shared memory in tiles of KT <= 128 per unit:
 //   S  = Q_tile aL_tile(u)^T        tcgen05.mma with a lane mask that only updates unit u's rows
 //   P  = exp2(scale*S - cL - m)     one thread per tile row, running max / sum in registers
 //   O += P Y_tile(u)                tcgen05.mma, A = P (bf16) from TMEM, same lane mask
-// Even and odd key tiles go to two softmax warpgroups with their own S/P buffer and accumulator
-// (split-KV); the epilogue warpgroup merges the two partial softmaxes, normalises and writes each
-// row to natural token order with 32-byte stores (the inverse layout map is the store address).
+// Key tiles alternate, across the groups too, between two softmax warpgroups with their own S/P buffer and accumulator
+// (split-KV; a group of one tile leaves the other side to the next group); the
+// epilogue warpgroup merges the two partial softmaxes, normalises and writes each row to natural token order with
+// 32-byte stores (the inverse layout map is the store address).
 //
-// Dense attention (kDense = true): a unit is 128 consecutive queries of one (batch, head), U = 1, key /
-// value tiles come straight from the KV cache, there is no bias and no lane mask.
+// KT is the number of keys divided evenly over the tiles that 128-key tiles would take, so that short caches (90 keys per
+// 3-frame chunk at framewise) load and multiply fewer padding keys, and the two rings hold as many tiles as fit.
 //
-// Warp roles (16 warps): 0 = key-side producer (queries, aL tiles, bias slices), 3 = value-tile
-// producer, 1 = PV-GEMM issuer (owns the TMEM allocation), 2 = S-GEMM issuer, 4..7 / 8..11 = softmax
-// warpgroups, 12..15 = epilogue warpgroup.  All roles run the same loops and meet only through
-// mbarriers with bounded waits; a timeout records a status code and the CTA unwinds.
+// Warp roles (16 warps): 0 = bias slices and aL tiles, 3 = Y tiles, 1 = PV-GEMM issuer (owns the TMEM allocation), 2 = the
+// groups' query rows and the S GEMMs, 4..7 / 8..11 = softmax warpgroups, 12..15 = epilogue warpgroup.  Roles 0 to 3 run as
+// whole warps with an elected issuing lane.  The query rows have one buffer: warp 2 reloads it as soon as its last S GEMM
+// of a group has completed, which the softmax and PV GEMMs of that group cover, while warp 0 is already loading the next
+// group's keys.  All roles meet only through mbarriers with bounded waits; a timeout records a status code and the CTA
+// unwinds.
 //
-// Arithmetic follows monarch_attn_ref_op (wan/modules/monarch_attn.py:1821-1829) and, for the dense
-// instantiation, softmax(q k^T * scale) v (wan/modules/attention.py:177-187).
+// What bounds it: reading the bridge (604 MB in 0.114 ms at framewise, 21 cached frames, 12 heads: 5.4 TB/s with the start-up
+// and the uneven last round, 6.3 in between; a bare TMA stream of the same tiles reaches 6.5), and at short caches, whose
+// bridge is in L2, the chain of a group (90 keys: 43 -> 29 us).  Against the form with queries spread over the four lane
+// quadrants, MMAs issued from one-lane code, two softmax passes and a warpgroup chosen by tile parity within the group:
+// a masked MMA took up to 165 cycles to issue, a query tile 32 boxes instead of 8, the bias reads met four-way bank
+// conflicts, and groups of one tile ran one after another.  4 videos, reduce2xh, 9 frames: 0.503 -> 0.388 ms;
+// reduce4xw2xh, 21 frames: 1.165 -> 1.008 ms.
+//
+// Arithmetic follows monarch_attn_ref_op (wan/modules/monarch_attn.py:1821-1829).
 #include "monarch_params.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -33,67 +41,53 @@ using namespace tc;
 
 namespace {
 
-constexpr int kAStages = 2;    // key (aL) tile ring, released as soon as the S GEMM has read a tile
-constexpr int kYStages = 3;    // value (Y) tile ring, released after the PV GEMM
+constexpr int kMaxStages = 8;              // tiles per ring, at most
 constexpr int kThreads = 512;
-constexpr int kKT = 128;                   // keys per tile
+constexpr int kKT = 128;                   // keys per tile, at most
 constexpr int kMaxU = 8;                   // units per group (the bias ring is sized for it)
+constexpr int kBiasPitch = kKT + 4;        // the rows of a warp may read two units' slices: different banks
 constexpr uint32_t kTmemCols = 512;
 // TMEM columns: S / P buffers of the two softmax warpgroups at 0 and 128, their accumulators at 256 and 384
 __host__ __device__ constexpr uint32_t col_s(int w) { return (uint32_t)w * 128u; }
 __host__ __device__ constexpr uint32_t col_o(int w) { return 256u + (uint32_t)w * 128u; }
-constexpr float kRescaleThreshold = 8.0f;  // log2 units: accumulators are rescaled only past this growth
+constexpr float kRescaleThreshold = 40.0f; // log2 units: the reference of a row moves only past this growth
 
 struct LTcParams {
     MonarchParams mp;
-    int n_units;     // column step: nbh * na * b2;  dense: B*H * ceil(n_q / 128)
+    int n_units;     // nbh * na * b2
     int U;           // units per group
-    int R4;          // tile rows per unit per lane quadrant
+    int R;           // tile rows per unit slot (128 / U, rounded down)
+    int kt;          // keys per tile (multiple of 16, <= 128)
+    int n_a, n_y;    // tiles in the aL and Y rings
     int q_rows_tma;  // the query rows of a unit are consecutive rows of the token grid: load them with TMA
-    int n_kv;        // dense: keys per (batch, head)
-    int q_tiles;     // dense: ceil(n_q / 128)
-    int write_lse;   // column step: also store the log-sum-exp of every query row (iterative variant)
-    int lse_only;    // column step: nothing but that (no value tiles, no PV GEMMs, no output rows)
+    int write_lse;   // also store the log-sum-exp of every query row (iterative variant, backward)
+    int lse_only;    // nothing but that (no value tiles, no PV GEMMs, no output rows)
     int* status;
 };
 
-
 struct __align__(16) Barriers {
-    alignas(16) float cl[4][kMaxU][kKT];   // bias slices, per unit slot: two ring slots for each softmax warpgroup
+    alignas(16) float cl[4][kMaxU][kBiasPitch];   // bias slices, per unit slot: a ring of four tiles
     float stats[2][2][128];                // [warpgroup][m | l][tile row]
     uint64_t q_full, q_empty;
-    uint64_t a_full[kAStages], a_empty[kAStages];
-    uint64_t y_full[kYStages], y_empty[kYStages];
+    uint64_t a_full[kMaxStages], a_empty[kMaxStages];
+    uint64_t y_full[kMaxStages], y_empty[kMaxStages];
     uint64_t cl_full[4], cl_empty[4];
-    uint64_t s_full[4], p_full[4], sp_free[4];   // [warpgroup * 2 + half]: dense attention works on 64-key halves of a tile
+    uint64_t s_full[2], p_full[2], sp_free[2];
     uint64_t pv_done[2];                   // all PV GEMMs issued so far into accumulator w have completed
-    uint64_t o_full, o_free;
+    uint64_t o_full[2];                    // by group parity
+    uint64_t o_free[2];                    // accumulator and statistics of warpgroup w have been read
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
 constexpr int kQBytes = 2 * 128 * 128;     // query tile, two 64-column halves
-constexpr int kTileBytes = 2 * kKT * 128;  // one key or value tile
-constexpr int kSmemBytes = 1024 + kQBytes + (kAStages + kYStages) * kTileBytes + (int)sizeof(Barriers) + 64;
+constexpr int kRing = 172 << 10;           // aL tiles, then Y tiles
+constexpr int kSmemBytes = 1024 + kQBytes + kRing + (int)sizeof(Barriers) + 64;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(ptr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
                  "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-}
-// tcgen05.mma with an output-lane mask: bit i of `dis` set = rows i, 32+i, 64+i, 96+i of D are NOT written.
-__device__ __forceinline__ void mma_ss_masked(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accum, uint32_t dis) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum), "r"(dis) : "memory");
-}
-__device__ __forceinline__ void mma_ts_masked(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accum, uint32_t dis) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "r"(dis) : "memory");
 }
 
 struct LUnit { int bhl, al, j; };
@@ -105,9 +99,8 @@ __device__ __forceinline__ LUnit decode_unit(const MonarchParams& p, int u) {
     return r;
 }
 
-// Column step: tal / ty = bridge aL / Y maps (box 64 x 128 keys x 1), tqr = query rows (5-D).
-// Dense:       tal / ty = K / V cache maps (4-D, box 64 x 1 x 128 tokens x 1), tqr = q map (same geometry).
-template <bool kDense, bool kCausal>
+// tal / ty = bridge aL / Y maps [group][key][column][128] (box 64 x 1 column x kt keys), tqr = query rows (5-D, box b1 rows).
+template <bool kCausal>
 __global__ void __launch_bounds__(kThreads, 1)
 monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap ty,
                     const __grid_constant__ CUtensorMap tqr, LTcParams lp) {
@@ -115,55 +108,48 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = base;
     unsigned char* a_s = q_s + kQBytes;
-    unsigned char* y_s = a_s + kAStages * kTileBytes;
-    Barriers* bars = reinterpret_cast<Barriers*>(y_s + kYStages * kTileBytes);
+    unsigned char* y_s = a_s + lp.n_a * lp.kt * 256;
+    Barriers* bars = reinterpret_cast<Barriers*>(a_s + kRing);
 
     const MonarchParams& p = lp.mp;
     const Blocking& blk = p.blk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int b1 = blk.b1, b2 = blk.b2;
-    // Dense attention splits every 128-key tile into two 64-key halves with an S / P buffer each (64 columns), so that
-    // the S GEMM of one half runs while the other half's softmax does; the column step, bound by its bridge reads,
-    // keeps whole tiles.
-    constexpr int kH = kDense ? 2 : 1;
-    constexpr int kNS = kKT / kH;
-    const int n_keys = kDense ? lp.n_kv : p.n_keys;
-    const int n_tiles_all = (n_keys + kKT - 1) / kKT;
-    // Key tiles a group of units has to walk.  Block-causal (no-cache path): the keys past the last cached
-    // group any of the group's units may see carry an infinite bias, so the walk stops before them.
-    auto group_tiles = [&](int u0, int nu) -> int {
-        if (!kCausal) return n_tiles_all;
-        int fmax = 0;
-        for (int us = 0; us < nu; ++us) {
-            const int a_abs = p.a0 + decode_unit(p, u0 + us).al;
-            fmax = max(fmax, min(p.F, (a_abs / p.causal_groups + 1) * p.causal_groups));
-        }
-        return (fmax * b1 + kKT - 1) / kKT;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
+    const int b1 = blk.b1, b2 = blk.b2, kt = lp.kt;
+    const int U = lp.U, R = lp.R;
+    const int half = kt * 128, tile_bytes = 2 * half;       // one 64-column half of a key or value tile, the whole tile
+    // Keys a unit may see, and the tiles a group of units has to walk.  Block-causal (no-cache path): a unit sees the
+    // cached groups up to the end of its own causal block; its tiles past that are neither loaded nor multiplied, and
+    // the keys past it within its last tile get weight zero (the row step leaves finite values there).
+    auto unit_keys = [&](int u) -> int {
+        if (!kCausal) return p.n_keys;
+        const int a_abs = p.a0 + (u / b2) % p.na;
+        return min(p.F, (a_abs / p.causal_groups + 1) * p.causal_groups) * b1;
     };
-    const long long tok_pitch = (long long)p.H * kHeadDim;
-    const int U = lp.U, R4 = lp.R4;
+    auto group_tiles = [&](int u0, int nu) -> int {
+        int most = p.n_keys;
+        if (kCausal) {
+            most = 0;
+            for (int us = 0; us < nu; ++us) most = max(most, unit_keys(u0 + us));
+        }
+        return (most + kt - 1) / kt;
+    };
     // this CTA's contiguous share of the unit list, walked in groups of at most U units
-    // (dense: units are dealt round-robin instead, so that the CTAs running at the same time share keys in L2)
-    const int u_begin = kDense ? (int)blockIdx.x : (int)((long long)lp.n_units * blockIdx.x / gridDim.x);
-    const int u_end = kDense ? lp.n_units : (int)((long long)lp.n_units * (blockIdx.x + 1) / gridDim.x);
-    const int u_step = kDense ? (int)gridDim.x : U;
+    const int u_begin = (int)((long long)lp.n_units * blockIdx.x / gridDim.x);
+    const int u_end = (int)((long long)lp.n_units * (blockIdx.x + 1) / gridDim.x);
 
+    if (warp == 2 && lane == 0) { prefetch_tmap(&tqr); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
         mbar_init(&bars->q_full, 1);
         mbar_init(&bars->q_empty, 1);
-        for (int s = 0; s < kAStages; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1); }
-        for (int s = 0; s < kYStages; ++s) { mbar_init(&bars->y_full[s], 1); mbar_init(&bars->y_empty[s], 1); }
-        for (int w = 0; w < 2; ++w) {
-            mbar_init(&bars->cl_full[w], 1); mbar_init(&bars->cl_full[w + 2], 1);
-            mbar_init(&bars->cl_empty[w], 128); mbar_init(&bars->cl_empty[w + 2], 128);
-            for (int hh = 0; hh < 2; ++hh) {
-                mbar_init(&bars->s_full[2 * w + hh], 1); mbar_init(&bars->p_full[2 * w + hh], 128);
-                mbar_init(&bars->sp_free[2 * w + hh], 1);
-            }
-            mbar_init(&bars->pv_done[w], 1);
+        for (int s = 0; s < kMaxStages; ++s) {
+            mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1);
+            mbar_init(&bars->y_full[s], 1); mbar_init(&bars->y_empty[s], 1);
         }
-        mbar_init(&bars->o_full, 1);
-        mbar_init(&bars->o_free, 128);
+        for (int s = 0; s < 4; ++s) { mbar_init(&bars->cl_full[s], 1); mbar_init(&bars->cl_empty[s], 128); }
+        for (int w = 0; w < 2; ++w) {
+            mbar_init(&bars->s_full[w], 1); mbar_init(&bars->p_full[w], 128); mbar_init(&bars->sp_free[w], 1);
+            mbar_init(&bars->pv_done[w], 1); mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128);
+        }
         bars->abort_flag = 0;
         mbar_init_fence();
     }
@@ -175,7 +161,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
-    // tile rows that belong to no unit are never written by a GEMM: give their logits a defined value
+    // tile rows that belong to no unit, and columns past kt, are never written by a GEMM: give their logits a defined value
     if (warp >= 4 && warp < 12) {
         uint32_t z[32];
 #pragma unroll
@@ -193,52 +179,77 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         bars->abort_flag = 1;
         atomicCAS(lp.status, 0, code);
     };
-    // lane mask of unit slot u: only its R4 lanes of each quadrant are written
-    auto dis_mask = [&](int u) -> uint32_t {
-        if (kDense) return 0u;
-        const uint32_t en = (R4 >= 32 ? 0xffffffffu : ((1u << R4) - 1u)) << (u * R4);
-        return ~en;
-    };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ key-side producer
-        if (lane == 0) { prefetch_tmap(&tal); prefetch_tmap(&tqr); }
-        int ga = 0, gc = 0;                  // running counters: aL tiles, groups
-        int cnt[2] = {0, 0};                 // tiles given to each softmax warpgroup so far
+        // ------------------------------------------------------------------ bias slices and key tiles
+        const uint32_t el = elect_one();
+        int sa = 0, pa = 1, gt = 0;              // ring slot and its phase, tiles of all groups so far
         bool ok = true;
-        for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += u_step, ++gc) {
-            const int nu = kDense ? 1 : min(U, u_end - u0);
-            const int n_tiles = group_tiles(u0, nu);
-            if (gc > 0) {
-                int okw = 1;
-                if (lane == 0) okw = mbar_wait(&bars->q_empty, (gc - 1) & 1) ? 1 : 0;
-                if (!__shfl_sync(0xffffffffu, okw, 0)) { fail(10); break; }
-            }
-            // ---- queries of the group
-            if (kDense) {
-                if (lane == 0) {
-                    const int qt = u0 % lp.q_tiles, bh = u0 / lp.q_tiles, b = bh / p.H, hd = bh - b * p.H;
-                    mbar_arrive_expect_tx(&bars->q_full, (uint32_t)kQBytes);
-                    tma_load_4d(q_s, &tqr, &bars->q_full, 0, hd, qt * 128, b);
-                    tma_load_4d(q_s + 128 * 128, &tqr, &bars->q_full, 64, hd, qt * 128, b);
+        for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
+                const int cslot = gt & 3;
+                if (!mbar_wait_u(&bars->cl_empty[cslot], ((gt >> 2) & 1) ^ 1)) { fail(13); ok = false; break; }
+                const int have = min(kt, p.n_keys_c - t * kt);                  // floats that exist (multiple of 4)
+                mbar_arrive_expect_tx_e(el, &bars->cl_full[cslot], (uint32_t)(nu * have * 4));
+                for (int us = 0; us < nu; ++us)
+                    bulk_load_e(el, bars->cl[cslot][us], p.cL + (long long)(u0 + us) * p.n_keys_c + t * kt, (uint32_t)(have * 4),
+                                &bars->cl_full[cslot]);
+                for (int us = 0; us < nu; ++us) {
+                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (!mbar_wait_u(&bars->a_empty[sa], pa)) { fail(11); ok = false; break; }
+                    const LUnit un = decode_unit(p, u0 + us);
+                    unsigned char* at = a_s + sa * tile_bytes;
+                    mbar_arrive_expect_tx_e(el, &bars->a_full[sa], (uint32_t)tile_bytes);
+                    tma_load_4d_e(el, at, &tal, &bars->a_full[sa], 0, un.j, t * kt, un.bhl * p.na + un.al);
+                    tma_load_4d_e(el, at + half, &tal, &bars->a_full[sa], 64, un.j, t * kt, un.bhl * p.na + un.al);
+                    if (++sa == lp.n_a) { sa = 0; pa ^= 1; }
                 }
-            } else if (lp.q_rows_tma) {
-                if (lane == 0) {
-                    const int nq = (b1 + R4 - 1) / R4;                       // quadrants that hold rows
-                    mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(nu * nq * R4 * 256));
+            }
+        }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ value tiles
+        if (!lp.lse_only) {
+            const uint32_t el = elect_one();
+            int sy = 0, py = 1;
+            bool ok = true;
+            for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
+                const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+                for (int t = 0; ok && t < n_tiles; ++t)
                     for (int us = 0; us < nu; ++us) {
+                        if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                        if (!mbar_wait_u(&bars->y_empty[sy], py)) { fail(12); ok = false; break; }
                         const LUnit un = decode_unit(p, u0 + us);
-                        const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-                        const int tok0 = blk.row_token(p.a0 + un.al, 0);
-                        const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
-                        for (int qd = 0; qd < nq; ++qd) {
-                            unsigned char* dst = q_s + (qd * 32 + us * R4) * 128;
-                            tma_load_5d(dst, &tqr, &bars->q_full, 0, hd, col, frow0 + qd * R4, b);
-                            tma_load_5d(dst + 128 * 128, &tqr, &bars->q_full, 64, hd, col, frow0 + qd * R4, b);
-                        }
+                        unsigned char* yt = y_s + sy * tile_bytes;
+                        mbar_arrive_expect_tx_e(el, &bars->y_full[sy], (uint32_t)tile_bytes);
+                        tma_load_4d_e(el, yt, &ty, &bars->y_full[sy], 0, un.j, t * kt, un.bhl * p.na + un.al);
+                        tma_load_4d_e(el, yt + half, &ty, &bars->y_full[sy], 64, un.j, t * kt, un.bhl * p.na + un.al);
+                        if (++sy == lp.n_y) { sy = 0; py ^= 1; }
                     }
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ query rows, S GEMMs
+        const uint32_t el = elect_one();
+        const uint32_t idesc_s = idesc_bf16(128, 0, 0, 0) | ((uint32_t)(kt >> 3) << 17);
+        const uint64_t q_desc = smem_desc_sw128(smem_addr(q_s), 16, 1024);
+        const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
+        auto load_q = [&](int u0) {
+            const int nu = min(U, u_end - u0);
+            if (lp.q_rows_tma) {
+                // the 128-byte swizzle is a function of the shared-memory address, so a box may land on any tile row
+                mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(nu * b1 * 256));
+                for (int us = 0; us < nu; ++us) {
+                    const LUnit un = decode_unit(p, u0 + us);
+                    const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+                    const int tok0 = blk.row_token(p.a0 + un.al, 0);
+                    const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
+                    unsigned char* dst = q_s + us * R * 128;
+                    tma_load_5d_e(el, dst, &tqr, &bars->q_full, 0, hd, col, frow0, b);
+                    tma_load_5d_e(el, dst + 128 * 128, &tqr, &bars->q_full, 64, hd, col, frow0, b);
                 }
             } else {
+                // query rows that are not consecutive rows of the token grid are gathered with plain loads
                 for (int us = 0; us < nu; ++us) {
                     const LUnit un = decode_unit(p, u0 + us);
                     const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
@@ -246,8 +257,8 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                     for (int idx = lane; idx < b1 * 16; idx += 32) {
                         const int i = idx >> 4, ch = idx & 15;
                         const uint4 val = *reinterpret_cast<const uint4*>(
-                            qb + (blk.row_token(p.a0 + un.al, i) + un.j) * tok_pitch + ch * 8);
-                        const int r = (i / R4) * 32 + us * R4 + (i % R4);
+                            qb + (long long)(blk.row_token(p.a0 + un.al, i) + un.j) * p.H * kHeadDim + ch * 8);
+                        const int r = us * R + i;
                         *reinterpret_cast<uint4*>(q_s + (ch >> 3) * (128 * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = val;
                     }
                 }
@@ -255,183 +266,74 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->q_full);
             }
-            // ---- per key tile: the bias slices of all units, then each unit's aL tile
-            for (int t = 0; ok && t < n_tiles; ++t) {
-                const int w = t & 1;
-                const int idx = cnt[w]++;
-                const int gt = cnt[0] + cnt[1] - 1;
-                if (!kDense) {
-                    // ring slot: two per softmax warpgroup, released by its threads after their last read
-                    const int cslot = w + 2 * (idx & 1);
-                    int okw = 1;
-                    if (lane == 0 && idx >= 2) okw = mbar_wait(&bars->cl_empty[cslot], ((idx >> 1) - 1) & 1) ? 1 : 0;
-                    if (!__shfl_sync(0xffffffffu, okw, 0)) { fail(13); ok = false; break; }
-                    const int have = min(kKT, p.n_keys_c - t * kKT);            // floats that exist (multiple of 4)
-                    if (have < kKT) {                                            // the rest masks its keys
-                        for (int us = 0; us < nu; ++us)
-                            for (int e = have + lane; e < kKT; e += 32) bars->cl[cslot][us][e] = INFINITY;
-                        __syncwarp();
-                    }
-                    if (lane == 0) {
-                        mbar_arrive_expect_tx(&bars->cl_full[cslot], (uint32_t)(nu * have * 4));
-                        for (int us = 0; us < nu; ++us) {
-                            const LUnit un = decode_unit(p, u0 + us);
-                            const long long aj = ((long long)un.bhl * p.na + un.al) * b2 + un.j;
-                            bulk_load(bars->cl[cslot][us], p.cL + aj * p.n_keys_c + t * kKT, (uint32_t)(have * 4), &bars->cl_full[cslot]);
-                        }
-                    }
-                }
-                for (int us = 0; us < nu; ++us, ++ga) {
-                    const int sa = ga % kAStages;
-                    int okw = 1;
-                    if (lane == 0 && ga >= kAStages) okw = mbar_wait(&bars->a_empty[sa], ((ga / kAStages) - 1) & 1) ? 1 : 0;
-                    if (!__shfl_sync(0xffffffffu, okw, 0)) { fail(11); ok = false; break; }
-                    if (lane == 0) {
-                        unsigned char* at = a_s + sa * kTileBytes;
-                        mbar_arrive_expect_tx(&bars->a_full[sa], (uint32_t)kTileBytes);
-                        if (kDense) {
-                            const int bh = u0 / lp.q_tiles, b = bh / p.H, hd = bh - b * p.H;
-                            tma_load_4d(at, &tal, &bars->a_full[sa], 0, hd, t * kKT, b);
-                            tma_load_4d(at + kKT * 128, &tal, &bars->a_full[sa], 64, hd, t * kKT, b);
-                        } else {
-                            const LUnit un = decode_unit(p, u0 + us);
-                            const int aj = (un.bhl * p.na + un.al) * b2 + un.j;
-                            tma_load_3d(at, &tal, &bars->a_full[sa], 0, t * kKT, aj);
-                            tma_load_3d(at + kKT * 128, &tal, &bars->a_full[sa], 64, t * kKT, aj);
-                        }
-                    }
-                }
-            }
-        }
-    } else if (warp == 3) {
-        // ------------------------------------------------------------------ value-tile producer
-        if (lane == 0 && !lp.lse_only) {
-            prefetch_tmap(&ty);
-            int gy = 0;
-            bool ok = true;
-            for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += u_step) {
-                const int nu = kDense ? 1 : min(U, u_end - u0);
-            const int n_tiles = group_tiles(u0, nu);
-                for (int t = 0; ok && t < n_tiles; ++t)
-                    for (int us = 0; us < nu; ++us, ++gy) {
-                        const int sy = gy % kYStages;
-                        if (gy >= kYStages && !mbar_wait(&bars->y_empty[sy], ((gy / kYStages) - 1) & 1)) { fail(12); ok = false; break; }
-                        unsigned char* yt = y_s + sy * kTileBytes;
-                        mbar_arrive_expect_tx(&bars->y_full[sy], (uint32_t)kTileBytes);
-                        if (kDense) {
-                            const int bh = u0 / lp.q_tiles, b = bh / p.H, hd = bh - b * p.H;
-                            tma_load_4d(yt, &ty, &bars->y_full[sy], 0, hd, t * kKT, b);
-                            tma_load_4d(yt + kKT * 128, &ty, &bars->y_full[sy], 64, hd, t * kKT, b);
-                        } else {
-                            const LUnit un = decode_unit(p, u0 + us);
-                            const int aj = (un.bhl * p.na + un.al) * b2 + un.j;
-                            tma_load_3d(yt, &ty, &bars->y_full[sy], 0, t * kKT, aj);
-                            tma_load_3d(yt + kKT * 128, &ty, &bars->y_full[sy], 64, t * kKT, aj);
-                        }
-                    }
-            }
-        }
-    } else if (warp == 2) {
-        // ------------------------------------------------------------------ S-GEMM issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = idesc_bf16(128, kNS, 0, 0);
-            const uint64_t q_desc = smem_desc_sw128(smem_addr(q_s), 16, 1024);
-            const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
-            int ga = 0, gc = 0, cnt[2] = {0, 0};
-            bool ok = true;
-            for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += u_step, ++gc) {
-                const int nu = kDense ? 1 : min(U, u_end - u0);
-            const int n_tiles = group_tiles(u0, nu);
-                if (!mbar_wait(&bars->q_full, gc & 1)) { fail(20); break; }
-                for (int t = 0; ok && t < n_tiles; ++t) {
-                    const int w = t & 1;
-                    const int idx = cnt[w]++;
-                    const int gt = cnt[0] + cnt[1] - 1;
-                    if (!kDense && idx >= 1 && !mbar_wait(&bars->sp_free[2 * w], (idx - 1) & 1)) { fail(25); ok = false; break; }
-                    for (int us = 0; us < nu; ++us, ++ga) {
-                        const int sa = ga % kAStages;
-                        if (!mbar_wait(&bars->a_full[sa], (ga / kAStages) & 1)) { fail(21); ok = false; break; }
-                        tc_fence_after();
-                        const uint64_t ad = a_desc0 + (uint64_t)((sa * kTileBytes) >> 4);
-                        const uint32_t dis = dis_mask(us);
-                        if (kDense) {
-                            for (int hh = 0; hh < 2; ++hh) {                   // keys [64 hh, 64 hh + 64) of the tile
-                                if (idx >= 1 && !mbar_wait(&bars->sp_free[2 * w + hh], (idx - 1) & 1)) { fail(25); ok = false; break; }
-                                tc_fence_after();
+        };
+        int sa = 0, pa = 0, gc = 0, gt = 0;
+        bool ok = true;
+        if (u_begin < u_end) load_q(u_begin);
+        for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            if (!mbar_wait_u(&bars->q_full, gc & 1)) { fail(20); break; }
+            for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
+                const int w = gt & 1;
+                if (!mbar_wait_u(&bars->sp_free[w], ((gt >> 1) & 1) ^ 1)) { fail(25); ok = false; break; }
+                for (int us = 0; us < nu; ++us) {
+                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (!mbar_wait_u(&bars->a_full[sa], pa)) { fail(21); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t ad = a_desc0 + (uint64_t)((sa * tile_bytes) >> 4);
+                    const LaneMask m = lane_mask_rows(us * R, R);
 #pragma unroll
-                                for (int ks = 0; ks < 8; ++ks) {
-                                    const uint32_t off = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;
-                                    mma_ss(tmem + col_s(w) + hh * kNS, q_desc + off, ad + off + (uint32_t)((hh * kNS * 128) >> 4), idesc_s, ks > 0);
-                                }
-                                mma_commit(&bars->s_full[2 * w + hh]);
-                            }
-                            if (!ok) break;
-                        } else {
-#pragma unroll
-                            for (int ks = 0; ks < 8; ++ks) {
-                                const uint32_t off = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;   // same geometry for both tiles
-                                mma_ss_masked(tmem + col_s(w), q_desc + off, ad + off, idesc_s, ks > 0, dis);
-                            }
-                        }
-                        mma_commit(&bars->a_empty[sa]);
+                    for (int ks = 0; ks < 8; ++ks) {
+                        const uint32_t qo = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;
+                        const uint32_t ao = ((ks >> 2) * half + (ks & 3) * 32) >> 4;
+                        mma_ss_masked_e(el, tmem + col_s(w), q_desc + qo, ad + ao, idesc_s, ks > 0, m);
                     }
-                    if (!ok) break;
-                    if (!kDense) mma_commit(&bars->s_full[2 * w]);
-                    if (t + 1 == n_tiles) mma_commit(&bars->q_empty);
+                    mma_commit_e(el, &bars->a_empty[sa]);
+                    if (++sa == lp.n_a) { sa = 0; pa ^= 1; }
                 }
+                if (!ok) break;
+                mma_commit_e(el, &bars->s_full[w]);
+            }
+            if (!ok) break;
+            if (u0 + U < u_end) {
+                mma_commit_e(el, &bars->q_empty);
+                if (!mbar_wait_u(&bars->q_empty, gc & 1)) { fail(10); break; }
+                load_q(u0 + U);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ PV-GEMM issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);
-            const uint64_t y_desc0 = smem_desc_sw128(smem_addr(y_s), kKT * 128, 1024);
-            int gy = 0, gc = 0, cnt[2] = {0, 0};
-            bool ok = true;
-            for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += u_step, ++gc) {
-                const int nu = kDense ? 1 : min(U, u_end - u0);
-            const int n_tiles = group_tiles(u0, nu);
-                for (int t = 0; ok && t < n_tiles; ++t) {
-                    const int w = t & 1;
-                    const int idx = cnt[w]++;
-                    const int gt = cnt[0] + cnt[1] - 1;
-                    if (!mbar_wait(&bars->p_full[2 * w], idx & 1)) { fail(22); ok = false; break; }
-                    // first GEMM of the group into this accumulator overwrites it: the previous group's
-                    // result must have been read
-                    if (t < 2 && gc > 0 && !mbar_wait(&bars->o_free, (gc - 1) & 1)) { fail(23); ok = false; break; }
-                    for (int us = 0; us < nu && !lp.lse_only; ++us, ++gy) {
-                        const int sy = gy % kYStages;
-                        if (!mbar_wait(&bars->y_full[sy], (gy / kYStages) & 1)) { fail(26); ok = false; break; }
-                        tc_fence_after();
-                        const uint64_t yd = y_desc0 + (uint64_t)((sy * kTileBytes) >> 4);
-                        const uint32_t dis = dis_mask(us);
-                        if (kDense) {
-                            for (int hh = 0; hh < 2; ++hh) {                   // the tile's two 64-key halves
-                                if (hh == 1 && !mbar_wait(&bars->p_full[2 * w + 1], idx & 1)) { fail(22); ok = false; break; }
-                                tc_fence_after();
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);
+        const uint64_t y_desc0 = smem_desc_sw128(smem_addr(y_s), half, 1024);
+        const int n_k = kt / 16;
+        int sy = 0, py = 0, gc = 0, gt = 0, used[2] = {0, 0};     // groups that accumulator w has taken part in
+        bool ok = true;
+        for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
+                const int w = gt & 1;
+                if (!mbar_wait_u(&bars->p_full[w], (gt >> 1) & 1)) { fail(22); ok = false; break; }
+                // first GEMM of the group into this accumulator overwrites it: the last result there must have been read
+                if (t < 2 && !mbar_wait_u(&bars->o_free[w], (used[w]++ & 1) ^ 1)) { fail(23); ok = false; break; }
+                for (int us = 0; us < nu && !lp.lse_only; ++us) {
+                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (!mbar_wait_u(&bars->y_full[sy], py)) { fail(26); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t yd = y_desc0 + (uint64_t)((sy * tile_bytes) >> 4);
+                    const LaneMask m = lane_mask_rows(us * R, R);
 #pragma unroll
-                                for (int kk = 0; kk < kNS / 16; ++kk)
-                                    mma_ts(tmem + col_o(w), tmem + col_s(w) + hh * kNS + kk * 8,
-                                           yd + (((hh * (kNS / 16) + kk) * 2048) >> 4), idesc_o, (t >= 2) || hh > 0 || (kk > 0));
-                                mma_commit(&bars->pv_done[w]);
-                                mma_commit(&bars->sp_free[2 * w + hh]);
-                            }
-                            if (!ok) break;
-                        } else {
-#pragma unroll
-                            for (int kk = 0; kk < kKT / 16; ++kk)
-                                mma_ts_masked(tmem + col_o(w), tmem + col_s(w) + kk * 8, yd + ((kk * 2048) >> 4), idesc_o,
-                                              (t >= 2) || (kk > 0), dis);
-                        }
-                        mma_commit(&bars->y_empty[sy]);
-                    }
-                    if (!ok) break;
-                    if (!kDense) {
-                        mma_commit(&bars->pv_done[w]);
-                        mma_commit(&bars->sp_free[2 * w]);
-                    }
-                    if (t + 1 == n_tiles) mma_commit(&bars->o_full);
+                    for (int kk = 0; kk < kKT / 16; ++kk)
+                        if (kk < n_k)
+                            mma_ts_masked_e(el, tmem + col_o(w), tmem + col_s(w) + kk * 8, yd + ((kk * 2048) >> 4), idesc_o,
+                                            (t >= 2) || (kk > 0), m);
+                    mma_commit_e(el, &bars->y_empty[sy]);
+                    if (++sy == lp.n_y) { sy = 0; py ^= 1; }
                 }
+                if (!ok) break;
+                mma_commit_e(el, &bars->pv_done[w]);
+                mma_commit_e(el, &bars->sp_free[w]);
+                if (t + 1 == n_tiles) mma_commit_e(el, &bars->o_full[gc & 1]);
             }
         }
     } else if (warp >= 4 && warp < 12) {
@@ -439,216 +341,178 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const int w = (warp - 4) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        const int us = kDense ? 0 : min(lane / R4, kMaxU - 1);       // unit slot whose bias this tile row uses
+        const int us = min(row / R, U - 1);                          // unit slot whose bias this tile row uses
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-        const uint32_t s_t0 = tmem + lane_sel + col_s(w);
+        const uint32_t s_t = tmem + lane_sel + col_s(w);
         const uint32_t o_t = tmem + lane_sel + col_o(w);
         const float scale_l2 = p.scale * kLog2e;
-        int gc = 0, idx = 0;                  // idx: tiles this warpgroup has handled so far
+        const uint64_t scale2 = f2_pack(scale_l2, scale_l2), nl2 = f2_pack(-kLog2e, -kLog2e);
+        int gt0 = 0, used = 0;                // tiles of the groups before this one; groups this warpgroup has taken part in
         bool ok = true;
-        for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += u_step, ++gc) {
-            const int n_tiles = group_tiles(u0, kDense ? 1 : min(U, u_end - u0));
+        for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += U) {
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            const int my_keys = us < nu ? unit_keys(u0 + us) : p.n_keys;
             float m_run = -INFINITY, l_run = 0.f;
             int my_tiles = 0;
-            for (int t = w; ok && t < n_tiles; t += 2) {
-              for (int hh = 0; hh < kH; ++hh) {                              // dense attention: the tile's two 64-key halves
-                const uint32_t s_t = s_t0 + hh * kNS;
-                const int valid = max(0, min(kNS, n_keys - t * kKT - hh * kNS));   // keys of this (half) tile that exist
-                if (!mbar_wait(&bars->s_full[2 * w + hh], idx & 1)) { fail(31); ok = false; break; }
-                const int cslot = w + 2 * (idx & 1);
+            for (int t = (gt0 & 1) ^ w; ok && t < n_tiles; t += 2) {
+                const int gt = gt0 + t, idx = gt >> 1;
+                const int lim = min(kt, my_keys - t * kt);           // keys of this tile that exist for this row
+                if (!mbar_wait(&bars->s_full[w], idx & 1)) { fail(31); ok = false; break; }
+                const int cslot = gt & 3;
                 const float* cs = bars->cl[cslot][us];
-                if (!kDense && !mbar_wait(&bars->cl_full[cslot], (idx >> 1) & 1)) { fail(33); ok = false; break; }
+                if (!mbar_wait(&bars->cl_full[cslot], (gt >> 2) & 1)) { fail(33); ok = false; break; }
                 tc_fence_after();
-                // pass 1: row maximum of the biased logits (log2 units)
-                const bool tail = kDense && valid < kNS;
-                const uint64_t scale2 = f2_pack(scale_l2, scale_l2), nl2 = f2_pack(-kLog2e, -kLog2e);
-                float lsum = 0.f;
-                bool spec_done = false;
-                if constexpr (kDense) {
-                    // After a warpgroup's first half tile the row maximum rarely moves past the rescale threshold, so
-                    // the half is first taken in ONE pass against the running reference; the packed P is only stored
-                    // if every row of the warp stayed below 2^threshold in total (then no weight exceeded it and the
-                    // two-pass path below would have produced the same bits), else the two passes run on the
-                    // untouched S.
-                    if (my_tiles > 0 && !tail) {
-                        const float nm = -m_run;
-                        const uint64_t nm2 = f2_pack(nm, nm);
-                        uint64_t ls2 = f2_pack(0.f, 0.f);
-                        uint32_t pk0[16], pk1[16];
-                        {
-                            uint32_t r[64];
-                            tmem_ld64(s_t, r);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int c = 0; c < 64; c += 2) {
-                                float d0, d1;
-                                f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), scale2, nm2), d0, d1);
-                                const float e0 = exp2f(d0), e1 = exp2f(d1);
-                                ls2 = f2_add(ls2, f2_pack(e0, e1));
-                                if (c < 32) pk0[c >> 1] = pack_bf16_alu(e0, e1);
-                                else pk1[(c - 32) >> 1] = pack_bf16_alu(e0, e1);
-                            }
-                        }
-                        float la, lb;
-                        f2_unpack(ls2, la, lb);
-                        const float ls = la + lb;
-                        if (!__any_sync(0xffffffffu, !(ls < 256.0f))) {      // 2^kRescaleThreshold; also catches inf / nan
-                            tmem_st16(s_t, pk0);
-                            tmem_st16(s_t + 16, pk1);
-                            tmem_wait_st();
-                            lsum = ls;
-                            spec_done = true;
-                        }
-                    }
-                }
-                if (!spec_done) {
-                float mx = -INFINITY;
+                // One pass over the tile, 32 keys at a time, against a reference m that is the maximum of the first 32 keys the
+                // row has seen: P is bf16 and the accumulators are fp32, so weights may exceed 1 without losing anything,
+                // and m only has to move when a logit outgrows it by 2^kRescaleThreshold.  The loop is not unrolled: its
+                // instructions are fetched from DRAM, behind the bridge traffic, each time the kernel starts.
+                uint64_t sum2 = f2_pack(0.f, 0.f);
 #pragma unroll 1
-                for (int c0 = 0; c0 < kNS; c0 += 64) {
-                    uint32_t r[64];
-                    tmem_ld64(s_t + c0, r);
-                    tmem_wait_ld();
-                    if (kDense && !tail) {
-                        // no bias: the maximum of the raw dot products (the scale is positive), two per instruction
-#pragma unroll
-                        for (int c = 0; c < 64; c += 2) mx = max3(mx, __uint_as_float(r[c]), __uint_as_float(r[c + 1]));
-                    } else if (kDense) {
-#pragma unroll
-                        for (int c = 0; c < 64; ++c)                         // keys past the end of the cache view
-                            mx = fmaxf(mx, c0 + c < valid ? __uint_as_float(r[c]) : -INFINITY);
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 64; c += 2) {                    // packed fp32 pairs: S * scale - log2(e) * cL
-                            const uint64_t bias2 = f2_mul(nl2, *reinterpret_cast<const uint64_t*>(&cs[c0 + c]));
-                            float x0, x1;
-                            f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), scale2, bias2), x0, x1);
-                            mx = max3(mx, x0, x1);
-                        }
-                    }
-                }
-                if (kDense) mx *= scale_l2;
-                // lazy rescale: keep the old reference while the maximum grew by less than the threshold
-                bool rescale = false;
-                float corr = 1.0f;
-                if (my_tiles == 0) {
-                    m_run = mx;
-                } else if (mx > m_run + kRescaleThreshold) {
-                    corr = exp2f(m_run - mx);
-                    m_run = mx;
-                    l_run *= corr;
-                    rescale = true;
-                }
-                if (__any_sync(0xffffffffu, rescale)) {
-                    // the accumulator may only be touched once the previous GEMMs into it have finished
-                    if (!mbar_wait(&bars->pv_done[w], (kH * idx + hh - 1) & 1)) { fail(32); ok = false; break; }
-                    tc_fence_after();
-#pragma unroll 1
-                    for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
+                for (int c0 = 0; c0 < kt; c0 += 32) {
+                    uint64_t x[16];                                  // biased logits, log2 units: S * scale - log2(e) * cL
+                    {
                         uint32_t r[32];
-                        tmem_ld32(o_t + c0, r);
+                        tmem_ld32(s_t + c0, r);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * corr);
-                        tmem_st32(o_t + c0, r);
+                        for (int c = 0; c < 16; c += 2) {
+                            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&cs[c0 + 2 * c]);
+                            x[c] = f2_fma(f2_pack(__uint_as_float(r[2 * c]), __uint_as_float(r[2 * c + 1])), scale2, f2_mul(nl2, b.x));
+                            x[c + 1] = f2_fma(f2_pack(__uint_as_float(r[2 * c + 2]), __uint_as_float(r[2 * c + 3])), scale2, f2_mul(nl2, b.y));
+                        }
                     }
-                    tmem_wait_st();
-                }
-                const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
-                // pass 2: P = exp2(logit - m), packed bf16 written back over the S columns already consumed
-                const uint64_t negm2 = f2_pack(neg_m, neg_m);
-                uint64_t lsum2 = f2_pack(0.f, 0.f);
+                    if (__any_sync(0xffffffffu, c0 + 32 > lim)) {     // keys that do not exist for this row
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) {
+                            float x0, x1;
+                            f2_unpack(x[c], x0, x1);
+                            x[c] = f2_pack(c0 + 2 * c < lim ? x0 : -INFINITY, c0 + 2 * c + 1 < lim ? x1 : -INFINITY);
+                        }
+                    }
+                    float mx = -INFINITY;
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        float x0, x1;
+                        f2_unpack(x[c], x0, x1);
+                        mx = max3(mx, x0, x1);
+                    }
+                    if (my_tiles == 0 && c0 == 0) {
+                        m_run = mx;
+                    } else if (__any_sync(0xffffffffu, mx > m_run + kRescaleThreshold)) {
+                        // move the reference of the rows that need it: what they have summed up so far, the P of this
+                        // tile's earlier keys and the accumulator are scaled down
+                        float corr = 1.0f;
+                        if (mx > m_run + kRescaleThreshold) {
+                            corr = exp2f(m_run - mx);
+                            m_run = mx;
+                        }
+                        l_run *= corr;
+                        sum2 = f2_mul(sum2, f2_pack(corr, corr));
 #pragma unroll 1
-                for (int c0 = 0; c0 < kNS; c0 += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(s_t + c0, r);
-                    tmem_wait_ld();
+                        for (int e0 = 0; e0 < c0 >> 1; e0 += 16) {
+                            uint32_t r[16];
+                            tmem_ld16(s_t + e0, r);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int c = 0; c < 16; ++c)
+                                r[c] = pack_bf16_alu(__uint_as_float(r[c] << 16) * corr, __uint_as_float(r[c] & 0xffff0000u) * corr);
+                            tmem_st16(s_t + e0, r);
+                        }
+                        if (my_tiles > 0) {
+                            // the accumulator may only be touched once the previous GEMMs into it have finished
+                            if (!mbar_wait(&bars->pv_done[w], (idx - 1) & 1)) { fail(32); ok = false; break; }
+                            tc_fence_after();
+#pragma unroll 1
+                            for (int e0 = 0; e0 < kHeadDim; e0 += 16) {
+                                uint32_t r[16];
+                                tmem_ld16(o_t + e0, r);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * corr);
+                                tmem_st16(o_t + e0, r);
+                            }
+                        }
+                        tmem_wait_st();
+                    }
+                    // P = exp2(x - m) as packed bf16 over the S columns already consumed, and its (unrounded) sum
+                    const float neg_m = m_run == -INFINITY ? 0.f : -m_run;
+                    const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
                     uint32_t pk[16];
 #pragma unroll
-                    for (int c = 0; c < 32; c += 2) {
-                        uint64_t shift2 = negm2;
-                        if (!kDense) shift2 = f2_fma(nl2, *reinterpret_cast<const uint64_t*>(&cs[c0 + c]), negm2);
+                    for (int c = 0; c < 16; ++c) {
                         float d0, d1;
-                        f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), scale2, shift2), d0, d1);
-                        float e0 = exp2f(d0), e1 = exp2f(d1);
-                        if (tail) {
-                            if (c0 + c >= valid) e0 = 0.f;
-                            if (c0 + c + 1 >= valid) e1 = 0.f;
-                        }
-                        lsum2 = f2_add(lsum2, f2_pack(e0, e1));
-                        pk[c >> 1] = pack_bf16_alu(e0, e1);
+                        f2_unpack(f2_add(x[c], neg_m2), d0, d1);
+                        const float e0 = exp2f(d0), e1 = exp2f(d1);
+                        sum2 = f2_add(sum2, f2_pack(e0, e1));
+                        pk[c] = pack_bf16_alu(e0, e1);
                     }
                     if (!lp.lse_only) tmem_st16(s_t + (c0 >> 1), pk);
                 }
+                if (!ok) break;
                 tmem_wait_st();
-                float lsum_hi;
-                f2_unpack(lsum2, lsum, lsum_hi);
-                lsum += lsum_hi;
-                }
-                if (!kDense) mbar_arrive(&bars->cl_empty[cslot]);
-                l_run += lsum;
+                float lo, hi;
+                f2_unpack(sum2, lo, hi);
+                mbar_arrive(&bars->cl_empty[cslot]);
+                l_run += lo + hi;
                 ++my_tiles;
-                if (hh == kH - 1) ++idx;
-                if (t + 2 >= n_tiles && hh == kH - 1) {   // this warpgroup's last tile of the group: publish (m, l)
-                    // the previous group's statistics must have been consumed
-                    if (gc > 0 && !mbar_wait(&bars->o_free, (gc - 1) & 1)) { fail(34); ok = false; break; }
+                if (t + 2 >= n_tiles) {                // this warpgroup's last tile of the group: publish (m, l)
+                    // the last statistics there must have been consumed
+                    if (!mbar_wait(&bars->o_free[w], (used++ & 1) ^ 1)) { fail(34); ok = false; break; }
                     bars->stats[w][0][row] = m_run;
                     bars->stats[w][1][row] = l_run;
                 }
                 tc_fence_before();
-                mbar_arrive(&bars->p_full[2 * w + hh]);
-              }
+                mbar_arrive(&bars->p_full[w]);
             }
+            gt0 += n_tiles;
         }
     } else if (warp >= 12) {
         // ------------------------------------------------------------------ epilogue warpgroup
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        const int us = kDense ? 0 : lane / R4;                       // unit slot of this tile row
-        const int i_row = kDense ? row : quad * R4 + lane % R4;      // query index of this tile row
+        const int us = row / R, i_row = row - us * R;                // unit slot and query index of this tile row
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-        int gc = 0;
-        for (int u0 = u_begin; u0 < u_end && !bars->abort_flag; u0 += u_step, ++gc) {
-            const int nu = kDense ? 1 : min(U, u_end - u0);
-            const int n_tiles = group_tiles(u0, nu);
-            if (!mbar_wait(&bars->o_full, gc & 1)) { fail(41); break; }
+        int gc = 0, gt0 = 0;
+        for (int u0 = u_begin; u0 < u_end && !bars->abort_flag; u0 += U, ++gc) {
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            if (!mbar_wait(&bars->o_full[gc & 1], (gc >> 1) & 1)) { fail(41); break; }
             tc_fence_after();
-            // even tiles went to warpgroup 0, odd tiles to warpgroup 1
-            const bool has1 = n_tiles > 1;
-            const float m0 = bars->stats[0][0][row], l0 = bars->stats[0][1][row];
-            const float m1 = has1 ? bars->stats[1][0][row] : -INFINITY, l1 = has1 ? bars->stats[1][1][row] : 0.f;
+            // the group's first tile went to warpgroup w_a, its second, if any, to the other; a row without a weight there
+            // takes nothing from it (its accumulator may never have been written)
+            const int w_a = gt0 & 1, w_b = w_a ^ 1;
+            gt0 += n_tiles;
+            const float m0 = bars->stats[w_a][0][row], l0 = bars->stats[w_a][1][row];
+            const float l1 = n_tiles > 1 ? bars->stats[w_b][1][row] : 0.f;
+            const bool has1 = l1 > 0.f;
+            const float m1 = has1 ? bars->stats[w_b][0][row] : -INFINITY;
             const float ms = fmaxf(m0, m1);
             const float w0 = exp2f(m0 - ms);
             const float w1 = has1 ? exp2f(m1 - ms) : 0.f;
-            const float inv = 1.0f / (w0 * l0 + w1 * l1);
-            bool row_ok;
+            const float den = w0 * l0 + (has1 ? w1 * l1 : 0.f);
+            const float inv = 1.0f / den;
+            const bool row_ok = us < nu && i_row < b1;
             __nv_bfloat16* out_row = nullptr;
-            if (kDense) {
-                const int qt = u0 % lp.q_tiles, bh = u0 / lp.q_tiles, b = bh / p.H, hd = bh - b * p.H;
-                const long long tok = (long long)qt * 128 + row;
-                row_ok = tok < p.n_q;
-                if (row_ok) out_row = p.out + (((long long)b * p.n_q + tok) * p.H + hd) * kHeadDim;
-            } else {
-                row_ok = us < nu && i_row < b1;
-                if (row_ok) {
-                    const LUnit un = decode_unit(p, u0 + us);
-                    const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-                    const long long tok = blk.row_token(p.a0 + un.al, i_row) + un.j;
-                    out_row = p.out_row(b, tok, hd);
-                    // iterative variant: the softmax's log-sum-exp (natural log) feeds the iteration update
-                    if (lp.write_lse) p.lse[(long long)(u0 + us) * b1 + i_row] = (ms + log2f(w0 * l0 + w1 * l1)) * 0.6931471805599453f;
-                }
+            if (row_ok) {
+                const LUnit un = decode_unit(p, u0 + us);
+                const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+                const long long tok = blk.row_token(p.a0 + un.al, i_row) + un.j;
+                out_row = p.out_row(b, tok, hd);
+                // iterative variant, backward: the softmax's log-sum-exp (natural log)
+                if (lp.write_lse) p.lse[(long long)(u0 + us) * b1 + i_row] = (ms + log2f(den)) * 0.6931471805599453f;
             }
+            const bool any1 = __any_sync(0xffffffffu, has1);
 #pragma unroll 1
             for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
                 uint32_t ra[32], rb[32];
                 if (!lp.lse_only) {
-                    tmem_ld32(tmem + lane_sel + col_o(0) + c0, ra);
-                    tmem_ld32(tmem + lane_sel + col_o(1) + c0, rb);
+                    tmem_ld32(tmem + lane_sel + col_o(w_a) + c0, ra);
+                    if (any1) tmem_ld32(tmem + lane_sel + col_o(w_b) + c0, rb);
                     tmem_wait_ld();
                 }
                 if (c0 + 32 == kHeadDim) {
                     tc_fence_before();
-                    mbar_arrive(&bars->o_free);               // accumulators and statistics are in registers
+                    mbar_arrive(&bars->o_free[w_a]);          // accumulators and statistics are in registers
+                    if (n_tiles > 1) mbar_arrive(&bars->o_free[w_b]);
                 }
                 if (row_ok && !lp.lse_only) {
 #pragma unroll
@@ -675,62 +539,39 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
 
 }  // namespace
 
+// Keys per tile of the column step: what 128-key tiles would take, divided evenly over them.
+int l_tile_keys(int n_keys) {
+    const int tiles = (n_keys + kKT - 1) / kKT;
+    return (((n_keys + tiles - 1) / tiles) + 15) & ~15;
+}
 
-// Launches the tensor-core column step for one chunk as a persistent grid.  maps = {aL, Y} with a
-// (64, 128 keys, 1) box and the 5-D query-row map (box rows = ceil(b1/4)).
-int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* maps /* aL, Y, q rows */, int* status, int num_sms,
-                     cudaStream_t s, int write_lse) {
+// Launches the tensor-core column step for one chunk as a persistent grid.  map_qrows = query rows, 5-D, box of b1 rows.
+int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s, int write_lse) {
     LaunchScope scope(kClsLStep, s);
     LTcParams lp;
     lp.mp = p;
     lp.n_units = p.nbh * p.na * p.blk.b2;
-    lp.R4 = (p.blk.b1 + 3) / 4;
-    lp.U = 32 / lp.R4;
-    if (lp.U < 1) lp.U = 1;
-    if (lp.U > kMaxU) lp.U = kMaxU;
+    lp.U = 128 / p.blk.b1 < kMaxU ? 128 / p.blk.b1 : kMaxU;
+    lp.R = 128 / lp.U;
+    lp.kt = l_tile_keys(p.n_keys);
+    // A value tile stays until its softmax and GEMM are done, a key tile only until its GEMM: two slots of five for keys
+    const int slots = kRing / (lp.kt * 256);
+    lp.n_a = (slots * 2 + 4) / 5 < kMaxStages ? (slots * 2 + 4) / 5 : kMaxStages;
+    lp.n_y = slots - lp.n_a < kMaxStages ? slots - lp.n_a : kMaxStages;
     lp.status = status;
-    // Query rows that are consecutive rows of the token grid come by TMA (the 128-byte swizzle is a function
-    // of the shared-memory address, so a box may land on any 128-byte row of the tile); other blockings
-    // are gathered by the producer warp with plain loads.
+    // Query rows that are consecutive rows of the token grid come by TMA; other blockings are gathered by the warp.
     lp.q_rows_tma = (p.blk.f_tied == 1 || p.blk.h_reduce == 1) ? 1 : 0;
-    lp.n_kv = 0;
-    lp.q_tiles = 0;
     lp.write_lse = write_lse != 0;
     lp.lse_only = write_lse == 2;
+    CUtensorMap maps[2];
+    if (int rc = make_bridge_tmap(&maps[0], p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, 1, lp.kt)) return rc;
+    if (int rc = make_bridge_tmap(&maps[1], p.Y, p.blk.b2, p.n_keys, p.nbh * p.na, 1, lp.kt)) return rc;
     const int n_groups = (lp.n_units + lp.U - 1) / lp.U;
     dim3 grid(n_groups < num_sms ? n_groups : num_sms);
-    auto kernel = p.causal_groups > 0 ? monarch_l_tc_kernel<false, true> : monarch_l_tc_kernel<false, false>;
+    auto kernel = p.causal_groups > 0 ? monarch_l_tc_kernel<true> : monarch_l_tc_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], maps[2], lp);
-    return (int)cudaGetLastError();
-}
-
-// Dense attention on the same kernel.  maps = {K, V, q}: 4-D (d, head, token, batch), box 64 x 1 x 128 x 1.
-int launch_dense_tc(const CUtensorMap* maps, __nv_bfloat16* out, int B, int H, int n_q, int n_kv, float scale, int* status,
-                    int num_sms, cudaStream_t s) {
-    LaunchScope scope(kClsDense, s);
-    LTcParams lp;
-    lp.mp = MonarchParams();
-    lp.mp.out = out;
-    lp.mp.H = H;
-    lp.mp.n_q = n_q;
-    lp.mp.scale = scale;
-    lp.mp.blk.b1 = 128;            // every tile row is a query
-    lp.mp.blk.b2 = 1;
-    lp.q_tiles = (n_q + 127) / 128;
-    lp.n_units = B * H * lp.q_tiles;
-    lp.U = 1;
-    lp.R4 = 32;
-    lp.n_kv = n_kv;
-    lp.q_rows_tma = 1;
-    lp.write_lse = 0;
-    lp.lse_only = 0;
-    lp.status = status;
-    dim3 grid(lp.n_units < num_sms ? lp.n_units : num_sms);
-    cudaError_t e = cudaFuncSetAttribute(monarch_l_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    monarch_l_tc_kernel<true, false><<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], maps[2], lp);
+    kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], *map_qrows, lp);
     return (int)cudaGetLastError();
 }
 

@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) monarch_r_kernel(MonarchParam
                         ok = f < (a_abs / p.causal_groups + 1) * p.causal_groups;
                     }
                     if (ok) {
-                        long long aj = ((long long)bhl * p.na + a_first) * b2 + r;
+                        const int gl = r / b2;
+                        const long long grp = (long long)bhl * p.na + a_first + gl;
                         uint4 val = *reinterpret_cast<const uint4*>(stg + rr * kLds + vec * 8);
-                        *reinterpret_cast<uint4*>(dst_base + (aj * p.n_keys + key) * kHeadDim + vec * 8) = val;
+                        *reinterpret_cast<uint4*>(dst_base + ((grp * p.n_keys + key) * b2 + r - gl * b2) * kHeadDim + vec * 8) = val;
                     }
                 }
             }

@@ -1,8 +1,8 @@
 // Monarch row step on the 5th-generation tensor cores (tcgen05 + TMEM), fed by TMA.
 //
 // Work is cut into units (batch*head, tile of stacked query groups, block row k, range of cached
-// groups f).  A tile stacks up to 128 query rows r = (query group a, column j); each group is padded
-// to a multiple of 8 rows so that its 128-byte-swizzled shared-memory image starts on a swizzle atom.
+// groups f).  A tile stacks up to 128 query rows r = (query group a, column j); each group takes 16, 32, 64 or 128 tile
+// rows, so that the 32 rows of an epilogue warp belong to one group (or are two whole groups of 16).
 // CTAs are persistent: each walks the unit list with a fixed stride and, for every (unit, f),
 // computes per query row a complete softmax over the b2 keys of K[f,k,:]:
 //   S  = Q_tile K[f,k]^T                 tcgen05.mma, both operands from shared memory (K-major)
@@ -12,17 +12,22 @@
 //   cL = sum_l P ln P                    from the softmax registers
 // and streams aL, Y (bf16) and cL to the chunk's bridge.
 //
-// Warp roles (19 warps): 0 = TMA producer, 1 = issuer of the [aL | Y] GEMMs (owns the TMEM
-// allocation), 2 = issuer of the S GEMMs,
-// 3..6 and 7..10 = two softmax warpgroups that take even / odd steps (each owns one of the two
-// S/P buffers in TMEM; a warp reaches TMEM lane quadrant warp % 4, and four consecutive warps cover
-// all four), 11..14 and 15..18 = two epilogue warpgroups (aL half / Y half of the
-// accumulator).  The S GEMM of step i+1 overlaps the softmax of step i; the output accumulator is
-// single buffered and handed back to the MMA warp as soon as both halves sit in registers.  Each
-// epilogue thread owns one bridge row and writes it straight from registers with 32-byte stores.  All roles run the same unit loop and meet
-// only through mbarriers whose phases follow running step counters, so the pipeline keeps flowing
-// across unit boundaries.  Every wait is bounded; on a timeout the CTA records a status code and
-// unwinds.
+// Warp roles (19 warps): 0 = TMA producer, 1 = issuer of the [aL | Y] GEMMs (owns the TMEM allocation), 2 = issuer of the S
+// GEMMs (all three run as whole warps with an elected issuing lane), 3..6 and 7..10 = two softmax warpgroups that take even
+// / odd steps (a warp reaches TMEM lane quadrant warp % 4, and four consecutive warps cover all four), 11..14 and 15..18 =
+// two epilogue warpgroups (aL half / Y half of the accumulator).  All roles run the same unit loop and meet only through
+// mbarriers whose phases follow running step counters, so the pipeline keeps flowing across unit boundaries.  Every wait
+// is bounded; on a timeout the CTA records a status code and unwinds.
+//
+// What bounds it: the bridge rows it writes, 512 bytes per (query row, cached group, block row).  Written by the epilogue
+// threads themselves (one 256-byte row per lane in 32-byte pieces) they go out at 25-27 KB per us and SM, 3.8 TB/s in all,
+// into L2 or DRAM alike; without the stores the same kernel takes a third to a half of the time.  So each epilogue warp packs
+// 32 rows x 64 columns to bf16 into a swizzled 4 KB staging buffer (two, in turn) and one lane hands it to the TMA store
+// engine.  With four S / P buffers in TMEM (the S GEMMs then run ahead of the softmax instead of waiting for the last P to
+// be consumed), one query tile and four 32 KB K / V stages: framewise, 21 cached frames, 12 heads 0.188 -> 0.167 ms;
+// reduce2xh, 9 frames, 4 videos 0.563 -> 0.500 ms; reduce4xw2xh, 21 frames 1.237 -> 1.135 ms (4.6 TB/s of DRAM traffic).
+// Tried and slower: 16 epilogue warps with a register split by setmaxnreg, separate accumulator hand-overs for the two
+// halves, one K / V tile for two query tiles, L2 prefetch of the K / V tiles.
 //
 // Arithmetic follows monarch_attn_ref_op (wan/modules/monarch_attn.py:1813-1823, 1828); the sqrt(s)
 // scaling of q and k is folded into the softmax scale, so aL here is the reference's aL / sqrt(s).
@@ -36,40 +41,45 @@ using namespace tc;
 
 namespace {
 
-constexpr int kStages = 8;            // K/V tile ring, at most (128 KB: 2 x 64 KB, 4 x 32 KB or 8 x 16 KB stages by block width)
+constexpr int kStages = 10;           // K/V tile ring, at most
 constexpr int kThreads = 608;          // 19 warps: one more would lower the register ceiling from 104 to 96
 constexpr int kTileRows = 128;
+constexpr int kMaxSBufs = 4;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColS0 = 0, kColS1 = 64, kColO = 128;   // O = [aL | Y], 256 columns
+constexpr uint32_t kColO = 256;        // O = [aL | Y], 256 columns; the S/P buffers lie below it
 
 struct RTcParams {
     MonarchParams mp;
-    int rows_per_group;    // b2 padded to a multiple of 8
+    int rows_per_group;    // b2 padded to 16, 32, 64 or 128: a warp's 32 tile rows belong to one group, or to two whole ones
     int groups_per_tile;   // 128 / rows_per_group
     int tiles;             // tiles per (batch*head) of the chunk
+    int fsplit, f_per;     // split of the F loop over units
     int n_units;           // nbh * tiles * b1 * fsplit
+    int col_kt;            // keys per tile of the column step (block-causal: it reads whole tiles)
     int* status;           // device status word (0 = ok)
 };
 
 
 struct RUnit {
     int bhl, tile, k, f_begin, n_it;
+    int f_limit;          // block-causal: cached groups the tile may see
 };
 
 template <bool kCausal>
 __device__ __forceinline__ RUnit decode_unit(const RTcParams& rp, int u) {
     const MonarchParams& p = rp.mp;
     RUnit r;
-    int fs = u % p.fsplit; u /= p.fsplit;
+    int fs = u % rp.fsplit; u /= rp.fsplit;
     r.k = u % p.blk.b1; u /= p.blk.b1;
     r.tile = u % rp.tiles;
     r.bhl = u / rp.tiles;
-    r.f_begin = fs * p.f_per;
-    int f_end = min(p.F, r.f_begin + p.f_per);
+    r.f_begin = fs * rp.f_per;
+    int f_end = min(p.F, r.f_begin + rp.f_per);
     if (kCausal) {
         // block-causal (no-cache path): the tile's last query group sees the most; later groups f are skipped
         const int a_hi = p.a0 + min((r.tile + 1) * rp.groups_per_tile, p.na) - 1;
-        f_end = min(f_end, (a_hi / p.causal_groups + 1) * p.causal_groups);
+        r.f_limit = min(p.F, (a_hi / p.causal_groups + 1) * p.causal_groups);
+        f_end = min(f_end, r.f_limit);
     }
     r.n_it = max(0, f_end - r.f_begin);               // 0: nothing to do, every role skips the unit
     return r;
@@ -79,9 +89,9 @@ struct __align__(8) Barriers {
     uint64_t q_full[2], q_empty[2];   // single pass: buffer 0, once per unit; iterative variant: one per step, alternating
     uint64_t kv_full[kStages];
     uint64_t kv_empty[kStages];
-    uint64_t s_full[2];
-    uint64_t p_full[2];
-    uint64_t sp_free[2];       // PV GEMM has consumed the P operand held in S/P buffer 0 / 1
+    uint64_t s_full[kMaxSBufs];
+    uint64_t p_full[kMaxSBufs];
+    uint64_t sp_free[kMaxSBufs];   // PV GEMM has consumed the P operand held in this S/P buffer
     uint64_t o_full;
     uint64_t o_free;
     uint32_t tmem_base;
@@ -90,14 +100,21 @@ struct __align__(8) Barriers {
 
 // shared memory carve-up (bytes from a 1024-aligned base)
 constexpr int kQBytes = 2 * kTileRows * 128;               // two 64-column halves
-constexpr int kStageBytes = 4 * 64 * 128;                  // K half 0, K half 1, V half 0, V half 1 (<= 64 rows each)
-constexpr int kSmemBytes = 1024 + 2 * kQBytes + 4 * kStageBytes + 256;   // two query tiles, 128 KB of K / V stages
+constexpr int kOutBytes = 8 * 2 * 32 * 128;                    // result staging: 32 rows x 64 columns per epilogue warp
+constexpr int kSmemData = 224 << 10;                       // query tiles | K / V ring | staging
+constexpr int kSmemBytes = 1024 + kSmemData + 512;
+static_assert(sizeof(Barriers) <= 512, "barriers follow the tiles");
 
-// 32-byte store of 16 bf16 to global memory (pointer 32-byte aligned).
-__device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) {
-    asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(ptr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+__device__ __forceinline__ void tma_store_4d_e(uint32_t el, const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %6, 0;\n"
+        "@e cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n}"
+        ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(el) : "memory");
 }
+// Bulk-group bookkeeping is per thread: lanes that issued nothing have nothing to commit or wait for.
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // kIter: a pass of the iterative variant after the first one.  The query operand is no longer the chunk's q
 // (one tile per unit) but the state aR[a,f,k,j,:] of the previous pass, which differs for every cached group f:
@@ -106,17 +123,14 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) 
 template <int N_S, bool kCausal, bool kIter>
 __global__ void __launch_bounds__(kThreads, 1)
 monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                    const __grid_constant__ CUtensorMap tv, RTcParams rp) {
+                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tal,
+                    const __grid_constant__ CUtensorMap ty, RTcParams rp) {
     static_assert(!kIter || (N_S <= 64 && !kCausal), "the iterative variant exists for block columns up to 64, no mask");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* q_s = base;
-    unsigned char* kv_s = q_s + 2 * kQBytes;                 // two query tiles: the next unit's loads while this one is worked on
-    Barriers* bars = reinterpret_cast<Barriers*>(kv_s + 4 * kStageBytes);
-
     const MonarchParams& p = rp.mp;
     const Blocking& blk = p.blk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int b1 = blk.b1, b2 = blk.b2;
     const int RG = rp.rows_per_group;
     constexpr int kHalf = N_S * 128;                    // bytes of one 64-column half of a K or V tile
@@ -124,19 +138,22 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     // accumulator move up in TMEM, and the softmax walks its row in 32-column chunks (see below).
     constexpr bool kWide = N_S > 64;
     // a stage holds K lo, K hi, V lo, V hi of N_S rows each: 16 KB up to 32 block columns, 32 KB up to 64, 64 KB beyond
-    constexpr int kStg = kWide ? 2 : (N_S <= 32 ? 8 : 4);
-    constexpr int kStgBytes = kWide ? 2 * kStageBytes : (N_S <= 32 ? kStageBytes / 2 : kStageBytes);
-    constexpr uint32_t cS1 = kWide ? 128u : kColS1, cO = kWide ? 256u : kColO;
-    // Single pass: the next unit's query tile loads into the other buffer while this unit is worked on (short units
-    // at small cache lengths otherwise wait for it); measured slower for narrow blocks (up to 32 columns), which keep one.
-    constexpr bool kQDouble = kIter || N_S > 32;
-    constexpr int kQBufs = kQDouble ? 2 : 1;
+    constexpr int kStgBytes = kWide ? 65536 : (N_S <= 32 ? 16384 : 32768);
+    constexpr int kSBufs = kWide ? 2 : 4;
+    constexpr uint32_t kSCols = kColO / kSBufs;          // TMEM columns per S/P buffer
+    constexpr int kQBufs = kIter ? 2 : 1;               // a query tile per unit, or per step
+    constexpr int kStg = (kSmemData - kQBufs * kQBytes - kOutBytes) / kStgBytes;
+    static_assert(kStg >= 2 && kStg <= kStages, "K / V ring");
+    unsigned char* q_s = base;
+    unsigned char* kv_s = q_s + kQBufs * kQBytes;
+    unsigned char* o_s = kv_s + kStg * kStgBytes;            // one 4 KB staging buffer per epilogue warp
+    Barriers* bars = reinterpret_cast<Barriers*>(base + kSmemData);
 
+    if (warp == 2 && lane == 0) { prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
         for (int s = 0; s < kStg; ++s) { mbar_init(&bars->kv_full[s], 1); mbar_init(&bars->kv_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars->s_full[s], 1); mbar_init(&bars->p_full[s], 128); }
-        for (int s = 0; s < 2; ++s) mbar_init(&bars->sp_free[s], 1);
+        for (int s = 0; s < kSBufs; ++s) { mbar_init(&bars->s_full[s], 1); mbar_init(&bars->p_full[s], 128); mbar_init(&bars->sp_free[s], 1); }
         mbar_init(&bars->o_full, 1);
         mbar_init(&bars->o_free, 256);
         bars->abort_flag = 0;
@@ -156,8 +173,8 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
+        {
+            const uint32_t el = elect_one();
             int g = 0, uc = 0;
             for (int u = u_first; u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
@@ -165,46 +182,41 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                 const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
                 const int g_first = un.tile * rp.groups_per_tile;
                 const int ng = min(rp.groups_per_tile, p.na - g_first);
-                if constexpr (!kIter) {
-                    const int qb = kQDouble ? (uc & 1) : 0;
-                    unsigned char* qd = q_s + qb * kQBytes;
-                    if (uc >= kQBufs && !mbar_wait(&bars->q_empty[qb], ((uc / kQBufs) - 1) & 1)) { fail(10); break; }
-                    mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(ng * RG * 256));
-                    for (int gi = 0; gi < ng; ++gi) {
-                        int tok = blk.row_token(p.a0 + g_first + gi, un.k);
-                        tma_load_4d(qd + gi * RG * 128, &tq, &bars->q_full[qb], 0, hd, tok, b);
-                        tma_load_4d(qd + kTileRows * 128 + gi * RG * 128, &tq, &bars->q_full[qb], 64, hd, tok, b);
-                    }
-                }
                 for (int i = 0; i < un.n_it; ++i, ++g) {
                     const int s = g % kStg;
-                    if constexpr (kIter) {
-                        // this step's query tile: the state rows (a, j) of (f, k), group by group
-                        const int qb = g & 1;
-                        if (g >= 2 && !mbar_wait(&bars->q_empty[qb], ((g >> 1) - 1) & 1)) { fail(10); break; }
-                        unsigned char* qd = q_s + qb * kQBytes;
-                        const int fk = (un.bhl * p.F + un.f_begin + i) * b1 + un.k;
-                        mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(ng * RG * 256));
-                        for (int gi = 0; gi < ng; ++gi) {
-                            tma_load_3d(qd + gi * RG * 128, &tq, &bars->q_full[qb], 0, (g_first + gi) * b2, fk);
-                            tma_load_3d(qd + kTileRows * 128 + gi * RG * 128, &tq, &bars->q_full[qb], 64, (g_first + gi) * b2, fk);
-                        }
-                    }
-                    if (g >= kStg && !mbar_wait(&bars->kv_empty[s], ((g / kStg) - 1) & 1)) { fail(11); break; }
+                    if (g >= kStg && !mbar_wait_u(&bars->kv_empty[s], ((g / kStg) - 1) & 1)) { fail(11); break; }
                     const int tok = ((un.f_begin + i) * b1 + un.k) * b2;
                     unsigned char* st = kv_s + s * kStgBytes;
-                    mbar_arrive_expect_tx(&bars->kv_full[s], (uint32_t)(4 * kHalf));
-                    tma_load_4d(st, &tk, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d(st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
-                    tma_load_4d(st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d(st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
+                    mbar_arrive_expect_tx_e(el, &bars->kv_full[s], (uint32_t)(4 * kHalf));
+                    tma_load_4d_e(el, st, &tk, &bars->kv_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
+                    tma_load_4d_e(el, st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
+                    if (!kIter && i > 0) continue;
+                    // the query tile: the unit's rows of q, or this step's state rows (a, j) of (f, k), group by group
+                    const int qc = kIter ? g : uc, qb = qc % kQBufs;
+                    if (qc >= kQBufs && !mbar_wait_u(&bars->q_empty[qb], ((qc / kQBufs) - 1) & 1)) { fail(10); break; }
+                    unsigned char* qd = q_s + qb * kQBytes;
+                    mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(ng * b2 * 256));
+                    for (int gi = 0; gi < ng; ++gi, qd += RG * 128) {
+                        if constexpr (kIter) {
+                            const int fk = (un.bhl * p.F + un.f_begin + i) * b1 + un.k;
+                            tma_load_3d_e(el, qd, &tq, &bars->q_full[qb], 0, (g_first + gi) * b2, fk);
+                            tma_load_3d_e(el, qd + kTileRows * 128, &tq, &bars->q_full[qb], 64, (g_first + gi) * b2, fk);
+                        } else {
+                            const int qtok = blk.row_token(p.a0 + g_first + gi, un.k);
+                            tma_load_4d_e(el, qd, &tq, &bars->q_full[qb], 0, hd, qtok, b);
+                            tma_load_4d_e(el, qd + kTileRows * 128, &tq, &bars->q_full[qb], 64, hd, qtok, b);
+                        }
+                    }
                 }
                 ++uc;
             }
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------------ S-GEMM issuer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc_s = idesc_bf16(kTileRows, N_S, 0, 0);
             // Descriptors differ from step to step only in the start-address field (16-byte units
             // in the low word), so they are built once and advanced with integer adds.
@@ -216,29 +228,29 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                 const RUnit un = decode_unit<kCausal>(rp, u);
                 if (kCausal && un.n_it == 0) continue;
                 if constexpr (!kIter) {
-                    if (!mbar_wait(&bars->q_full[kQDouble ? (uc & 1) : 0], (uc / kQBufs) & 1)) { fail(20); break; }
+                    if (!mbar_wait_u(&bars->q_full[0], uc & 1)) { fail(20); break; }
                 }
                 for (int i = 0; i < un.n_it; ++i, ++g) {
                     const int s = g % kStg;
                     if constexpr (kIter) {
-                        if (!mbar_wait(&bars->q_full[g & 1], (g >> 1) & 1)) { fail(20); ok = false; break; }
+                        if (!mbar_wait_u(&bars->q_full[g & 1], (g >> 1) & 1)) { fail(20); ok = false; break; }
                     }
-                    if (!mbar_wait(&bars->kv_full[s], (g / kStg) & 1)) { fail(21); ok = false; break; }
-                    if (g >= 2 && !mbar_wait(&bars->sp_free[g & 1], ((g >> 1) - 1) & 1)) { fail(25); ok = false; break; }
+                    if (!mbar_wait_u(&bars->kv_full[s], (g / kStg) & 1)) { fail(21); ok = false; break; }
+                    if (g >= kSBufs && !mbar_wait_u(&bars->sp_free[g % kSBufs], ((g / kSBufs) - 1) & 1)) { fail(25); ok = false; break; }
                     tc_fence_after();
                     const uint64_t kd = k_desc0 + (uint64_t)((s * kStgBytes) >> 4);
-                    const uint32_t d = tmem + ((g & 1) ? cS1 : kColS0);
+                    const uint32_t d = tmem + (g % kSBufs) * kSCols;
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t q_off = ((ks >> 2) * (kTileRows * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t k_off = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss(d, q_desc + (uint32_t)((((kIter ? g : (kQDouble ? uc : 0)) & 1) * kQBytes) >> 4) + q_off, kd + k_off, idesc_s, ks > 0);
+                        mma_ss_e(el, d, q_desc + (uint32_t)(((kIter ? g & 1 : 0) * kQBytes) >> 4) + q_off, kd + k_off, idesc_s, ks > 0);
                     }
-                    mma_commit(&bars->s_full[g & 1]);
+                    mma_commit_e(el, &bars->s_full[g % kSBufs]);
                     if constexpr (kIter) {
-                        mma_commit(&bars->q_empty[g & 1]);                 // this step's query tile has been read
+                        mma_commit_e(el, &bars->q_empty[g & 1]);                 // this step's query tile has been read
                     } else {
-                        if (i + 1 == un.n_it) mma_commit(&bars->q_empty[kQDouble ? (uc & 1) : 0]);   // last read of this unit's Q tile
+                        if (i + 1 == un.n_it) mma_commit_e(el, &bars->q_empty[0]);   // last read of this unit's Q tile
                     }
                 }
                 ++uc;
@@ -246,7 +258,8 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ PV-GEMM issuer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             // [aL | Y] in one N = 256 GEMM; the passes of the iterative variant that only need aL and cL stop at N = 128
             const uint32_t idesc_o = p.write_Y ? idesc_bf16(kTileRows, 2 * kHeadDim, 0, 1) : idesc_bf16(kTileRows, kHeadDim, 0, 1);
             constexpr int ksteps_pv = N_S / 16;
@@ -256,18 +269,18 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
                 for (int i = 0; i < un.n_it; ++i, ++g) {
-                    if (!mbar_wait(&bars->p_full[g & 1], (g >> 1) & 1)) { fail(22); ok = false; break; }
-                    if (g > 0 && !mbar_wait(&bars->o_free, (g - 1) & 1)) { fail(23); ok = false; break; }
+                    if (!mbar_wait_u(&bars->p_full[g % kSBufs], (g / kSBufs) & 1)) { fail(22); ok = false; break; }
+                    if (g > 0 && !mbar_wait_u(&bars->o_free, (g - 1) & 1)) { fail(23); ok = false; break; }
                     tc_fence_after();
                     const int s = g % kStg;
                     const uint64_t bd = kv_desc_mn0 + (uint64_t)((s * kStgBytes) >> 4);
-                    const uint32_t p_t = tmem + ((g & 1) ? cS1 : kColS0);
+                    const uint32_t p_t = tmem + (g % kSBufs) * kSCols;
 #pragma unroll
                     for (int kk = 0; kk < ksteps_pv; ++kk)
-                        mma_ts(tmem + cO, p_t + kk * 8, bd + ((kk * 2048) >> 4), idesc_o, kk > 0);
-                    mma_commit(&bars->o_full);
-                    mma_commit(&bars->kv_empty[s]);
-                    mma_commit(&bars->sp_free[g & 1]);
+                        mma_ts_e(el, tmem + kColO, p_t + kk * 8, bd + ((kk * 2048) >> 4), idesc_o, kk > 0);
+                    mma_commit_e(el, &bars->o_full);
+                    mma_commit_e(el, &bars->kv_empty[s]);
+                    mma_commit_e(el, &bars->sp_free[g % kSBufs]);
                 }
             }
         }
@@ -278,7 +291,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         const int row = quad * 32 + lane;               // tile row == TMEM lane
         const int gl = row / RG, j = row - gl * RG;
         const float scale_l2 = p.mult0 * kLog2e;
-        const uint32_t s_t = tmem + ((uint32_t)(quad * 32) << 16) + (wg ? cS1 : kColS0);
+        const uint32_t s_t0 = tmem + ((uint32_t)(quad * 32) << 16);
         int g = 0;
         bool ok = true;
         for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
@@ -301,7 +314,9 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                         scale_row = p.scale * kLog2e * fminf(1.0f / (p.cR[ci] + 1e-6f), 1e4f);
                     }
                 }
-                if (!mbar_wait(&bars->s_full[wg], (g >> 1) & 1)) { fail(31); ok = false; break; }
+                const int sb = g % kSBufs;
+                const uint32_t s_t = s_t0 + sb * kSCols;
+                if (!mbar_wait(&bars->s_full[sb], (g / kSBufs) & 1)) { fail(31); ok = false; break; }
                 tc_fence_after();
                 if (warp_active) {
                     if constexpr (!kWide) {
@@ -443,7 +458,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                     }
                 }
                 tc_fence_before();
-                mbar_arrive(&bars->p_full[wg]);
+                mbar_arrive(&bars->p_full[sb]);
             }
         }
     } else if (warp >= 11) {
@@ -451,7 +466,13 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         const int which = (warp - 11) >> 2;              // 0: aL (columns 0..127 of O), 1: Y (columns 128..255)
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        const uint32_t o_t = tmem + ((uint32_t)(quad * 32) << 16) + cO + which * kHeadDim;
+        const uint32_t o_t = tmem + ((uint32_t)(quad * 32) << 16) + kColO + which * kHeadDim;
+        const uint32_t el = elect_one();
+        // this warp's staging: 32 tile rows x 64 columns, 128-byte swizzle; its rows of a group start at column j0
+        unsigned char* const st = o_s + (warp - 11) * 8192;
+        unsigned char* const st_row = st + lane * 128;
+        const int gl0 = quad * 32 / RG, j0 = quad * 32 - gl0 * RG, n_box = RG == 16 ? 2 : 1;
+        const CUtensorMap* const om = which ? &ty : &tal;
         int g = 0;
         bool ok = true;
         for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
@@ -462,41 +483,58 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             for (int i = 0; ok && i < un.n_it; ++i, ++g) {
                 if (!mbar_wait(&bars->o_full, g & 1)) { fail(41); ok = false; break; }
                 tc_fence_after();
-                // This thread's bridge row: 256 bytes at (aj, key), written as 32-byte vectors.
-                const int gl = row / RG, j = row - gl * RG;
-                const bool row_ok = warp_active && gl < ng && j < b2 && (which == 0 || p.write_Y);
-                const long long aj = ((long long)un.bhl * p.na + g_first + gl) * b2 + j;
                 const int key = (un.f_begin + i) * b1 + un.k;
-                __nv_bfloat16* const out_row = (which ? p.Y : p.aL) + (aj * p.n_keys + key) * kHeadDim;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {                 // 64 columns at a time
-                    uint32_t ra[32], rb[32];
-                    if (warp_active && (which == 0 || p.write_Y)) {
-                        tmem_ld32(o_t + h * 64, ra);
-                        tmem_ld32(o_t + h * 64 + 32, rb);
-                        tmem_wait_ld();
-                    }
-                    if (h == 1) {
-                        tc_fence_before();
-                        mbar_arrive(&bars->o_free);            // accumulator may be overwritten from here on
-                    }
-                    if (row_ok) {
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const uint32_t (&r)[32] = c ? rb : ra;
-#pragma unroll
-                            for (int v8 = 0; v8 < 2; ++v8) {
-                                uint32_t w[8];
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    w[e] = pack_bf16_alu(__uint_as_float(r[v8 * 16 + 2 * e]), __uint_as_float(r[v8 * 16 + 2 * e + 1]));
-                                st_global_v8(out_row + h * 64 + c * 32 + v8 * 16, w);
-                            }
-                        }
-                    }
+                const bool work = warp_active && (which == 0 || p.write_Y);
+                if (!work) {
+                    tc_fence_before();
+                    mbar_arrive(&bars->o_free);
+                    continue;
                 }
+                uint32_t ra[32], rb[32];
+                // 64 columns from registers to this warp's staging rows, and on to the bridge
+                auto put = [&](int h) {
+                    tma_store_wait_read();                     // the previous box has been read
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint32_t (&r)[32] = c < 4 ? ra : rb;
+                        uint32_t w[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            w[e] = pack_bf16(__uint_as_float(r[(c & 3) * 8 + 2 * e]), __uint_as_float(r[(c & 3) * 8 + 2 * e + 1]));
+                        *reinterpret_cast<uint4*>(st_row + h * 4096 + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    for (int x = 0; x < n_box; ++x)
+                        if (gl0 + x < ng)
+                            tma_store_4d_e(el, om, st + h * 4096 + x * 2048, h * 64, j0, key, un.bhl * p.na + g_first + gl0 + x);
+                    tma_store_commit();
+                };
+                tmem_ld32(o_t, ra);
+                tmem_ld32(o_t + 32, rb);
+                tmem_wait_ld();
+                put(0);
+                tmem_ld32(o_t + 64, ra);
+                tmem_ld32(o_t + 96, rb);
+                tmem_wait_ld();
+                tc_fence_before();
+                mbar_arrive(&bars->o_free);                    // accumulator may be overwritten from here on
+                put(1);
+            }
+            if (kCausal && which == 1 && warp_active && un.n_it > 0 && un.f_begin + un.n_it == un.f_limit) {
+                // The column step reads whole tiles of col_kt keys and gives the keys past the limit weight zero: their Y
+                // rows must hold finite numbers.  The unit that computed the tile's last cached group writes them.
+                const int gl = row / RG, j = row - gl * RG;
+                const int end = min(p.n_keys, (un.f_limit * b1 + rp.col_kt - 1) / rp.col_kt * rp.col_kt);
+                for (int key = un.f_limit * b1 + un.k; key < end; key += b1)
+                    if (gl < ng && j < b2) {
+                        uint4* y = reinterpret_cast<uint4*>(p.Y + ((((long long)un.bhl * p.na + g_first + gl) * p.n_keys + key) * b2 + j) * kHeadDim);
+                        for (int c = 0; c < kHeadDim / 8; ++c) y[c] = make_uint4(0, 0, 0, 0);
+                    }
             }
         }
+        tma_store_wait_all();
     }
 
     tc_fence_before();
@@ -509,25 +547,45 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 
 // Launches the tensor-core row step for one chunk as a persistent grid.  `status` is a device int the
 // kernel sets on an internal timeout.
-int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or the aR state), k, v */, int rows_per_group,
-                     int n_s, int* status, int num_sms, cudaStream_t s) {
+int l_tile_keys(int n_keys);
+
+int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or the aR state), k, v */, int n_s, int* status,
+                     int num_sms, cudaStream_t s) {
     LaunchScope scope(kClsRStep, s);
     RTcParams rp;
     rp.mp = p;
-    rp.rows_per_group = rows_per_group;
-    rp.groups_per_tile = kTileRows / rows_per_group;
+    const int b2 = p.blk.b2;
+    rp.rows_per_group = b2 <= 16 ? 16 : (b2 <= 32 ? 32 : (b2 <= 64 ? 64 : 128));
+    rp.groups_per_tile = kTileRows / rp.rows_per_group;
+    rp.col_kt = l_tile_keys(p.n_keys);
     rp.tiles = (p.na + rp.groups_per_tile - 1) / rp.groups_per_tile;
-    rp.n_units = p.nbh * rp.tiles * p.blk.b1 * p.fsplit;
+    {
+        // Persistent CTAs take whole units round-robin, so the launch lasts (units per CTA, rounded up) x (steps per
+        // unit).  Pick the split of the F loop that makes that smallest, with at least three steps per unit (every unit
+        // reloads its query tile) and an extra step's worth charged per unit for that reload.
+        long long best = -1;
+        for (int fs = 1; fs <= (p.F / 3 > 1 ? p.F / 3 : 1); ++fs) {
+            const int per = (p.F + fs - 1) / fs, splits = (p.F + per - 1) / per;
+            const long long units = (long long)p.nbh * rp.tiles * p.blk.b1 * splits;
+            const long long cost = ((units + num_sms - 1) / num_sms) * (per + 1);
+            if (best < 0 || cost < best) { best = cost; rp.f_per = per; rp.fsplit = splits; }
+        }
+    }
+    rp.n_units = p.nbh * rp.tiles * p.blk.b1 * rp.fsplit;
     rp.status = status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
     // wide blocks: two 64 KB K / V stages instead of five 32 KB ones
     const bool iter = p.use_aR != 0;
     if (iter && (n_s > 64 || p.causal_groups > 0)) return SFM_ERR_UNSUPPORTED;
     const int smem_bytes = kSmemBytes;
+    // result stores: one box = 64 channels of up to 32 columns of one key
+    CUtensorMap out_maps[2];
+    for (int i = 0; i < 2; ++i)
+        if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, rp.rows_per_group < 32 ? rp.rows_per_group : 32, 1)) return rc;
     auto go = [&](auto kernel) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<grid, kThreads, smem_bytes, s>>>(maps[0], maps[1], maps[2], rp);
+        kernel<<<grid, kThreads, smem_bytes, s>>>(maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
         return 0;
     };
     int rc;

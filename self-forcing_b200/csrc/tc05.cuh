@@ -204,6 +204,102 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
+// ----------------------------------------------------------------------------- warp-uniform issue
+// The roles that issue TMA copies and MMAs run as whole warps with uniform control flow; only the issuing instruction
+// itself is predicated on one elected lane (`el`, from elect_one, the same lane for a role's whole life: a commit covers
+// what its own thread has issued).  Descriptors, masks and coordinates then live in uniform registers.  Issued from an
+// `if (lane == 0)` block they are moved there one by one for each instruction: a masked N = 128 MMA then takes 120-165
+// cycles instead of the tensor pipe's 64, an unmasked one 77.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t el;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(el));
+    return el;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// All lanes wait; the answer is the warp's (false if any lane gave up).
+__device__ __forceinline__ bool mbar_wait_u(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_e(uint32_t el, uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n.reg .pred e;\nsetp.ne.b32 e, %2, 0;\n@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}"
+                 ::"r"(smem_addr(bar)), "r"(bytes), "r"(el) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_e(uint32_t el, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %6, 0;\n"
+        "@e cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n}"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(el)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_e(uint32_t el, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
+                                              int c2, int c3) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %7, 0;\n"
+        "@e cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n}"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+        "r"(el) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_e(uint32_t el, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
+                                              int c2, int c3, int c4) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %8, 0;\n"
+        "@e cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n}"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+        "r"(c4), "r"(el) : "memory");
+}
+__device__ __forceinline__ void bulk_load_e(uint32_t el, void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("{\n.reg .pred e;\nsetp.ne.b32 e, %4, 0;\n"
+                 "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}"
+                 ::"r"(smem_addr(smem_dst)), "l"(gmem_src), "r"(bytes), "r"(smem_addr(bar)), "r"(el) : "memory");
+}
+__device__ __forceinline__ void mma_ss_e(uint32_t el, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n.reg .pred p, e;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 e, %5, 0;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum), "r"(el) : "memory");
+}
+__device__ __forceinline__ void mma_ts_e(uint32_t el, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n.reg .pred p, e;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 e, %5, 0;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "r"(el) : "memory");
+}
+// Output-lane mask: bit i of dis[w] set = row 32 w + i of D is not written.
+struct LaneMask { uint32_t dis[4]; };
+// Writes rows [row0, row0 + n) only.
+__device__ __forceinline__ LaneMask lane_mask_rows(int row0, int n) {
+    LaneMask m;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int lo = max(row0 - 32 * w, 0), hi = min(row0 + n - 32 * w, 32);
+        const uint32_t below_hi = hi >= 32 ? 0xffffffffu : (hi > 0 ? (1u << hi) - 1u : 0u);
+        const uint32_t below_lo = lo >= 32 ? 0xffffffffu : (1u << lo) - 1u;
+        m.dis[w] = ~(below_hi & ~below_lo);
+    }
+    return m;
+}
+__device__ __forceinline__ void mma_ss_masked_e(uint32_t el, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accum, const LaneMask& m) {
+    asm volatile(
+        "{\n.reg .pred p, e;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 e, %9, 0;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum), "r"(m.dis[0]), "r"(m.dis[1]), "r"(m.dis[2]),
+        "r"(m.dis[3]), "r"(el) : "memory");
+}
+__device__ __forceinline__ void mma_ts_masked_e(uint32_t el, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accum, const LaneMask& m) {
+    asm volatile(
+        "{\n.reg .pred p, e;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 e, %9, 0;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "r"(m.dis[0]), "r"(m.dis[1]), "r"(m.dis[2]),
+        "r"(m.dis[3]), "r"(el) : "memory");
+}
+__device__ __forceinline__ void mma_commit_e(uint32_t el, uint64_t* bar) {
+    asm volatile("{\n.reg .pred e;\nsetp.ne.b32 e, %1, 0;\n"
+                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}"
+                 ::"r"(smem_addr(bar)), "r"(el) : "memory");
+}
+
 }  // namespace tc
 
 // ----------------------------------------------------------------------------- host: tensor maps
@@ -217,5 +313,8 @@ EncodeTiledFn get_encode_tiled();
 // inner box of 64 elements.
 int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                    const uint32_t* box);
+
+// Bridge tensor aL or Y, [group][key][column][128]; one box = 64 channels x box_cols columns x box_keys keys of one group.
+int make_bridge_tmap(CUtensorMap* out, const void* base, int b2, int n_keys, int groups, int box_cols, int box_keys);
 
 }  // namespace sfm

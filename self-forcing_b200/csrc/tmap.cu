@@ -32,4 +32,12 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
     return r == CUDA_SUCCESS ? SFM_OK : SFM_ERR_BAD_SHAPE;
 }
 
+int make_bridge_tmap(CUtensorMap* out, const void* base, int b2, int n_keys, int groups, int box_cols, int box_keys) {
+    const uint64_t row = (uint64_t)kHeadDim * 2;
+    const uint64_t dims[4] = {(uint64_t)kHeadDim, (uint64_t)b2, (uint64_t)n_keys, (uint64_t)groups};
+    const uint64_t str[3] = {row, b2 * row, (uint64_t)n_keys * b2 * row};
+    const uint32_t box[4] = {64, (uint32_t)box_cols, (uint32_t)box_keys, 1};
+    return make_tmap_bf16(out, base, 4, dims, str, box);
+}
+
 }  // namespace sfm

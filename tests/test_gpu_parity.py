@@ -260,6 +260,56 @@ def test_monarch_baseline_config1_T20_vs_golden(sfb, golden):
     check_close(z[0, ::97, ::5, :], torch.from_numpy(golden["c1_T20_z_sample"]), "config 1, T=20")
 
 
+# (h, w, f_tied, h_reduce, w_reduce, frames cached): keys that divide into tiles of 80 / 112 / 48 keys with a remainder in
+# the last one, block rows with 1, 2, 5, 6 and 8 units per query tile, block columns at the edges of the row step's
+# groups of 16, 32, 64 and 128 tile rows
+TILE_EDGES = [(24, 12, 1, 1, 1, 6), (20, 16, 1, 1, 1, 21), (21, 17, 1, 1, 1, 21), (25, 32, 1, 1, 1, 6), (16, 33, 1, 1, 1, 3),
+              (8, 64, 1, 1, 1, 6), (5, 65, 1, 1, 1, 9), (22, 20, 3, 1, 1, 6), (64, 6, 1, 1, 1, 3), (6, 8, 1, 2, 4, 6)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("edge", TILE_EDGES, ids=lambda e: "h{}w{}_ft{}hr{}wr{}_F{}".format(*e))
+def test_monarch_tile_edges(sfb, edge):
+    h, w, ft, hr, wr, frames = edge
+    rng = np.random.default_rng(h * 1000 + w)
+    n, n_kv = 3 * h * w, frames * h * w
+    mk = lambda *s: bf(cases.randn(rng, *s))
+    c = dict(blocking=(ft, hr, wr, h, w), q=mk(1, n, 3, 128), nk=mk(1, n, 3, 128), nv=mk(1, n, 3, 128),
+             kbuf=mk(1, n_kv, 3, 128), vbuf=mk(1, n_kv, 3, 128), start=n_kv - n, end=n_kv, n_kv=n_kv, sm_scale=128 ** -0.5)
+    check_close(run_gpu_cache(sfb, c)[0], run_oracle_cache(c)[0], str(edge))
+
+
+@pytest.mark.gpu
+def test_monarch_column_reference_moves(sfb):
+    """Column logits that outgrow those of the first keys by far more than 2^40, so that the column step's softmax
+    reference moves within a tile and between tiles.  The keys of a block row are equal and small integers times signs and
+    the block has 8 columns, so the row step's averages are exact and only the column softmax is tested."""
+    rng = np.random.default_rng(77)
+    h, w, frames, H = 6, 8, 42, 2
+    sign = torch.from_numpy(rng.choice([-1.0, 1.0], size=(1, frames, h, 1, H, 128)).astype(np.float32))
+    k = (sign * torch.arange(frames).view(1, frames, 1, 1, 1, 1)).expand(1, frames, h, w, H, 128).reshape(1, -1, H, 128)
+    q, v = bf(cases.randn(rng, 1, 3 * h * w, H, 128)), bf(cases.randn(rng, 1, frames * h * w, H, 128))
+    n = 3 * h * w
+    c = dict(blocking=(1, 1, 1, h, w), q=q, nk=bf(k[:, -n:]), nv=v[:, -n:], kbuf=bf(k), vbuf=v, start=k.shape[1] - n,
+             end=k.shape[1], n_kv=k.shape[1], sm_scale=128 ** -0.5)
+    check_close(run_gpu_cache(sfb, c)[0], run_oracle_cache(c)[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grid", [(6, 8, 1, 1, 1), (20, 16, 1, 1, 1), (12, 10, 3, 1, 1)])
+def test_block_causal_does_not_read_old_scratch(sfb, grid):
+    """The block-causal call leaves parts of its scratch unwritten: what they held before must not matter."""
+    h, w, ft, hr, wr = grid
+    rng = np.random.default_rng(78)
+    q, k, v = (bf(cases.randn(rng, 1, 9 * h * w, 2, 128)).cuda() for _ in range(3))
+    call = lambda: sfb.monarch_attn(q, k, v, ft, hr, wr, h, w, block_causal_size=3 * h * w)
+    call()
+    for ws in sfb.ops._workspaces.values():
+        ws[256:].fill_(0xFF)                                  # NaN in every type
+    ref = orc.monarch_attn(q.float().cpu(), k.float().cpu(), v.float().cpu(), ft, hr, wr, h, w, block_causal_size=3 * h * w)
+    check_close(call(), ref)
+
+
 # ------------------------------------------------------------------------------- no-cache entry point
 @pytest.mark.parametrize("ci", range(4))
 def test_monarch_nocache_and_block_causal(sfb, ci):
