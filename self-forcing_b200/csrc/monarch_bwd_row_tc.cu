@@ -91,7 +91,7 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
 
     const MonarchParams& p = rp.mp;
     const Blocking& blk = p.blk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int b1 = blk.b1, b2 = blk.b2;
     const int RG = rp.rows_per_group;
     const int F = p.F;
@@ -127,7 +127,8 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tda); prefetch_tmap(&tdy);
             int g = 0, uc = 0;
             bool ok = true;
@@ -136,39 +137,40 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
                 const int g_first = un.tile * rp.groups_per_tile;
                 const int ng = min(rp.groups_per_tile, p.na - g_first);
-                if (uc > 0 && !mbar_wait(&bars->q_empty, (uc - 1) & 1)) { fail(10); break; }
-                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(ng * b2 * 256));           // the padding rows stay zero
+                if (uc > 0 && !mbar_wait_u(&bars->q_empty, (uc - 1) & 1)) { fail(10); break; }
+                mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(ng * b2 * 256));           // the padding rows stay zero
                 for (int gi = 0; gi < ng; ++gi) {
                     const int tok = blk.row_token(p.a0 + g_first + gi, un.k);
-                    tma_load_4d(q_s + gi * RG * 128, &tq, &bars->q_full, 0, hd, tok, b);
-                    tma_load_4d(q_s + kRows * 128 + gi * RG * 128, &tq, &bars->q_full, 64, hd, tok, b);
+                    tma_load_4d_e(el, q_s + gi * RG * 128, &tq, &bars->q_full, 0, hd, tok, b);
+                    tma_load_4d_e(el, q_s + kRows * 128 + gi * RG * 128, &tq, &bars->q_full, 64, hd, tok, b);
                 }
                 for (int f = 0; f < F; ++f, ++g) {
                     const int s = g & 1;
-                    if (g >= 2 && !mbar_wait(&bars->kv_empty[s], ((g >> 1) - 1) & 1)) { fail(11); ok = false; break; }
+                    if (g >= 2 && !mbar_wait_u(&bars->kv_empty[s], ((g >> 1) - 1) & 1)) { fail(11); ok = false; break; }
                     const int tok = (f * b1 + un.k) * b2;
                     unsigned char* st = kv_s + s * kKVStage;
-                    mbar_arrive_expect_tx(&bars->kv_full[s], (uint32_t)(4 * kHalf));
-                    tma_load_4d(st, &tk, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d(st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
-                    tma_load_4d(st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d(st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
-                    if (g >= 1 && !mbar_wait(&bars->da_empty, (g - 1) & 1)) { fail(12); ok = false; break; }
+                    mbar_arrive_expect_tx_e(el, &bars->kv_full[s], (uint32_t)(4 * kHalf));
+                    tma_load_4d_e(el, st, &tk, &bars->kv_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
+                    tma_load_4d_e(el, st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
+                    if (g >= 1 && !mbar_wait_u(&bars->da_empty, (g - 1) & 1)) { fail(12); ok = false; break; }
                     const int key = f * b1 + un.k;
-                    mbar_arrive_expect_tx(&bars->da_full, (uint32_t)(2 * ng * RG * 256));
+                    mbar_arrive_expect_tx_e(el, &bars->da_full, (uint32_t)(2 * ng * RG * 256));
                     for (int gi = 0; gi < ng; ++gi) {
                         const int grp = un.bhl * p.na + g_first + gi;
-                        tma_load_4d(da_s + gi * RG * 128, &tda, &bars->da_full, 0, 0, key, grp);
-                        tma_load_4d(da_s + kRows * 128 + gi * RG * 128, &tda, &bars->da_full, 64, 0, key, grp);
-                        tma_load_4d(dy_s + gi * RG * 128, &tdy, &bars->da_full, 0, 0, key, grp);
-                        tma_load_4d(dy_s + kRows * 128 + gi * RG * 128, &tdy, &bars->da_full, 64, 0, key, grp);
+                        tma_load_4d_e(el, da_s + gi * RG * 128, &tda, &bars->da_full, 0, 0, key, grp);
+                        tma_load_4d_e(el, da_s + kRows * 128 + gi * RG * 128, &tda, &bars->da_full, 64, 0, key, grp);
+                        tma_load_4d_e(el, dy_s + gi * RG * 128, &tdy, &bars->da_full, 0, 0, key, grp);
+                        tma_load_4d_e(el, dy_s + kRows * 128 + gi * RG * 128, &tdy, &bars->da_full, 64, 0, key, grp);
                     }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc_s = idesc_bf16(kRows, N_S, 0, 0);            // S, dR
             constexpr uint32_t idesc_q = idesc_bf16(kRows, kHeadDim, 0, 1);        // dQ: A from TMEM, B MN-major
             constexpr uint32_t idesc_k = idesc_bf16(kRows, kHeadDim, 1, 1);        // dK, dV: both MN-major
@@ -185,12 +187,12 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
             int g = 0, uc = 0, gd = 0;
             bool ok = true;
             for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
-                if (!mbar_wait(&bars->q_full, uc & 1)) { fail(20); break; }
+                if (!mbar_wait_u(&bars->q_full, uc & 1)) { fail(20); break; }
                 for (int f = 0; f < F; ++f, ++g) {
                     const int s = g & 1;
                     const bool kvw = wants_kv(f);
-                    if (!mbar_wait(&bars->kv_full[s], (g >> 1) & 1)) { fail(21); ok = false; break; }
-                    if (g >= 1 && !mbar_wait(&bars->sdr_free, (g - 1) & 1)) { fail(22); ok = false; break; }
+                    if (!mbar_wait_u(&bars->kv_full[s], (g >> 1) & 1)) { fail(21); ok = false; break; }
+                    if (g >= 1 && !mbar_wait_u(&bars->sdr_free, (g - 1) & 1)) { fail(22); ok = false; break; }
                     tc_fence_after();
                     const uint64_t kd = kv_k0 + (uint64_t)((s * kKVStage) >> 4);
                     const uint64_t vd = kd + (uint64_t)((2 * kHalf) >> 4);
@@ -198,51 +200,51 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss(tmem + kCS, q_k + qo, kd + ko, idesc_s, ks > 0);
+                        mma_ss_e(el, tmem + kCS, q_k + qo, kd + ko, idesc_s, ks > 0);
                     }
-                    mma_commit(&bars->s_full);
-                    if (!mbar_wait(&bars->da_full, g & 1)) { fail(23); ok = false; break; }
+                    mma_commit_e(el, &bars->s_full);
+                    if (!mbar_wait_u(&bars->da_full, g & 1)) { fail(23); ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss(tmem + kCDR, da_k + qo, kd + ko, idesc_s, ks > 0);
+                        mma_ss_e(el, tmem + kCDR, da_k + qo, kd + ko, idesc_s, ks > 0);
                     }
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss(tmem + kCDR, dy_k + qo, vd + ko, idesc_s, 1u);
+                        mma_ss_e(el, tmem + kCDR, dy_k + qo, vd + ko, idesc_s, 1u);
                     }
-                    mma_commit(&bars->dr_full);
-                    if (!kvw) mma_commit(&bars->da_empty);          // nothing else reads the row tiles this step
-                    if (!mbar_wait(&bars->p_full, g & 1)) { fail(24); ok = false; break; }
-                    if (f == 0 && uc >= 1 && !mbar_wait(&bars->dq_free, (uc - 1) & 1)) { fail(25); ok = false; break; }
+                    mma_commit_e(el, &bars->dr_full);
+                    if (!kvw) mma_commit_e(el, &bars->da_empty);          // nothing else reads the row tiles this step
+                    if (!mbar_wait_u(&bars->p_full, g & 1)) { fail(24); ok = false; break; }
+                    if (f == 0 && uc >= 1 && !mbar_wait_u(&bars->dq_free, (uc - 1) & 1)) { fail(25); ok = false; break; }
                     tc_fence_after();
                     const uint64_t kmn = kv_mn0 + (uint64_t)((s * kKVStage) >> 4);
 #pragma unroll
                     for (int kk = 0; kk < N_S / 16; ++kk)      // dQ (+)= (scale dz) K
-                        mma_ts(tmem + kCDQ, tmem + kCDR + kk * 8, kmn + ((kk * 2048) >> 4), idesc_q, (f > 0 || kk > 0) ? 1u : 0u);
+                        mma_ts_e(el, tmem + kCDQ, tmem + kCDR + kk * 8, kmn + ((kk * 2048) >> 4), idesc_q, (f > 0 || kk > 0) ? 1u : 0u);
                     if (kvw) {
-                        if (gd >= 1 && !mbar_wait(&bars->dkv_free, (gd - 1) & 1)) { fail(26); ok = false; break; }
+                        if (gd >= 1 && !mbar_wait_u(&bars->dkv_free, (gd - 1) & 1)) { fail(26); ok = false; break; }
                         tc_fence_after();
 #pragma unroll
                         for (int kk = 0; kk < kRows / 16; ++kk)     // dK = R^T daL_tile
-                            mma_ss(tmem + kCDK, r_mn + ((kk * 2048) >> 4), da_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
+                            mma_ss_e(el, tmem + kCDK, r_mn + ((kk * 2048) >> 4), da_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
 #pragma unroll
                         for (int kk = 0; kk < kRows / 16; ++kk)     // dK += (scale dz)^T Q_tile
-                            mma_ss(tmem + kCDK, z_mn + ((kk * 2048) >> 4), q_mn + ((kk * 2048) >> 4), idesc_k, 1u);
+                            mma_ss_e(el, tmem + kCDK, z_mn + ((kk * 2048) >> 4), q_mn + ((kk * 2048) >> 4), idesc_k, 1u);
 #pragma unroll
                         for (int kk = 0; kk < kRows / 16; ++kk)     // dV = R^T dY_tile
-                            mma_ss(tmem + kCDV, r_mn + ((kk * 2048) >> 4), dy_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
-                        mma_commit(&bars->dkv_full);
-                        mma_commit(&bars->da_empty);
+                            mma_ss_e(el, tmem + kCDV, r_mn + ((kk * 2048) >> 4), dy_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
+                        mma_commit_e(el, &bars->dkv_full);
+                        mma_commit_e(el, &bars->da_empty);
                         ++gd;
                     }
-                    mma_commit(&bars->sdr_free);
-                    mma_commit(&bars->kv_empty[s]);
-                    if (f + 1 == F) { mma_commit(&bars->dq_full); mma_commit(&bars->q_empty); }
+                    mma_commit_e(el, &bars->sdr_free);
+                    mma_commit_e(el, &bars->kv_empty[s]);
+                    if (f + 1 == F) { mma_commit_e(el, &bars->dq_full); mma_commit_e(el, &bars->q_empty); }
                 }
             }
         }

@@ -122,7 +122,7 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
     BBarriers* bars = reinterpret_cast<BBarriers*>(ds_s + 2 * kDsTile);
 
     const Blocking& blk = p.blk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int b1 = blk.b1;
     const int n_keys = p.n_keys;
     const int n_tiles = (n_keys + kKB - 1) / kKB;
@@ -159,7 +159,8 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) { prefetch_tmap(&tal); prefetch_tmap(&ty); prefetch_tmap(&tqr); prefetch_tmap(&tdo); }
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tal); prefetch_tmap(&ty); prefetch_tmap(&tqr); prefetch_tmap(&tdo);
         int g = 0, uc = 0;                                       // tiles loaded, slabs started
         bool ok = true;
         for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u, ++uc) {
@@ -168,26 +169,23 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
             const int grp = un.bhl * p.A + un.a;
             const int qb = kQBufs == 2 ? (uc & 1) : 0;
             unsigned char* qt = qd_s + qb * kQdBuf;
-            auto load_tiles = [&](int t_begin, int t_end) {      // lane 0 only
+            auto load_tiles = [&](int t_begin, int t_end) {
                 for (int t = t_begin; t < t_end; ++t, ++g) {
                     const int s = g % kStgB;
-                    if (g >= kStgB && !mbar_wait(&bars->a_empty[s], ((g / kStgB) - 1) & 1)) { fail(11); ok = false; break; }
+                    if (g >= kStgB && !mbar_wait_u(&bars->a_empty[s], ((g / kStgB) - 1) & 1)) { fail(11); ok = false; break; }
                     unsigned char* st = a_s + s * kBStage;
-                    mbar_arrive_expect_tx(&bars->a_full[s], (uint32_t)kBStage);
-                    tma_load_4d(st, &tal, &bars->a_full[s], 0, un.j, t * kKB, grp);
-                    tma_load_4d(st + kKB * 128, &tal, &bars->a_full[s], 64, un.j, t * kKB, grp);
-                    tma_load_4d(st + kBTile, &ty, &bars->a_full[s], 0, un.j, t * kKB, grp);
-                    tma_load_4d(st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, un.j, t * kKB, grp);
+                    mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kBStage);
+                    tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                    tma_load_4d_e(el, st + kKB * 128, &tal, &bars->a_full[s], 64, un.j, t * kKB, grp);
+                    tma_load_4d_e(el, st + kBTile, &ty, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                    tma_load_4d_e(el, st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, un.j, t * kKB, grp);
                 }
             };
             // the slab's first tile does not wait for the query-side buffer
-            if (lane == 0) load_tiles(0, 1);
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            load_tiles(0, 1);
             if (!ok) break;
             if (uc >= kQBufs) {
-                int okw = 1;
-                if (lane == 0) okw = mbar_wait(&bars->q_empty[qb], ((uc / kQBufs) - 1) & 1) ? 1 : 0;
-                if (!__shfl_sync(0xffffffffu, okw, 0)) { fail(10); break; }
+                if (!mbar_wait_u(&bars->q_empty[qb], ((uc / kQBufs) - 1) & 1)) { fail(10); break; }
             }
             for (int i = lane; i < NC * kNI; i += 32) {
                 float l2 = INFINITY, dl = 0.f;
@@ -200,27 +198,26 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 bars->delta[qb][i] = dl;
             }
             __syncwarp();
-            if (lane == 0) {
+            {
                 // 32 consecutive rows of the token grid per chunk; rows past the slab's b1 hold other tokens (or the
                 // fill value) and are masked by an infinite log-sum-exp
-                mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(NC * 4 * p.q_box_rows * 128));
+                mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(NC * 4 * p.q_box_rows * 128));
                 const int tok0 = blk.row_token(un.a, 0);
                 const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
                 for (int c = 0; c < NC; ++c) {
                     unsigned char* dq_ = qt + c * kQdBuf;
-                    tma_load_5d(dq_, &tqr, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d(dq_ + kQdHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d(dq_ + kQdTile, &tdo, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d(dq_ + kQdTile + kQdHalf, &tdo, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
+                    tma_load_5d_e(el, dq_, &tqr, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
+                    tma_load_5d_e(el, dq_ + kQdHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
+                    tma_load_5d_e(el, dq_ + kQdTile, &tdo, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
+                    tma_load_5d_e(el, dq_ + kQdTile + kQdHalf, &tdo, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
                 }
                 load_tiles(1, n_tiles);
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            g = __shfl_sync(0xffffffffu, g, 0);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc_s = idesc_bf16(128, kNI, 0, 0);            // S^T, dP^T
             constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);       // dY, daL: A from TMEM, B MN-major
             constexpr uint32_t idesc_q = idesc_bf16(128, 64, 1, 1);             // dq^T: both operands MN-major
@@ -235,9 +232,9 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 const int gt = g / NC, c = g - gt * NC;
                 const int uc = gt / n_tiles, t = gt - uc * n_tiles, w = g & 1, s = gt % kStgB;
                 const int qb = kQBufs == 2 ? (uc & 1) : 0;
-                if (t == 0 && c == 0 && !mbar_wait(&bars->q_full[qb], (uc / kQBufs) & 1)) { fail(20); return false; }
-                if (c == 0 && !mbar_wait(&bars->a_full[s], (gt / kStgB) & 1)) { fail(21); return false; }
-                if (g >= 2 && !mbar_wait(&bars->sd_free[w], ((g >> 1) - 1) & 1)) { fail(22); return false; }
+                if (t == 0 && c == 0 && !mbar_wait_u(&bars->q_full[qb], (uc / kQBufs) & 1)) { fail(20); return false; }
+                if (c == 0 && !mbar_wait_u(&bars->a_full[s], (gt / kStgB) & 1)) { fail(21); return false; }
+                if (g >= 2 && !mbar_wait_u(&bars->sd_free[w], ((g >> 1) - 1) & 1)) { fail(22); return false; }
                 tc_fence_after();
                 const uint64_t al = a_k0 + (uint64_t)((s * kBStage) >> 4);
                 const uint64_t yy = al + (uint64_t)(kBTile >> 4);
@@ -247,15 +244,15 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint32_t ao = ((ks >> 2) * (kKB * 128) + (ks & 3) * 32) >> 4;
                     const uint32_t qo = ((ks >> 2) * kQdHalf + (ks & 3) * 32) >> 4;
-                    mma_ss(tmem + bc_s(w), al + ao, qq + qo, idesc_s, ks > 0);
+                    mma_ss_e(el, tmem + bc_s(w), al + ao, qq + qo, idesc_s, ks > 0);
                 }
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint32_t ao = ((ks >> 2) * (kKB * 128) + (ks & 3) * 32) >> 4;
                     const uint32_t qo = ((ks >> 2) * kQdHalf + (ks & 3) * 32) >> 4;
-                    mma_ss(tmem + bc_dp(w), yy + ao, dd + qo, idesc_s, ks > 0);
+                    mma_ss_e(el, tmem + bc_dp(w), yy + ao, dd + qo, idesc_s, ks > 0);
                 }
-                mma_commit(&bars->s_full[w]);
+                mma_commit_e(el, &bars->s_full[w]);
                 return true;
             };
             int drains[2] = {0, 0};               // accumulator hand-overs to each warpgroup so far
@@ -270,34 +267,34 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 const int gt = g / NC, c = g - gt * NC;
                 const int uc = gt / n_tiles, t = gt - uc * n_tiles, w = g & 1, s = gt % kStgB;
                 const int qb = kQBufs == 2 ? (uc & 1) : 0;
-                if (!mbar_wait(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
+                if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
                 // the accumulators are shared by all tiles: the previous tile's must have been drained
-                if (c == 0 && gt >= 1 && !mbar_wait(&bars->acc_free[last_drainer], (drains[last_drainer] - 1) & 1)) { fail(24); break; }
-                if (t == 0 && c == 0 && uc >= 1 && !mbar_wait(&bars->dq_free, (uc - 1) & 1)) { fail(25); break; }
+                if (c == 0 && gt >= 1 && !mbar_wait_u(&bars->acc_free[last_drainer], (drains[last_drainer] - 1) & 1)) { fail(24); break; }
+                if (t == 0 && c == 0 && uc >= 1 && !mbar_wait_u(&bars->dq_free, (uc - 1) & 1)) { fail(25); break; }
                 tc_fence_after();
                 const uint64_t qn = q_mn0 + (uint64_t)(((qb + c) * kQdBuf) >> 4);
                 const uint64_t dn = qn + (uint64_t)(kQdTile >> 4);
 #pragma unroll
                 for (int kk = 0; kk < kNI / 16; ++kk)          // dY_tile (+)= P^T dOut
-                    mma_ts(tmem + kColDY, tmem + bc_s(w) + kk * 8, dn + ((kk * 2048) >> 4), idesc_o, (c > 0 || kk > 0) ? 1u : 0u);
+                    mma_ts_e(el, tmem + kColDY, tmem + bc_s(w) + kk * 8, dn + ((kk * 2048) >> 4), idesc_o, (c > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
                 for (int kk = 0; kk < kNI / 16; ++kk)          // daL_tile (+)= (scale dS)^T Q
-                    mma_ts(tmem + kColDaL, tmem + bc_dp(w) + kk * 8, qn + ((kk * 2048) >> 4), idesc_o, (c > 0 || kk > 0) ? 1u : 0u);
+                    mma_ts_e(el, tmem + kColDaL, tmem + bc_dp(w) + kk * 8, qn + ((kk * 2048) >> 4), idesc_o, (c > 0 || kk > 0) ? 1u : 0u);
                 const uint64_t am = a_mn0 + (uint64_t)((s * kBStage) >> 4);
                 const uint64_t dsd = ds0 + (uint64_t)((w * kDsTile) >> 4);
                 // dq^T of chunk c (+)= aL_tile^T (scale dS)^T: 64 output columns of which the upper 32 receive zeros
                 // (and, on a slab's first tile, are set to zero before the next chunk sets its own)
 #pragma unroll
                 for (int kk = 0; kk < kKB / 16; ++kk)
-                    mma_ss(tmem + kColDq + c * kNI, am + ((kk * 2048) >> 4), dsd + ((kk * 2048) >> 4), idesc_q, (t > 0 || kk > 0) ? 1u : 0u);
+                    mma_ss_e(el, tmem + kColDq + c * kNI, am + ((kk * 2048) >> 4), dsd + ((kk * 2048) >> 4), idesc_q, (t > 0 || kk > 0) ? 1u : 0u);
                 if (c == NC - 1) {
-                    mma_commit(&bars->acc_full[w]);
+                    mma_commit_e(el, &bars->acc_full[w]);
                     ++drains[w];
                     last_drainer = w;
-                    mma_commit(&bars->a_empty[s]);
+                    mma_commit_e(el, &bars->a_empty[s]);
                 }
-                mma_commit(&bars->sd_free[w]);
-                if (t + 1 == n_tiles && c == NC - 1) { mma_commit(&bars->dq_full); mma_commit(&bars->q_empty[qb]); }
+                mma_commit_e(el, &bars->sd_free[w]);
+                if (t + 1 == n_tiles && c == NC - 1) { mma_commit_e(el, &bars->dq_full); mma_commit_e(el, &bars->q_empty[qb]); }
                 if (g + 1 < total && !ahead && !issue_s(g + 1)) { ok = false; break; }
             }
         }

@@ -84,7 +84,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
 
     const MonarchParams& p = ip.mp;
     const Blocking& blk = p.blk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int b1 = blk.b1, b2 = blk.b2;
     const int n_keys = p.n_keys;
     const int n_tiles = (n_keys + kKTile - 1) / kKTile;
@@ -118,7 +118,8 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) { prefetch_tmap(&tal); prefetch_tmap(&tqr); }
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tal); prefetch_tmap(&tqr);
         int g = 0, uc = 0;
         bool ok = true;
         for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u, ++uc) {
@@ -127,20 +128,18 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             const int qb = uc & 1;
             unsigned char* qd_s = q_s + qb * kItQBytes;
             if (uc >= 2) {
-                int okw = 1;
-                if (lane == 0) okw = mbar_wait(&bars->q_empty[qb], ((uc >> 1) - 1) & 1) ? 1 : 0;
-                if (!__shfl_sync(0xffffffffu, okw, 0)) { fail(10); break; }
+                if (!mbar_wait_u(&bars->q_empty[qb], ((uc >> 1) - 1) & 1)) { fail(10); break; }
             }
             for (int i = lane; i < 128; i += 32)
                 bars->lse2[qb][i] = i < b1 ? kLog2e * p.lse[(long long)u * b1 + i] : INFINITY;
             if (ip.q_rows_tma) {
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&bars->q_full[qb], (uint32_t)(b1 * 256));
+                {
+                    mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(b1 * 256));
                     const int tok0 = blk.row_token(p.a0 + un.al, 0);
                     const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
-                    tma_load_5d(qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
-                    tma_load_5d(qd_s + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
+                    tma_load_5d_e(el, qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
+                    tma_load_5d_e(el, qd_s + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
                 }
             } else {
                 const __nv_bfloat16* qg = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
@@ -154,22 +153,21 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->q_full[qb]);
             }
-            if (lane == 0) {
+            {
                 for (int t = 0; t < n_tiles; ++t, ++g) {
                     const int s = g % kAStg;
-                    if (g >= kAStg && !mbar_wait(&bars->a_empty[s], ((g / kAStg) - 1) & 1)) { fail(11); ok = false; break; }
+                    if (g >= kAStg && !mbar_wait_u(&bars->a_empty[s], ((g / kAStg) - 1) & 1)) { fail(11); ok = false; break; }
                     unsigned char* st = a_s + s * kItTileBytes;
-                    mbar_arrive_expect_tx(&bars->a_full[s], (uint32_t)kItTileBytes);
-                    tma_load_4d(st, &tal, &bars->a_full[s], 0, un.j, t * kKTile, un.bhl * p.na + un.al);
-                    tma_load_4d(st + kKTile * 128, &tal, &bars->a_full[s], 64, un.j, t * kKTile, un.bhl * p.na + un.al);
+                    mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kItTileBytes);
+                    tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKTile, un.bhl * p.na + un.al);
+                    tma_load_4d_e(el, st + kKTile * 128, &tal, &bars->a_full[s], 64, un.j, t * kKTile, un.bhl * p.na + un.al);
                 }
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            g = __shfl_sync(0xffffffffu, g, 0);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc_s = idesc_bf16(128, N_I, 0, 0);
             constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);
             const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
@@ -179,35 +177,35 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             bool ok = true;
             auto issue_s = [&](int g) -> bool {                  // S^T of tile g
                 const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1, s = g % kAStg, qb = uc & 1;
-                if (t == 0 && !mbar_wait(&bars->q_full[qb], (uc >> 1) & 1)) { fail(20); return false; }
-                if (!mbar_wait(&bars->a_full[s], (g / kAStg) & 1)) { fail(21); return false; }
-                if (g >= 2 && !mbar_wait(&bars->sp_free[w], ((g >> 1) - 1) & 1)) { fail(22); return false; }
+                if (t == 0 && !mbar_wait_u(&bars->q_full[qb], (uc >> 1) & 1)) { fail(20); return false; }
+                if (!mbar_wait_u(&bars->a_full[s], (g / kAStg) & 1)) { fail(21); return false; }
+                if (g >= 2 && !mbar_wait_u(&bars->sp_free[w], ((g >> 1) - 1) & 1)) { fail(22); return false; }
                 tc_fence_after();
                 const uint64_t ad = a_desc0 + (uint64_t)((s * kItTileBytes) >> 4);
                 const uint64_t qd = qk_desc0 + (uint64_t)((qb * kItQBytes) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint32_t off = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;
-                    mma_ss(tmem + it_col_s(w), ad + off, qd + off, idesc_s, ks > 0);
+                    mma_ss_e(el, tmem + it_col_s(w), ad + off, qd + off, idesc_s, ks > 0);
                 }
-                mma_commit(&bars->s_full[w]);
-                mma_commit(&bars->a_empty[s]);
+                mma_commit_e(el, &bars->s_full[w]);
+                mma_commit_e(el, &bars->a_empty[s]);
                 return true;
             };
             if (total > 0) ok = issue_s(0);
             for (int g = 0; ok && g < total && !bars->abort_flag; ++g) {
                 if (g + 1 < total && !issue_s(g + 1)) { ok = false; break; }
                 const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1, qb = uc & 1;
-                if (!mbar_wait(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
-                if (g >= 2 && !mbar_wait(&bars->o_free[w], ((g >> 1) - 1) & 1)) { fail(24); break; }
+                if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
+                if (g >= 2 && !mbar_wait_u(&bars->o_free[w], ((g >> 1) - 1) & 1)) { fail(24); break; }
                 tc_fence_after();
                 const uint64_t qd = qn_desc0 + (uint64_t)((qb * kItQBytes) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < N_I / 16; ++kk)
-                    mma_ts(tmem + it_col_o(w), tmem + it_col_s(w) + kk * 8, qd + ((kk * 2048) >> 4), idesc_o, kk > 0);
-                mma_commit(&bars->o_full[w]);
-                mma_commit(&bars->sp_free[w]);
-                if (t + 1 == n_tiles) mma_commit(&bars->q_empty[qb]);       // last read of this unit's query tile
+                    mma_ts_e(el, tmem + it_col_o(w), tmem + it_col_s(w) + kk * 8, qd + ((kk * 2048) >> 4), idesc_o, kk > 0);
+                mma_commit_e(el, &bars->o_full[w]);
+                mma_commit_e(el, &bars->sp_free[w]);
+                if (t + 1 == n_tiles) mma_commit_e(el, &bars->q_empty[qb]);       // last read of this unit's query tile
             }
         }
     } else if (warp >= 4) {
