@@ -90,6 +90,32 @@ int sfm_rope_cache_write(const void* q, const void* k, const void* v, void* q_ou
                          int start_frame, int monarch_order, void* stream);
 
 /*
+ * One layer call on the KV cache: the cache write of the new tokens (sfm_rope_cache_write, or its normalising / evicting
+ * forms) and the attention over the cache view (sfm_monarch_fwd, or sfm_dense_fwd with the tokens in natural order), all
+ * arguments in one struct so that a binding passes a single pointer.
+ *   q, k, v      [B, n_q | n_new, H, D] natural order; k, v contiguous, q too when q_rot is given, else batch stride
+ *                q_batch_stride
+ *   q_rot        [B, n_q, H, D]: normalised and rotated q (n_q = n_new); NULL: q is attended as it is
+ *   rope, norm_q_weight, norm_k_weight, roll_*   as in sfm_rope_cache_write_roll; each may be NULL / 0
+ *   k_cache, v_cache   the cache view [B, n_kv, H, D], batch stride cache_batch_stride; n_kv includes the new tokens
+ *   out          [B, n_q, H, D] contiguous;  workspace: sfm_monarch_workspace_bytes(..., 0) bytes (unused when dense)
+ * Replaces: the cache branch of CausalWanSelfAttention.forward between the projections
+ * (wan/modules/causal_model.py:900-1103), and monarch_attn_with_kv_cache (wan/modules/monarch_attn.py:1778-1796).
+ */
+typedef struct SfmKvCall {
+    const void *q, *k, *v, *norm_q_weight, *norm_k_weight;
+    void *q_rot, *k_cache, *v_cache;
+    const void *rope;
+    void *out, *workspace, *stream;
+    int64_t q_batch_stride, cache_batch_stride;
+    uint64_t workspace_bytes;
+    float eps, sm_scale;
+    int32_t B, H, D, n_q, n_new, n_kv, start_idx, roll_dst, roll_shift, start_frame;
+    int32_t f_tied, h_reduce, w_reduce, h, w, num_iters, dense, reserved;
+} SfmKvCall;
+int sfm_kv_attention(const void* call);
+
+/*
  * Stand-alone 3-axis RoPE of one tensor x [B, L, H, D] -> out (same shape): the first
  * frames*h*w tokens are rotated as a frames x h x w grid whose frame positions start at
  * start_frame; the rest are copied.  rope = device table from sfm_rope_table.

@@ -18,6 +18,7 @@ SIGNATURES = {
     "sfm_build_maps": (C.c_int, [C.c_void_p, C.c_void_p] + [C.c_int] * 6),
     "sfm_rope_table": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_double]),
     "sfm_rope_cache_write": (C.c_int, [C.c_void_p] * 6 + [C.c_int64, C.c_void_p] + [C.c_int] * 12 + [C.c_void_p]),
+    "sfm_kv_attention": (C.c_int, [C.c_char_p]),
     "sfm_rope_apply": (C.c_int, [C.c_void_p] * 3 + [C.c_int] * 8 + [C.c_void_p]),
     "sfm_monarch_workspace_bytes": (C.c_size_t, [C.c_int] * 11 + [C.c_size_t]),
     "sfm_monarch_fwd": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p,

@@ -1,14 +1,17 @@
 // extern "C" entry points for the Monarch forward and their host-side planning.
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 
 #include "monarch_params.cuh"
+#include "profile.cuh"
 #include "tc05.cuh"
 
 using namespace sfm;
 
 namespace sfm {
-int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps, int n_s, int* status, int num_sms, cudaStream_t s);
+int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps, int n_s, int* status, int clear_status, int num_sms,
+                     cudaStream_t s);
 int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s, int write_lse);
 int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s);
 }
@@ -142,17 +145,13 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
     if (pl.blk.b2 > kB2Max && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
     // only the tensor-core column step knows how to scatter its rows
     if (os && os->world > 1 && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
-    int num_sms = 148;
-    {
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    }
+    const int num_sms = device_sms();
     int* status = reinterpret_cast<int*>(base + pl.off_status);
     CUtensorMap maps[5];     // q, K, V, query rows, iteration state
     const int n_s = (pl.blk.b2 + 15) & ~15;
-    {
-        // Every path starts from a clear status word: the workspace may be recycled memory, and the kernels
-        // without bounded waits (iterative variant, block rows above 128) never write it.
+    // Every path starts from a clear status word: the workspace may be recycled memory.  The tensor-core path's first
+    // kernel clears it; the mma.sync kernels have no bounded waits and never write it.
+    if (!use_tc) {
         cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), stream);
         if (e != cudaSuccess) return (int)e;
     }
@@ -204,7 +203,7 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
                 if (use_tc) {
                     // later passes of the iterative variant read their query operand from the state aR
                     CUtensorMap rmaps[3] = {p.use_aR ? maps[4] : maps[0], maps[1], maps[2]};
-                    if ((rc = launch_r_step_tc(p, rmaps, n_s, status, num_sms, stream))) return rc;
+                    if ((rc = launch_r_step_tc(p, rmaps, n_s, status, bh0 == 0 && a0 == 0 && it == 0, num_sms, stream))) return rc;
                 } else {
                     if ((rc = launch_r_step(p, stream))) return rc;
                 }
@@ -257,11 +256,7 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
     p.blk = blk;
     p.bh0 = bh0; p.nbh = nbh; p.a0 = 0; p.na = p.A;
     p.use_aR = 0; p.write_Y = 1;
-    int num_sms = 148;
-    {
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    }
+    const int num_sms = device_sms();
     const int n_s = (blk.b2 + 15) & ~15;
     const size_t slabs = (size_t)nbh * p.A * blk.b2;
     int rc;
@@ -279,7 +274,7 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
     if ((rc = make_tmap_bf16(&maps[1], kc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
-    if ((rc = launch_r_step_tc(p, maps, n_s, status, num_sms, stream))) return rc;
+    if ((rc = launch_r_step_tc(p, maps, n_s, status, 0, num_sms, stream))) return rc;
     if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
     *p_out = p;
     return SFM_OK;
@@ -407,6 +402,31 @@ extern "C" int sfm_monarch_nocache_fwd(const void* q, const void* k, const void*
                        bridge_budget_bytes, (cudaStream_t)stream);
 }
 
+extern "C" int sfm_kv_attention(const void* call) {
+    if (!call) return SFM_ERR_NULL_POINTER;
+    SfmKvCall c;
+    memcpy(&c, call, sizeof(c));
+    if (!c.k || !c.v || !c.q || (c.q_rot && !c.rope)) return SFM_ERR_NULL_POINTER;
+    const int order = c.dense ? 0 : 1;
+    int rc = c.roll_shift > 0 || c.norm_q_weight || c.norm_k_weight
+                 ? sfm_rope_cache_write_roll(c.q_rot ? c.q : nullptr, c.k, c.v, c.norm_q_weight, c.norm_k_weight, c.eps, c.q_rot,
+                                             c.k_cache, c.v_cache, c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new,
+                                             c.H, c.D, c.start_idx, c.roll_dst, c.roll_shift, c.f_tied, c.h_reduce,
+                                             c.w_reduce, c.h, c.w, c.start_frame, order, c.stream)
+                 : sfm_rope_cache_write(c.q_rot ? c.q : nullptr, c.k, c.v, c.q_rot, c.k_cache, c.v_cache,
+                                        c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new, c.H, c.D, c.start_idx,
+                                        c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.start_frame, order, c.stream);
+    if (rc) return rc;
+    const void* q = c.q_rot ? c.q_rot : c.q;
+    const int64_t q_bs = c.q_rot ? (int64_t)c.n_q * c.H * c.D : c.q_batch_stride;
+    if (c.dense)
+        return sfm_dense_fwd(q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.B, c.H, c.D, c.n_q, c.n_kv, c.sm_scale,
+                             c.stream);
+    return run_monarch(q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.workspace, c.workspace_bytes, c.B, c.H, c.D,
+                       c.n_q, c.n_kv, c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.sm_scale, c.num_iters, 0, 0,
+                       (cudaStream_t)c.stream);
+}
+
 // ---------------------------------------------------------------------------------------------
 // launch accounting / per-kernel timing
 // ---------------------------------------------------------------------------------------------
@@ -414,7 +434,6 @@ extern "C" int sfm_monarch_nocache_fwd(const void* q, const void* k, const void*
 #include <mutex>
 #include <vector>
 
-#include "profile.cuh"
 
 namespace {
 std::atomic<long long> g_launches[kNumClasses];

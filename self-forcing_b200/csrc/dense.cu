@@ -2,6 +2,8 @@
 // "regular" configuration.  Host side of the tensor-core kernel in dense_tc.cu.
 //
 // Stands in for flash_attention / attention (wan/modules/attention.py:34-187).
+#include <atomic>
+
 #include "common.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -29,13 +31,16 @@ extern "C" int sfm_dense_fwd(const void* q, int64_t q_batch_stride, const void* 
     auto mis = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
     if (mis(q) || mis(k) || mis(v) || mis(out) || (q_batch_stride % 8) || (kv_batch_stride % 8)) return SFM_ERR_ALIGNMENT;
 
-    int dev = 0, num_sms = 148;
+    static std::atomic<int*> words[64];                     // the status word's address, looked up once per device
+    int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    int* status = nullptr;
-    e = cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_dense_status);
-    if (e != cudaSuccess) return (int)e;
+    int* status = dev >= 0 && dev < 64 ? words[dev].load(std::memory_order_relaxed) : nullptr;
+    if (!status) {
+        e = cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_dense_status);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) words[dev].store(status, std::memory_order_relaxed);
+    }
 
     const uint64_t row = (uint64_t)kHeadDim * 2, tok = (uint64_t)H * row;
     uint64_t dq[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_q, (uint64_t)B};
@@ -48,7 +53,8 @@ extern "C" int sfm_dense_fwd(const void* q, int64_t q_batch_stride, const void* 
     if ((rc = make_tmap_bf16(&maps[0], k, 4, dk, sk, box))) return rc;
     if ((rc = make_tmap_bf16(&maps[1], v, 4, dk, sk, box))) return rc;
     if ((rc = make_tmap_bf16(&maps[2], q, 4, dq, sq, box))) return rc;
-    return launch_dense_tc(maps, (__nv_bfloat16*)out, B, H, n_q, n_kv, sm_scale, status, num_sms, (cudaStream_t)stream);
+    return launch_dense_tc(maps, (__nv_bfloat16*)out, B, H, n_q, n_kv, sm_scale, status, device_sms(),
+                           (cudaStream_t)stream);
 }
 
 // Waits for `stream`, then reports (and clears) the status word of the dense-attention kernels on the

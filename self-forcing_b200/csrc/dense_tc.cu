@@ -387,8 +387,7 @@ int launch_dense_tc(const CUtensorMap* maps, __nv_bfloat16* out, int B, int H, i
     p.scale = scale;
     p.status = status;
     dim3 grid(p.n_units < num_sms ? p.n_units : num_sms);
-    cudaError_t e = cudaFuncSetAttribute(dense_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
+    if (int rc = opt_in_smem((const void*)dense_tc_kernel, kSmemBytes)) return rc;
     dense_tc_kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], maps[2], p);
     return (int)cudaGetLastError();
 }

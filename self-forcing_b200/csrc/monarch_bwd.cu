@@ -798,11 +798,7 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
 
     cudaStream_t s = (cudaStream_t)stream;
     const int BH = B * H;
-    int num_sms = 148;
-    {
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    }
+    const int num_sms = device_sms();
     // one status word per call: a kernel that gives up on a bounded wait sets it, nothing clears it before the end
     if (cudaMemsetAsync(ws, 0, sizeof(int), s) != cudaSuccess) return SFM_ERR_UNSUPPORTED;
     for (int bh0 = 0; bh0 < BH; bh0 += pl.nbh) {

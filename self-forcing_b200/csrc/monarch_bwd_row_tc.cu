@@ -493,8 +493,7 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     if (int rc = make_bridge_tmap(&bridge[0], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, rp.rows_per_group, 1)) return rc;
     if (int rc = make_bridge_tmap(&bridge[1], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, rp.rows_per_group, 1)) return rc;
     auto go = [&](auto kernel) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRBSmem);
-        if (e != cudaSuccess) return (int)e;
+        if (int rc = opt_in_smem((const void*)kernel, kRBSmem)) return rc;
         kernel<<<grid, kThreadsRB, kRBSmem, s>>>(maps[0], maps[1], maps[2], bridge[0], bridge[1], rp);
         return 0;
     };

@@ -465,8 +465,7 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     if (int rc = make_bridge_tmap(&bridge[0], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
     if (int rc = make_bridge_tmap(&bridge[1], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
     auto go = [&](auto kernel, int smem) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
+        if (int rc = opt_in_smem((const void*)kernel, smem)) return rc;
         kernel<<<grid, kThreadsB, smem, s>>>(bridge[0], bridge[1], maps[0], maps[1], p);
         return 0;
     };

@@ -299,8 +299,7 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kItSmemBytes);
-        if (e != cudaSuccess) return (int)e;
+        if (int rc = opt_in_smem((const void*)kernel, kItSmemBytes)) return rc;
         kernel<<<grid, kThreadsIt, kItSmemBytes, s>>>(map_al, *map_qrows, ip);
         return 0;
     };

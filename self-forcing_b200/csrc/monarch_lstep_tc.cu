@@ -569,8 +569,7 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     const int n_groups = (lp.n_units + lp.U - 1) / lp.U;
     dim3 grid(n_groups < num_sms ? n_groups : num_sms);
     auto kernel = p.causal_groups > 0 ? monarch_l_tc_kernel<true> : monarch_l_tc_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
+    if (int rc = opt_in_smem((const void*)kernel, kSmemBytes)) return rc;
     kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], *map_qrows, lp);
     return (int)cudaGetLastError();
 }

@@ -57,6 +57,7 @@ struct RTcParams {
     int n_units;           // nbh * tiles * b1 * fsplit
     int col_kt;            // keys per tile of the column step (block-causal: it reads whole tiles)
     int* status;           // device status word (0 = ok)
+    int clear_status;      // the call's first launch starts it from zero
 };
 
 
@@ -169,6 +170,8 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         bars->abort_flag = 1;
         atomicCAS(rp.status, 0, code);
     };
+    // no wait can run out before block 0 has started
+    if (rp.clear_status && blockIdx.x == 0 && tid == 0) *rp.status = 0;
     const int u_first = blockIdx.x, u_stride = gridDim.x;
 
     if (warp == 0) {
@@ -550,7 +553,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 int l_tile_keys(int n_keys);
 
 int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or the aR state), k, v */, int n_s, int* status,
-                     int num_sms, cudaStream_t s) {
+                     int clear_status, int num_sms, cudaStream_t s) {
     LaunchScope scope(kClsRStep, s);
     RTcParams rp;
     rp.mp = p;
@@ -573,6 +576,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     }
     rp.n_units = p.nbh * rp.tiles * p.blk.b1 * rp.fsplit;
     rp.status = status;
+    rp.clear_status = clear_status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
     // wide blocks: two 64 KB K / V stages instead of five 32 KB ones
     const bool iter = p.use_aR != 0;
@@ -583,8 +587,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     for (int i = 0; i < 2; ++i)
         if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, rp.rows_per_group < 32 ? rp.rows_per_group : 32, 1)) return rc;
     auto go = [&](auto kernel) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-        if (e != cudaSuccess) return (int)e;
+        if (int rc = opt_in_smem((const void*)kernel, smem_bytes)) return rc;
         kernel<<<grid, kThreads, smem_bytes, s>>>(maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
         return 0;
     };

@@ -15,4 +15,9 @@ struct LaunchScope {
     int slot_;
 };
 
+// Host-side facts that do not change, asked of the runtime once per device: the number of SMs of the current device,
+// and a kernel's opt-in to `bytes` of dynamic shared memory.
+int device_sms();
+int opt_in_smem(const void* kernel, int bytes);
+
 }  // namespace sfm

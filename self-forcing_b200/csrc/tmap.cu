@@ -1,10 +1,46 @@
-// Host-side construction of TMA tensor maps (driver entry point fetched through the runtime).
+// Host side shared by the launchers: per-device facts, and the construction of TMA tensor maps (driver entry point fetched through the runtime).
 #include <cudaTypedefs.h>
 
+#include <atomic>
+#include <mutex>
+#include <unordered_map>
+
 #include "common.cuh"
+#include "profile.cuh"
 #include "tc05.cuh"
 
 namespace sfm {
+
+namespace {
+constexpr int kMaxDevices = 64;
+}
+
+int device_sms() {
+    static std::atomic<int> sms[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    int n = sms[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+        sms[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+int opt_in_smem(const void* kernel, int bytes) {
+    static std::mutex mutex;
+    static std::unordered_map<const void*, uint64_t> done;       // devices (bits) that know the kernel's size
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    const uint64_t bit = 1ull << (dev & 63);
+    std::lock_guard<std::mutex> lock(mutex);
+    uint64_t& mask = done[kernel];
+    if (mask & bit) return 0;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) mask |= bit;
+    return (int)e;
+}
 
 EncodeTiledFn get_encode_tiled() {
     static EncodeTiledFn fn = nullptr;

@@ -157,18 +157,11 @@ def self_attention_kv(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: 
             roll = (dst - step.cache_start, src - dst)
         else:
             cache._roll(step.roll)
-    curr_k = cache.k[:, step.cache_start:step.cache_start + step.local_end]
-    curr_v = cache.v[:, step.cache_start:step.cache_start + step.local_end]
-    is_init = cfg.use_dense_init and curr_k.shape[1] == 3 * frame_tokens
+    is_init = cfg.use_dense_init and step.local_end == 3 * frame_tokens
     dense = cfg.disable_monarch or is_init
-    f_tied = 1 if cfg.use_framewise else 3
-    q_rot = ops.norm_rope_cache_write(q, k, v, curr_k, curr_v, step.local_start, start_frame, f_tied, cfg.h_reduce,
-                                      cfg.w_reduce, gh, gw, freqs=freqs, norm_q_weight=norm_q_weight,
-                                      norm_k_weight=norm_k_weight, eps=cfg.eps, monarch_order=not dense, roll=roll)
-    if dense:
-        out = ops.dense_attention_on_cache(q_rot, curr_k, curr_v, sm_scale)
-    else:
-        out = ops.monarch_attention_on_cache(q_rot, curr_k, curr_v, f_tied, cfg.h_reduce, cfg.w_reduce, gh, gw,
-                                             sm_scale, cfg.num_iters)
+    out = ops.layer_attention(q, k, v, cache.k, cache.v, step.cache_start, step.local_end, step.local_start, start_frame,
+                              1 if cfg.use_framewise else 3, cfg.h_reduce, cfg.w_reduce, gh, gw, dense=dense, freqs=freqs,
+                              norm_q_weight=norm_q_weight, norm_k_weight=norm_k_weight, eps=cfg.eps, roll=roll,
+                              sm_scale=sm_scale, num_iters=cfg.num_iters)
     cache._store(step)
     return out

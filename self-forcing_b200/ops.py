@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from typing import Dict, Optional, Tuple
 
 import numpy as np
@@ -26,6 +27,9 @@ def _stream() -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else None
+
+
 def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
     return C.c_void_p(0 if t is None else t.data_ptr())
 
@@ -33,7 +37,7 @@ def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
 def _require(t: torch.Tensor, name: str) -> None:
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise RuntimeError(f"{name} must be a CUDA tensor: this package has no CPU path")
-    if t.dtype != torch.bfloat16:
+    if t.dtype is not torch.bfloat16:
         raise TypeError(f"{name} must be bfloat16, got {t.dtype}")
     if t.dim() != 4 or t.shape[-1] != 128:
         raise ValueError(f"{name} must be [B, N, H, 128], got {tuple(t.shape)}")
@@ -63,7 +67,8 @@ def _workspace(device: torch.device, nbytes: int, tag: str = "monarch") -> torch
     the least recently used one is dropped beyond that (a buffer was allocated on the stream that uses it, so
     PyTorch's allocator hands its memory out again in that stream's order only), and release_workspaces()
     drops them all."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), int(_stream().value or 0), tag)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (index, _raw_stream(index), tag)
     ws = _workspaces.pop(key, None)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=device)
@@ -89,20 +94,20 @@ def _watch_status(ws: torch.Tensor) -> None:
     launch on that workspace leaves a set word alone only until the next call clears it, so a persistent
     fault is reported within _WATCH_EVERY calls and a transient one may pass unseen: the synchronous
     check (SFM_CHECK_STATUS=1, or check_device_status()) is the strict form."""
-    key = ws.device.index if ws.device.index is not None else torch.cuda.current_device()
+    key = ws.get_device()
     state = _status_mirror.get(key)
     if state is None:
-        state = [torch.zeros(1, dtype=torch.int32).pin_memory(), 0]
+        host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        state = [host, 0, C.c_int32.from_address(host.data_ptr())]
         _status_mirror[key] = state
-    host = state[0]
-    code = int(host[0])
+    code = state[2].value
     if code != 0:
-        host[0] = 0
+        state[2].value = 0
         raise RuntimeError(f"an earlier Monarch attention call on this GPU recorded device status {code} "
                            "(a kernel gave up on a bounded wait); its output is not valid")
     state[1] += 1
     if state[1] % _WATCH_EVERY == 0:
-        host.copy_(ws[:4].view(torch.int32), non_blocking=True)
+        state[0].copy_(ws[:4].view(torch.int32), non_blocking=True)
 
 
 def check_device_status(device=None) -> None:
@@ -182,15 +187,59 @@ def _monarch_fwd(q, k_cache, v_cache, f_tied, h_reduce, w_reduce, h, w, sm_scale
         nbytes = 256
     ws = _workspace(q.device, nbytes)
     out = torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
-    rc = lib.sfm_monarch_fwd(_ptr(q), _batch_stride(q), _ptr(k_cache), _ptr(v_cache), _batch_stride(k_cache),
-                             _ptr(out), _ptr(ws), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w,
-                             float(sm_scale), int(num_iters), 0, _stream())
+    rc = lib.sfm_monarch_fwd(q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache),
+                             out.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w,
+                             float(sm_scale), int(num_iters), 0, _raw_stream(q.get_device()))
     _lib.check(rc, "sfm_monarch_fwd")
+    _after_call(ws)
+    return out
+
+
+def _after_call(ws):
     if os.environ.get("SFM_CHECK_STATUS") == "1":      # debugging aid: synchronises the stream
-        _lib.check(lib.sfm_workspace_status(_ptr(ws), _stream()), "sfm_workspace_status")
+        _lib.check(_lib.load().sfm_workspace_status(ws.data_ptr(), _raw_stream(ws.get_device())), "sfm_workspace_status")
     else:
         _watch_status(ws)
+
+
+# SfmKvCall of include/sfmonarch.h
+_KV_CALL = struct.Struct("@12P2qQ2f18i")
+
+
+def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, sm_scale, num_iters, dense=False, rope=None,
+                  start_frame=0, wq=None, wk=None, eps=0.0, roll_dst=0, roll_shift=0):
+    """One call of the library: the new tokens' cache write (with ``rope``: normalised if weights are given, rotated, and q
+    too), then attention over the cache view of ``n_kv`` tokens at ``kc_ptr`` / ``vc_ptr``.  The tensors have been checked;
+    k, v (and q, if it is rotated) are contiguous."""
+    B, n_q, H, D = q.shape
+    device = q.get_device()
+    stream = _raw_stream(device)
+    q_rot = torch.empty_like(q) if rope is not None else None
+    out = torch.empty_like(q) if q.is_contiguous() else torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
+    ws = None if dense else _workspaces.get((device, stream, "monarch"))
+    for attempt in (0, 1):
+        if not dense and (ws is None or attempt):
+            nbytes = _lib.load().sfm_monarch_workspace_bytes(B, H, D, n_q, n_kv, *blocking, num_iters, 0)
+            ws = _workspace(q.device, nbytes or 256)      # unsupported sizes: let the entry point name the error
+        call = _KV_CALL.pack(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), 0 if wq is None else wq.data_ptr(), 0 if wk is None else wk.data_ptr(),
+            0 if q_rot is None else q_rot.data_ptr(), kc_ptr, vc_ptr, 0 if rope is None else rope.data_ptr(), out.data_ptr(),
+            0 if dense else ws.data_ptr(), stream, q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws.numel(),
+            eps, sm_scale, B, H, D, n_q, k.shape[1], n_kv, start_idx, roll_dst, roll_shift, start_frame, *blocking, num_iters,
+            dense, 0)
+        rc = _lib.load().sfm_kv_attention(call)
+        if rc != _ERR_WORKSPACE or attempt:               # the cached scratch may be too small for this call: get more, once
+            break
+    if rc:
+        _lib.check(rc, "sfm_kv_attention")
+    if not dense:
+        _after_call(ws)
+    elif os.environ.get("SFM_CHECK_STATUS") == "1":
+        _lib.check(_lib.load().sfm_dense_status(stream), "sfm_dense_status")
     return out
+
+
+_ERR_WORKSPACE = -5
 
 
 def monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h_reduce, w_reduce, h, w, sm_scale=None,
@@ -233,10 +282,7 @@ def monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h
                              h_reduce, w_reduce, h, w, float(sm_scale), g0, g1, int(causal_groups), budget_bytes,
                              _stream())
     _lib.check(rc, "sfm_monarch_bwd")
-    if os.environ.get("SFM_CHECK_STATUS") == "1":      # debugging aid: synchronises the stream
-        _lib.check(lib.sfm_workspace_status(_ptr(ws), _stream()), "sfm_workspace_status")
-    else:
-        _watch_status(ws)
+    _after_call(ws)
     return dq, dk, dv
 
 
@@ -332,12 +378,9 @@ def monarch_attn_with_kv_cache(q, k_cache, v_cache, new_k, new_v, start_idx, end
     q = _as_token_major(q)
     new_k = new_k.contiguous()
     new_v = new_v.contiguous()
-    rc = _lib.load().sfm_rope_cache_write(_ptr(None), _ptr(new_k), _ptr(new_v), _ptr(None), _ptr(k_cache),
-                                          _ptr(v_cache), _batch_stride(k_cache), _ptr(None), B, n_new, H, D,
-                                          int(start_idx), f_tied, h_reduce, w_reduce, h, w, 0, 1, _stream())
-    _lib.check(rc, "sfm_rope_cache_write")
     _mark_written(k_cache, v_cache)
-    return _monarch_fwd(q, k_cache, v_cache, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters)
+    return _kv_attention(q, new_k, new_v, k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), k_cache.shape[1],
+                         int(start_idx), (f_tied, h_reduce, w_reduce, h, w), float(sm_scale), int(num_iters))
 
 
 def norm_rope_cache_write(q, k, v, k_cache, v_cache, start_idx, start_frame, f_tied, h_reduce, w_reduce, h, w,
@@ -391,6 +434,46 @@ def norm_rope_cache_write(q, k, v, k_cache, v_cache, start_idx, start_frame, f_t
     return q_rot
 
 
+def _norm_weight(weight, width, device):
+    if weight.dtype is not torch.bfloat16 or not weight.is_contiguous() or weight.device != device:
+        weight = weight.detach().to(device=device, dtype=torch.bfloat16).contiguous()
+    if weight.numel() != width:
+        raise ValueError("norm weights must have H*D elements")
+    return weight
+
+
+def layer_attention(q, k, v, k_full, v_full, cache_start, n_kv, start_idx, start_frame, f_tied, h_reduce, w_reduce, h, w,
+                    dense=False, freqs=None, norm_q_weight=None, norm_k_weight=None, eps=1e-6, roll=None, sm_scale=None,
+                    num_iters=1):
+    """norm_rope_cache_write followed by attention (Monarch, or dense with the cache in natural order) over the view
+    [cache_start, cache_start + n_kv) of the cache tensors ``k_full`` / ``v_full``, in one call of the library.
+    ``start_idx`` and ``roll`` are relative to the view."""
+    for t, name in ((q, "q"), (k, "k"), (v, "v")):
+        _require(t, name)
+    _cache_view_ok(k_full, "k_cache")
+    _cache_view_ok(v_full, "v_cache")
+    B, n, H, D = q.shape
+    if k.shape != q.shape or v.shape != q.shape or start_idx < 0 or start_idx + n > n_kv or cache_start + n_kv > k_full.shape[1]:
+        raise ValueError("q, k, v shapes or the cache extent do not match")
+    if k_full.shape != v_full.shape or _batch_stride(k_full) != _batch_stride(v_full) or k_full.shape[0] != B or k_full.shape[2] != H:
+        raise ValueError("k_cache and v_cache must share shape and strides")
+    if (norm_q_weight is None) != (norm_k_weight is None):
+        raise ValueError("give both norm weights or neither")
+    wq = wk = None
+    if norm_q_weight is not None:
+        wq, wk = _norm_weight(norm_q_weight, H * D, q.device), _norm_weight(norm_k_weight, H * D, q.device)
+    dst, shift = (0, 0) if roll is None else (int(roll[0]), int(roll[1]))
+    if start_idx + shift > n_kv:
+        raise ValueError("the eviction shift reads past the cache view")
+    tab = _rope_table_from_freqs(freqs, q.device)
+    offset = cache_start * (H * D * 2)
+    _mark_written(k_full, v_full)
+    return _kv_attention(q.contiguous(), k.contiguous(), v.contiguous(), k_full.data_ptr() + offset, v_full.data_ptr() + offset,
+                         _batch_stride(k_full), n_kv, start_idx, (f_tied, h_reduce, w_reduce, h, w),
+                         float(D ** -0.5 if sm_scale is None else sm_scale), num_iters, dense, tab, start_frame, wq, wk, float(eps),
+                         dst, shift)
+
+
 def rope_monarch_attn_with_kv_cache(q, k, v, k_cache, v_cache, start_idx, end_idx, start_frame, f_tied, h_reduce,
                                     w_reduce, h, w, freqs=None, sm_scale=None, num_iters=1):
     """Fused front end: q, k are the UN-rotated projections.  One kernel applies the 3-axis RoPE
@@ -409,13 +492,10 @@ def rope_monarch_attn_with_kv_cache(q, k, v, k_cache, v_cache, start_idx, end_id
         sm_scale = D ** -0.5
     tab = _rope_table_from_freqs(freqs, q.device)
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    q_rot = torch.empty_like(q)
-    rc = _lib.load().sfm_rope_cache_write(_ptr(q), _ptr(k), _ptr(v), _ptr(q_rot), _ptr(k_cache), _ptr(v_cache),
-                                          _batch_stride(k_cache), _ptr(tab), B, n_q, H, D, int(start_idx), f_tied,
-                                          h_reduce, w_reduce, h, w, int(start_frame), 1, _stream())
-    _lib.check(rc, "sfm_rope_cache_write")
     _mark_written(k_cache, v_cache)
-    return _monarch_fwd(q_rot, k_cache, v_cache, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters)
+    return _kv_attention(q, k, v, k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), k_cache.shape[1],
+                         int(start_idx), (f_tied, h_reduce, w_reduce, h, w), float(sm_scale), int(num_iters), rope=tab,
+                         start_frame=int(start_frame))
 
 
 def _ptr_array(ptrs):
