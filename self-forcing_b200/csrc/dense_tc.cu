@@ -100,6 +100,8 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    pdl_trigger();
+    pdl_wait();
 
     auto fail = [&](int code) {
         bars->abort_flag = 1;
@@ -388,8 +390,7 @@ int launch_dense_tc(const CUtensorMap* maps, __nv_bfloat16* out, int B, int H, i
     p.status = status;
     dim3 grid(p.n_units < num_sms ? p.n_units : num_sms);
     if (int rc = opt_in_smem((const void*)dense_tc_kernel, kSmemBytes)) return rc;
-    dense_tc_kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], maps[2], p);
-    return (int)cudaGetLastError();
+    return launch_pdl((long long)p.n_units * n_kv <= 64ll * kKT * num_sms, dense_tc_kernel, grid, kThreads, kSmemBytes, s, maps[0], maps[1], maps[2], p);
 }
 
 }  // namespace sfm

@@ -80,6 +80,8 @@ rope_cache_write_kernel(const __grid_constant__ PeerSrc src, int src_tokens, int
                         int roll_dst, int roll_shift, int rope_tok0) {
     constexpr int kVecPerRow = kHeadDim / 8;  // 16
     constexpr int kLanes = 32 * kWarps;       // lanes per item
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red_s[kLayoutThreads / 32];
     const int warp = threadIdx.x >> 5;
     const int l = threadIdx.x & (kLanes - 1);                   // lane within the item's group
@@ -253,16 +255,15 @@ int rope_cache_write_impl(const PeerSrc& src, bool have_q, int src_tokens, int s
     if (B > 65535) return SFM_ERR_BAD_SHAPE;
     LaunchScope scope(kClsLayout, (cudaStream_t)stream);
     auto go = [&](auto kernel) {
-        kernel<<<grid, kLayoutThreads, 0, (cudaStream_t)stream>>>(
-            src, src_tokens, src_heads, head0, (uint4*)q_out, (uint4*)k_cache, (uint4*)v_cache, cache_batch_stride / 8,
-            (const float2*)rope, B, n_new, H, start_idx, blk, start_frame, monarch_order, p0, p1,
-            (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, eps, roll_dst, roll_shift, rope_tok0 < 0 ? 0 : rope_tok0);
+        return launch_pdl(true, kernel, grid, kLayoutThreads, 0, (cudaStream_t)stream, src, src_tokens, src_heads, head0,
+                          (uint4*)q_out, (uint4*)k_cache, (uint4*)v_cache, cache_batch_stride / 8, (const float2*)rope, B, n_new,
+                          H, start_idx, blk, start_frame, monarch_order, p0, p1, (const __nv_bfloat16*)wq,
+                          (const __nv_bfloat16*)wk, eps, roll_dst, roll_shift, rope_tok0 < 0 ? 0 : rope_tok0);
     };
-    if (!in_regs) go(rope_cache_write_kernel<4, false>);
-    else if (warps == 1) go(rope_cache_write_kernel<1, true>);
-    else if (warps == 2) go(rope_cache_write_kernel<2, true>);
-    else go(rope_cache_write_kernel<4, true>);
-    return (int)cudaGetLastError();
+    if (!in_regs) return go(rope_cache_write_kernel<4, false>);
+    if (warps == 1) return go(rope_cache_write_kernel<1, true>);
+    if (warps == 2) return go(rope_cache_write_kernel<2, true>);
+    return go(rope_cache_write_kernel<4, true>);
 }
 }  // namespace
 

@@ -110,6 +110,8 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    pdl_trigger();
+    pdl_wait();
 
     auto fail = [&](int code) {
         bars->abort_flag = 1;
@@ -300,8 +302,7 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel) -> int {
         if (int rc = opt_in_smem((const void*)kernel, kItSmemBytes)) return rc;
-        kernel<<<grid, kThreadsIt, kItSmemBytes, s>>>(map_al, *map_qrows, ip);
-        return 0;
+        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, kItSmemBytes, s, map_al, *map_qrows, ip);
     };
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {

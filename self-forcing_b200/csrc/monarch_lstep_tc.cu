@@ -174,6 +174,8 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
 
     auto fail = [&](int code) {
         bars->abort_flag = 1;
@@ -551,7 +553,11 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     LTcParams lp;
     lp.mp = p;
     lp.n_units = p.nbh * p.na * p.blk.b2;
+    // as many units per group as the tile holds, but no more than it takes to give every SM one: the units of a group
+    // follow one another through the MMA pipe and the rings (two heads on a 6 x 8 grid: 18 -> 11 us)
+    const int share = (lp.n_units + num_sms - 1) / num_sms;
     lp.U = 128 / p.blk.b1 < kMaxU ? 128 / p.blk.b1 : kMaxU;
+    if (lp.U > share) lp.U = share;
     lp.R = 128 / lp.U;
     lp.kt = l_tile_keys(p.n_keys);
     // A value tile stays until its softmax and GEMM are done, a key tile only until its GEMM: two slots of five for keys
@@ -570,8 +576,8 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     dim3 grid(n_groups < num_sms ? n_groups : num_sms);
     auto kernel = p.causal_groups > 0 ? monarch_l_tc_kernel<true> : monarch_l_tc_kernel<false>;
     if (int rc = opt_in_smem((const void*)kernel, kSmemBytes)) return rc;
-    kernel<<<grid, kThreads, kSmemBytes, s>>>(maps[0], maps[1], *map_qrows, lp);
-    return (int)cudaGetLastError();
+    const bool is_short = (long long)n_groups * ((p.n_keys + lp.kt - 1) / lp.kt) <= 16ll * num_sms;
+    return launch_pdl(is_short, kernel, grid, kThreads, kSmemBytes, s, maps[0], maps[1], *map_qrows, lp);
 }
 
 }  // namespace sfm

@@ -170,6 +170,8 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         bars->abort_flag = 1;
         atomicCAS(rp.status, 0, code);
     };
+    pdl_trigger();
+    pdl_wait();
     // no wait can run out before block 0 has started
     if (rp.clear_status && blockIdx.x == 0 && tid == 0) *rp.status = 0;
     const int u_first = blockIdx.x, u_stride = gridDim.x;
@@ -564,13 +566,13 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     rp.tiles = (p.na + rp.groups_per_tile - 1) / rp.groups_per_tile;
     {
         // Persistent CTAs take whole units round-robin, so the launch lasts (units per CTA, rounded up) x (steps per
-        // unit).  Pick the split of the F loop that makes that smallest, with at least three steps per unit (every unit
-        // reloads its query tile) and an extra step's worth charged per unit for that reload.
+        // unit).  Pick the split of the F loop that makes that smallest, with one and a half steps charged per unit for the
+        // reload of its query tile.
         long long best = -1;
-        for (int fs = 1; fs <= (p.F / 3 > 1 ? p.F / 3 : 1); ++fs) {
+        for (int fs = 1; fs <= p.F; ++fs) {
             const int per = (p.F + fs - 1) / fs, splits = (p.F + per - 1) / per;
             const long long units = (long long)p.nbh * rp.tiles * p.blk.b1 * splits;
-            const long long cost = ((units + num_sms - 1) / num_sms) * (per + 1);
+            const long long cost = ((units + num_sms - 1) / num_sms) * (2 * per + 3);
             if (best < 0 || cost < best) { best = cost; rp.f_per = per; rp.fsplit = splits; }
         }
     }
@@ -588,8 +590,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
         if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, rp.rows_per_group < 32 ? rp.rows_per_group : 32, 1)) return rc;
     auto go = [&](auto kernel) -> int {
         if (int rc = opt_in_smem((const void*)kernel, smem_bytes)) return rc;
-        kernel<<<grid, kThreads, smem_bytes, s>>>(maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
-        return 0;
+        return launch_pdl(rp.n_units * rp.f_per <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
     };
     int rc;
     const bool causal = p.causal_groups > 0;

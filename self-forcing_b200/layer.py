@@ -140,7 +140,7 @@ def self_attention_kv(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: 
     norm_q / norm_k when the two weights are given).  ``grid`` = (frames, height, width) of the chunk
     in tokens.  Updates ``cache`` in place and returns the attention output [B, n, H, 128], the
     tensor the reference flattens and feeds to ``self.o`` (causal_model.py:1105-1107)."""
-    frames, gh, gw = (int(x) for x in grid)
+    frames, gh, gw = map(int, grid)
     B, n, H, D = q.shape
     frame_tokens = gh * gw
     if n != frames * frame_tokens:

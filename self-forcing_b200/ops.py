@@ -43,6 +43,14 @@ def _require(t: torch.Tensor, name: str) -> None:
         raise ValueError(f"{name} must be [B, N, H, 128], got {tuple(t.shape)}")
 
 
+_BF16 = torch.bfloat16
+
+
+def _good(t) -> bool:
+    """What _require asks for, without saying what is wrong."""
+    return isinstance(t, torch.Tensor) and t.dtype is _BF16 and t.is_cuda and t.dim() == 4 and t.shape[3] == 128
+
+
 def _token_major(t: torch.Tensor) -> bool:
     """[B, N, H, D] with dense (N, H, D) strides; the batch stride is free."""
     _, n, h, d = t.shape
@@ -54,7 +62,8 @@ def _as_token_major(t: torch.Tensor) -> torch.Tensor:
 
 
 def _batch_stride(t: torch.Tensor) -> int:
-    return t.stride(0) if t.shape[0] > 1 else t.shape[1] * t.shape[2] * t.shape[3]
+    shape = t.shape
+    return t.stride(0) if shape[0] > 1 else shape[1] * shape[2] * shape[3]
 
 
 _MAX_WORKSPACES = 8
@@ -128,7 +137,7 @@ def _rope_table_from_freqs(freqs: Optional[torch.Tensor], device: torch.device) 
     """Device table [1024, 64, 2] fp32 = (cos, sin).  Built from the model's complex128
     ``freqs`` buffer when given (causal_model.py:1352-1357), else by the library."""
     if freqs is None:
-        key = ("lib", device)
+        key = ("lib", device.index)
         tab = _rope_tables.get(key)
         if tab is None:
             host = np.empty((1024, 64, 2), dtype=np.float32)
@@ -172,7 +181,8 @@ def build_maps(n_tokens, f_tied, h_reduce, w_reduce, h, w):
 
 
 def _cache_view_ok(c: torch.Tensor, name: str) -> None:
-    _require(c, name)
+    if not _good(c):
+        _require(c, name)
     if not _token_major(c):
         raise ValueError(f"{name} must keep dense (token, head, dim) strides: it is written in place")
 
@@ -363,8 +373,9 @@ def monarch_attn_with_kv_cache(q, k_cache, v_cache, new_k, new_v, start_idx, end
             raise NotImplementedError("the backward pass exists for num_iters == 1 only")
         return _MonarchWithKVCacheFn.apply(q, new_k, new_v, k_cache, v_cache, start_idx, end_idx,
                                            (f_tied, h_reduce, w_reduce, h, w), sm_scale, grad_only_new_kv)
-    for t, name in ((q, "q"), (new_k, "new_k"), (new_v, "new_v")):
-        _require(t, name)
+    if not (_good(q) and _good(new_k) and _good(new_v)):
+        for t, name in ((q, "q"), (new_k, "new_k"), (new_v, "new_v")):
+            _require(t, name)
     _cache_view_ok(k_cache, "k_cache")
     _cache_view_ok(v_cache, "v_cache")
     if k_cache.stride() != v_cache.stride() or k_cache.shape != v_cache.shape:
@@ -448,14 +459,18 @@ def layer_attention(q, k, v, k_full, v_full, cache_start, n_kv, start_idx, start
     """norm_rope_cache_write followed by attention (Monarch, or dense with the cache in natural order) over the view
     [cache_start, cache_start + n_kv) of the cache tensors ``k_full`` / ``v_full``, in one call of the library.
     ``start_idx`` and ``roll`` are relative to the view."""
-    for t, name in ((q, "q"), (k, "k"), (v, "v")):
-        _require(t, name)
-    _cache_view_ok(k_full, "k_cache")
-    _cache_view_ok(v_full, "v_cache")
-    B, n, H, D = q.shape
-    if k.shape != q.shape or v.shape != q.shape or start_idx < 0 or start_idx + n > n_kv or cache_start + n_kv > k_full.shape[1]:
+    if not (_good(q) and _good(k) and _good(v)):
+        for t, name in ((q, "q"), (k, "k"), (v, "v")):
+            _require(t, name)
+    if not (_good(k_full) and _good(v_full) and k_full.is_contiguous() and v_full.is_contiguous()):
+        _cache_view_ok(k_full, "k_cache")
+        _cache_view_ok(v_full, "v_cache")
+    shape, cache_shape = q.shape, k_full.shape
+    B, n, H, D = shape
+    if k.shape != shape or v.shape != shape or start_idx < 0 or start_idx + n > n_kv or cache_start + n_kv > cache_shape[1]:
         raise ValueError("q, k, v shapes or the cache extent do not match")
-    if k_full.shape != v_full.shape or _batch_stride(k_full) != _batch_stride(v_full) or k_full.shape[0] != B or k_full.shape[2] != H:
+    cache_bs = _batch_stride(k_full)
+    if v_full.shape != cache_shape or _batch_stride(v_full) != cache_bs or cache_shape[0] != B or cache_shape[2] != H:
         raise ValueError("k_cache and v_cache must share shape and strides")
     if (norm_q_weight is None) != (norm_k_weight is None):
         raise ValueError("give both norm weights or neither")
@@ -469,7 +484,7 @@ def layer_attention(q, k, v, k_full, v_full, cache_start, n_kv, start_idx, start
     offset = cache_start * (H * D * 2)
     _mark_written(k_full, v_full)
     return _kv_attention(q.contiguous(), k.contiguous(), v.contiguous(), k_full.data_ptr() + offset, v_full.data_ptr() + offset,
-                         _batch_stride(k_full), n_kv, start_idx, (f_tied, h_reduce, w_reduce, h, w),
+                         cache_bs, n_kv, start_idx, (f_tied, h_reduce, w_reduce, h, w),
                          float(D ** -0.5 if sm_scale is None else sm_scale), num_iters, dense, tab, start_frame, wq, wk, float(eps),
                          dst, shift)
 
