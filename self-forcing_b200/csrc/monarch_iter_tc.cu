@@ -11,10 +11,15 @@
 //   S^T [128 keys x N_I]  = aL_tile [128 x 128] * Q_j^T                    tcgen05.mma, both operands in shared memory
 //   P^T                   = exp(...) per element, bf16, written back over S^T in TMEM; cR = row sums (registers)
 //   aR_tile [128 x 128]   = P^T * Q_j                                      tcgen05.mma, A from TMEM, B = Q_j MN-major
-// N_I = block rows padded to 16.  Warp roles (12 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2-3 idle,
-// 4-7 and 8-11 = two warpgroups that take even / odd tiles: softmax-like pass, then drain of the accumulator and
-// one 256-byte aR row per thread (32-byte stores).  Persistent CTAs take contiguous shares of the unit list; all
-// roles walk the same (unit, tile) sequence and meet through mbarriers with bounded waits.
+// N_I = block rows padded to 16.  Warp roles (16 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), both with an elected
+// issuing lane, 2-3 idle, 4-7 and 8-11 = two warpgroups that take even / odd tiles for the softmax-like pass, 12-15 = drain
+// warpgroup: accumulator -> bf16 -> swizzled staging (two 4 KB buffers per warp) -> TMA store of 32 keys x 64 channels.
+// Persistent CTAs take contiguous shares of the unit list; all roles walk the same (unit, tile) sequence and meet through
+// mbarriers with bounded waits.
+//
+// What bounds it: with 90 keys per unit (first chunk) the chain of a tile, with longer caches the aR rows, 256 bytes per
+// key a whole (query group, column) set apart.  With the working warpgroups storing them themselves, one row per lane, the
+// 19 updates of a 20-pass call took 787 us, now 747.
 #include "monarch_params.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -26,7 +31,7 @@ using namespace tc;
 namespace {
 
 constexpr int kAStg = 3;                  // aL tile ring
-constexpr int kThreadsIt = 384;
+constexpr int kThreadsIt = 512;
 constexpr int kKTile = 128;               // keys per tile
 constexpr uint32_t kTmemColsIt = 512;
 __host__ __device__ constexpr uint32_t it_col_s(int w) { return (uint32_t)w * 128u; }
@@ -44,25 +49,21 @@ struct __align__(16) ItBarriers {
     uint64_t q_full[2], q_empty[2];
     uint64_t a_full[kAStg], a_empty[kAStg];
     uint64_t s_full[2], p_full[2], sp_free[2];
-    uint64_t o_full[2], o_free[2];
+    uint64_t o_full[2], o_free[2];          // accumulator w
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
 constexpr int kItQBytes = 2 * 128 * 128;      // one query tile: two 64-column halves of 128 rows
 constexpr int kItTileBytes = 2 * kKTile * 128;
-constexpr int kItSmemBytes = 1024 + 2 * kItQBytes + kAStg * kItTileBytes + (int)sizeof(ItBarriers) + 64;
+constexpr int kItOutBytes = 4 * 2 * 4096;       // staging of the drain warps
+constexpr int kItSmemBytes = 1024 + 2 * kItQBytes + kAStg * kItTileBytes + kItOutBytes + (int)sizeof(ItBarriers) + 64;
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void st_global_v8_it(void* ptr, const uint32_t (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(ptr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-}
-
 struct ItUnit { int bhl, al, j; };
 __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
     ItUnit r;
@@ -72,15 +73,18 @@ __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
     return r;
 }
 
-// tal = bridge aL map (box 64 x 1 column x 128 keys), tqr = query rows (5-D, box of b1 rows).
+// tal = bridge aL map (box 64 x 1 column x 128 keys), tqr = query rows (5-D, box of b1 rows), tar = state aR
+// [bh][key][query group, column][128] (box 64 x 1 x 32 keys).
 template <int N_I>
 __global__ void __launch_bounds__(kThreadsIt, 1)
-monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap tqr, ItParams ip) {
+monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap tqr,
+                       const __grid_constant__ CUtensorMap tar, ItParams ip) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = base;                                   // two query tiles
     unsigned char* a_s = q_s + 2 * kItQBytes;
-    ItBarriers* bars = reinterpret_cast<ItBarriers*>(a_s + kAStg * kItTileBytes);
+    unsigned char* o_s = a_s + kAStg * kItTileBytes;
+    ItBarriers* bars = reinterpret_cast<ItBarriers*>(o_s + kItOutBytes);
 
     const MonarchParams& p = ip.mp;
     const Blocking& blk = p.blk;
@@ -210,14 +214,13 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                 if (t + 1 == n_tiles) mma_commit_e(el, &bars->q_empty[qb]);       // last read of this unit's query tile
             }
         }
-    } else if (warp >= 4) {
+    } else if (warp >= 4 && warp < 12) {
         // ------------------------------------------------------------------ the two working warpgroups
         const int w = (warp - 4) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                       // TMEM lane == key within the tile
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         const uint32_t s_t = tmem + lane_sel + it_col_s(w);
-        const uint32_t o_t = tmem + lane_sel + it_col_o(w);
         const float scale_l2 = p.scale * kLog2e;
         const int total = (u_end - u_begin) * n_tiles;
         bool ok = true;
@@ -250,35 +253,55 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             tc_fence_before();
             mbar_arrive(&bars->p_full[w]);
 
-            // ---- drain the accumulator: this thread's aR row
-            if (!mbar_wait(&bars->o_full[w], (g >> 1) & 1)) { fail(41); break; }
+            if (valid) {
+                const ItUnit un = it_decode(p, u);
+                p.cR[(((long long)un.bhl * n_keys + key) * p.na + un.al) * b2 + un.j] = csum;
+            }
+        }
+    } else if (warp >= 12) {
+        // ------------------------------------------------------------------ drain warpgroup
+        const uint32_t el = elect_one();
+        const int quad = warp & 3;
+        const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+        unsigned char* const st = o_s + quad * 8192;
+        unsigned char* const st_row = st + lane * 128;
+        const int total = (u_end - u_begin) * n_tiles;
+        for (int g = 0; g < total && !bars->abort_flag; ++g) {
+            const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1;
+            const ItUnit un = it_decode(p, u_begin + uc);
+            const uint32_t o_t = tmem + lane_sel + it_col_o(w);
+            const int key0 = t * kKTile + quad * 32;
+            if (!mbar_wait_u(&bars->o_full[w], (g >> 1) & 1)) { fail(41); break; }
             tc_fence_after();
-            const ItUnit un = it_decode(p, u);
-            const int f = key / b1, k = key - f * b1;
-            const long long ridx = ((((long long)un.bhl * p.F + f) * b1 + k) * p.na + un.al) * b2 + un.j;
-            __nv_bfloat16* dst = p.aR + ridx * kHeadDim;
-#pragma unroll 1
-            for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(o_t + c0, r);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                       // 64 columns at a time
+                uint32_t ra[32], rb[32];
+                tmem_ld32(o_t + h * 64, ra);
+                tmem_ld32(o_t + h * 64 + 32, rb);
                 tmem_wait_ld();
-                if (c0 + 32 == kHeadDim) {
+                if (h == 1) {
                     tc_fence_before();
                     mbar_arrive(&bars->o_free[w]);
                 }
-                if (valid) {
+                if (key0 >= n_keys) continue;                   // keys past the end of the last tile
+                tma_store_wait_read();
+                __syncwarp();
 #pragma unroll
-                    for (int v8 = 0; v8 < 2; ++v8) {
-                        uint32_t wv[8];
+                for (int c = 0; c < 8; ++c) {
+                    const uint32_t (&r)[32] = c < 4 ? ra : rb;
+                    uint32_t wv[4];
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            wv[e] = pack_bf16(__uint_as_float(r[v8 * 16 + 2 * e]), __uint_as_float(r[v8 * 16 + 2 * e + 1]));
-                        st_global_v8_it(dst + c0 + v8 * 16, wv);
-                    }
+                    for (int e = 0; e < 4; ++e)
+                        wv[e] = pack_bf16(__uint_as_float(r[(c & 3) * 8 + 2 * e]), __uint_as_float(r[(c & 3) * 8 + 2 * e + 1]));
+                    *reinterpret_cast<uint4*>(st_row + h * 4096 + ((c ^ (lane & 7)) << 4)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
                 }
+                fence_async_smem();
+                __syncwarp();
+                tma_store_4d_e(el, &tar, st + h * 4096, h * 64, un.al * b2 + un.j, key0, un.bhl);
+                tma_store_commit();
             }
-            if (valid) p.cR[ridx] = csum;
         }
+        tma_store_wait_all();
     }
 
     tc_fence_before();
@@ -297,12 +320,14 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     ip.n_units = p.nbh * p.na * p.blk.b2;
     CUtensorMap map_al;
     if (int rc = make_bridge_tmap(&map_al, p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, 1, kKTile)) return rc;
+    CUtensorMap map_ar;
+    if (int rc = make_bridge_tmap(&map_ar, p.aR, p.na * p.blk.b2, p.n_keys, p.nbh, 1, 32)) return rc;
     ip.q_rows_tma = (p.blk.f_tied == 1 || p.blk.h_reduce == 1) ? 1 : 0;
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel) -> int {
         if (int rc = opt_in_smem((const void*)kernel, kItSmemBytes)) return rc;
-        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, kItSmemBytes, s, map_al, *map_qrows, ip);
+        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, kItSmemBytes, s, map_al, *map_qrows, map_ar, ip);
     };
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {

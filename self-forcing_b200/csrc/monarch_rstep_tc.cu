@@ -106,17 +106,6 @@ constexpr int kSmemData = 224 << 10;                       // query tiles | K / 
 constexpr int kSmemBytes = 1024 + kSmemData + 512;
 static_assert(sizeof(Barriers) <= 512, "barriers follow the tiles");
 
-__device__ __forceinline__ void tma_store_4d_e(uint32_t el, const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3) {
-    asm volatile(
-        "{\n.reg .pred e;\nsetp.ne.b32 e, %6, 0;\n"
-        "@e cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n}"
-        ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(el) : "memory");
-}
-// Bulk-group bookkeeping is per thread: lanes that issued nothing have nothing to commit or wait for.
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // kIter: a pass of the iterative variant after the first one.  The query operand is no longer the chunk's q
 // (one tile per unit) but the state aR[a,f,k,j,:] of the previous pass, which differs for every cached group f:
 // one tile per STEP, loaded through `tq` = a 3-D map of aR ([bh*F*b1][na*b2][128]) into two alternating

@@ -264,6 +264,18 @@ __device__ __forceinline__ void mma_ts_e(uint32_t el, uint32_t d_tmem, uint32_t 
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "r"(el) : "memory");
 }
+// Tiled store shared -> global; the staging rows must have been made visible to the async proxy (fence_async_smem).
+__device__ __forceinline__ void tma_store_4d_e(uint32_t el, const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %6, 0;\n"
+        "@e cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n}"
+        ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(el) : "memory");
+}
+// Bulk-group bookkeeping is per thread: lanes that issued nothing have nothing to commit or wait for.
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// At most one store's staging is still unread: with two buffers in turn, the next one to be filled is free.
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Output-lane mask: bit i of dis[w] set = row 32 w + i of D is not written.
 struct LaneMask { uint32_t dis[4]; };
 // Writes rows [row0, row0 + n) only.
