@@ -361,6 +361,22 @@ int sfm_monarch_bwd(const void* q, int64_t q_batch_stride,
                     int causal_groups, size_t budget_bytes, void* stream);
 
 /*
+ * sfm_monarch_bwd in the form autograd wants it: dq [B, n_q, H, D] bf16 (the fp32 sum, rounded once), dk / dv with their
+ * tokens in natural order.  The group range covers whole tied frame sets (multiples of h_reduce * w_reduce).  Returns
+ * SFM_ERR_UNSUPPORTED, with nothing launched, for the shapes that sfm_monarch_bwd runs on its fp32 kernels.
+ * Replaces: the same, with the inverse permutation of dk / dv and the cast of dq that follow it
+ * (wan/modules/monarch_attn.py:1462-1470).
+ */
+int sfm_monarch_bwd_natural(const void* q, int64_t q_batch_stride,
+                            const void* k_cache, const void* v_cache, int64_t kv_batch_stride,
+                            const void* dout, void* dq, void* dk, void* dv,
+                            void* workspace, size_t workspace_bytes,
+                            int B, int H, int D, int n_q, int n_kv,
+                            int f_tied, int h_reduce, int w_reduce, int h, int w,
+                            float sm_scale, int kv_group_begin, int kv_group_end,
+                            size_t budget_bytes, void* stream);
+
+/*
  * Launch accounting and optional per-kernel timing.  Kernel classes: 0 layout / RoPE /
  * cache write, 1 Monarch row step, 2 Monarch column step, 3 Monarch iteration update,
  * 4 dense attention, 5 Monarch backward (SFM_NUM_KERNEL_CLASSES of them).

@@ -45,8 +45,8 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
                       int* status, int num_sms, cudaStream_t s);
 size_t bwd_row_tc_partial_bytes(const MonarchParams& mp, int g0, int g1);
 int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* dcL, float* dq, float* part_k,
-                      float* part_v, __nv_bfloat16* dk, __nv_bfloat16* dv, int g0, int g1, int* status, int num_sms,
-                      cudaStream_t s);
+                      float* part_v, __nv_bfloat16* dk, __nv_bfloat16* dv, int g0, int g1, __nv_bfloat16* dq_bf16, int natural,
+                      int* status, int num_sms, cudaStream_t s);
 namespace {
 
 using bf16 = __nv_bfloat16;
@@ -742,11 +742,12 @@ extern "C" size_t sfm_monarch_bwd_workspace_bytes(int B, int H, int D, int n_q, 
     return pl.total;
 }
 
-extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
-                               int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
-                               size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
-                               int w_reduce, int h, int w, float sm_scale, int kv_group_begin, int kv_group_end,
-                               int causal_groups, size_t budget_bytes, void* stream) {
+// train: dq is bf16 and the tokens of dk / dv are in natural order; tensor-core path only.
+static int monarch_bwd(bool train, const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
+                       int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
+                       size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
+                       int w_reduce, int h, int w, float sm_scale, int kv_group_begin, int kv_group_end,
+                       int causal_groups, size_t budget_bytes, void* stream) {
     if (!q || !k_cache || !v_cache || !dout || !dq || !workspace) return SFM_ERR_NULL_POINTER;
     BwdPlan pl;
     if (int rc = make_bwd_plan(&pl, B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes)) return rc;
@@ -782,6 +783,9 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
     const char* force_fp32 = getenv("SFM_BWD_FP32");
     const bool use_tc = causal_groups == 0 && blk.b1 <= 96 && blk.b2 <= 64 && (blk.f_tied == 1 || blk.h_reduce == 1) &&
                         !(force_fp32 && force_fp32[0] == '1');
+    const char* row_fp32 = getenv("SFM_BWD_ROW_FP32");          // keeps the fp32 row kernel
+    if (train && (!use_tc || (row_fp32 && row_fp32[0] == '1') || kv_group_begin % blk.gpt || kv_group_end % blk.gpt))
+        return SFM_ERR_UNSUPPORTED;
 
     const int T = blk.b1 <= 16 ? 2 : (blk.b1 <= 32 ? 4 : (blk.b1 <= 64 ? 8 : 16));
     const int LT = blk.b2 <= 64 ? 16 : 32;
@@ -820,6 +824,7 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
             float* delta = (float*)(ws + o); o = up256(o + rows * sizeof(float));
             p.dq2 = (float*)(ws + o); o = up256(o + rows * kHeadDim * sizeof(float));
             if (o > workspace_bytes) return SFM_ERR_WORKSPACE;
+            if (train) p.dq = p.dq2;                          // the fp32 shares stay in the scratch
             MonarchParams mp;
             CUtensorMap maps[8];
             int rc = forward_tc_slice(q, q_batch_stride, k_cache, v_cache, kv_batch_stride, out_s, aLb, Yb, cL, lse, status,
@@ -842,17 +847,17 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
             }
             if ((rc = launch_bwd_col_tc(mp, maps + 4, delta, dcL, p.dq, status, num_sms, s))) return rc;
             p.aLb = aLb; p.Yb = Yb; p.dcL = dcL; p.dcl_pitch = n_keys_c;
-            // Row-step backward on tcgen05 when its per-tile dK / dV partials fit what is left of the workspace;
-            // SFM_BWD_ROW_FP32=1 keeps the fp32 row kernel.
-            const char* row_fp32 = getenv("SFM_BWD_ROW_FP32");
+            // Row-step backward on tcgen05 when its per-tile dK / dV partials fit what is left of the workspace
             const size_t part = up256(bwd_row_tc_partial_bytes(mp, p.g0, p.g1));
             if (!(row_fp32 && row_fp32[0] == '1') && o + 2 * part <= workspace_bytes) {
                 float* part_k = (float*)(ws + o);
                 float* part_v = (float*)(ws + o + part);
-                if ((rc = launch_bwd_row_tc(mp, maps, dcL, p.dq, part_k, part_v, p.dk, p.dv, p.g0, p.g1, status, num_sms, s)))
+                if ((rc = launch_bwd_row_tc(mp, maps, dcL, p.dq, part_k, part_v, p.dk, p.dv, p.g0, p.g1,
+                                            train ? (bf16*)dq : nullptr, train, status, num_sms, s)))
                     return rc;
                 continue;
             }
+            if (train) return SFM_ERR_WORKSPACE;
         } else {
         {
             LaunchScope scope(kClsBackward, s);
@@ -877,4 +882,24 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
         }
     }
     return cudaGetLastError() == cudaSuccess ? SFM_OK : SFM_ERR_UNSUPPORTED;
+}
+
+extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
+                               int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
+                               size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
+                               int w_reduce, int h, int w, float sm_scale, int kv_group_begin, int kv_group_end,
+                               int causal_groups, size_t budget_bytes, void* stream) {
+    return monarch_bwd(false, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
+                       B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, kv_group_begin, kv_group_end,
+                       causal_groups, budget_bytes, stream);
+}
+
+extern "C" int sfm_monarch_bwd_natural(const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
+                                       int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
+                                       size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied,
+                                       int h_reduce, int w_reduce, int h, int w, float sm_scale, int kv_group_begin,
+                                       int kv_group_end, size_t budget_bytes, void* stream) {
+    return monarch_bwd(true, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
+                       B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, kv_group_begin, kv_group_end, 0,
+                       budget_bytes, stream);
 }

@@ -22,6 +22,10 @@
 // Warp roles (12 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2-3 idle, 4-7 = element-wise warpgroup,
 // 8-11 = drain warpgroup (dK / dV per step, dQ per unit).  Every wait is bounded and reports through the status word.
 //
+// The training call takes dq in bf16 and dk / dv with their tokens in natural order from here: cast and permutation as
+// passes of their own over the same rows, and the permutation's table sent from the host (which waits for the GPU) made up
+// 125 of the 1050 us of a call with 4680 queries and 18720 cached tokens.
+//
 // Stands in for the Triton kernel _al_cl_y_bwd (wan/modules/monarch_attn.py:403-596), without its atomic adds.
 #include "monarch_params.cuh"
 #include "profile.cuh"
@@ -42,6 +46,7 @@ struct BwdRowParams {
     MonarchParams mp;              // q, kc, vc, blocking, slice; mp.aL / mp.Y hold daL / dY
     const float* dcL;              // [slab][n_keys_c]
     float* dq;                     // natural order fp32, already holds the column step's share
+    __nv_bfloat16* dq_bf16;        // the sum goes here, rounded, instead of back to dq (null: back to dq)
     float* part_k;                 // [tile][nbh][n_sel tokens][128] fp32 partial dK (n_sel = (g1 - g0) * b1 * b2)
     float* part_v;
     int g0, g1;                    // cached groups whose dK / dV are wanted
@@ -427,7 +432,10 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                         float4 o = *reinterpret_cast<float4*>(dqr + c0 + 4 * v);
                         o.x += __uint_as_float(r[4 * v]); o.y += __uint_as_float(r[4 * v + 1]);
                         o.z += __uint_as_float(r[4 * v + 2]); o.w += __uint_as_float(r[4 * v + 3]);
-                        *reinterpret_cast<float4*>(dqr + c0 + 4 * v) = o;
+                        if (rp.dq_bf16)
+                            *reinterpret_cast<uint2*>(rp.dq_bf16 + (dqr - rp.dq) + c0 + 4 * v) = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
+                        else
+                            *reinterpret_cast<float4*>(dqr + c0 + 4 * v) = o;
                     }
                 }
             }
@@ -439,10 +447,11 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
     if (warp == 1) tmem_dealloc(tmem, kTmemColsRB);
 }
 
-// dk / dv [B, n_sel, H, 128] bf16 (Monarch order) = sum over the tiles' fp32 partials, in tile order.
+// dk / dv [B, n_sel, H, 128] bf16 (Monarch order, or the tokens in natural order) = sum over the tiles' fp32 partials, in tile order.
 __global__ void __launch_bounds__(256) bwd_merge_kv_kernel(const float* __restrict__ part_k, const float* __restrict__ part_v,
                                                            __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                                           int tiles, int nbh, long long n_sel, int H, int bh0) {
+                                                           int tiles, int nbh, long long n_sel, int H, int bh0,
+                                                           Blocking blk, int natural) {
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;          // one float4 of one (bh_local, token)
     const long long per_bh = n_sel * (kHeadDim / 4);
     if (idx >= per_bh * nbh) return;
@@ -459,7 +468,12 @@ __global__ void __launch_bounds__(256) bwd_merge_kv_kernel(const float* __restri
         k.x += a.x; k.y += a.y; k.z += a.z; k.w += a.w;
         v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
     }
-    const long long out = (((long long)b * n_sel + tok) * H + hd) * kHeadDim + c4 * 4;
+    long long tok_out = tok;
+    if (natural) {
+        const int g = (int)tok / (blk.b1 * blk.b2), in_g = (int)tok - g * blk.b1 * blk.b2, r = in_g / blk.b2;
+        tok_out = blk.row_token(g, r) + in_g - r * blk.b2;
+    }
+    const long long out = (((long long)b * n_sel + tok_out) * H + hd) * kHeadDim + c4 * 4;
     *reinterpret_cast<uint2*>(dk + out) = make_uint2(pack_bf16(k.x, k.y), pack_bf16(k.z, k.w));
     *reinterpret_cast<uint2*>(dv + out) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
 }
@@ -475,12 +489,12 @@ size_t bwd_row_tc_partial_bytes(const MonarchParams& mp, int g0, int g1) {
 
 // Row-step backward for one slice.  maps = {q, K, V} (the forward's).
 int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* dcL, float* dq, float* part_k,
-                      float* part_v, __nv_bfloat16* dk, __nv_bfloat16* dv, int g0, int g1, int* status, int num_sms,
-                      cudaStream_t s) {
+                      float* part_v, __nv_bfloat16* dk, __nv_bfloat16* dv, int g0, int g1, __nv_bfloat16* dq_bf16, int natural,
+                      int* status, int num_sms, cudaStream_t s) {
     if (mp.blk.b2 > 64) return SFM_ERR_UNSUPPORTED;
     BwdRowParams rp;
     rp.mp = mp;
-    rp.dcL = dcL; rp.dq = dq; rp.part_k = part_k; rp.part_v = part_v;
+    rp.dcL = dcL; rp.dq = dq; rp.dq_bf16 = dq_bf16; rp.part_k = part_k; rp.part_v = part_v;
     rp.g0 = g0; rp.g1 = g1;
     rp.rows_per_group = (mp.blk.b2 + 7) & ~7;
     rp.groups_per_tile = kRows / rp.rows_per_group;
@@ -515,7 +529,7 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
         const long long n_sel = (long long)(g1 - g0) * mp.blk.b1 * mp.blk.b2;
         const long long n = n_sel * (kHeadDim / 4) * mp.nbh;
         bwd_merge_kv_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(part_k, part_v, dk, dv, rp.tiles, mp.nbh, n_sel, mp.H,
-                                                                       mp.bh0);
+                                                                       mp.bh0, mp.blk, natural);
         if (cudaGetLastError() != cudaSuccess) return SFM_ERR_UNSUPPORTED;
     }
     return SFM_OK;

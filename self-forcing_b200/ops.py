@@ -249,7 +249,7 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
     return out
 
 
-_ERR_WORKSPACE = -5
+_ERR_UNSUPPORTED, _ERR_WORKSPACE = -3, -5
 
 
 def monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h_reduce, w_reduce, h, w, sm_scale=None,
@@ -274,26 +274,66 @@ def monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h
         raise ValueError("grad_out must have q's shape")
     B, n_q, H, D = q.shape
     n_kv = k_cache.shape[1]
-    if sm_scale is None:
-        sm_scale = D ** -0.5
     q = _as_token_major(q)
     grad_out = grad_out.contiguous()
     lib = _lib.load()
-    nbytes = lib.sfm_monarch_bwd_workspace_bytes(B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes)
-    ws = _workspace(q.device, max(int(nbytes), 256), "monarch_bwd")
+    ws = _bwd_workspace(q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes)
     group = (f_tied * h * w) // (h_reduce * w_reduce)
     g0, g1 = (0, n_kv // group) if kv_groups is None else (int(kv_groups[0]), int(kv_groups[1]))
     dq = torch.empty((B, n_q, H, D), dtype=torch.float32, device=q.device)
     dk = torch.empty((B, max(g1 - g0, 0) * group, H, D), dtype=q.dtype, device=q.device)
     dv = torch.empty_like(dk)
-    rc = lib.sfm_monarch_bwd(_ptr(q), _batch_stride(q), _ptr(k_cache), _ptr(v_cache), _batch_stride(k_cache),
-                             _ptr(grad_out), _ptr(dq), _ptr(dk) if dk.numel() else None,
-                             _ptr(dv) if dv.numel() else None, _ptr(ws), ws.numel(), B, H, D, n_q, n_kv, f_tied,
-                             h_reduce, w_reduce, h, w, float(sm_scale), g0, g1, int(causal_groups), budget_bytes,
-                             _stream())
+    rc = lib.sfm_monarch_bwd(q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache),
+                             grad_out.data_ptr(), dq.data_ptr(), dk.data_ptr() if dk.numel() else None,
+                             dv.data_ptr() if dv.numel() else None, ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied,
+                             h_reduce, w_reduce, h, w, float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1,
+                             int(causal_groups), budget_bytes, _raw_stream(q.get_device()))
     _lib.check(rc, "sfm_monarch_bwd")
     _after_call(ws)
     return dq, dk, dv
+
+
+def _bwd_workspace(q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes=0):
+    B, n_q, H, D = q.shape
+    nbytes = _lib.load().sfm_monarch_bwd_workspace_bytes(B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes)
+    return _workspace(q.device, max(int(nbytes), 256), "monarch_bwd")
+
+
+def _backward_natural(q, k_cache, v_cache, grad_out, blocking, sm_scale, g0, g1):
+    """(dq bf16, dk, dv with their tokens in natural order) of the cached groups [g0, g1), or None for shapes the
+    tensor-core backward does not take.  The tensors are those a forward call of this module has accepted."""
+    B, n_q, H, D = q.shape
+    n_kv = k_cache.shape[1]
+    q, grad_out = _as_token_major(q), grad_out.contiguous()
+    ws = _bwd_workspace(q, n_kv, *blocking)
+    f_tied, h_reduce, w_reduce, h, w = blocking
+    dq = torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
+    dk = torch.empty((B, (g1 - g0) * (f_tied * h * w) // (h_reduce * w_reduce), H, D), dtype=q.dtype, device=q.device)
+    dv = torch.empty_like(dk)
+    rc = _lib.load().sfm_monarch_bwd_natural(
+        q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), grad_out.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce,
+        h, w, float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1, 0, _raw_stream(q.get_device()))
+    if rc == _ERR_UNSUPPORTED:
+        return None
+    _lib.check(rc, "sfm_monarch_bwd_natural")
+    _after_call(ws)
+    return dq, dk, dv
+
+
+_nat2mon_index: Dict[tuple, torch.Tensor] = {}
+
+
+def _nat2mon_on_device(n_tokens, blocking, device):
+    """The permutation as an index tensor on the GPU; the last few are kept (a copy from the host waits for the GPU)."""
+    key = (n_tokens, blocking, device.index)
+    idx = _nat2mon_index.get(key)
+    if idx is None:
+        idx = torch.from_numpy(build_maps(n_tokens, *blocking)[0].astype(np.int64)).to(device)
+        while len(_nat2mon_index) >= _MAX_WORKSPACES:
+            _nat2mon_index.pop(next(iter(_nat2mon_index)))
+        _nat2mon_index[key] = idx
+    return idx
 
 
 class _MonarchWithKVCacheFn(torch.autograd.Function):
@@ -319,11 +359,15 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
         n_kv = k_cache.shape[1]
         want_cache = not only_new and (ctx.needs_input_grad[3] or ctx.needs_input_grad[4])
         g0, g1 = (0, n_kv // group) if want_cache else (start // group, -(-end // group))
-        dq, dk, dv = monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out.to(q.dtype), f_tied, h_reduce,
+        grad_out = grad_out.to(q.dtype)
+        if not want_cache and start % (f_tied * h * w) == 0:
+            grads = _backward_natural(q, k_cache, v_cache, grad_out, blocking, sm_scale, g0, g1)
+            if grads is not None:
+                return (*grads, None, None, None, None, None, None, None)
+        dq, dk, dv = monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h_reduce,
                                                          w_reduce, h, w, sm_scale, (g0, g1))
         lo = start - g0 * group
-        nat2mon, _ = build_maps(end - start, f_tied, h_reduce, w_reduce, h, w)
-        idx = torch.from_numpy(nat2mon.astype(np.int64)).to(q.device)
+        idx = _nat2mon_on_device(end - start, blocking, q.device)
         d_new_k = dk[:, lo:lo + end - start].index_select(1, idx)
         d_new_v = dv[:, lo:lo + end - start].index_select(1, idx)
         # The reference hands back the gradient with respect to the cache CONTENT after its in-place write,
@@ -350,8 +394,7 @@ class _MonarchNoCacheFn(torch.autograd.Function):
         blocking, sm_scale, causal_groups = ctx.args
         dq, dk, dv = monarch_attn_with_kv_cache_backward(q, k_mon, v_mon, grad_out.to(q.dtype), *blocking, sm_scale,
                                                          causal_groups=causal_groups)
-        nat2mon, _ = build_maps(k_mon.shape[1], *blocking)
-        idx = torch.from_numpy(nat2mon.astype(np.int64)).to(q.device)
+        idx = _nat2mon_on_device(k_mon.shape[1], blocking, q.device)
         return dq, dk.index_select(1, idx), dv.index_select(1, idx), None, None, None
 
 
