@@ -72,7 +72,7 @@ _MAX_WORKSPACES = 8
 def _workspace(device: torch.device, nbytes: int, tag: str = "monarch") -> torch.Tensor:
     """Scratch for the row-step results, cached per (GPU, stream, kind): calls queued on one stream run in
     order and may share it, calls on different streams may overlap and must not.  A buffer only grows (up to
-    the bridge budget, 1 GiB by default, plus the call's fixed part); at most _MAX_WORKSPACES buffers are kept,
+    the bridge budget, 4 GiB by default, plus the call's fixed part); at most _MAX_WORKSPACES buffers are kept,
     the least recently used one is dropped beyond that (a buffer was allocated on the stream that uses it, so
     PyTorch's allocator hands its memory out again in that stream's order only), and release_workspaces()
     drops them all."""
