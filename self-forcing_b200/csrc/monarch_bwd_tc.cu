@@ -19,10 +19,16 @@
 // dY and daL accumulate over the chunks of a tile in TMEM, dq^T has 32 columns per chunk and accumulates over the
 // tiles.  dY and daL are written over Y and aL in place (a tile is in shared memory before its rows are overwritten).
 //
-// Warp roles (12 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2-3 idle, 4-7 and 8-11 = two warpgroups
-// that take even / odd (tile, chunk) steps (element-wise pass; the group that had a tile's last chunk then drains
-// the dY / daL accumulators and adds up dcL, and after a slab's last tile stores its dq).  Persistent CTAs over contiguous shares of the slab list.
-// All waits are bounded and report through the status word.
+// Warp roles (16 warps): 0 = aL / Y tiles, 1 = MMA issuer (owns TMEM), 2 = query side, 3 idle, 4-7 and 8-11 = two warpgroups that take even
+// / odd (tile, chunk) steps (element-wise pass), 12-15 = drain warpgroup: a tile's dY / daL, rounded, into the shared memory of
+// its Y / aL tile, which nothing reads any more, and from there by TMA store over Y / aL; dcL; after a slab's last tile its
+// dq.  The issuer takes the next step's S GEMMs before this step's gradient GEMMs only if that tile is already there: the tile
+// ring has two stages, and a stage is free again when its tile's results have left it.  Persistent CTAs over contiguous shares
+// of the slab list.  All waits are bounded and report through the status word.
+//
+// What bounds it: the bridge, read and written (378 + 318 MB at 4680 queries, 18720 cached tokens, 12 heads).  With the results
+// stored one 256-byte row per lane by the element-wise warpgroups, between two of their steps, and one warp loading tiles and
+// query side, where a slab's log-sum-exps held up its tiles, it took 236 us, now 142 (4.9 TB/s); with the drain warpgroup alone, 205.
 //
 // Stands in for the Triton kernel _z_bwd and its preprocess (wan/modules/monarch_attn.py:852-886, 1034-1222).
 #include <algorithm>
@@ -38,7 +44,7 @@ using namespace tc;
 namespace {
 
 constexpr int kStgB = 2;                     // (aL, Y) tile-pair ring
-constexpr int kThreadsB = 384;
+constexpr int kThreadsB = 512;
 constexpr int kKB = 128;                     // keys per tile
 constexpr int kNI = 32;                      // query rows per chunk
 constexpr int kMaxNC = 3;                    // chunks per slab: block rows up to 96
@@ -49,12 +55,8 @@ __host__ __device__ constexpr uint32_t bc_dp(int w) { return (uint32_t)w * 64u +
 constexpr uint32_t kColDaL = 128, kColDY = 256, kColDq = 384;
 
 struct BwdColParams {
-    const __nv_bfloat16* q;        // natural order [B, n_q, H, 128]
-    long long q_bs;
     const float* delta;            // [B, n_q, H]: dOut . out per token and head
     const float* lse;              // [slab][b1]
-    __nv_bfloat16* aL;             // bridge [group][n_keys][column][128]: aL in, daL out
-    __nv_bfloat16* Y;              // bridge: Y in, dY out
     const float* cL;               // [slab][n_keys_c]
     float* dcL;                    // [slab][n_keys_c]
     float* dq;                     // natural order [B, n_q, H, 128] fp32
@@ -77,11 +79,11 @@ constexpr int kDsTile = kKB * 128;                 // (scale dS)^T copy: 128 key
 struct __align__(16) BBarriers {
     float lse2[2][kMaxNC * kNI];
     float delta[2][kMaxNC * kNI];
-    float dsum[2][kMaxNC][kKB];             // [tile parity][chunk][key]: -dcL shares of the chunks
+    float dsum[4][kMaxNC][kKB];             // [tile & 3][chunk][key]: -dcL shares of the chunks
     uint64_t q_full[2], q_empty[2];
     uint64_t a_full[kStgB], a_empty[kStgB];
     uint64_t s_full[2], p_full[2], sd_free[2];
-    uint64_t acc_full[2], acc_free[2];      // per warpgroup: a parity wait may lag its barrier by one phase only
+    uint64_t acc_full, acc_free;
     uint64_t dq_full, dq_free;
     uint32_t tmem_base;
     volatile int abort_flag;
@@ -94,11 +96,6 @@ __host__ __device__ constexpr int b_smem_bytes(int nc) {
 }
 
 __device__ __forceinline__ void tmem_st16b(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
-__device__ __forceinline__ void stg_v8(void* ptr, const uint32_t (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(ptr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-}
-
 struct BUnit { int bhl, a, j; };
 __device__ __forceinline__ BUnit b_decode(const BwdColParams& p, int u) {
     BUnit r;
@@ -108,10 +105,11 @@ __device__ __forceinline__ BUnit b_decode(const BwdColParams& p, int u) {
     return r;
 }
 
-// tal / ty = bridge maps (box 64 x 1 column x 128 keys); tqr / tdo = query rows of q / dOut (5-D, box of 32 rows).
+// tal / ty = bridge maps (box 64 x 1 column x 128 keys), sal / sy the same with boxes of 32 keys; tqr / tdo = query rows of q / dOut (5-D, box of 32 rows).
 template <int NC>
 __global__ void __launch_bounds__(kThreadsB, 1)
 monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap ty,
+                          const __grid_constant__ CUtensorMap sal, const __grid_constant__ CUtensorMap sy,
                           const __grid_constant__ CUtensorMap tqr, const __grid_constant__ CUtensorMap tdo,
                           BwdColParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -133,11 +131,11 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
 
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
-        for (int s = 0; s < kStgB; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1); }
+        for (int s = 0; s < kStgB; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 4); }
         for (int w = 0; w < 2; ++w) {
             mbar_init(&bars->s_full[w], 1); mbar_init(&bars->p_full[w], 128); mbar_init(&bars->sd_free[w], 1);
         }
-        for (int w = 0; w < 2; ++w) { mbar_init(&bars->acc_full[w], 1); mbar_init(&bars->acc_free[w], 128); }
+        mbar_init(&bars->acc_full, 1); mbar_init(&bars->acc_free, 128);
         mbar_init(&bars->dq_full, 1); mbar_init(&bars->dq_free, 128);
         bars->abort_flag = 0;
         mbar_init_fence();
@@ -158,60 +156,63 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
     };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ producer
+        // ------------------------------------------------------------------ tile loads
         const uint32_t el = elect_one();
-        prefetch_tmap(&tal); prefetch_tmap(&ty); prefetch_tmap(&tqr); prefetch_tmap(&tdo);
-        int g = 0, uc = 0;                                       // tiles loaded, slabs started
+        prefetch_tmap(&tal); prefetch_tmap(&ty); prefetch_tmap(&sal); prefetch_tmap(&sy);
+        int g = 0;                                               // tiles loaded
         bool ok = true;
-        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u, ++uc) {
+        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
+            const BUnit un = b_decode(p, u);
+            const int grp = un.bhl * p.A + un.a;
+            for (int t = 0; t < n_tiles; ++t, ++g) {
+                const int s = g % kStgB;
+                if (g >= kStgB && !mbar_wait_u(&bars->a_empty[s], ((g / kStgB) - 1) & 1)) { fail(11); ok = false; break; }
+                unsigned char* st = a_s + s * kBStage;
+                mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kBStage);
+                tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                tma_load_4d_e(el, st + kKB * 128, &tal, &bars->a_full[s], 64, un.j, t * kKB, grp);
+                tma_load_4d_e(el, st + kBTile, &ty, &bars->a_full[s], 0, un.j, t * kKB, grp);
+                tma_load_4d_e(el, st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, un.j, t * kKB, grp);
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ query side: rows of q and dOut, lse, delta
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tqr); prefetch_tmap(&tdo);
+        int uc = 0;                                              // slabs started
+        for (int u = u_begin; u < u_end && !bars->abort_flag; ++u, ++uc) {
             const BUnit un = b_decode(p, u);
             const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-            const int grp = un.bhl * p.A + un.a;
             const int qb = kQBufs == 2 ? (uc & 1) : 0;
             unsigned char* qt = qd_s + qb * kQdBuf;
-            auto load_tiles = [&](int t_begin, int t_end) {
-                for (int t = t_begin; t < t_end; ++t, ++g) {
-                    const int s = g % kStgB;
-                    if (g >= kStgB && !mbar_wait_u(&bars->a_empty[s], ((g / kStgB) - 1) & 1)) { fail(11); ok = false; break; }
-                    unsigned char* st = a_s + s * kBStage;
-                    mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kBStage);
-                    tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKB, grp);
-                    tma_load_4d_e(el, st + kKB * 128, &tal, &bars->a_full[s], 64, un.j, t * kKB, grp);
-                    tma_load_4d_e(el, st + kBTile, &ty, &bars->a_full[s], 0, un.j, t * kKB, grp);
-                    tma_load_4d_e(el, st + kBTile + kKB * 128, &ty, &bars->a_full[s], 64, un.j, t * kKB, grp);
-                }
-            };
-            // the slab's first tile does not wait for the query-side buffer
-            load_tiles(0, 1);
-            if (!ok) break;
-            if (uc >= kQBufs) {
-                if (!mbar_wait_u(&bars->q_empty[qb], ((uc / kQBufs) - 1) & 1)) { fail(10); break; }
-            }
-            for (int i = lane; i < NC * kNI; i += 32) {
-                float l2 = INFINITY, dl = 0.f;
+            const int tok0 = blk.row_token(un.a, 0) + un.j;      // the slab's rows are consecutive rows of the token grid
+            float l2[NC], dl[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int i = c * kNI + lane;
+                l2[c] = INFINITY; dl[c] = 0.f;
                 if (i < b1) {
-                    const long long tok = blk.row_token(un.a, i) + un.j;
-                    l2 = kLog2e * p.lse[(long long)u * b1 + i];
-                    dl = p.delta[((long long)b * p.n_q + tok) * p.H + hd];
+                    l2[c] = kLog2e * p.lse[(long long)u * b1 + i];
+                    dl[c] = p.delta[((long long)b * p.n_q + tok0 + i * blk.w) * p.H + hd];
                 }
-                bars->lse2[qb][i] = l2;
-                bars->delta[qb][i] = dl;
+            }
+            if (uc >= kQBufs && !mbar_wait_u(&bars->q_empty[qb], ((uc / kQBufs) - 1) & 1)) { fail(10); break; }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                bars->lse2[qb][c * kNI + lane] = l2[c];
+                bars->delta[qb][c * kNI + lane] = dl[c];
             }
             __syncwarp();
-            {
-                // 32 consecutive rows of the token grid per chunk; rows past the slab's b1 hold other tokens (or the
-                // fill value) and are masked by an infinite log-sum-exp
-                mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(NC * 4 * p.q_box_rows * 128));
-                const int tok0 = blk.row_token(un.a, 0);
-                const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
-                for (int c = 0; c < NC; ++c) {
-                    unsigned char* dq_ = qt + c * kQdBuf;
-                    tma_load_5d_e(el, dq_, &tqr, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d_e(el, dq_ + kQdHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d_e(el, dq_ + kQdTile, &tdo, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
-                    tma_load_5d_e(el, dq_ + kQdTile + kQdHalf, &tdo, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
-                }
-                load_tiles(1, n_tiles);
+            // 32 consecutive rows of the token grid per chunk; rows past the slab's b1 hold other tokens (or the
+            // fill value) and are masked by an infinite log-sum-exp
+            mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(NC * 4 * p.q_box_rows * 128));
+            const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w;
+            for (int c = 0; c < NC; ++c) {
+                unsigned char* dq_ = qt + c * kQdBuf;
+                tma_load_5d_e(el, dq_, &tqr, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
+                tma_load_5d_e(el, dq_ + kQdHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
+                tma_load_5d_e(el, dq_ + kQdTile, &tdo, &bars->q_full[qb], 0, hd, col, frow0 + c * kNI, b);
+                tma_load_5d_e(el, dq_ + kQdTile + kQdHalf, &tdo, &bars->q_full[qb], 64, hd, col, frow0 + c * kNI, b);
             }
         }
     } else if (warp == 1) {
@@ -255,21 +256,28 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 mma_commit_e(el, &bars->s_full[w]);
                 return true;
             };
-            int drains[2] = {0, 0};               // accumulator hand-overs to each warpgroup so far
-            int last_drainer = 0;
+            // the tile (and, at a slab's start, the query rows) of step g have arrived
+            auto ready = [&](int g) -> bool {
+                const int gt = g / NC, c = g - gt * NC;
+                const int uc = gt / n_tiles, t = gt - uc * n_tiles, s = gt % kStgB;
+                if (c != 0) return true;
+                return mbar_test_u(&bars->a_full[s], (gt / kStgB) & 1) &&
+                       (t != 0 || mbar_test_u(&bars->q_full[kQBufs == 2 ? (uc & 1) : 0], (uc / kQBufs) & 1));
+            };
             if (total > 0) ok = issue_s(0);
             for (int g = 0; ok && g < total && !bars->abort_flag; ++g) {
                 // The S GEMMs of the next step are issued ahead of this step's, except across a slab boundary when the
                 // query-side rows are single buffered: the next slab's rows can only load once this slab's last
                 // GEMMs have released the buffer, so waiting for them here would never end.
-                const bool ahead = g + 1 < total && !(kQBufs == 1 && (g + 1) % (n_tiles * NC) == 0);
+                // Nor when the next tile is not there yet: it may be waiting for a stage that this step's tile follows.
+                const bool ahead = g + 1 < total && !(kQBufs == 1 && (g + 1) % (n_tiles * NC) == 0) && ready(g + 1);
                 if (ahead && !issue_s(g + 1)) { ok = false; break; }
                 const int gt = g / NC, c = g - gt * NC;
                 const int uc = gt / n_tiles, t = gt - uc * n_tiles, w = g & 1, s = gt % kStgB;
                 const int qb = kQBufs == 2 ? (uc & 1) : 0;
                 if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
                 // the accumulators are shared by all tiles: the previous tile's must have been drained
-                if (c == 0 && gt >= 1 && !mbar_wait_u(&bars->acc_free[last_drainer], (drains[last_drainer] - 1) & 1)) { fail(24); break; }
+                if (c == 0 && gt >= 1 && !mbar_wait_u(&bars->acc_free, (gt - 1) & 1)) { fail(24); break; }
                 if (t == 0 && c == 0 && uc >= 1 && !mbar_wait_u(&bars->dq_free, (uc - 1) & 1)) { fail(25); break; }
                 tc_fence_after();
                 const uint64_t qn = q_mn0 + (uint64_t)(((qb + c) * kQdBuf) >> 4);
@@ -287,34 +295,31 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
 #pragma unroll
                 for (int kk = 0; kk < kKB / 16; ++kk)
                     mma_ss_e(el, tmem + kColDq + c * kNI, am + ((kk * 2048) >> 4), dsd + ((kk * 2048) >> 4), idesc_q, (t > 0 || kk > 0) ? 1u : 0u);
-                if (c == NC - 1) {
-                    mma_commit_e(el, &bars->acc_full[w]);
-                    ++drains[w];
-                    last_drainer = w;
-                    mma_commit_e(el, &bars->a_empty[s]);
-                }
+                if (c == NC - 1) mma_commit_e(el, &bars->acc_full);
                 mma_commit_e(el, &bars->sd_free[w]);
                 if (t + 1 == n_tiles && c == NC - 1) { mma_commit_e(el, &bars->dq_full); mma_commit_e(el, &bars->q_empty[qb]); }
                 if (g + 1 < total && !ahead && !issue_s(g + 1)) { ok = false; break; }
             }
         }
-    } else if (warp >= 4) {
+    } else if (warp >= 4 && warp < 12) {
         // ------------------------------------------------------------------ the two working warpgroups
         const int w = (warp - 4) >> 2;
         const int quad = warp & 3;
-        const int row = quad * 32 + lane;                       // TMEM lane: key within the tile (d for the dq drain)
+        const int row = quad * 32 + lane;                       // TMEM lane: key within the tile
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         const float scale_l2 = p.scale * kLog2e;
         unsigned char* ds_row = ds_s + w * kDsTile + row * 128;
-        int my_drains = 0;
+        auto load_cl = [&](int g) -> float {                    // step g's bias of this thread's key
+            const int gt = g / NC, uc = gt / n_tiles, key = (gt - uc * n_tiles) * kKB + row;
+            return g < total && key < n_keys ? kLog2e * p.cL[(long long)(u_begin + uc) * p.n_keys_c + key] : INFINITY;
+        };
+        float cl_next = load_cl(w);
         for (int g = w; g < total && !bars->abort_flag; g += 2) {
             const int gt = g / NC, c = g - gt * NC;
-            const int uc = gt / n_tiles, t = gt - uc * n_tiles;
+            const int uc = gt / n_tiles;
             const int qb = kQBufs == 2 ? (uc & 1) : 0;
-            const int u = u_begin + uc;
-            const int key = t * kKB + row;
-            const bool valid = key < n_keys;
-            const float cl2 = valid ? kLog2e * p.cL[(long long)u * p.n_keys_c + key] : INFINITY;
+            const float cl2 = cl_next;
+            cl_next = load_cl(g + 2);
             if (!mbar_wait(&bars->s_full[w], (g >> 1) & 1)) { fail(31); break; }
             tc_fence_after();
             uint32_t rs[kNI], rd[kNI];
@@ -341,74 +346,88 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
                 *reinterpret_cast<uint4*>(ds_row + ((cc ^ (row & 7)) << 4)) = make_uint4(pd[4 * cc], pd[4 * cc + 1], pd[4 * cc + 2], pd[4 * cc + 3]);
-            bars->dsum[gt & 1][c][row] = dsum;
+            bars->dsum[gt & 3][c][row] = dsum;
             fence_async_smem();
             tmem_wait_st();
             tc_fence_before();
             mbar_arrive(&bars->p_full[w]);
-            if (c != NC - 1) continue;
-
-            // ---- the tile's last chunk: drain dY and daL, one 256-byte row each, written over Y and aL
-            if (!mbar_wait(&bars->acc_full[w], my_drains & 1)) { fail(41); break; }
-            ++my_drains;
+        }
+    } else if (warp >= 12) {
+        // ------------------------------------------------------------------ drain warpgroup
+        const uint32_t el = elect_one();
+        const int quad = warp & 3;
+        const int row = quad * 32 + lane;                       // TMEM lane: key within the tile (d for dq)
+        const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+        const int n_gt = (u_end - u_begin) * n_tiles;
+        for (int gt = 0; gt < n_gt && !bars->abort_flag; ++gt) {
+            const int uc = gt / n_tiles, t = gt - uc * n_tiles, s = gt % kStgB;
+            const int u = u_begin + uc;
+            const BUnit un = b_decode(p, u);
+            const int key0 = t * kKB + quad * 32;
+            if (!mbar_wait_u(&bars->acc_full, gt & 1)) { fail(41); break; }
             tc_fence_after();
-            if (valid) {
+            if (key0 + lane < n_keys) {
                 float acc = 0.f;                     // the chunks' shares in a fixed order
 #pragma unroll
-                for (int cc = 0; cc < NC; ++cc) acc += bars->dsum[gt & 1][cc][row];
-                p.dcL[(long long)u * p.n_keys_c + key] = -acc;
+                for (int cc = 0; cc < NC; ++cc) acc += bars->dsum[gt & 3][cc][row];
+                p.dcL[(long long)u * p.n_keys_c + key0 + lane] = -acc;
             }
-            const BUnit un = b_decode(p, u);
-            const long long ro = ((((long long)un.bhl * p.A + un.a) * n_keys + key) * blk.b2 + un.j) * kHeadDim;
+            // this warp's 32 keys, 64 columns at a time: daL over the aL tile, dY over the Y tile
 #pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                __nv_bfloat16* dst = (half ? p.Y : p.aL) + ro;
-                const uint32_t col0 = half ? kColDY : kColDaL;
-#pragma unroll 1
-                for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem + lane_sel + col0 + c0, r);
-                    tmem_wait_ld();
-                    if (half == 1 && c0 + 32 == kHeadDim) {
-                        tc_fence_before();
-                        mbar_arrive(&bars->acc_free[w]);
-                    }
-                    if (valid) {
-#pragma unroll
-                        for (int v8 = 0; v8 < 2; ++v8) {
-                            uint32_t wv[8];
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                wv[e] = pack_bf16(__uint_as_float(r[v8 * 16 + 2 * e]), __uint_as_float(r[v8 * 16 + 2 * e + 1]));
-                            stg_v8(dst + c0 + v8 * 16, wv);
-                        }
-                    }
+            for (int h = 0; h < 4; ++h) {
+                unsigned char* const st = a_s + s * kBStage + h * (kKB * 128) + quad * 4096;
+                uint32_t ra[32], rb[32];
+                const uint32_t col0 = (h < 2 ? kColDaL : kColDY) + (h & 1) * 64;
+                tmem_ld32(tmem + lane_sel + col0, ra);
+                tmem_ld32(tmem + lane_sel + col0 + 32, rb);
+                tmem_wait_ld();
+                if (h == 3) {
+                    tc_fence_before();
+                    mbar_arrive(&bars->acc_free);
                 }
+                if (key0 >= n_keys) continue;        // keys past the end of the last tile
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint32_t (&r)[32] = c < 4 ? ra : rb;
+                    uint32_t wv[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        wv[e] = pack_bf16(__uint_as_float(r[(c & 3) * 8 + 2 * e]), __uint_as_float(r[(c & 3) * 8 + 2 * e + 1]));
+                    *reinterpret_cast<uint4*>(st + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+                }
+                fence_async_smem();
+                __syncwarp();
+                tma_store_4d_e(el, h < 2 ? &sal : &sy, st, (h & 1) * 64, un.j, key0, un.bhl * p.A + un.a);
+                tma_store_commit();
             }
+            tma_store_wait_read_all();
+            __syncwarp();
+            if (el) mbar_arrive(&bars->a_empty[s]);
             // ---- last tile of the slab: its dq (TMEM lane = d, column = query row)
             if (t + 1 == n_tiles) {
-                if (!mbar_wait(&bars->dq_full, uc & 1)) { fail(42); break; }
+                if (!mbar_wait_u(&bars->dq_full, uc & 1)) { fail(42); break; }
                 tc_fence_after();
-                uint32_t r[NC][kNI];
-#pragma unroll
-                for (int cc = 0; cc < NC; ++cc) tmem_ld32(tmem + lane_sel + kColDq + cc * kNI, r[cc]);
-                tmem_wait_ld();
-                tc_fence_before();
-                mbar_arrive(&bars->dq_free);
                 const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-#pragma unroll
+                const long long pitch = (long long)blk.w * p.H * kHeadDim;
+                float* const dq0 = p.dq + (((long long)b * p.n_q + blk.row_token(un.a, 0) + un.j) * p.H + hd) * kHeadDim + row;
+#pragma unroll 1
                 for (int cc = 0; cc < NC; ++cc) {
+                    uint32_t r[kNI];
+                    tmem_ld32(tmem + lane_sel + kColDq + cc * kNI, r);
+                    tmem_wait_ld();
+                    if (cc == NC - 1) {
+                        tc_fence_before();
+                        mbar_arrive(&bars->dq_free);
+                    }
 #pragma unroll
                     for (int ii = 0; ii < kNI; ++ii) {
                         const int i = cc * kNI + ii;
-                        if (i < b1) {
-                            const long long tok = blk.row_token(un.a, i) + un.j;
-                            p.dq[(((long long)b * p.n_q + tok) * p.H + hd) * kHeadDim + row] = __uint_as_float(r[cc][ii]);
-                        }
+                        if (i < b1) dq0[i * pitch] = __uint_as_float(r[ii]);
                     }
                 }
             }
         }
+        tma_store_wait_all();
     }
 
     tc_fence_before();
@@ -448,8 +467,8 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     if (mp.blk.b1 > kMaxNC * kNI) return SFM_ERR_UNSUPPORTED;
     LaunchScope scope(kClsBackward, s);
     BwdColParams p;
-    p.q = mp.q; p.q_bs = mp.q_bs; p.delta = delta; p.lse = mp.lse;
-    p.aL = mp.aL; p.Y = mp.Y; p.cL = mp.cL; p.dcL = dcL; p.dq = dq;
+    p.delta = delta; p.lse = mp.lse;
+    p.cL = mp.cL; p.dcL = dcL; p.dq = dq;
     p.H = mp.H; p.n_q = mp.n_q; p.A = mp.na; p.n_keys = mp.n_keys; p.n_keys_c = mp.n_keys_c;
     p.bh0 = mp.bh0; p.nbh = mp.nbh;
     p.n_units = mp.nbh * mp.na * mp.blk.b2;
@@ -461,12 +480,14 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     p.status = status;
     dim3 grid(p.n_units < num_sms ? p.n_units : num_sms);
     const int nc = (mp.blk.b1 + kNI - 1) / kNI;
-    CUtensorMap bridge[2];
+    CUtensorMap bridge[4];
     if (int rc = make_bridge_tmap(&bridge[0], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
     if (int rc = make_bridge_tmap(&bridge[1], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, kKB)) return rc;
+    if (int rc = make_bridge_tmap(&bridge[2], mp.aL, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, 32)) return rc;
+    if (int rc = make_bridge_tmap(&bridge[3], mp.Y, mp.blk.b2, mp.n_keys, mp.nbh * mp.na, 1, 32)) return rc;
     auto go = [&](auto kernel, int smem) -> int {
         if (int rc = opt_in_smem((const void*)kernel, smem)) return rc;
-        kernel<<<grid, kThreadsB, smem, s>>>(bridge[0], bridge[1], maps[0], maps[1], p);
+        kernel<<<grid, kThreadsB, smem, s>>>(bridge[0], bridge[1], bridge[2], bridge[3], maps[0], maps[1], p);
         return 0;
     };
     int rc = nc == 1 ? go(monarch_bwd_col_tc_kernel<1>, b_smem_bytes(1))

@@ -220,6 +220,13 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (i
 __device__ __forceinline__ bool mbar_wait_u(uint64_t* bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
+// Has the phase completed?  No waiting.
+__device__ __forceinline__ bool mbar_test_u(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, done != 0);
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx_e(uint32_t el, uint64_t* bar, uint32_t bytes) {
     asm volatile("{\n.reg .pred e;\nsetp.ne.b32 e, %2, 0;\n@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}"
                  ::"r"(smem_addr(bar)), "r"(bytes), "r"(el) : "memory");
@@ -275,6 +282,8 @@ __device__ __forceinline__ void tma_store_4d_e(uint32_t el, const CUtensorMap* m
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // At most one store's staging is still unread: with two buffers in turn, the next one to be filled is free.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// No store's staging is still unread.
+__device__ __forceinline__ void tma_store_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Output-lane mask: bit i of dis[w] set = row 32 w + i of D is not written.
 struct LaneMask { uint32_t dis[4]; };
