@@ -9,18 +9,28 @@
 // Units are those of the forward row step: (batch*head, tile of stacked query groups, block row k), each walking
 // all cached groups f; per step
 //   S  = Q_tile K^T                 dR = daL_tile K^T + dY_tile V^T        three tcgen05.mma chains, operands in shared memory
-//   R, dz                           one thread per query row (R recomputed exactly as in the forward)
-//   dQ (+)= (scale dz) K            A = scale dz as bf16 in TMEM, B = the K tile MN-major; accumulates over f in TMEM
+//   R, dz                           two threads per query row, half of the block's columns each (R as in the forward)
+//   dQ (+)= (scale dz) K            A = a bf16 copy of scale dz in shared memory, B = the K tile MN-major; accumulates over f
 //   dK = R^T daL_tile + (scale dz)^T Q_tile,   dV = R^T dY_tile
-//                                   A = bf16 copies of R / scale dz in shared memory read MN-major (M = key l, padded to
-//                                   128 with a block of zeros), B = the row tiles read MN-major; only for the cached
-//                                   groups whose dK / dV are wanted
+//                                   A = bf16 copies of R / scale dz in shared memory read MN-major (M = key l; lanes 64 to
+//                                   127 get what lies behind the copy and are never read), B = the row tiles read
+//                                   MN-major; only for the cached groups whose dK / dV are wanted, which come first where they are the
+//                                   last ones
 // dK / dV of a (f, k) get one contribution per tile of query groups: each tile writes fp32 partials to its own
 // buffer and a small kernel adds them in a fixed order and rounds to bf16 (no atomics).  dQ rows are owned by one
 // unit each and added to what the column step's backward left in dq.
 //
-// Warp roles (12 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2-3 idle, 4-7 = element-wise warpgroup,
-// 8-11 = drain warpgroup (dK / dV per step, dQ per unit).  Every wait is bounded and reports through the status word.
+// Warp roles (16 warps): 0 = K, V, daL and dY tiles, 1 = S and dR GEMMs (owns TMEM), 2 = query tiles, 3 = gradient GEMMs, 4-11 = element-wise
+// pass (warps w and w + 4 share rows), 12-15 = drain warpgroup (dK / dV per step, dQ per unit).  Every wait is bounded and
+// reports through the status word.
+//
+// What bounds it: the chain of a step (S, dR, element-wise pass, dQ), with daL and dY (53 KB a step) read meanwhile: their
+// tiles share a ring of three, so that one and a half steps' are held at a time.  The element-wise pass takes each weight's
+// exponential once and the sums from the expanded form, sum R dR = sum R (daL.K + dY.V) + dcL (sum R ln R + 1).  4680
+// queries, 18720 cached tokens, 12 heads, dK / dV of the last quarter: 286 us with one issuing warp, one thread per row and
+// results stored a row per lane; 234 with two threads per row and S / dR released once read; 215 with the gradient GEMMs
+// issued by a warp of their own (a single issuer waits for the next K tile with this step's results in hand, and that tile
+// for a stage they hold); 177 with the transposed drain.
 //
 // The training call takes dq in bf16 and dk / dv with their tokens in natural order from here: cast and permutation as
 // passes of their own over the same rows, and the permutation's table sent from the host (which waits for the GPU) made up
@@ -37,10 +47,11 @@ using namespace tc;
 
 namespace {
 
-constexpr int kThreadsRB = 384;
+constexpr int kThreadsRB = 512;
 constexpr int kRows = 128;
 constexpr uint32_t kTmemColsRB = 512;
 constexpr uint32_t kCS = 0, kCDR = 64, kCDQ = 128, kCDK = 256, kCDV = 384;
+static_assert(kCDV == kCDK + kHeadDim, "drained together");
 
 struct BwdRowParams {
     MonarchParams mp;              // q, kc, vc, blocking, slice; mp.aL / mp.Y hold daL / dY
@@ -54,20 +65,39 @@ struct BwdRowParams {
     int* status;
 };
 
-struct __align__(8) RBBarriers {
+constexpr int kRowSlots = 3;
+struct __align__(16) RBBarriers {
+    float4 stats[2][2][kRows];                             // [step parity][half][row]: max, sum, sum of e ln e, sum of e dR
     uint64_t q_full, q_empty;
-    uint64_t kv_full[2], kv_empty[2];
-    uint64_t da_full, da_empty;
-    uint64_t s_full, dr_full, p_full, sdr_free;
+    uint64_t k_full[2], k_empty[2], v_full, v_empty;
+    uint64_t rt_full[kRowSlots], rt_empty[kRowSlots];      // daL and dY tiles in turn
+    uint64_t s_full, dr_full, sdr_read, p_full, rz_free;   // S, dR: written, in registers; R, dz copies: written, free
+    uint64_t x_full[4];                                    // the row statistics of the two halves, per lane quadrant
     uint64_t dkv_full, dkv_free, dq_full, dq_free;
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
 constexpr int kQB = 2 * kRows * 128;                 // a row tile: two 64-column halves of 128 rows (32 KB)
-constexpr int kKVStage = 4 * 64 * 128;               // K lo, K hi, V lo, V hi (<= 64 rows each)
+constexpr int kKVTile = 2 * 64 * 128;                // a K or V tile: two 64-column halves of at most 64 rows (16 KB)
 constexpr int kStageT = kRows * 128;                 // R or dz copy: 128 rows x 64 bf16 (16 KB)
-constexpr int kRBSmem = 1024 + kQB + 2 * kKVStage + 2 * kQB + 3 * kStageT + (int)sizeof(RBBarriers) + 64;
+constexpr int kOutStage = 32 * 64;                   // a drain warp's staging: 32 rows of 16 fp32 columns
+constexpr int kRBSmem = 1024 + kQB + 3 * kKVTile + 2 * kStageT + kRowSlots * kQB + 4 * kOutStage + (int)sizeof(RBBarriers) + 64;
+static_assert(kRBSmem <= 227 * 1024, "shared memory");
+
+// N columns, N a multiple of 8 up to 32
+template <int N>
+__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[N]) {
+    if constexpr (N == 32) tmem_ld32(taddr, r);
+    else {
+        if constexpr (N & 16) tmem_ld16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
+        if constexpr (N & 8) tmem_ld8(taddr + (N & 16), *reinterpret_cast<uint32_t(*)[8]>(&r[N & 16]));
+    }
+}
+
+__device__ __forceinline__ void red_add_v4(float* ptr, const float4& v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(ptr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
 
 struct RBUnit { int bhl, tile, k; };
 __device__ __forceinline__ RBUnit rb_decode(const BwdRowParams& rp, int u) {
@@ -87,12 +117,12 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = base;
-    unsigned char* kv_s = q_s + kQB;                       // 2 stages
-    unsigned char* da_s = kv_s + 2 * kKVStage;             // daL tile
-    unsigned char* dy_s = da_s + kQB;                      // dY tile
-    unsigned char* r_s = dy_s + kQB;                       // R copy | dz copy | zeros
+    unsigned char* kv_s = q_s + kQB;                       // two K tiles, one V tile
+    unsigned char* r_s = kv_s + 3 * kKVTile;              // R copy | dz copy
     unsigned char* z_s = r_s + kStageT;
-    RBBarriers* bars = reinterpret_cast<RBBarriers*>(r_s + 3 * kStageT);
+    unsigned char* rt_s = z_s + kStageT;                   // daL / dY tiles
+    unsigned char* o_s = rt_s + kRowSlots * kQB;           // drain staging
+    RBBarriers* bars = reinterpret_cast<RBBarriers*>(o_s + 4 * kOutStage);
 
     const MonarchParams& p = rp.mp;
     const Blocking& blk = p.blk;
@@ -103,18 +133,20 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
     constexpr int kHalf = N_S * 128;
 
     if (tid == 0) {
-        mbar_init(&bars->q_full, 1); mbar_init(&bars->q_empty, 1);
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars->kv_full[s], 1); mbar_init(&bars->kv_empty[s], 1); }
-        mbar_init(&bars->da_full, 1); mbar_init(&bars->da_empty, 1);
-        mbar_init(&bars->s_full, 1); mbar_init(&bars->dr_full, 1); mbar_init(&bars->p_full, 128);
-        mbar_init(&bars->sdr_free, 1);
+        mbar_init(&bars->q_full, 1); mbar_init(&bars->q_empty, 2);
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1); }
+        mbar_init(&bars->v_full, 1); mbar_init(&bars->v_empty, 1);
+        for (int s = 0; s < kRowSlots; ++s) { mbar_init(&bars->rt_full[s], 1); mbar_init(&bars->rt_empty[s], 1); }
+        mbar_init(&bars->s_full, 1); mbar_init(&bars->dr_full, 1); mbar_init(&bars->p_full, 256);
+        mbar_init(&bars->sdr_read, 256); mbar_init(&bars->rz_free, 1);
+        for (int i = 0; i < 4; ++i) mbar_init(&bars->x_full[i], 64);
         mbar_init(&bars->dkv_full, 1); mbar_init(&bars->dkv_free, 128);
         mbar_init(&bars->dq_full, 1); mbar_init(&bars->dq_free, 128);
         bars->abort_flag = 0;
         mbar_init_fence();
     }
     // tile rows no load writes and the padding of the R / dz copies must read as zero
-    for (int i = tid; i < (kQB + 2 * kKVStage + 2 * kQB + 3 * kStageT) / 16; i += kThreadsRB)
+    for (int i = tid; i < (kQB + 3 * kKVTile + 2 * kStageT + kRowSlots * kQB) / 16; i += kThreadsRB)
         reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 1) { tmem_alloc(&bars->tmem_base, kTmemColsRB); tmem_relinquish(); }
     fence_async_smem();
@@ -128,248 +160,314 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
         atomicCAS(rp.status, 0, code);
     };
     const int u_first = blockIdx.x, u_stride = gridDim.x;
-    auto wants_kv = [&](int f) { return f >= rp.g0 && f < rp.g1; };
+    // The groups of a unit, last one first: a training call wants dK / dV of the last ones, and the query tile is then free
+    // from the last step's S GEMM on.  The order does not depend on which are wanted (nor then does dQ's rounding).
+    auto group_of = [&](int i) { return F - 1 - i; };
+    auto wants_kv = [&](int i) { const int f = group_of(i); return f >= rp.g0 && f < rp.g1; };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ producer
-        {
-            const uint32_t el = elect_one();
-            prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tda); prefetch_tmap(&tdy);
-            int g = 0, uc = 0;
-            bool ok = true;
-            for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
-                const RBUnit un = rb_decode(rp, u);
-                const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-                const int g_first = un.tile * rp.groups_per_tile;
-                const int ng = min(rp.groups_per_tile, p.na - g_first);
-                if (uc > 0 && !mbar_wait_u(&bars->q_empty, (uc - 1) & 1)) { fail(10); break; }
-                mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(ng * b2 * 256));           // the padding rows stay zero
-                for (int gi = 0; gi < ng; ++gi) {
-                    const int tok = blk.row_token(p.a0 + g_first + gi, un.k);
-                    tma_load_4d_e(el, q_s + gi * RG * 128, &tq, &bars->q_full, 0, hd, tok, b);
-                    tma_load_4d_e(el, q_s + kRows * 128 + gi * RG * 128, &tq, &bars->q_full, 64, hd, tok, b);
-                }
-                for (int f = 0; f < F; ++f, ++g) {
-                    const int s = g & 1;
-                    if (g >= 2 && !mbar_wait_u(&bars->kv_empty[s], ((g >> 1) - 1) & 1)) { fail(11); ok = false; break; }
-                    const int tok = (f * b1 + un.k) * b2;
-                    unsigned char* st = kv_s + s * kKVStage;
-                    mbar_arrive_expect_tx_e(el, &bars->kv_full[s], (uint32_t)(4 * kHalf));
-                    tma_load_4d_e(el, st, &tk, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
-                    tma_load_4d_e(el, st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
-                    if (g >= 1 && !mbar_wait_u(&bars->da_empty, (g - 1) & 1)) { fail(12); ok = false; break; }
-                    const int key = f * b1 + un.k;
-                    mbar_arrive_expect_tx_e(el, &bars->da_full, (uint32_t)(2 * ng * RG * 256));
+        // ------------------------------------------------------------------ K, V, daL, dY
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tda); prefetch_tmap(&tdy);
+        int g = 0, sr = 0, pr = 1;
+        bool ok = true;
+        for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
+            const RBUnit un = rb_decode(rp, u);
+            const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+            const int g_first = un.tile * rp.groups_per_tile;
+            const int ng = min(rp.groups_per_tile, p.na - g_first);
+            for (int i = 0; ok && i < F; ++i, ++g) {
+                const int s = g & 1, f = group_of(i);
+                if (g >= 2 && !mbar_wait_u(&bars->k_empty[s], ((g >> 1) - 1) & 1)) { fail(11); ok = false; break; }
+                const int tok = (f * b1 + un.k) * b2;
+                unsigned char* kt = kv_s + s * kKVTile;
+                unsigned char* vt = kv_s + 2 * kKVTile;
+                mbar_arrive_expect_tx_e(el, &bars->k_full[s], (uint32_t)(2 * kHalf));
+                tma_load_4d_e(el, kt, &tk, &bars->k_full[s], 0, hd, tok, b);
+                tma_load_4d_e(el, kt + kHalf, &tk, &bars->k_full[s], 64, hd, tok, b);
+                const int key = f * b1 + un.k;
+                for (int which = 0; which < 2; ++which) {
+                    if (which) {
+                        if (g >= 1 && !mbar_wait_u(&bars->v_empty, (g - 1) & 1)) { fail(13); ok = false; break; }
+                        mbar_arrive_expect_tx_e(el, &bars->v_full, (uint32_t)(2 * kHalf));
+                        tma_load_4d_e(el, vt, &tv, &bars->v_full, 0, hd, tok, b);
+                        tma_load_4d_e(el, vt + kHalf, &tv, &bars->v_full, 64, hd, tok, b);
+                    }
+                    if (!mbar_wait_u(&bars->rt_empty[sr], pr)) { fail(12); ok = false; break; }
+                    unsigned char* rt = rt_s + sr * kQB;
+                    mbar_arrive_expect_tx_e(el, &bars->rt_full[sr], (uint32_t)(ng * RG * 256));
                     for (int gi = 0; gi < ng; ++gi) {
                         const int grp = un.bhl * p.na + g_first + gi;
-                        tma_load_4d_e(el, da_s + gi * RG * 128, &tda, &bars->da_full, 0, 0, key, grp);
-                        tma_load_4d_e(el, da_s + kRows * 128 + gi * RG * 128, &tda, &bars->da_full, 64, 0, key, grp);
-                        tma_load_4d_e(el, dy_s + gi * RG * 128, &tdy, &bars->da_full, 0, 0, key, grp);
-                        tma_load_4d_e(el, dy_s + kRows * 128 + gi * RG * 128, &tdy, &bars->da_full, 64, 0, key, grp);
+                        tma_load_4d_e(el, rt + gi * RG * 128, which ? &tdy : &tda, &bars->rt_full[sr], 0, 0, key, grp);
+                        tma_load_4d_e(el, rt + kRows * 128 + gi * RG * 128, which ? &tdy : &tda, &bars->rt_full[sr], 64, 0, key, grp);
                     }
+                    if (++sr == kRowSlots) { sr = 0; pr ^= 1; }
                 }
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ query tiles
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tq);
+        int uc = 0;
+        for (int u = u_first; u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
+            const RBUnit un = rb_decode(rp, u);
+            const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+            const int g_first = un.tile * rp.groups_per_tile;
+            const int ng = min(rp.groups_per_tile, p.na - g_first);
+            if (uc > 0 && !mbar_wait_u(&bars->q_empty, (uc - 1) & 1)) { fail(10); break; }
+            mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(ng * b2 * 256));           // the padding rows stay zero
+            for (int gi = 0; gi < ng; ++gi) {
+                const int tok = blk.row_token(p.a0 + g_first + gi, un.k);
+                tma_load_4d_e(el, q_s + gi * RG * 128, &tq, &bars->q_full, 0, hd, tok, b);
+                tma_load_4d_e(el, q_s + kRows * 128 + gi * RG * 128, &tq, &bars->q_full, 64, hd, tok, b);
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        {
-            const uint32_t el = elect_one();
-            constexpr uint32_t idesc_s = idesc_bf16(kRows, N_S, 0, 0);            // S, dR
-            constexpr uint32_t idesc_q = idesc_bf16(kRows, kHeadDim, 0, 1);        // dQ: A from TMEM, B MN-major
-            constexpr uint32_t idesc_k = idesc_bf16(kRows, kHeadDim, 1, 1);        // dK, dV: both MN-major
-            const uint64_t q_k = smem_desc_sw128(smem_addr(q_s), 16, 1024);
-            const uint64_t q_mn = smem_desc_sw128(smem_addr(q_s), kRows * 128, 1024);
-            const uint64_t da_k = smem_desc_sw128(smem_addr(da_s), 16, 1024);
-            const uint64_t da_mn = smem_desc_sw128(smem_addr(da_s), kRows * 128, 1024);
-            const uint64_t dy_k = smem_desc_sw128(smem_addr(dy_s), 16, 1024);
-            const uint64_t dy_mn = smem_desc_sw128(smem_addr(dy_s), kRows * 128, 1024);
-            const uint64_t kv_k0 = smem_desc_sw128(smem_addr(kv_s), 16, 1024);
-            const uint64_t kv_mn0 = smem_desc_sw128(smem_addr(kv_s), kHalf, 1024);
-            const uint64_t r_mn = smem_desc_sw128(smem_addr(r_s), 2 * kStageT, 1024);      // second M block = the zeros
-            const uint64_t z_mn = smem_desc_sw128(smem_addr(z_s), kStageT, 1024);
-            int g = 0, uc = 0, gd = 0;
-            bool ok = true;
-            for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
-                if (!mbar_wait_u(&bars->q_full, uc & 1)) { fail(20); break; }
-                for (int f = 0; f < F; ++f, ++g) {
-                    const int s = g & 1;
-                    const bool kvw = wants_kv(f);
-                    if (!mbar_wait_u(&bars->kv_full[s], (g >> 1) & 1)) { fail(21); ok = false; break; }
-                    if (g >= 1 && !mbar_wait_u(&bars->sdr_free, (g - 1) & 1)) { fail(22); ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t kd = kv_k0 + (uint64_t)((s * kKVStage) >> 4);
-                    const uint64_t vd = kd + (uint64_t)((2 * kHalf) >> 4);
+        // ------------------------------------------------------------------ S and dR GEMMs
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_s = idesc_bf16(kRows, N_S, 0, 0);
+        const uint64_t q_k = smem_desc_sw128(smem_addr(q_s), 16, 1024);
+        const uint64_t rt_k0 = smem_desc_sw128(smem_addr(rt_s), 16, 1024);
+        const uint64_t kv_k0 = smem_desc_sw128(smem_addr(kv_s), 16, 1024);
+        const uint64_t vd = kv_k0 + (uint64_t)((2 * kKVTile) >> 4);
+        int g = 0, uc = 0, sr = 0, pr = 0;
+        bool ok = true;
+        for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
+            if (!mbar_wait_u(&bars->q_full, uc & 1)) { fail(20); break; }
+            for (int i = 0; i < F; ++i, ++g) {
+                const int s = g & 1;
+                const bool kvw = wants_kv(i);
+                if (!mbar_wait_u(&bars->k_full[s], (g >> 1) & 1)) { fail(21); ok = false; break; }
+                if (g >= 1 && !mbar_wait_u(&bars->sdr_read, (g - 1) & 1)) { fail(22); ok = false; break; }
+                tc_fence_after();
+                const uint64_t kd = kv_k0 + (uint64_t)((s * kKVTile) >> 4);
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
-                        const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
-                        const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss_e(el, tmem + kCS, q_k + qo, kd + ko, idesc_s, ks > 0);
-                    }
-                    mma_commit_e(el, &bars->s_full);
-                    if (!mbar_wait_u(&bars->da_full, g & 1)) { fail(23); ok = false; break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
-                        const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
-                        const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss_e(el, tmem + kCDR, da_k + qo, kd + ko, idesc_s, ks > 0);
-                    }
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
-                        const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
-                        const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss_e(el, tmem + kCDR, dy_k + qo, vd + ko, idesc_s, 1u);
-                    }
-                    mma_commit_e(el, &bars->dr_full);
-                    if (!kvw) mma_commit_e(el, &bars->da_empty);          // nothing else reads the row tiles this step
-                    if (!mbar_wait_u(&bars->p_full, g & 1)) { fail(24); ok = false; break; }
-                    if (f == 0 && uc >= 1 && !mbar_wait_u(&bars->dq_free, (uc - 1) & 1)) { fail(25); ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t kmn = kv_mn0 + (uint64_t)((s * kKVStage) >> 4);
-#pragma unroll
-                    for (int kk = 0; kk < N_S / 16; ++kk)      // dQ (+)= (scale dz) K
-                        mma_ts_e(el, tmem + kCDQ, tmem + kCDR + kk * 8, kmn + ((kk * 2048) >> 4), idesc_q, (f > 0 || kk > 0) ? 1u : 0u);
-                    if (kvw) {
-                        if (gd >= 1 && !mbar_wait_u(&bars->dkv_free, (gd - 1) & 1)) { fail(26); ok = false; break; }
-                        tc_fence_after();
-#pragma unroll
-                        for (int kk = 0; kk < kRows / 16; ++kk)     // dK = R^T daL_tile
-                            mma_ss_e(el, tmem + kCDK, r_mn + ((kk * 2048) >> 4), da_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
-#pragma unroll
-                        for (int kk = 0; kk < kRows / 16; ++kk)     // dK += (scale dz)^T Q_tile
-                            mma_ss_e(el, tmem + kCDK, z_mn + ((kk * 2048) >> 4), q_mn + ((kk * 2048) >> 4), idesc_k, 1u);
-#pragma unroll
-                        for (int kk = 0; kk < kRows / 16; ++kk)     // dV = R^T dY_tile
-                            mma_ss_e(el, tmem + kCDV, r_mn + ((kk * 2048) >> 4), dy_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
-                        mma_commit_e(el, &bars->dkv_full);
-                        mma_commit_e(el, &bars->da_empty);
-                        ++gd;
-                    }
-                    mma_commit_e(el, &bars->sdr_free);
-                    mma_commit_e(el, &bars->kv_empty[s]);
-                    if (f + 1 == F) { mma_commit_e(el, &bars->dq_full); mma_commit_e(el, &bars->q_empty); }
+                for (int ks = 0; ks < 8; ++ks) {
+                    const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
+                    const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
+                    mma_ss_e(el, tmem + kCS, q_k + qo, kd + ko, idesc_s, ks > 0);
                 }
+                mma_commit_e(el, &bars->s_full);
+                if (i + 1 == F) mma_commit_e(el, &bars->q_empty);
+#pragma unroll 1
+                for (int which = 0; which < 2; ++which) {
+                    if (!mbar_wait_u(&bars->rt_full[sr], pr)) { fail(23); ok = false; break; }
+                    if (which && !mbar_wait_u(&bars->v_full, g & 1)) { fail(27); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t rd = rt_k0 + (uint64_t)((sr * kQB) >> 4);
+                    const uint64_t bd = which ? vd : kd;
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) {
+                        const uint32_t qo = ((ks >> 2) * (kRows * 128) + (ks & 3) * 32) >> 4;
+                        const uint32_t ko = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
+                        mma_ss_e(el, tmem + kCDR, rd + qo, bd + ko, idesc_s, (which || ks > 0) ? 1u : 0u);
+                    }
+                    if (!kvw) mma_commit_e(el, &bars->rt_empty[sr]);      // nothing else reads the row tiles this step
+                    if (++sr == kRowSlots) { sr = 0; pr ^= 1; }
+                }
+                if (!ok) break;
+                mma_commit_e(el, &bars->dr_full);
+                mma_commit_e(el, &bars->v_empty);
             }
         }
-    } else if (warp >= 4 && warp < 8) {
-        // ------------------------------------------------------------------ element-wise warpgroup: one query row per thread
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ gradient GEMMs
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_q = idesc_bf16(kRows, kHeadDim, 0, 1);        // dQ: B MN-major
+        constexpr uint32_t idesc_k = idesc_bf16(kRows, kHeadDim, 1, 1);        // dK, dV: both MN-major
+        const uint64_t q_mn = smem_desc_sw128(smem_addr(q_s), kRows * 128, 1024);
+        const uint64_t rt_mn0 = smem_desc_sw128(smem_addr(rt_s), kRows * 128, 1024);
+        const uint64_t kv_mn0 = smem_desc_sw128(smem_addr(kv_s), kHalf, 1024);
+        const uint64_t r_mn = smem_desc_sw128(smem_addr(r_s), kStageT, 1024);
+        const uint64_t z_mn = smem_desc_sw128(smem_addr(z_s), kStageT, 1024);
+        const uint64_t z_k = smem_desc_sw128(smem_addr(z_s), 16, 1024);
+        const int q_last = rp.g1 > rp.g0 ? F - 1 - rp.g0 : 0;        // from here on these GEMMs leave the query tile alone
+        int g = 0, uc = 0, gd = 0, sr = 0;
+        bool ok = true;
+        for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride, ++uc) {
+            for (int i = 0; i < F; ++i, ++g) {
+                const int s = g & 1, da = sr, dy = da + 1 == kRowSlots ? 0 : da + 1;
+                sr = dy + 1 == kRowSlots ? 0 : dy + 1;
+                if (!mbar_wait_u(&bars->p_full, g & 1)) { fail(24); ok = false; break; }
+                if (i == 0 && uc >= 1 && !mbar_wait_u(&bars->dq_free, (uc - 1) & 1)) { fail(25); ok = false; break; }
+                tc_fence_after();
+                const uint64_t kmn = kv_mn0 + (uint64_t)((s * kKVTile) >> 4);
+#pragma unroll
+                for (int kk = 0; kk < N_S / 16; ++kk)      // dQ (+)= (scale dz) K
+                    mma_ss_e(el, tmem + kCDQ, z_k + ((kk * 32) >> 4), kmn + ((kk * 2048) >> 4), idesc_q, (i > 0 || kk > 0) ? 1u : 0u);
+                mma_commit_e(el, &bars->k_empty[s]);
+                if (wants_kv(i)) {
+                    if (gd >= 1 && !mbar_wait_u(&bars->dkv_free, (gd - 1) & 1)) { fail(26); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t da_mn = rt_mn0 + (uint64_t)((da * kQB) >> 4), dy_mn = rt_mn0 + (uint64_t)((dy * kQB) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < kRows / 16; ++kk)     // dK = R^T daL_tile
+                        mma_ss_e(el, tmem + kCDK, r_mn + ((kk * 2048) >> 4), da_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
+                    mma_commit_e(el, &bars->rt_empty[da]);
+#pragma unroll
+                    for (int kk = 0; kk < kRows / 16; ++kk)     // dV = R^T dY_tile
+                        mma_ss_e(el, tmem + kCDV, r_mn + ((kk * 2048) >> 4), dy_mn + ((kk * 2048) >> 4), idesc_k, kk > 0);
+                    mma_commit_e(el, &bars->rt_empty[dy]);
+#pragma unroll
+                    for (int kk = 0; kk < kRows / 16; ++kk)     // dK += (scale dz)^T Q_tile
+                        mma_ss_e(el, tmem + kCDK, z_mn + ((kk * 2048) >> 4), q_mn + ((kk * 2048) >> 4), idesc_k, 1u);
+                    mma_commit_e(el, &bars->dkv_full);
+                    ++gd;
+                }
+                if (i == q_last) mma_commit_e(el, &bars->q_empty);
+                mma_commit_e(el, &bars->rz_free);
+                if (i + 1 == F) mma_commit_e(el, &bars->dq_full);
+            }
+        }
+    } else if (warp >= 4 && warp < 12) {
+        // ------------------------------------------------------------------ element-wise pass: half a query row per thread
+        constexpr int kC = N_S / 2;                             // columns per thread
+        const int half = (warp - 4) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const int gl = row / RG, j = row - gl * RG;
-        const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+        const int n_valid = b2 - half * kC;                     // of this thread's columns
+        const uint32_t s_t = tmem + ((uint32_t)(quad * 32) << 16) + kCS + half * kC;
+        const uint32_t dr_t = s_t + (kCDR - kCS);
         const float scale_l2 = p.mult0 * kLog2e;
+        const uint64_t scale2 = f2_pack(scale_l2, scale_l2);
         unsigned char* r_row = r_s + row * 128;
         unsigned char* z_row = z_s + row * 128;
+        auto load_dcl = [&](int u, int i) -> float {
+            if (u >= rp.n_units) return 0.f;
+            const RBUnit un = rb_decode(rp, u);
+            const int al = un.tile * rp.groups_per_tile + gl;
+            if (gl >= rp.groups_per_tile || al >= p.na || j >= b2) return 0.f;
+            return rp.dcL[(((long long)un.bhl * p.na + al) * b2 + j) * p.n_keys_c + group_of(i) * b1 + un.k];
+        };
+        float dcl_next = load_dcl(u_first, 0);
         int g = 0;
         bool ok = true;
         for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
             const RBUnit un = rb_decode(rp, u);
-            const int g_first = un.tile * rp.groups_per_tile;
-            const int ng = min(rp.groups_per_tile, p.na - g_first);
-            const bool row_ok = gl < ng && j < b2;
-            const long long slab = ((long long)un.bhl * p.na + g_first + gl) * b2 + j;
-            for (int f = 0; f < F; ++f, ++g) {
-                const float dcl = row_ok ? rp.dcL[slab * p.n_keys_c + f * b1 + un.k] : 0.f;
-                if (!mbar_wait(&bars->s_full, g & 1)) { fail(31); ok = false; break; }
+            const bool row_ok = gl < min(rp.groups_per_tile, p.na - un.tile * rp.groups_per_tile) && j < b2;
+            for (int i = 0; i < F; ++i, ++g) {
+                const float dcl = dcl_next;
+                dcl_next = i + 1 < F ? load_dcl(u, i + 1) : load_dcl(u + u_stride, 0);
+                if (!mbar_wait_u(&bars->s_full, g & 1)) { fail(31); ok = false; break; }
                 tc_fence_after();
-                uint32_t raw[N_S], dr[N_S];
-                if constexpr (N_S == 64) {
-                    tmem_ld32(tmem + lane_sel + kCS, *reinterpret_cast<uint32_t(*)[32]>(&raw[0]));
-                    tmem_ld32(tmem + lane_sel + kCS + 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[32]));
-                } else if constexpr (N_S == 48) {
-                    tmem_ld32(tmem + lane_sel + kCS, *reinterpret_cast<uint32_t(*)[32]>(&raw[0]));
-                    tmem_ld16(tmem + lane_sel + kCS + 32, *reinterpret_cast<uint32_t(*)[16]>(&raw[32]));
-                } else if constexpr (N_S == 32) {
-                    tmem_ld32(tmem + lane_sel + kCS, *reinterpret_cast<uint32_t(*)[32]>(&raw[0]));
-                } else {
-                    tmem_ld16(tmem + lane_sel + kCS, *reinterpret_cast<uint32_t(*)[16]>(&raw[0]));
-                }
-                tmem_wait_ld();
-                float mx = -INFINITY;
+                uint64_t d2[kC / 2], e[kC / 2], x[kC / 2];      // log2 of the weight over this half's maximum, weight, dR
+                {
+                    uint32_t r[kC];
+                    tmem_ld_n(s_t, r);
+                    tmem_wait_ld();
+                    if (n_valid < kC) {
 #pragma unroll
-                for (int c = 0; c < N_S; ++c) {
-                    if (c >= b2) raw[c] = 0xf149f2cau;                 // -1e30: weight zero
-                    mx = fmaxf(mx, __uint_as_float(raw[c]));
-                }
-                const float m2 = mx * scale_l2;
-                float z = 0.f;
+                        for (int c = 0; c < kC; ++c)
+                            if (c >= n_valid) r[c] = 0xf149f2cau;   // -1e30: weight zero
+                    }
 #pragma unroll
-                for (int c = 0; c < N_S; ++c) z += exp2f(fmaf(__uint_as_float(raw[c]), scale_l2, -m2));
-                const float inv_z = 1.0f / z, l2z = __log2f(z);
-                if (!mbar_wait(&bars->dr_full, g & 1)) { fail(32); ok = false; break; }
+                    for (int c = 0; c < kC; c += 2) d2[c / 2] = f2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1]));
+                }
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int c = 0; c < kC / 2; ++c) {
+                    float x0, x1;
+                    f2_unpack(d2[c], x0, x1);
+                    mx[c & 3] = max3(mx[c & 3], x0, x1);
+                }
+                // a half without columns must not take its fill value for a maximum
+                const float m2 = fmaxf(max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) * scale_l2, -1e20f);
+                const uint64_t neg_m2 = f2_pack(-m2, -m2);
+                uint64_t z2 = f2_pack(0.f, 0.f), el2 = z2, ex2 = z2;      // sums of e, e log2 e, e (daL . K + dY . V)
+#pragma unroll
+                for (int c = 0; c < kC / 2; ++c) {
+                    d2[c] = f2_fma(d2[c], scale2, neg_m2);
+                    float x0, x1;
+                    f2_unpack(d2[c], x0, x1);
+                    e[c] = f2_pack(exp2f(x0), exp2f(x1));
+                    z2 = f2_add(z2, e[c]);
+                    el2 = f2_fma(e[c], d2[c], el2);
+                }
+                float lo, hi;
+                f2_unpack(z2, lo, hi);
+                const float z = lo + hi;
+                f2_unpack(el2, lo, hi);
+                const float el = lo + hi;
+                if (!mbar_wait_u(&bars->dr_full, g & 1)) { fail(32); ok = false; break; }
                 tc_fence_after();
-                if constexpr (N_S == 64) {
-                    tmem_ld32(tmem + lane_sel + kCDR, *reinterpret_cast<uint32_t(*)[32]>(&dr[0]));
-                    tmem_ld32(tmem + lane_sel + kCDR + 32, *reinterpret_cast<uint32_t(*)[32]>(&dr[32]));
-                } else if constexpr (N_S == 48) {
-                    tmem_ld32(tmem + lane_sel + kCDR, *reinterpret_cast<uint32_t(*)[32]>(&dr[0]));
-                    tmem_ld16(tmem + lane_sel + kCDR + 32, *reinterpret_cast<uint32_t(*)[16]>(&dr[32]));
-                } else if constexpr (N_S == 32) {
-                    tmem_ld32(tmem + lane_sel + kCDR, *reinterpret_cast<uint32_t(*)[32]>(&dr[0]));
-                } else {
-                    tmem_ld16(tmem + lane_sel + kCDR, *reinterpret_cast<uint32_t(*)[16]>(&dr[0]));
+                {
+                    uint32_t r[kC];
+                    tmem_ld_n(dr_t, r);
+                    tmem_wait_ld();
+                    tc_fence_before();
+                    mbar_arrive(&bars->sdr_read);
+                    if (n_valid < kC) {
+#pragma unroll
+                        for (int c = 0; c < kC; ++c)
+                            if (c >= n_valid) r[c] = 0u;
+                    }
+#pragma unroll
+                    for (int c = 0; c < kC; c += 2) {
+                        x[c / 2] = f2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1]));
+                        ex2 = f2_fma(e[c / 2], x[c / 2], ex2);
+                    }
                 }
-                tmem_wait_ld();
-                // dR_l = (daL . K_l + dY . V_l) + dcL (ln R_l + 1); sum_l R_l dR_l
-                float dot = 0.f;
+                f2_unpack(ex2, lo, hi);
+                const float ex = lo + hi;
+                bars->stats[g & 1][half][row] = make_float4(m2, z, el, ex);
+                mbar_arrive(&bars->x_full[quad]);
+                if (!mbar_wait_u(&bars->x_full[quad], g & 1)) { fail(33); ok = false; break; }
+                const float4 o = bars->stats[g & 1][half ^ 1][row];
+                // both halves against the row's maximum
+                const float mr = fmaxf(m2, o.x), dm = m2 - mr, dmo = o.x - mr;
+                const float a = exp2f(dm), ao = exp2f(dmo);
+                const float zr = a * z + ao * o.y, inv_z = 1.0f / zr, l2z = __log2f(zr);
+                const float rlr = (a * fmaf(z, dm, el) + ao * fmaf(o.y, dmo, o.z)) * inv_z - l2z;     // sum of R log2 R
+                const float dcl2 = dcl * 0.6931471805599453f;
+                // dR_l = (daL . K_l + dY . V_l) + dcL (ln R_l + 1); the sum of R dR from its parts
+                const float dot = fmaf(dcl2, rlr, (a * ex + ao * o.w) * inv_z);
+                const float rs = row_ok ? a * inv_z : 0.f;      // rows of no unit must not reach dK / dV
+                const float off = fmaf(dcl2, dm - l2z, -dot);   // dR - sum = x + dcl2 d2 + off (dcL itself cancels)
+                const uint64_t rs2 = f2_pack(rs, rs), zs2 = f2_pack(rs * p.scale, rs * p.scale);
+                const uint64_t dc2 = f2_pack(dcl2, dcl2), off2 = f2_pack(off, off);
+                if (g >= 1 && !mbar_wait_u(&bars->rz_free, (g - 1) & 1)) { fail(34); ok = false; break; }
+                const bool kvw = wants_kv(i);
 #pragma unroll
-                for (int c = 0; c < N_S; ++c) {
-                    const float d2 = fmaf(__uint_as_float(raw[c]), scale_l2, -m2);     // log2 of the unnormalised weight
-                    const float rr = exp2f(d2) * inv_z;
-                    const float lnr = (d2 - l2z) * 0.6931471805599453f;
-                    const float x = c < b2 ? fmaf(dcl, lnr + 1.0f, __uint_as_float(dr[c])) : 0.f;
-                    dr[c] = __float_as_uint(x);
-                    dot = fmaf(rr, x, dot);
-                }
-                uint32_t pr[N_S / 2], pz[N_S / 2];
+                for (int c8 = 0; c8 < kC / 2; c8 += 4) {
+                    uint32_t pr[4], pz[4];
 #pragma unroll
-                for (int c = 0; c < N_S; c += 2) {
-                    float r0 = exp2f(fmaf(__uint_as_float(raw[c]), scale_l2, -m2)) * inv_z;
-                    float r1 = exp2f(fmaf(__uint_as_float(raw[c + 1]), scale_l2, -m2)) * inv_z;
-                    float z0 = r0 * (__uint_as_float(dr[c]) - dot) * p.scale;
-                    float z1 = r1 * (__uint_as_float(dr[c + 1]) - dot) * p.scale;
-                    if (!row_ok) { r0 = 0.f; r1 = 0.f; z0 = 0.f; z1 = 0.f; }   // rows of no unit must not reach dK / dV
-                    pr[c >> 1] = pack_bf16(r0, r1);
-                    pz[c >> 1] = pack_bf16(z0, z1);
-                }
-                // scale dz as the TMEM operand of the dQ GEMM (over the dR columns already read)
-                if constexpr (N_S == 64) {
-                    tmem_st32(tmem + lane_sel + kCDR, pz);
-                } else if constexpr (N_S == 32) {
-                    tmem_st16(tmem + lane_sel + kCDR, pz);
-                } else if constexpr (N_S == 48) {
-                    tmem_st16(tmem + lane_sel + kCDR, *reinterpret_cast<uint32_t(*)[16]>(&pz[0]));
-                    uint32_t t2[16];
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) t2[c] = c < 8 ? pz[16 + c] : 0u;
-                    tmem_st16(tmem + lane_sel + kCDR + 16, t2);
-                } else {
-                    uint32_t t2[16];
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) t2[c] = c < 8 ? pz[c] : 0u;
-                    tmem_st16(tmem + lane_sel + kCDR, t2);
-                }
-                // bf16 copies of the R and scale dz rows for the dK / dV GEMMs (128-byte swizzled rows)
-#pragma unroll
-                for (int c = 0; c < N_S / 8; ++c) {
-                    const int pc = (c ^ (row & 7)) << 4;
-                    *reinterpret_cast<uint4*>(r_row + pc) = make_uint4(pr[4 * c], pr[4 * c + 1], pr[4 * c + 2], pr[4 * c + 3]);
-                    *reinterpret_cast<uint4*>(z_row + pc) = make_uint4(pz[4 * c], pz[4 * c + 1], pz[4 * c + 2], pz[4 * c + 3]);
+                    for (int c = 0; c < 4; ++c) {
+                        float v0, v1;
+                        f2_unpack(f2_mul(f2_mul(e[c8 + c], zs2), f2_fma(dc2, d2[c8 + c], f2_add(x[c8 + c], off2))), v0, v1);
+                        pz[c] = pack_bf16(v0, v1);
+                        f2_unpack(f2_mul(e[c8 + c], rs2), v0, v1);
+                        pr[c] = pack_bf16(v0, v1);
+                    }
+                    const int pc = (((half * kC + 2 * c8) >> 3) ^ (row & 7)) << 4;
+                    if (kvw) *reinterpret_cast<uint4*>(r_row + pc) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
+                    *reinterpret_cast<uint4*>(z_row + pc) = make_uint4(pz[0], pz[1], pz[2], pz[3]);
                 }
                 fence_async_smem();
-                tmem_wait_st();
-                tc_fence_before();
                 mbar_arrive(&bars->p_full);
             }
         }
-    } else if (warp >= 8) {
+    } else if (warp >= 12) {
         // ------------------------------------------------------------------ drain warpgroup
+        // Rows come out of TMEM one per lane; through a small transposition in shared memory they go out 64 bytes at a time,
+        // four lanes a row, instead of 32 rows per store instruction.
         const int quad = warp & 3;
-        const int row = quad * 32 + lane;                       // dK / dV: key l; dQ: query row
-        const int gl = row / RG, j = row - gl * RG;
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+        unsigned char* const st = o_s + quad * kOutStage;
+        const int l_row = lane >> 2, l_col = (lane & 3) * 4;     // of each group of 8 rows, of each block of 16 columns
+        auto transpose = [&](const uint32_t (&r)[16], float4 (&v)[4]) {
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int rr = it * 8 + l_row;
+                v[it] = *reinterpret_cast<const float4*>(st + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+            }
+        };
         const long long n_sel = (long long)(rp.g1 - rp.g0) * b1 * b2;
         int uc = 0, gd = 0;
         bool ok = true;
@@ -378,65 +476,74 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
             const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
             const int g_first = un.tile * rp.groups_per_tile;
             const int ng = min(rp.groups_per_tile, p.na - g_first);
-            for (int f = 0; f < F; ++f) {
-                if (!wants_kv(f)) continue;
-                if (!mbar_wait(&bars->dkv_full, gd & 1)) { fail(41); ok = false; break; }
+            for (int i = 0; i < F; ++i) {
+                if (!wants_kv(i)) continue;
+                if (!mbar_wait_u(&bars->dkv_full, gd & 1)) { fail(41); ok = false; break; }
                 tc_fence_after();
-                const long long prow = (((long long)un.tile * p.nbh + un.bhl) * n_sel + ((long long)(f - rp.g0) * b1 + un.k) * b2 + row) * kHeadDim;
+                // the keys of the block, at most 64, are on the first two warps' lanes
+                if (quad * 32 < b2 && quad < 2) {
+                    const long long row0 = ((long long)un.tile * p.nbh + un.bhl) * n_sel + ((long long)(group_of(i) - rp.g0) * b1 + un.k) * b2;
+                    const long long o0 = (row0 + quad * 32 + l_row) * kHeadDim + l_col;
 #pragma unroll 1
-                for (int half = 0; half < 2; ++half) {
-                    float* dst = (half ? rp.part_v : rp.part_k) + prow;
-                    const uint32_t col0 = half ? kCDV : kCDK;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
-                        uint32_t r[32];
-                        if (quad < 2) {                        // keys live on lanes 0..63
-                            tmem_ld32(tmem + lane_sel + col0 + c0, r);
-                            tmem_wait_ld();
-                        }
-                        if (half == 1 && c0 + 32 == kHeadDim) {
-                            tc_fence_before();
-                            mbar_arrive(&bars->dkv_free);
-                        }
-                        if (quad < 2 && row < b2) {
+                    for (int c0 = 0; c0 < 2 * kHeadDim; c0 += 16) {
+                        float* dst = (c0 < kHeadDim ? rp.part_k : rp.part_v) + o0 + (c0 & (kHeadDim - 1));
+                        uint32_t r[16];
+                        float4 v[4];
+                        tmem_ld16(tmem + lane_sel + kCDK + c0, r);          // dV's columns follow dK's
+                        tmem_wait_ld();
+                        transpose(r, v);
 #pragma unroll
-                            for (int v = 0; v < 8; ++v)
-                                *reinterpret_cast<uint4*>(dst + c0 + 4 * v) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-                        }
+                        for (int it = 0; it < 4; ++it)
+                            if (quad * 32 + it * 8 + l_row < b2) *reinterpret_cast<float4*>(dst + it * 8 * kHeadDim) = v[it];
                     }
+                    tc_fence_before();
                 }
+                mbar_arrive(&bars->dkv_free);
                 ++gd;
             }
             if (!ok) break;
             // ---- the unit's dQ rows: added to the column step's share
-            if (!mbar_wait(&bars->dq_full, uc & 1)) { fail(42); break; }
-            tc_fence_after();
-            const bool row_ok = gl < ng && j < b2;
-            float* dqr = nullptr;
-            if (row_ok) {
-                const long long tok = blk.row_token(p.a0 + g_first + gl, un.k) + j;
-                dqr = rp.dq + (((long long)b * p.n_q + tok) * p.H + hd) * kHeadDim;
+            long long off[4];                                    // of this lane's rows; negative: no row
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int row = quad * 32 + it * 8 + l_row, gl = row / RG, j = row - gl * RG;
+                const int tok = gl < ng && j < b2 ? blk.row_token(p.a0 + g_first + gl, un.k) + j : -1;
+                off[it] = tok < 0 ? -1 : (((long long)b * p.n_q + tok) * p.H + hd) * kHeadDim + l_col;
             }
+            float4 share[4];
+            auto load_share = [&](int c0) {
+#pragma unroll
+                for (int it = 0; it < 4; ++it)
+                    if (rp.dq_bf16 && off[it] >= 0) share[it] = *reinterpret_cast<const float4*>(rp.dq + off[it] + c0);
+            };
+            load_share(0);
+            if (!mbar_wait_u(&bars->dq_full, uc & 1)) { fail(42); break; }
+            tc_fence_after();
 #pragma unroll 1
-            for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem + lane_sel + kCDQ + c0, r);
+            for (int c0 = 0; c0 < kHeadDim; c0 += 16) {
+                uint32_t r[16];
+                float4 v[4];
+                tmem_ld16(tmem + lane_sel + kCDQ + c0, r);
                 tmem_wait_ld();
-                if (c0 + 32 == kHeadDim) {
+                if (c0 + 16 == kHeadDim) {
                     tc_fence_before();
                     mbar_arrive(&bars->dq_free);
                 }
-                if (row_ok) {
+                transpose(r, v);
+                if (rp.dq_bf16) {
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        float4 o = *reinterpret_cast<float4*>(dqr + c0 + 4 * v);
-                        o.x += __uint_as_float(r[4 * v]); o.y += __uint_as_float(r[4 * v + 1]);
-                        o.z += __uint_as_float(r[4 * v + 2]); o.w += __uint_as_float(r[4 * v + 3]);
-                        if (rp.dq_bf16)
-                            *reinterpret_cast<uint2*>(rp.dq_bf16 + (dqr - rp.dq) + c0 + 4 * v) = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
-                        else
-                            *reinterpret_cast<float4*>(dqr + c0 + 4 * v) = o;
+                    for (int it = 0; it < 4; ++it) {
+                        v[it].x += share[it].x; v[it].y += share[it].y; v[it].z += share[it].z; v[it].w += share[it].w;
                     }
+                    if (c0 + 16 < kHeadDim) load_share(c0 + 16);
+                }
+#pragma unroll
+                for (int it = 0; it < 4; ++it) {
+                    if (off[it] < 0) continue;
+                    if (rp.dq_bf16)
+                        *reinterpret_cast<uint2*>(rp.dq_bf16 + off[it] + c0) = make_uint2(pack_bf16(v[it].x, v[it].y), pack_bf16(v[it].z, v[it].w));
+                    else
+                        red_add_v4(rp.dq + off[it] + c0, v[it]);         // the only addition to these words
                 }
             }
         }

@@ -59,11 +59,6 @@ constexpr int kItTileBytes = 2 * kKTile * 128;
 constexpr int kItOutBytes = 4 * 2 * 4096;       // staging of the drain warps
 constexpr int kItSmemBytes = 1024 + 2 * kItQBytes + kAStg * kItTileBytes + kItOutBytes + (int)sizeof(ItBarriers) + 64;
 
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
 struct ItUnit { int bhl, al, j; };
 __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
     ItUnit r;
