@@ -14,6 +14,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps, int n_s, i
                      cudaStream_t s);
 int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s, int write_lse);
 int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s);
+bool l_iter_own_lse(const MonarchParams& p);
 }
 
 namespace {
@@ -218,9 +219,9 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
                         if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 0))) return rc;
                     } else if ((rc = launch_l_step(p, 0, stream))) return rc;
                 } else if (iter_tc) {
-                    // the column step's softmax statistics (its output row is overwritten by the last pass), then
+                    // the column step's softmax statistics, unless the update takes them itself, then
                     // the update of the state
-                    if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 2))) return rc;
+                    if (!l_iter_own_lse(p) && (rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 2))) return rc;
                     if ((rc = launch_l_iter_tc(p, &maps[3], status, num_sms, stream))) return rc;
                 } else {
                     if ((rc = launch_l_step(p, 1, stream))) return rc;

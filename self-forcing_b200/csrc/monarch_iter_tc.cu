@@ -11,15 +11,19 @@
 //   S^T [128 keys x N_I]  = aL_tile [128 x 128] * Q_j^T                    tcgen05.mma, both operands in shared memory
 //   P^T                   = exp(...) per element, bf16, written back over S^T in TMEM; cR = row sums (registers)
 //   aR_tile [128 x 128]   = P^T * Q_j                                      tcgen05.mma, A from TMEM, B = Q_j MN-major
-// N_I = block rows padded to 16.  Warp roles (16 warps): 0 = TMA producer, 1 = MMA issuer (owns TMEM), both with an elected
-// issuing lane, 2-3 idle, 4-7 and 8-11 = two warpgroups that take even / odd tiles for the softmax-like pass, 12-15 = drain
+// N_I = block rows padded to 16.  The log-sum-exp of a query comes from a column step run before this kernel, or, when all
+// keys fit one tile, from the tile itself: every warp has 32 keys on its lanes and takes each query's maximum and sum over
+// them, and the four warps of a tile exchange them.
+// Warp roles (16 warps): 0 = aL tiles, 1 = S^T GEMMs (owns TMEM), 2 = query rows and log-sum-exps, 3 = aR GEMMs, all with an
+// elected issuing lane, 4-7 and 8-11 = two warpgroups that take even / odd tiles for the softmax-like pass, 12-15 = drain
 // warpgroup: accumulator -> bf16 -> swizzled staging (two 4 KB buffers per warp) -> TMA store of 32 keys x 64 channels.
 // Persistent CTAs take contiguous shares of the unit list; all roles walk the same (unit, tile) sequence and meet through
 // mbarriers with bounded waits.
 //
-// What bounds it: with 90 keys per unit (first chunk) the chain of a tile, with longer caches the aR rows, 256 bytes per
-// key a whole (query group, column) set apart.  With the working warpgroups storing them themselves, one row per lane, the
-// 19 updates of a 20-pass call took 787 us, now 747.
+// What bounds it: with one tile per unit, the chain of a unit and its loads; with longer caches the aR rows, 256 bytes per
+// key a whole (query group, column) set apart.  With one loading warp (each unit's rows waited for its predecessor's
+// log-sum-exps to arrive from memory), one issuer, two query tiles and the log-sum-exps from a pass of the column step, 20
+// passes over a 4680-token chunk, 12 heads, took 1711 us, now 1005 (update 40 -> 27 us each, the pass, 27 us, gone).
 #include "monarch_params.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -30,7 +34,6 @@ using namespace tc;
 
 namespace {
 
-constexpr int kAStg = 3;                  // aL tile ring
 constexpr int kThreadsIt = 512;
 constexpr int kKTile = 128;               // keys per tile
 constexpr uint32_t kTmemColsIt = 512;
@@ -41,23 +44,52 @@ struct ItParams {
     MonarchParams mp;
     int n_units;       // nbh * na * b2
     int q_rows_tma;    // query rows of a unit are consecutive rows of the token grid
+    int own_lse;       // one tile per unit: the queries' log-sum-exps are taken from it
     int* status;
 };
 
+// Query tiles and aL tiles held at a time: units of one tile are short, and a query tile stays until its aR GEMM is done.
+__host__ __device__ constexpr int it_nq(int n_i) { return n_i <= 64 ? 4 : 2; }
+__host__ __device__ constexpr int it_na(int n_i) { return n_i <= 32 ? 4 : 3; }
+
+template <int N_I>
 struct __align__(16) ItBarriers {
-    float lse2[2][128];                   // log2(e) * lse of the unit's queries, +inf past b1
-    uint64_t q_full[2], q_empty[2];
-    uint64_t a_full[kAStg], a_empty[kAStg];
-    uint64_t s_full[2], p_full[2], sp_free[2];
+    float lse2[it_nq(N_I)][N_I];            // per query tile (log-sum-exps that come from memory)
+    float2 part[2][4][N_I];                 // [warpgroup][lane quadrant][query]: maximum, sum over the quadrant's keys
+    float lse2_own[8][N_I];                 // [working warp]: log-sum-exps of its tile's queries
+    uint64_t q_full[it_nq(N_I)], q_empty[it_nq(N_I)];
+    uint64_t a_full[it_na(N_I)], a_empty[it_na(N_I)];
+    uint64_t s_full[2], p_full[2], sp_free[2], x_full[2];
     uint64_t o_full[2], o_free[2];          // accumulator w
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
-constexpr int kItQBytes = 2 * 128 * 128;      // one query tile: two 64-column halves of 128 rows
 constexpr int kItTileBytes = 2 * kKTile * 128;
 constexpr int kItOutBytes = 4 * 2 * 4096;       // staging of the drain warps
-constexpr int kItSmemBytes = 1024 + 2 * kItQBytes + kAStg * kItTileBytes + kItOutBytes + (int)sizeof(ItBarriers) + 64;
+template <int N_I>
+constexpr int it_smem_bytes() {
+    return 1024 + it_nq(N_I) * N_I * 256 + it_na(N_I) * kItTileBytes + kItOutBytes + (int)sizeof(ItBarriers<N_I>) + 64;
+}
+
+// Sum over the warp of 16 values per lane: lane l gets the sum of v[l & 15].
+__device__ __forceinline__ float column_sums(float (&v)[16], int lane) {
+#pragma unroll
+    for (int off = 8; off; off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < off; ++i) {
+            const float send = up ? v[i] : v[i + off], keep = up ? v[i + off] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
 
 struct ItUnit { int bhl, al, j; };
 __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
@@ -76,10 +108,12 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                        const __grid_constant__ CUtensorMap tar, ItParams ip) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* q_s = base;                                   // two query tiles
-    unsigned char* a_s = q_s + 2 * kItQBytes;
-    unsigned char* o_s = a_s + kAStg * kItTileBytes;
-    ItBarriers* bars = reinterpret_cast<ItBarriers*>(o_s + kItOutBytes);
+    constexpr int NQ = it_nq(N_I), NA = it_na(N_I);
+    constexpr int kQHalf = N_I * 128, kQTile = 2 * kQHalf;       // a query tile: two 64-column halves
+    unsigned char* q_s = base;
+    unsigned char* a_s = q_s + NQ * kQTile;
+    unsigned char* o_s = a_s + NA * kItTileBytes;
+    ItBarriers<N_I>* bars = reinterpret_cast<ItBarriers<N_I>*>(o_s + kItOutBytes);
 
     const MonarchParams& p = ip.mp;
     const Blocking& blk = p.blk;
@@ -92,17 +126,17 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
     const int u_end = (int)((long long)ip.n_units * (blockIdx.x + 1) / gridDim.x);
 
     if (tid == 0) {
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
-        for (int s = 0; s < kAStg; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1); }
+        for (int s = 0; s < NQ; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
+        for (int s = 0; s < NA; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1); }
         for (int w = 0; w < 2; ++w) {
             mbar_init(&bars->s_full[w], 1); mbar_init(&bars->p_full[w], 128); mbar_init(&bars->sp_free[w], 1);
-            mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128);
+            mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128); mbar_init(&bars->x_full[w], 128);
         }
         bars->abort_flag = 0;
         mbar_init_fence();
     }
     // query rows that no load writes must hold finite numbers (their weights are zero)
-    for (int i = tid; i < 2 * kItQBytes / 16; i += kThreadsIt) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < NQ * kQTile / 16; i += kThreadsIt) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 1) { tmem_alloc(&bars->tmem_base, kTmemColsIt); tmem_relinquish(); }
     fence_async_smem();
     tc_fence_before();
@@ -118,89 +152,108 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
     };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ producer
+        // ------------------------------------------------------------------ aL tiles
         const uint32_t el = elect_one();
-        prefetch_tmap(&tal); prefetch_tmap(&tqr);
-        int g = 0, uc = 0;
+        prefetch_tmap(&tal);
+        int s = 0, ph = 1;
         bool ok = true;
-        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u, ++uc) {
+        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
+            const ItUnit un = it_decode(p, u);
+            for (int t = 0; t < n_tiles; ++t) {
+                if (!mbar_wait_u(&bars->a_empty[s], ph)) { fail(11); ok = false; break; }
+                unsigned char* st = a_s + s * kItTileBytes;
+                mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kItTileBytes);
+                tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKTile, un.bhl * p.na + un.al);
+                tma_load_4d_e(el, st + kKTile * 128, &tal, &bars->a_full[s], 64, un.j, t * kKTile, un.bhl * p.na + un.al);
+                if (++s == NA) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ query rows, log-sum-exps
+        const uint32_t el = elect_one();
+        prefetch_tmap(&tqr);
+        int qb = 0, ph = 1;
+        for (int u = u_begin; u < u_end && !bars->abort_flag; ++u) {
             const ItUnit un = it_decode(p, u);
             const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-            const int qb = uc & 1;
-            unsigned char* qd_s = q_s + qb * kItQBytes;
-            if (uc >= 2) {
-                if (!mbar_wait_u(&bars->q_empty[qb], ((uc >> 1) - 1) & 1)) { fail(10); break; }
+            unsigned char* qd_s = q_s + qb * kQTile;
+            constexpr int kL = (N_I + 31) / 32;
+            float l2[kL];
+            if (!ip.own_lse) {
+#pragma unroll
+                for (int c = 0; c < kL; ++c)
+                    l2[c] = c * 32 + lane < b1 ? kLog2e * p.lse[(long long)u * b1 + c * 32 + lane] : INFINITY;
             }
-            for (int i = lane; i < 128; i += 32)
-                bars->lse2[qb][i] = i < b1 ? kLog2e * p.lse[(long long)u * b1 + i] : INFINITY;
-            if (ip.q_rows_tma) {
+            if (!mbar_wait_u(&bars->q_empty[qb], ph)) { fail(10); break; }
+            if (!ip.own_lse) {
+#pragma unroll
+                for (int c = 0; c < kL; ++c)
+                    if (c * 32 + lane < N_I) bars->lse2[qb][c * 32 + lane] = l2[c];
                 __syncwarp();
-                {
-                    mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(b1 * 256));
-                    const int tok0 = blk.row_token(p.a0 + un.al, 0);
-                    const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
-                    tma_load_5d_e(el, qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
-                    tma_load_5d_e(el, qd_s + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
-                }
+            }
+            if (ip.q_rows_tma) {
+                mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(b1 * 256));
+                const int tok0 = blk.row_token(p.a0 + un.al, 0);
+                const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
+                tma_load_5d_e(el, qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
+                tma_load_5d_e(el, qd_s + kQHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
             } else {
                 const __nv_bfloat16* qg = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
                 for (int idx = lane; idx < b1 * 16; idx += 32) {
                     const int i = idx >> 4, ch = idx & 15;
                     const uint4 val = *reinterpret_cast<const uint4*>(
                         qg + (blk.row_token(p.a0 + un.al, i) + un.j) * tok_pitch + ch * 8);
-                    *reinterpret_cast<uint4*>(qd_s + (ch >> 3) * (128 * 128) + i * 128 + (((ch & 7) ^ (i & 7)) << 4)) = val;
+                    *reinterpret_cast<uint4*>(qd_s + (ch >> 3) * kQHalf + i * 128 + (((ch & 7) ^ (i & 7)) << 4)) = val;
                 }
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->q_full[qb]);
             }
-            {
-                for (int t = 0; t < n_tiles; ++t, ++g) {
-                    const int s = g % kAStg;
-                    if (g >= kAStg && !mbar_wait_u(&bars->a_empty[s], ((g / kAStg) - 1) & 1)) { fail(11); ok = false; break; }
-                    unsigned char* st = a_s + s * kItTileBytes;
-                    mbar_arrive_expect_tx_e(el, &bars->a_full[s], (uint32_t)kItTileBytes);
-                    tma_load_4d_e(el, st, &tal, &bars->a_full[s], 0, un.j, t * kKTile, un.bhl * p.na + un.al);
-                    tma_load_4d_e(el, st + kKTile * 128, &tal, &bars->a_full[s], 64, un.j, t * kKTile, un.bhl * p.na + un.al);
-                }
-            }
+            if (++qb == NQ) { qb = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        {
-            const uint32_t el = elect_one();
-            constexpr uint32_t idesc_s = idesc_bf16(128, N_I, 0, 0);
-            constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);
-            const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
-            const uint64_t qk_desc0 = smem_desc_sw128(smem_addr(q_s), 16, 1024);             // K-major (S GEMM)
-            const uint64_t qn_desc0 = smem_desc_sw128(smem_addr(q_s), 128 * 128, 1024);      // MN-major (aR GEMM)
-            const int total = (u_end - u_begin) * n_tiles;
-            bool ok = true;
-            auto issue_s = [&](int g) -> bool {                  // S^T of tile g
-                const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1, s = g % kAStg, qb = uc & 1;
-                if (t == 0 && !mbar_wait_u(&bars->q_full[qb], (uc >> 1) & 1)) { fail(20); return false; }
-                if (!mbar_wait_u(&bars->a_full[s], (g / kAStg) & 1)) { fail(21); return false; }
-                if (g >= 2 && !mbar_wait_u(&bars->sp_free[w], ((g >> 1) - 1) & 1)) { fail(22); return false; }
+        // ------------------------------------------------------------------ S^T GEMMs
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_s = idesc_bf16(128, N_I, 0, 0);
+        const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
+        const uint64_t q_desc0 = smem_desc_sw128(smem_addr(q_s), 16, 1024);              // K-major
+        int g = 0, qb = 0, qp = 0, s = 0, ph = 0;
+        bool ok = true;
+        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
+            if (!mbar_wait_u(&bars->q_full[qb], qp)) { fail(20); break; }
+            for (int t = 0; t < n_tiles; ++t, ++g) {
+                const int w = g & 1;
+                if (!mbar_wait_u(&bars->a_full[s], ph)) { fail(21); ok = false; break; }
+                if (g >= 2 && !mbar_wait_u(&bars->sp_free[w], ((g >> 1) - 1) & 1)) { fail(22); ok = false; break; }
                 tc_fence_after();
                 const uint64_t ad = a_desc0 + (uint64_t)((s * kItTileBytes) >> 4);
-                const uint64_t qd = qk_desc0 + (uint64_t)((qb * kItQBytes) >> 4);
+                const uint64_t qd = q_desc0 + (uint64_t)((qb * kQTile) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t off = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;
-                    mma_ss_e(el, tmem + it_col_s(w), ad + off, qd + off, idesc_s, ks > 0);
+                    const uint32_t ao = ((ks >> 2) * (kKTile * 128) + (ks & 3) * 32) >> 4;
+                    const uint32_t qo = ((ks >> 2) * kQHalf + (ks & 3) * 32) >> 4;
+                    mma_ss_e(el, tmem + it_col_s(w), ad + ao, qd + qo, idesc_s, ks > 0);
                 }
                 mma_commit_e(el, &bars->s_full[w]);
                 mma_commit_e(el, &bars->a_empty[s]);
-                return true;
-            };
-            if (total > 0) ok = issue_s(0);
-            for (int g = 0; ok && g < total && !bars->abort_flag; ++g) {
-                if (g + 1 < total && !issue_s(g + 1)) { ok = false; break; }
-                const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1, qb = uc & 1;
-                if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); break; }
-                if (g >= 2 && !mbar_wait_u(&bars->o_free[w], ((g >> 1) - 1) & 1)) { fail(24); break; }
+                if (++s == NA) { s = 0; ph ^= 1; }
+            }
+            if (++qb == NQ) { qb = 0; qp ^= 1; }
+        }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ aR GEMMs
+        const uint32_t el = elect_one();
+        constexpr uint32_t idesc_o = idesc_bf16(128, kHeadDim, 0, 1);
+        const uint64_t q_desc0 = smem_desc_sw128(smem_addr(q_s), kQHalf, 1024);          // MN-major
+        int g = 0, qb = 0;
+        bool ok = true;
+        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
+            for (int t = 0; t < n_tiles; ++t, ++g) {
+                const int w = g & 1;
+                if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); ok = false; break; }
+                if (g >= 2 && !mbar_wait_u(&bars->o_free[w], ((g >> 1) - 1) & 1)) { fail(24); ok = false; break; }
                 tc_fence_after();
-                const uint64_t qd = qn_desc0 + (uint64_t)((qb * kItQBytes) >> 4);
+                const uint64_t qd = q_desc0 + (uint64_t)((qb * kQTile) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < N_I / 16; ++kk)
                     mma_ts_e(el, tmem + it_col_o(w), tmem + it_col_s(w) + kk * 8, qd + ((kk * 2048) >> 4), idesc_o, kk > 0);
@@ -208,6 +261,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                 mma_commit_e(el, &bars->sp_free[w]);
                 if (t + 1 == n_tiles) mma_commit_e(el, &bars->q_empty[qb]);       // last read of this unit's query tile
             }
+            if (++qb == NQ) qb = 0;
         }
     } else if (warp >= 4 && warp < 12) {
         // ------------------------------------------------------------------ the two working warpgroups
@@ -218,17 +272,52 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
         const uint32_t s_t = tmem + lane_sel + it_col_s(w);
         const float scale_l2 = p.scale * kLog2e;
         const int total = (u_end - u_begin) * n_tiles;
-        bool ok = true;
-        for (int g = w; ok && g < total && !bars->abort_flag; g += 2) {
-            const int uc = g / n_tiles, t = g - uc * n_tiles, qb = uc & 1;
+        // bias of tile g's key on this lane, in log2 units; a key past the end gets weight zero
+        auto load_cl = [&](int g) -> float {
+            const int uc = g / n_tiles, key = (g - uc * n_tiles) * kKTile + row;
+            return g < total && key < n_keys ? kLog2e * p.cL[(long long)(u_begin + uc) * p.n_keys_c + key] : INFINITY;
+        };
+        float cl_next = load_cl(w);
+        for (int g = w; g < total && !bars->abort_flag; g += 2) {
+            const int uc = g / n_tiles, t = g - uc * n_tiles;
             const int u = u_begin + uc;
             const int key = t * kKTile + row;
             const bool valid = key < n_keys;
-            // bias of this key in log2 units; a key past the end gets weight zero
-            const float cl2 = valid ? kLog2e * p.cL[(long long)u * p.n_keys_c + key] : INFINITY;
-            if (!mbar_wait(&bars->s_full[w], (g >> 1) & 1)) { fail(31); break; }
+            const float cl2 = cl_next;
+            cl_next = load_cl(g + 2);
+            if (!mbar_wait_u(&bars->s_full[w], (g >> 1) & 1)) { fail(31); break; }
             tc_fence_after();
-            const float* lse2 = bars->lse2[qb];
+            const float* lse2 = bars->lse2[uc % NQ];
+            if (ip.own_lse) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < N_I; c0 += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(s_t + c0, r);
+                    tmem_wait_ld();
+                    float e[16], m = 0.f;                       // m: of query c0 + (lane & 15)
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        const float x = fmaf(__uint_as_float(r[c]), scale_l2, -cl2);
+                        const float mc = fmaxf(warp_max(x), -1e30f);        // finite also if none of these keys exists
+                        if ((lane & 15) == c) m = mc;
+                        e[c] = exp2f(x - mc);
+                    }
+                    const float sum = column_sums(e, lane);
+                    if (lane < 16) bars->part[w][quad][c0 + lane] = make_float2(m, sum);
+                }
+                mbar_arrive(&bars->x_full[w]);
+                if (!mbar_wait_u(&bars->x_full[w], (g >> 1) & 1)) { fail(32); break; }
+                float* own = bars->lse2_own[warp - 4];
+#pragma unroll
+                for (int c = lane; c < N_I; c += 32) {
+                    const float2 a = bars->part[w][0][c], b = bars->part[w][1][c], d = bars->part[w][2][c], e = bars->part[w][3][c];
+                    const float m = fmaxf(fmaxf(a.x, b.x), fmaxf(d.x, e.x));
+                    const float z = a.y * exp2f(a.x - m) + b.y * exp2f(b.x - m) + d.y * exp2f(d.x - m) + e.y * exp2f(e.x - m);
+                    own[c] = c < b1 ? m + __log2f(z) : INFINITY;
+                }
+                __syncwarp();
+                lse2 = own;
+            }
             float csum = 0.f;
 #pragma unroll 1
             for (int c0 = 0; c0 < N_I; c0 += 16) {
@@ -306,6 +395,10 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
 
 }  // namespace
 
+// The update takes the queries' log-sum-exps itself when the keys fit one tile: with more tiles it would have to go over them
+// twice, as the column step's pass before it does.
+bool l_iter_own_lse(const MonarchParams& p) { return p.n_keys <= kKTile; }
+
 // Launches the tensor-core iteration update for one chunk.  map_qrows = query rows, 5-D, box of b1 rows.
 int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* status, int num_sms, cudaStream_t s) {
     if (p.blk.b1 > 128) return SFM_ERR_UNSUPPORTED;
@@ -318,22 +411,23 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     CUtensorMap map_ar;
     if (int rc = make_bridge_tmap(&map_ar, p.aR, p.na * p.blk.b2, p.n_keys, p.nbh, 1, 32)) return rc;
     ip.q_rows_tma = (p.blk.f_tied == 1 || p.blk.h_reduce == 1) ? 1 : 0;
+    ip.own_lse = l_iter_own_lse(p);
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
-    auto go = [&](auto kernel) -> int {
-        if (int rc = opt_in_smem((const void*)kernel, kItSmemBytes)) return rc;
-        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, kItSmemBytes, s, map_al, *map_qrows, map_ar, ip);
+    auto go = [&](auto kernel, int smem) -> int {
+        if (int rc = opt_in_smem((const void*)kernel, smem)) return rc;
+        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, smem, s, map_al, *map_qrows, map_ar, ip);
     };
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {
-        case 16: rc = go(monarch_iter_tc_kernel<16>); break;
-        case 32: rc = go(monarch_iter_tc_kernel<32>); break;
-        case 48: rc = go(monarch_iter_tc_kernel<48>); break;
-        case 64: rc = go(monarch_iter_tc_kernel<64>); break;
-        case 80: rc = go(monarch_iter_tc_kernel<80>); break;
-        case 96: rc = go(monarch_iter_tc_kernel<96>); break;
-        case 112: rc = go(monarch_iter_tc_kernel<112>); break;
-        case 128: rc = go(monarch_iter_tc_kernel<128>); break;
+        case 16: rc = go(monarch_iter_tc_kernel<16>, it_smem_bytes<16>()); break;
+        case 32: rc = go(monarch_iter_tc_kernel<32>, it_smem_bytes<32>()); break;
+        case 48: rc = go(monarch_iter_tc_kernel<48>, it_smem_bytes<48>()); break;
+        case 64: rc = go(monarch_iter_tc_kernel<64>, it_smem_bytes<64>()); break;
+        case 80: rc = go(monarch_iter_tc_kernel<80>, it_smem_bytes<80>()); break;
+        case 96: rc = go(monarch_iter_tc_kernel<96>, it_smem_bytes<96>()); break;
+        case 112: rc = go(monarch_iter_tc_kernel<112>, it_smem_bytes<112>()); break;
+        case 128: rc = go(monarch_iter_tc_kernel<128>, it_smem_bytes<128>()); break;
         default: return SFM_ERR_UNSUPPORTED;
     }
     if (rc) return rc;

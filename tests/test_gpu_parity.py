@@ -251,6 +251,20 @@ def test_monarch_iterative_small(sfb, ci, iters):
     check_close(z, z_ref, f"{c['name']} T={iters}")
 
 
+# (h, w, f_tied, h_reduce, w_reduce, frames cached): 128 and 129 keys (one tile, two tiles), block rows of 16 to 120, query
+# rows that are gathered
+@pytest.mark.parametrize("edge", [(32, 8, 1, 1, 1, 4), (43, 8, 1, 1, 1, 3), (16, 16, 1, 1, 1, 8), (40, 6, 3, 1, 1, 3), (20, 8, 3, 2, 1, 3),
+                                  (3, 8, 1, 1, 1, 3)], ids=lambda e: "h{}w{}_ft{}hr{}wr{}_F{}".format(*e))
+def test_monarch_iterative_tile_edges(sfb, edge):
+    h, w, ft, hr, wr, frames = edge
+    rng = np.random.default_rng(h * 1000 + w)
+    n, n_kv = 3 * h * w, frames * h * w
+    mk = lambda *s: bf(cases.randn(rng, *s))
+    c = dict(blocking=(ft, hr, wr, h, w), q=mk(1, n, 3, 128), nk=mk(1, n, 3, 128), nv=mk(1, n, 3, 128),
+             kbuf=mk(1, n_kv, 3, 128), vbuf=mk(1, n_kv, 3, 128), start=n_kv - n, end=n_kv, n_kv=n_kv, sm_scale=128 ** -0.5)
+    check_close(run_gpu_cache(sfb, c, 3)[0], run_oracle_cache(c, 3)[0], str(edge))
+
+
 def test_monarch_baseline_config1_T20_vs_golden(sfb, golden):
     c = cases.c1_case()
     kc = torch.zeros(1, c["chunk"], 12, 128, dtype=torch.bfloat16, device="cuda")
