@@ -106,7 +106,7 @@ typedef struct SfmKvCall {
     const void *q, *k, *v, *norm_q_weight, *norm_k_weight;
     void *q_rot, *k_cache, *v_cache;
     const void *rope;
-    void *out, *workspace, *stream;
+    void *out, *workspace, *stream, *lse;
     int64_t q_batch_stride, cache_batch_stride;
     uint64_t workspace_bytes;
     float eps, sm_scale;
@@ -114,6 +114,8 @@ typedef struct SfmKvCall {
     int32_t f_tied, h_reduce, w_reduce, h, w, num_iters, dense, reserved;
 } SfmKvCall;
 int sfm_kv_attention(const void* call);
+/* lse (or null; Monarch attention with num_iters 1 and block rows up to 128): fp32 [B * H][n_q], every query's log-sum-exp
+ * over its column's keys, in the order (query group, column, block row) that sfm_monarch_bwd_natural takes. */
 
 /*
  * Stand-alone 3-axis RoPE of one tensor x [B, L, H, D] -> out (same shape): the first
@@ -364,11 +366,14 @@ int sfm_monarch_bwd(const void* q, int64_t q_batch_stride,
  * sfm_monarch_bwd in the form autograd wants it: dq [B, n_q, H, D] bf16 (the fp32 sum, rounded once), dk / dv with their
  * tokens in natural order.  The group range covers whole tied frame sets (multiples of h_reduce * w_reduce).  Returns
  * SFM_ERR_UNSUPPORTED, with nothing launched, for the shapes that sfm_monarch_bwd runs on its fp32 kernels.
+ * out, lse: the forward's output [B, n_q, H, D] and log-sum-exps (sfm_kv_attention); with both given the column step is not
+ * run again.
  * Replaces: the same, with the inverse permutation of dk / dv and the cast of dq that follow it
  * (wan/modules/monarch_attn.py:1462-1470).
  */
 int sfm_monarch_bwd_natural(const void* q, int64_t q_batch_stride,
                             const void* k_cache, const void* v_cache, int64_t kv_batch_stride,
+                            const void* out, const float* lse,
                             const void* dout, void* dq, void* dk, void* dv,
                             void* workspace, size_t workspace_bytes,
                             int B, int H, int D, int n_q, int n_kv,

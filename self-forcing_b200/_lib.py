@@ -44,7 +44,7 @@ SIGNATURES = {
     "sfm_monarch_bwd_workspace_bytes": (C.c_size_t, [C.c_int] * 10 + [C.c_size_t]),
     "sfm_monarch_bwd": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64] + [C.c_void_p] * 5 +
                         [C.c_size_t] + [C.c_int] * 10 + [C.c_float, C.c_int, C.c_int, C.c_int, C.c_size_t, C.c_void_p]),
-    "sfm_monarch_bwd_natural": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64] + [C.c_void_p] * 5 +
+    "sfm_monarch_bwd_natural": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64] + [C.c_void_p] * 7 +
                                 [C.c_size_t] + [C.c_int] * 10 + [C.c_float, C.c_int, C.c_int, C.c_size_t, C.c_void_p]),
     "sfm_workspace_status": (C.c_int, [C.c_void_p, C.c_void_p]),
     "sfm_static_scratch_status": (C.c_int, [C.c_void_p]),

@@ -96,7 +96,7 @@ struct OutShards {
 int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out, void* ws,
                 size_t ws_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce, int w_reduce,
                 int h, int w, float sm_scale, int num_iters, int causal_groups, size_t budget, cudaStream_t stream,
-                const OutShards* os = nullptr) {
+                const OutShards* os = nullptr, float* lse = nullptr) {
     if (!q || !kc || !vc || !ws) return SFM_ERR_NULL_POINTER;
     if (!os && !out) return SFM_ERR_NULL_POINTER;
     if (os) {
@@ -148,6 +148,7 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
     // for block rows up to 128 and block columns up to 64; everything else runs on the mma.sync kernels.
     const bool iter_tc = num_iters > 1 && pl.blk.b1 <= 128 && pl.blk.b2 <= kB2Max;
     const bool use_tc = (num_iters == 1 && (causal_groups == 0 || pl.blk.b1 <= 128)) || iter_tc;
+    if (lse && (num_iters != 1 || pl.blk.b1 > 128)) return SFM_ERR_UNSUPPORTED;
     // block columns above 64 exist on the tensor-core kernels only (single pass, block rows up to 128)
     if (pl.blk.b2 > kB2Max && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
     // only the tensor-core column step knows how to scatter its rows
@@ -216,7 +217,9 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
                 }
                 if (last) {
                     if (use_tc && pl.blk.b1 <= 128) {
-                        if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, 0))) return rc;
+                        // a chunk's rows are consecutive: whole (batch, head) pairs, or query groups of one
+                        if (lse) p.lse = lse + ((size_t)bh0 * pl.A + a0) * pl.blk.b1 * pl.blk.b2;
+                        if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
                     } else if ((rc = launch_l_step(p, 0, stream))) return rc;
                 } else if (iter_tc) {
                     // the column step's softmax statistics, unless the update takes them itself, then
@@ -239,11 +242,11 @@ namespace sfm {
 // Single-pass forward on the tensor-core kernels for the (batch, head) pairs [bh0, bh0 + nbh) with all query
 // groups at once, into caller-given bridge buffers (aL, Y: bf16 [bh_local * A + a][n_keys][b2][128], cL: fp32 [slab][n_keys_c],
 // slab = (bh_local * A + a) * b2 + j) and, optionally, the column step's log-sum-exp per query row
-// (lse: fp32 [slab][b1]).  The backward uses it to recompute what the forward did not keep.  Returns the launch
+// (lse: fp32 [slab][b1]); without `column` the row step only.  The backward uses it to recompute what the forward did not keep.  Returns the launch
 // parameters and the tensor maps of q, K, V and the query rows for the kernels that follow.
 int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out,
                      __nv_bfloat16* aL, __nv_bfloat16* Y, float* cL, float* lse, int* status, int B, int H, int n_q,
-                     int n_kv, const Blocking& blk, float scale, int bh0, int nbh, MonarchParams* p_out,
+                     int n_kv, const Blocking& blk, float scale, int bh0, int nbh, bool column, MonarchParams* p_out,
                      CUtensorMap* maps, cudaStream_t stream) {
     if (blk.b1 > 128 || blk.b2 > kB2MaxTc) return SFM_ERR_UNSUPPORTED;
     const int group = blk.b1 * blk.b2;
@@ -282,7 +285,7 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
     if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
     if ((rc = launch_r_step_tc(p, maps, n_s, status, 0, num_sms, stream))) return rc;
-    if ((rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
+    if (column && (rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
     *p_out = p;
     return SFM_OK;
 }
@@ -431,7 +434,7 @@ extern "C" int sfm_kv_attention(const void* call) {
                              c.stream);
     return run_monarch(q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.workspace, c.workspace_bytes, c.B, c.H, c.D,
                        c.n_q, c.n_kv, c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.sm_scale, c.num_iters, 0, 0,
-                       (cudaStream_t)c.stream);
+                       (cudaStream_t)c.stream, nullptr, (float*)c.lse);
 }
 
 // ---------------------------------------------------------------------------------------------

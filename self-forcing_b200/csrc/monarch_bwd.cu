@@ -38,7 +38,7 @@
 namespace sfm {
 int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out,
                      __nv_bfloat16* aL, __nv_bfloat16* Y, float* cL, float* lse, int* status, int B, int H, int n_q,
-                     int n_kv, const Blocking& blk, float scale, int bh0, int nbh, MonarchParams* p_out,
+                     int n_kv, const Blocking& blk, float scale, int bh0, int nbh, bool column, MonarchParams* p_out,
                      CUtensorMap* maps, cudaStream_t stream);
 int launch_bwd_delta(const void* dout, const void* out, float* delta, long long rows, cudaStream_t s);
 int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* delta, float* dcL, float* dq,
@@ -742,8 +742,9 @@ extern "C" size_t sfm_monarch_bwd_workspace_bytes(int B, int H, int D, int n_q, 
     return pl.total;
 }
 
-// train: dq is bf16 and the tokens of dk / dv are in natural order; tensor-core path only.
-static int monarch_bwd(bool train, const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
+// train: dq is bf16 and the tokens of dk / dv are in natural order; tensor-core path only.  out_fwd, lse_fwd: what the forward
+// left (both or neither).
+static int monarch_bwd(bool train, const void* out_fwd, const float* lse_fwd, const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
                        int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
                        size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
                        int w_reduce, int h, int w, float sm_scale, int kv_group_begin, int kv_group_end,
@@ -827,12 +828,14 @@ static int monarch_bwd(bool train, const void* q, int64_t q_batch_stride, const 
             if (train) p.dq = p.dq2;                          // the fp32 shares stay in the scratch
             MonarchParams mp;
             CUtensorMap maps[8];
+            const bool have_fwd = out_fwd && lse_fwd;
+            if (have_fwd) lse = const_cast<float*>(lse_fwd) + (size_t)bh0 * n_q;
             int rc = forward_tc_slice(q, q_batch_stride, k_cache, v_cache, kv_batch_stride, out_s, aLb, Yb, cL, lse, status,
-                                      B, H, n_q, n_kv, blk, sm_scale, bh0, nbh, &mp, maps, s);
+                                      B, H, n_q, n_kv, blk, sm_scale, bh0, nbh, !have_fwd, &mp, maps, s);
             if (rc) return rc;
             // delta = dOut . out for every (token, head); the scratch output holds this slice's heads only, the
             // other heads' products are never read
-            if ((rc = launch_bwd_delta(dout, out_s, delta, (long long)rows, s))) return rc;
+            if ((!have_fwd || bh0 == 0) && (rc = launch_bwd_delta(dout, have_fwd ? out_fwd : out_s, delta, (long long)rows, s))) return rc;
             // query rows of q and dOut for the column kernel: (d, head, column, row of the token grid, batch), boxes of
             // 32 consecutive grid rows (fewer when the whole call has fewer)
             {
@@ -889,17 +892,17 @@ extern "C" int sfm_monarch_bwd(const void* q, int64_t q_batch_stride, const void
                                size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
                                int w_reduce, int h, int w, float sm_scale, int kv_group_begin, int kv_group_end,
                                int causal_groups, size_t budget_bytes, void* stream) {
-    return monarch_bwd(false, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
+    return monarch_bwd(false, nullptr, nullptr, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
                        B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, kv_group_begin, kv_group_end,
                        causal_groups, budget_bytes, stream);
 }
 
 extern "C" int sfm_monarch_bwd_natural(const void* q, int64_t q_batch_stride, const void* k_cache, const void* v_cache,
-                                       int64_t kv_batch_stride, const void* dout, void* dq, void* dk, void* dv, void* workspace,
-                                       size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied,
+                                       int64_t kv_batch_stride, const void* out, const float* lse, const void* dout, void* dq,
+                                       void* dk, void* dv, void* workspace, size_t workspace_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied,
                                        int h_reduce, int w_reduce, int h, int w, float sm_scale, int kv_group_begin,
                                        int kv_group_end, size_t budget_bytes, void* stream) {
-    return monarch_bwd(true, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
+    return monarch_bwd(true, out, lse, q, q_batch_stride, k_cache, v_cache, kv_batch_stride, dout, dq, dk, dv, workspace, workspace_bytes,
                        B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, kv_group_begin, kv_group_end, 0,
                        budget_bytes, stream);
 }

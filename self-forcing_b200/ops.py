@@ -213,11 +213,11 @@ def _after_call(ws):
 
 
 # SfmKvCall of include/sfmonarch.h
-_KV_CALL = struct.Struct("@12P2qQ2f18i")
+_KV_CALL = struct.Struct("@13P2qQ2f18i")
 
 
 def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, sm_scale, num_iters, dense=False, rope=None,
-                  start_frame=0, wq=None, wk=None, eps=0.0, roll_dst=0, roll_shift=0):
+                  start_frame=0, wq=None, wk=None, eps=0.0, roll_dst=0, roll_shift=0, lse=None):
     """One call of the library: the new tokens' cache write (with ``rope``: normalised if weights are given, rotated, and q
     too), then attention over the cache view of ``n_kv`` tokens at ``kc_ptr`` / ``vc_ptr``.  The tensors have been checked;
     k, v (and q, if it is rotated) are contiguous."""
@@ -234,7 +234,7 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
         call = _KV_CALL.pack(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), 0 if wq is None else wq.data_ptr(), 0 if wk is None else wk.data_ptr(),
             0 if q_rot is None else q_rot.data_ptr(), kc_ptr, vc_ptr, 0 if rope is None else rope.data_ptr(), out.data_ptr(),
-            0 if dense else ws.data_ptr(), stream, q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws.numel(),
+            0 if dense else ws.data_ptr(), stream, 0 if lse is None else lse.data_ptr(), q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws.numel(),
             eps, sm_scale, B, H, D, n_q, k.shape[1], n_kv, start_idx, roll_dst, roll_shift, start_frame, *blocking, num_iters,
             dense, 0)
         rc = _lib.load().sfm_kv_attention(call)
@@ -299,9 +299,9 @@ def _bwd_workspace(q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes=0):
     return _workspace(q.device, max(int(nbytes), 256), "monarch_bwd")
 
 
-def _backward_natural(q, k_cache, v_cache, grad_out, blocking, sm_scale, g0, g1):
+def _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1):
     """(dq bf16, dk, dv with their tokens in natural order) of the cached groups [g0, g1), or None for shapes the
-    tensor-core backward does not take.  The tensors are those a forward call of this module has accepted."""
+    tensor-core backward does not take.  out, lse: what the forward left, or None.  The tensors are those a forward call of this module has accepted."""
     B, n_q, H, D = q.shape
     n_kv = k_cache.shape[1]
     q, grad_out = _as_token_major(q), grad_out.contiguous()
@@ -311,9 +311,10 @@ def _backward_natural(q, k_cache, v_cache, grad_out, blocking, sm_scale, g0, g1)
     dk = torch.empty((B, (g1 - g0) * (f_tied * h * w) // (h_reduce * w_reduce), H, D), dtype=q.dtype, device=q.device)
     dv = torch.empty_like(dk)
     rc = _lib.load().sfm_monarch_bwd_natural(
-        q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), grad_out.data_ptr(),
-        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce,
-        h, w, float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1, 0, _raw_stream(q.get_device()))
+        q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache),
+        None if out is None else out.data_ptr(), None if lse is None else lse.data_ptr(), grad_out.data_ptr(), dq.data_ptr(),
+        dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w,
+        float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1, 0, _raw_stream(q.get_device()))
     if rc == _ERR_UNSUPPORTED:
         return None
     _lib.check(rc, "sfm_monarch_bwd_natural")
@@ -343,10 +344,17 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, new_k, new_v, k_cache, v_cache, start_idx, end_idx, blocking, sm_scale, grad_only_new_kv):
         f_tied, h_reduce, w_reduce, h, w = blocking
+        # the backward of the new tokens' gradients takes the queries' log-sum-exps and the output from here (block rows that
+        # its kernels do not take have no use for them)
+        lse = None
+        if grad_only_new_kv and f_tied * h <= 96 * h_reduce:
+            lse = torch.empty(q.shape[:-1], dtype=torch.float32, device=q.device)
         out = monarch_attn_with_kv_cache(q.detach(), k_cache.detach(), v_cache.detach(), new_k.detach(), new_v.detach(),
                                          start_idx, end_idx, f_tied, h_reduce, w_reduce, h, w, sm_scale, 1,
-                                         _no_grad=True)
+                                         _no_grad=True, _lse=lse)
         ctx.save_for_backward(q, k_cache, v_cache)
+        # not a saved tensor: the caller may change the output in place, and the backward then does without it
+        ctx.forward_out = (out.detach(), out._version, lse) if lse is not None else None
         ctx.args = (int(start_idx), int(end_idx), blocking, sm_scale, bool(grad_only_new_kv))
         return out
 
@@ -361,7 +369,10 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
         g0, g1 = (0, n_kv // group) if want_cache else (start // group, -(-end // group))
         grad_out = grad_out.to(q.dtype)
         if not want_cache and start % (f_tied * h * w) == 0:
-            grads = _backward_natural(q, k_cache, v_cache, grad_out, blocking, sm_scale, g0, g1)
+            out, version, lse = ctx.forward_out or (None, 0, None)
+            if out is not None and out._version != version:
+                out = lse = None
+            grads = _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1)
             if grads is not None:
                 return (*grads, None, None, None, None, None, None, None)
         dq, dk, dv = monarch_attn_with_kv_cache_backward(q, k_cache, v_cache, grad_out, f_tied, h_reduce,
@@ -400,7 +411,7 @@ class _MonarchNoCacheFn(torch.autograd.Function):
 
 # ------------------------------------------------------------------------------------- public
 def monarch_attn_with_kv_cache(q, k_cache, v_cache, new_k, new_v, start_idx, end_idx, f_tied, h_reduce, w_reduce,
-                               h, w, sm_scale=None, num_iters=1, grad_only_new_kv=False, _no_grad=False):
+                               h, w, sm_scale=None, num_iters=1, grad_only_new_kv=False, _no_grad=False, _lse=None):
     """Same contract as the reference's monarch_attn_with_kv_cache (monarch_attn.py:1778-1796):
     new_k / new_v are written, in Monarch block order, into k_cache / v_cache[:, start_idx:end_idx]
     IN PLACE, then q attends the whole cache view.  q, new_k, new_v: [B, n, H, 128] bf16 (already
@@ -434,7 +445,7 @@ def monarch_attn_with_kv_cache(q, k_cache, v_cache, new_k, new_v, start_idx, end
     new_v = new_v.contiguous()
     _mark_written(k_cache, v_cache)
     return _kv_attention(q, new_k, new_v, k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), k_cache.shape[1],
-                         int(start_idx), (f_tied, h_reduce, w_reduce, h, w), float(sm_scale), int(num_iters))
+                         int(start_idx), (f_tied, h_reduce, w_reduce, h, w), float(sm_scale), int(num_iters), lse=_lse)
 
 
 def norm_rope_cache_write(q, k, v, k_cache, v_cache, start_idx, start_frame, f_tied, h_reduce, w_reduce, h, w,

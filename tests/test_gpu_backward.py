@@ -161,17 +161,20 @@ def test_backward_group_range(sfb):
     assert dk3.shape[1] == 0 and dv3.shape[1] == 0
 
 
+@pytest.mark.parametrize("change_out", [False, True])
 @pytest.mark.parametrize("blocking,frames_q,cached", [((1, 1, 1, 4, 24), 1, 3), ((1, 2, 4, 6, 48), 3, 4), ((2, 1, 1, 33, 16), 2, 3),
                                                       ((1, 1, 1, 5, 64), 3, 3)])
-def test_natural_order_backward(sfb, blocking, frames_q, cached):
+def test_natural_order_backward(sfb, blocking, frames_q, cached, change_out):
     """The training call's gradients (dq in bf16, dk / dv of the new tokens in natural order) are those of the full
-    backward, cast and permuted."""
+    backward, cast and permuted, also when the caller changes the output in place before the backward."""
     c = make_case(blocking, frames_q, cached, B=2, H=2, seed=8480)
     _, kv, vv = gpu_cache(sfb, c)
     dq, dk, dv = sfb.monarch_attn_with_kv_cache_backward(c["q"].cuda(), kv, vv, c["g"].cuda(), *blocking, sm_scale=c["sm_scale"])
     leaves = [c[n].cuda().requires_grad_() for n in ("q", "nk", "nv")]
     z = sfb.monarch_attn_with_kv_cache(leaves[0], kv, vv, *leaves[1:], c["start"], c["end"], *blocking, sm_scale=c["sm_scale"],
                                        grad_only_new_kv=True)
+    if change_out:
+        z.mul_(1.0)
     z.backward(c["g"].cuda())
     ft, hr, wr, h, w = blocking
     assert torch.equal(leaves[0].grad, bf(dq))
