@@ -120,18 +120,20 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     // Keys a unit may see, and the tiles a group of units has to walk.  Block-causal (no-cache path): a unit sees the
     // cached groups up to the end of its own causal block; its tiles past that are neither loaded nor multiplied, and
     // the keys past it within its last tile get weight zero (the row step leaves finite values there).
-    auto unit_keys = [&](int u) -> int {
-        if (!kCausal) return p.n_keys;
-        const int a_abs = p.a0 + (u / b2) % p.na;
-        return min(p.F, (a_abs / p.causal_groups + 1) * p.causal_groups) * b1;
+    auto group_keys = [&](int al) -> int {                 // of query group al of the slice
+        return kCausal ? min(p.F, ((p.a0 + al) / p.causal_groups + 1) * p.causal_groups) * b1 : p.n_keys;
     };
-    auto group_tiles = [&](int u0, int nu) -> int {
-        int most = p.n_keys;
-        if (kCausal) {
-            most = 0;
-            for (int us = 0; us < nu; ++us) most = max(most, unit_keys(u0 + us));
-        }
-        return (most + kt - 1) / kt;
+    // The units of a group belong to one query group or to two (U <= b2 if block-causal): the second from unit `split` on.
+    // Worked out once per group: with four integer divisions per tile and unit in every role, a block-causal clip of 12 frames,
+    // 12 heads took 267 us, without 214.
+    struct GroupKeys { int first, second, split; __device__ __forceinline__ int of(int us) const { return us < split ? first : second; } };
+    auto keys_of = [&](int u0) -> GroupKeys {
+        if (!kCausal) return {p.n_keys, p.n_keys, kMaxU};
+        const int slab = u0 / b2, al = slab % p.na;
+        return {group_keys(al), group_keys(al + 1 == p.na ? 0 : al + 1), b2 - (u0 - slab * b2)};
+    };
+    auto group_tiles = [&](const GroupKeys& gk, int nu) -> int {
+        return ((kCausal && gk.split < nu ? max(gk.first, gk.second) : gk.first) + kt - 1) / kt;
     };
     // this CTA's contiguous share of the unit list, walked in groups of at most U units
     const int u_begin = (int)((long long)lp.n_units * blockIdx.x / gridDim.x);
@@ -188,7 +190,8 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         int sa = 0, pa = 1, gt = 0;              // ring slot and its phase, tiles of all groups so far
         bool ok = true;
         for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            const GroupKeys gk = keys_of(u0);
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int cslot = gt & 3;
                 if (!mbar_wait_u(&bars->cl_empty[cslot], ((gt >> 2) & 1) ^ 1)) { fail(13); ok = false; break; }
@@ -198,7 +201,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                     bulk_load_e(el, bars->cl[cslot][us], p.cL + (long long)(u0 + us) * p.n_keys_c + t * kt, (uint32_t)(have * 4),
                                 &bars->cl_full[cslot]);
                 for (int us = 0; us < nu; ++us) {
-                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (kCausal && t * kt >= gk.of(us)) continue;
                     if (!mbar_wait_u(&bars->a_empty[sa], pa)) { fail(11); ok = false; break; }
                     const LUnit un = decode_unit(p, u0 + us);
                     unsigned char* at = a_s + sa * tile_bytes;
@@ -216,10 +219,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
             int sy = 0, py = 1;
             bool ok = true;
             for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
-                const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+                const GroupKeys gk = keys_of(u0);
+                const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
                 for (int t = 0; ok && t < n_tiles; ++t)
                     for (int us = 0; us < nu; ++us) {
-                        if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                        if (kCausal && t * kt >= gk.of(us)) continue;
                         if (!mbar_wait_u(&bars->y_empty[sy], py)) { fail(12); ok = false; break; }
                         const LUnit un = decode_unit(p, u0 + us);
                         unsigned char* yt = y_s + sy * tile_bytes;
@@ -273,13 +277,14 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         bool ok = true;
         if (u_begin < u_end) load_q(u_begin);
         for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            const GroupKeys gk = keys_of(u0);
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
             if (!mbar_wait_u(&bars->q_full, gc & 1)) { fail(20); break; }
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;
                 if (!mbar_wait_u(&bars->sp_free[w], ((gt >> 1) & 1) ^ 1)) { fail(25); ok = false; break; }
                 for (int us = 0; us < nu; ++us) {
-                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (kCausal && t * kt >= gk.of(us)) continue;
                     if (!mbar_wait_u(&bars->a_full[sa], pa)) { fail(21); ok = false; break; }
                     tc_fence_after();
                     const uint64_t ad = a_desc0 + (uint64_t)((sa * tile_bytes) >> 4);
@@ -312,14 +317,15 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         int sy = 0, py = 0, gc = 0, gt = 0, used[2] = {0, 0};     // groups that accumulator w has taken part in
         bool ok = true;
         for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            const GroupKeys gk = keys_of(u0);
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;
                 if (!mbar_wait_u(&bars->p_full[w], (gt >> 1) & 1)) { fail(22); ok = false; break; }
                 // first GEMM of the group into this accumulator overwrites it: the last result there must have been read
                 if (t < 2 && !mbar_wait_u(&bars->o_free[w], (used[w]++ & 1) ^ 1)) { fail(23); ok = false; break; }
                 for (int us = 0; us < nu && !lp.lse_only; ++us) {
-                    if (kCausal && t * kt >= unit_keys(u0 + us)) continue;
+                    if (kCausal && t * kt >= gk.of(us)) continue;
                     if (!mbar_wait_u(&bars->y_full[sy], py)) { fail(26); ok = false; break; }
                     tc_fence_after();
                     const uint64_t yd = y_desc0 + (uint64_t)((sy * tile_bytes) >> 4);
@@ -352,8 +358,9 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         int gt0 = 0, used = 0;                // tiles of the groups before this one; groups this warpgroup has taken part in
         bool ok = true;
         for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += U) {
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
-            const int my_keys = us < nu ? unit_keys(u0 + us) : p.n_keys;
+            const GroupKeys gk = keys_of(u0);
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int my_keys = us < nu ? gk.of(us) : p.n_keys;
             float m_run = -INFINITY, l_run = 0.f;
             int my_tiles = 0;
             for (int t = (gt0 & 1) ^ w; ok && t < n_tiles; t += 2) {
@@ -476,7 +483,8 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         int gc = 0, gt0 = 0;
         for (int u0 = u_begin; u0 < u_end && !bars->abort_flag; u0 += U, ++gc) {
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(u0, nu);
+            const GroupKeys gk = keys_of(u0);
+            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
             if (!mbar_wait(&bars->o_full[gc & 1], (gc >> 1) & 1)) { fail(41); break; }
             tc_fence_after();
             // the group's first tile went to warpgroup w_a, its second, if any, to the other; a row without a weight there
@@ -541,10 +549,25 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
 
 }  // namespace
 
-// Keys per tile of the column step: what 128-key tiles would take, divided evenly over them.
-int l_tile_keys(int n_keys) {
-    const int tiles = (n_keys + kKT - 1) / kKT;
-    return (((n_keys + tiles - 1) / tiles) + 15) & ~15;
+// Keys per tile of the column step: what 128-key tiles would take, divided evenly over them.  Block-causal units see 1, 2, ...
+// causal blocks of keys, and the row step writes what the tiles that they reach hold: there the size that holds least, a
+// tile counting as 8 keys more than it has (12 frames of 30 x 52 in blocks of three, 90 keys: 96 a tile instead of 128, 17 % less).
+int l_tile_keys(const MonarchParams& p) {
+    const int even = (p.n_keys + kKT - 1) / kKT;
+    int best = (((p.n_keys + even - 1) / even) + 15) & ~15;
+    if (p.causal_groups > 0) {
+        long long least = 0;
+        for (int kt = kKT; kt >= 64; kt -= 16) {
+            long long held = 0;
+            for (int keys = 0; keys < p.n_keys;) {
+                keys = keys + p.causal_groups * p.blk.b1 < p.n_keys ? keys + p.causal_groups * p.blk.b1 : p.n_keys;
+                const int tiles = (keys + kt - 1) / kt;
+                held += (tiles * kt < p.n_keys ? tiles * kt : p.n_keys) + 8 * tiles;
+            }
+            if (kt == kKT || held < least) { least = held; best = kt; }
+        }
+    }
+    return best;
 }
 
 // Launches the tensor-core column step for one chunk as a persistent grid.  map_qrows = query rows, 5-D, box of b1 rows.
@@ -558,8 +581,9 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     const int share = (lp.n_units + num_sms - 1) / num_sms;
     lp.U = 128 / p.blk.b1 < kMaxU ? 128 / p.blk.b1 : kMaxU;
     if (lp.U > share) lp.U = share;
+    if (p.causal_groups > 0 && lp.U > p.blk.b2) lp.U = p.blk.b2;
     lp.R = 128 / lp.U;
-    lp.kt = l_tile_keys(p.n_keys);
+    lp.kt = l_tile_keys(p);
     // A value tile stays until its softmax and GEMM are done, a key tile only until its GEMM: two slots of five for keys
     const int slots = kRing / (lp.kt * 256);
     lp.n_a = (slots * 2 + 4) / 5 < kMaxStages ? (slots * 2 + 4) / 5 : kMaxStages;

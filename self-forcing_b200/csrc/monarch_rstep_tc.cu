@@ -541,7 +541,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 
 // Launches the tensor-core row step for one chunk as a persistent grid.  `status` is a device int the
 // kernel sets on an internal timeout.
-int l_tile_keys(int n_keys);
+int l_tile_keys(const MonarchParams& p);
 
 int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or the aR state), k, v */, int n_s, int* status,
                      int clear_status, int num_sms, cudaStream_t s) {
@@ -551,7 +551,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     const int b2 = p.blk.b2;
     rp.rows_per_group = b2 <= 16 ? 16 : (b2 <= 32 ? 32 : (b2 <= 64 ? 64 : 128));
     rp.groups_per_tile = kTileRows / rp.rows_per_group;
-    rp.col_kt = l_tile_keys(p.n_keys);
+    rp.col_kt = l_tile_keys(p);
     rp.tiles = (p.na + rp.groups_per_tile - 1) / rp.groups_per_tile;
     {
         // Persistent CTAs take whole units round-robin, so the launch lasts (units per CTA, rounded up) x (steps per

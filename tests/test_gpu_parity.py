@@ -325,6 +325,17 @@ def test_block_causal_does_not_read_old_scratch(sfb, grid):
 
 
 # ------------------------------------------------------------------------------- no-cache entry point
+# (h, w, frames): fewer block columns than a column tile takes units (4, 3), groups of units across query groups and across
+# heads, 3 h keys a causal block in tiles of 64 to 128
+@pytest.mark.parametrize("grid", [(16, 4, 9), (9, 3, 12), (30, 11, 12), (22, 9, 6), (43, 5, 9)], ids=lambda g: "h{}w{}_F{}".format(*g))
+def test_block_causal_unit_groups(sfb, grid):
+    h, w, frames = grid
+    rng = np.random.default_rng(h * 100 + w)
+    q, k, v = (bf(cases.randn(rng, 2, frames * h * w, 3, 128)) for _ in range(3))
+    got = sfb.monarch_attn(q.cuda(), k.cuda(), v.cuda(), 1, 1, 1, h, w, block_causal_size=3 * h * w)
+    check_close(got, orc.monarch_attn(q.float(), k.float(), v.float(), 1, 1, 1, h, w, block_causal_size=3 * h * w), str(grid))
+
+
 @pytest.mark.parametrize("ci", range(4))
 def test_monarch_nocache_and_block_causal(sfb, ci):
     name, ft, hr, wr, h, w = cases.SMALL_BLOCKINGS[ci]
