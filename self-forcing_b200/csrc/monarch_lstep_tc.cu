@@ -135,9 +135,18 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     auto group_tiles = [&](const GroupKeys& gk, int nu) -> int {
         return ((kCausal && gk.split < nu ? max(gk.first, gk.second) : gk.first) + kt - 1) / kt;
     };
-    // this CTA's contiguous share of the unit list, walked in groups of at most U units
-    const int u_begin = (int)((long long)lp.n_units * blockIdx.x / gridDim.x);
-    const int u_end = (int)((long long)lp.n_units * (blockIdx.x + 1) / gridDim.x);
+    // This CTA's groups, of U consecutive units each: the grid goes through the unit list together, from its end, one group per
+    // CTA a round, and the units left over are dealt out evenly.
+    // Neighbouring columns, whose bridge rows are neighbours in memory, are then read at the same time, and what the row step
+    // wrote last is read first, partly from L2: against a contiguous share per CTA the clip above went from 502 to 475 us, 40
+    // heads with 21 frames from 1052 to 1030, 12 frames from 225 to 222.
+    const int round = (int)gridDim.x * U, n_full = lp.n_units / round, rest = lp.n_units - n_full * round;
+    const int rest0 = (int)((long long)rest * blockIdx.x / gridDim.x), rest1 = (int)((long long)rest * (blockIdx.x + 1) / gridDim.x);
+    const int n_my = n_full + (rest1 > rest0 ? 1 : 0);
+    auto group_at = [&](int gi, int& nu) -> int {          // first unit and number of units
+        nu = gi < n_full ? U : rest1 - rest0;
+        return gi < n_full ? lp.n_units - (gi + 1) * round + (int)blockIdx.x * U : rest0;
+    };
 
     if (warp == 2 && lane == 0) { prefetch_tmap(&tqr); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
@@ -189,9 +198,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const uint32_t el = elect_one();
         int sa = 0, pa = 1, gt = 0;              // ring slot and its phase, tiles of all groups so far
         bool ok = true;
-        for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
+        for (int gi = 0; ok && gi < n_my; ++gi) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int n_tiles = group_tiles(gk, nu);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int cslot = gt & 3;
                 if (!mbar_wait_u(&bars->cl_empty[cslot], ((gt >> 2) & 1) ^ 1)) { fail(13); ok = false; break; }
@@ -218,9 +229,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
             const uint32_t el = elect_one();
             int sy = 0, py = 1;
             bool ok = true;
-            for (int u0 = u_begin; ok && u0 < u_end; u0 += U) {
+            for (int gi = 0; ok && gi < n_my; ++gi) {
+                int nu;
+                const int u0 = group_at(gi, nu);
                 const GroupKeys gk = keys_of(u0);
-                const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+                const int n_tiles = group_tiles(gk, nu);
                 for (int t = 0; ok && t < n_tiles; ++t)
                     for (int us = 0; us < nu; ++us) {
                         if (kCausal && t * kt >= gk.of(us)) continue;
@@ -240,8 +253,9 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const uint32_t idesc_s = idesc_bf16(128, 0, 0, 0) | ((uint32_t)(kt >> 3) << 17);
         const uint64_t q_desc = smem_desc_sw128(smem_addr(q_s), 16, 1024);
         const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
-        auto load_q = [&](int u0) {
-            const int nu = min(U, u_end - u0);
+        auto load_q = [&](int gi) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             if (lp.q_rows_tma) {
                 // the 128-byte swizzle is a function of the shared-memory address, so a box may land on any tile row
                 mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(nu * b1 * 256));
@@ -275,10 +289,12 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         };
         int sa = 0, pa = 0, gc = 0, gt = 0;
         bool ok = true;
-        if (u_begin < u_end) load_q(u_begin);
-        for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
+        if (n_my > 0) load_q(0);
+        for (int gi = 0; ok && gi < n_my; ++gi, ++gc) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int n_tiles = group_tiles(gk, nu);
             if (!mbar_wait_u(&bars->q_full, gc & 1)) { fail(20); break; }
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;
@@ -302,10 +318,10 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                 mma_commit_e(el, &bars->s_full[w]);
             }
             if (!ok) break;
-            if (u0 + U < u_end) {
+            if (gi + 1 < n_my) {
                 mma_commit_e(el, &bars->q_empty);
                 if (!mbar_wait_u(&bars->q_empty, gc & 1)) { fail(10); break; }
-                load_q(u0 + U);
+                load_q(gi + 1);
             }
         }
     } else if (warp == 1) {
@@ -316,9 +332,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const int n_k = kt / 16;
         int sy = 0, py = 0, gc = 0, gt = 0, used[2] = {0, 0};     // groups that accumulator w has taken part in
         bool ok = true;
-        for (int u0 = u_begin; ok && u0 < u_end; u0 += U, ++gc) {
+        for (int gi = 0; ok && gi < n_my; ++gi, ++gc) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int n_tiles = group_tiles(gk, nu);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;
                 if (!mbar_wait_u(&bars->p_full[w], (gt >> 1) & 1)) { fail(22); ok = false; break; }
@@ -357,9 +375,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const uint64_t scale2 = f2_pack(scale_l2, scale_l2), nl2 = f2_pack(-kLog2e, -kLog2e);
         int gt0 = 0, used = 0;                // tiles of the groups before this one; groups this warpgroup has taken part in
         bool ok = true;
-        for (int u0 = u_begin; ok && u0 < u_end && !bars->abort_flag; u0 += U) {
+        for (int gi = 0; ok && gi < n_my && !bars->abort_flag; ++gi) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int n_tiles = group_tiles(gk, nu);
             const int my_keys = us < nu ? gk.of(us) : p.n_keys;
             float m_run = -INFINITY, l_run = 0.f;
             int my_tiles = 0;
@@ -482,9 +502,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const int us = row / R, i_row = row - us * R;                // unit slot and query index of this tile row
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         int gc = 0, gt0 = 0;
-        for (int u0 = u_begin; u0 < u_end && !bars->abort_flag; u0 += U, ++gc) {
+        for (int gi = 0; gi < n_my && !bars->abort_flag; ++gi, ++gc) {
+            int nu;
+            const int u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
-            const int nu = min(U, u_end - u0), n_tiles = group_tiles(gk, nu);
+            const int n_tiles = group_tiles(gk, nu);
             if (!mbar_wait(&bars->o_full[gc & 1], (gc >> 1) & 1)) { fail(41); break; }
             tc_fence_after();
             // the group's first tile went to warpgroup w_a, its second, if any, to the other; a row without a weight there
