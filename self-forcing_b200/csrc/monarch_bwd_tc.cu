@@ -23,8 +23,8 @@
 // / odd (tile, chunk) steps (element-wise pass), 12-15 = drain warpgroup: a tile's dY / daL, rounded, into the shared memory of
 // its Y / aL tile, which nothing reads any more, and from there by TMA store over Y / aL; dcL; after a slab's last tile its
 // dq.  The issuer takes the next step's S GEMMs before this step's gradient GEMMs only if that tile is already there: the tile
-// ring has two stages, and a stage is free again when its tile's results have left it.  Persistent CTAs over contiguous shares
-// of the slab list.  All waits are bounded and report through the status word.
+// ring has two stages, and a stage is free again when its tile's results have left it.  Persistent CTAs, one slab each a
+// round.  All waits are bounded and report through the status word.
 //
 // What bounds it: the bridge, read and written (378 + 318 MB at 4680 queries, 18720 cached tokens, 12 heads).  With the results
 // stored one 256-byte row per lane by the element-wise warpgroups, between two of their steps, and one warp loading tiles and
@@ -124,9 +124,12 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
     const int b1 = blk.b1;
     const int n_keys = p.n_keys;
     const int n_tiles = (n_keys + kKB - 1) / kKB;
-    const int u_begin = (int)((long long)p.n_units * blockIdx.x / gridDim.x);
-    const int u_end = (int)((long long)p.n_units * (blockIdx.x + 1) / gridDim.x);
-    const int total = (u_end - u_begin) * n_tiles * NC;            // (slab, tile, chunk) steps of this CTA
+    // The grid goes through the slabs together, from the last one: neighbouring columns are neighbours in the bridge, what the
+    // row step wrote last is read first, and what is written last here the row step's backward reads first
+    // (all backward kernels at the size above 289 -> 282 us against a contiguous share per CTA).
+    const int n_my = (p.n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    auto unit_at = [&](int uc) -> int { return p.n_units - 1 - (uc * (int)gridDim.x + (int)blockIdx.x); };
+    const int total = n_my * n_tiles * NC;                         // (slab, tile, chunk) steps of this CTA
     constexpr int kQBufs = NC == 1 ? 2 : 1;
 
     if (tid == 0) {
@@ -161,8 +164,8 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
         prefetch_tmap(&tal); prefetch_tmap(&ty); prefetch_tmap(&sal); prefetch_tmap(&sy);
         int g = 0;                                               // tiles loaded
         bool ok = true;
-        for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
-            const BUnit un = b_decode(p, u);
+        for (int uc = 0; ok && uc < n_my && !bars->abort_flag; ++uc) {
+            const BUnit un = b_decode(p, unit_at(uc));
             const int grp = un.bhl * p.A + un.a;
             for (int t = 0; t < n_tiles; ++t, ++g) {
                 const int s = g % kStgB;
@@ -179,8 +182,8 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
         // ------------------------------------------------------------------ query side: rows of q and dOut, lse, delta
         const uint32_t el = elect_one();
         prefetch_tmap(&tqr); prefetch_tmap(&tdo);
-        int uc = 0;                                              // slabs started
-        for (int u = u_begin; u < u_end && !bars->abort_flag; ++u, ++uc) {
+        for (int uc = 0; uc < n_my && !bars->abort_flag; ++uc) {
+            const int u = unit_at(uc);
             const BUnit un = b_decode(p, u);
             const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
             const int qb = kQBufs == 2 ? (uc & 1) : 0;
@@ -311,7 +314,7 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
         unsigned char* ds_row = ds_s + w * kDsTile + row * 128;
         auto load_cl = [&](int g) -> float {                    // step g's bias of this thread's key
             const int gt = g / NC, uc = gt / n_tiles, key = (gt - uc * n_tiles) * kKB + row;
-            return g < total && key < n_keys ? kLog2e * p.cL[(long long)(u_begin + uc) * p.n_keys_c + key] : INFINITY;
+            return g < total && key < n_keys ? kLog2e * p.cL[(long long)unit_at(uc) * p.n_keys_c + key] : INFINITY;
         };
         float cl_next = load_cl(w);
         for (int g = w; g < total && !bars->abort_flag; g += 2) {
@@ -358,10 +361,10 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                       // TMEM lane: key within the tile (d for dq)
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-        const int n_gt = (u_end - u_begin) * n_tiles;
+        const int n_gt = n_my * n_tiles;
         for (int gt = 0; gt < n_gt && !bars->abort_flag; ++gt) {
             const int uc = gt / n_tiles, t = gt - uc * n_tiles, s = gt % kStgB;
-            const int u = u_begin + uc;
+            const int u = unit_at(uc);
             const BUnit un = b_decode(p, u);
             const int key0 = t * kKB + quad * 32;
             if (!mbar_wait_u(&bars->acc_full, gt & 1)) { fail(41); break; }
