@@ -95,7 +95,6 @@ __host__ __device__ constexpr int b_smem_bytes(int nc) {
     return 1024 + qd_bytes(nc) + kStgB * kBStage + 2 * kDsTile + (int)sizeof(BBarriers) + 64;
 }
 
-__device__ __forceinline__ void tmem_st16b(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
 struct BUnit { int bhl, a, j; };
 __device__ __forceinline__ BUnit b_decode(const BwdColParams& p, int u) {
     BUnit r;
@@ -343,8 +342,8 @@ monarch_bwd_col_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_
                 pp[cc >> 1] = pack_bf16(p0, p1);
                 pd[cc >> 1] = pack_bf16(d0 * p.scale, d1 * p.scale);
             }
-            tmem_st16b(tmem + lane_sel + bc_s(w), pp);
-            tmem_st16b(tmem + lane_sel + bc_dp(w), pd);
+            tmem_st16(tmem + lane_sel + bc_s(w), pp);
+            tmem_st16(tmem + lane_sel + bc_dp(w), pd);
             // bf16 copy of this key's (scale dS) row for the dq GEMM: 64 bytes of data, 128-byte swizzled row
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
