@@ -16,7 +16,7 @@
 //                                   127 get what lies behind the copy and are never read), B = the row tiles read
 //                                   MN-major; only for the cached groups whose dK / dV are wanted, which come first where they are the
 //                                   last ones
-// dK / dV of a (f, k) get one contribution per tile of query groups: each tile writes fp32 partials to its own
+// dK / dV of a (f, k) get one contribution per tile of query groups: with more than one, each tile writes fp32 partials to its own
 // buffer and a small kernel adds them in a fixed order and rounds to bf16 (no atomics).  dQ rows are owned by one
 // unit each and added to what the column step's backward left in dq.
 //
@@ -60,6 +60,9 @@ struct BwdRowParams {
     __nv_bfloat16* dq_bf16;        // the sum goes here, rounded, instead of back to dq (null: back to dq)
     float* part_k;                 // [tile][nbh][n_sel tokens][128] fp32 partial dK (n_sel = (g1 - g0) * b1 * b2)
     float* part_v;
+    __nv_bfloat16* dk;             // the results, written from here when there is one tile (no partials, no merge)
+    __nv_bfloat16* dv;
+    int natural;                   // their tokens' order
     int g0, g1;                    // cached groups whose dK / dV are wanted
     int rows_per_group, groups_per_tile, tiles, n_units;
     int* status;
@@ -109,7 +112,9 @@ __device__ __forceinline__ RBUnit rb_decode(const BwdRowParams& rp, int u) {
 }
 
 // tq, tk, tv: the forward's maps of q, K, V; tda, tdy: bridge maps of daL / dY (box 64 x rows_per_group columns x 1 key).
-template <int N_S>
+// kOneTile: all query groups fit one tile, whose dK / dV are the results (24 x 32 tokens, 2 videos, 12 heads, 6 frames cached:
+// training call 380 -> 358 us against partials and a merge).
+template <int N_S, bool kOneTile>
 __global__ void __launch_bounds__(kThreadsRB, 1)
 monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                           const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tda,
@@ -484,17 +489,29 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 if (quad * 32 < b2 && quad < 2) {
                     const long long row0 = ((long long)un.tile * p.nbh + un.bhl) * n_sel + ((long long)(group_of(i) - rp.g0) * b1 + un.k) * b2;
                     const long long o0 = (row0 + quad * 32 + l_row) * kHeadDim + l_col;
+                    // with one tile: the results themselves, in the order asked for
+                    const int fi = group_of(i) - rp.g0, tok0 = rp.natural ? blk.row_token(fi, un.k) : (fi * b1 + un.k) * b2;
+                    const long long d0 = (((long long)b * n_sel + tok0 + quad * 32 + l_row) * p.H + hd) * kHeadDim + l_col;
 #pragma unroll 1
                     for (int c0 = 0; c0 < 2 * kHeadDim; c0 += 16) {
-                        float* dst = (c0 < kHeadDim ? rp.part_k : rp.part_v) + o0 + (c0 & (kHeadDim - 1));
                         uint32_t r[16];
                         float4 v[4];
                         tmem_ld16(tmem + lane_sel + kCDK + c0, r);          // dV's columns follow dK's
                         tmem_wait_ld();
                         transpose(r, v);
+                        if constexpr (kOneTile) {
+                            __nv_bfloat16* dst = (c0 < kHeadDim ? rp.dk : rp.dv) + d0 + (c0 & (kHeadDim - 1));
 #pragma unroll
-                        for (int it = 0; it < 4; ++it)
-                            if (quad * 32 + it * 8 + l_row < b2) *reinterpret_cast<float4*>(dst + it * 8 * kHeadDim) = v[it];
+                            for (int it = 0; it < 4; ++it)
+                                if (quad * 32 + it * 8 + l_row < b2)
+                                    *reinterpret_cast<uint2*>(dst + (long long)it * 8 * p.H * kHeadDim) =
+                                        make_uint2(pack_bf16(v[it].x, v[it].y), pack_bf16(v[it].z, v[it].w));
+                        } else {
+                            float* dst = (c0 < kHeadDim ? rp.part_k : rp.part_v) + o0 + (c0 & (kHeadDim - 1));
+#pragma unroll
+                            for (int it = 0; it < 4; ++it)
+                                if (quad * 32 + it * 8 + l_row < b2) *reinterpret_cast<float4*>(dst + it * 8 * kHeadDim) = v[it];
+                        }
                     }
                     tc_fence_before();
                 }
@@ -591,7 +608,7 @@ size_t bwd_row_tc_partial_bytes(const MonarchParams& mp, int g0, int g1) {
     const int rows_per_group = (mp.blk.b2 + 7) & ~7;
     const int gpt = kRows / rows_per_group;
     const int tiles = (mp.na + gpt - 1) / gpt;
-    return (size_t)tiles * mp.nbh * (size_t)(g1 - g0) * mp.blk.b1 * mp.blk.b2 * kHeadDim * sizeof(float);
+    return tiles == 1 ? 0 : (size_t)tiles * mp.nbh * (size_t)(g1 - g0) * mp.blk.b1 * mp.blk.b2 * kHeadDim * sizeof(float);
 }
 
 // Row-step backward for one slice.  maps = {q, K, V} (the forward's).
@@ -602,6 +619,7 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     BwdRowParams rp;
     rp.mp = mp;
     rp.dcL = dcL; rp.dq = dq; rp.dq_bf16 = dq_bf16; rp.part_k = part_k; rp.part_v = part_v;
+    rp.dk = dk; rp.dv = dv; rp.natural = natural;
     rp.g0 = g0; rp.g1 = g1;
     rp.rows_per_group = (mp.blk.b2 + 7) & ~7;
     rp.groups_per_tile = kRows / rp.rows_per_group;
@@ -622,16 +640,16 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     {
         LaunchScope scope(kClsBackward, s);
         switch (n_s) {
-            case 16: rc = go(monarch_bwd_row_tc_kernel<16>); break;
-            case 32: rc = go(monarch_bwd_row_tc_kernel<32>); break;
-            case 48: rc = go(monarch_bwd_row_tc_kernel<48>); break;
-            case 64: rc = go(monarch_bwd_row_tc_kernel<64>); break;
+            case 16: rc = rp.tiles == 1 ? go(monarch_bwd_row_tc_kernel<16, true>) : go(monarch_bwd_row_tc_kernel<16, false>); break;
+            case 32: rc = rp.tiles == 1 ? go(monarch_bwd_row_tc_kernel<32, true>) : go(monarch_bwd_row_tc_kernel<32, false>); break;
+            case 48: rc = rp.tiles == 1 ? go(monarch_bwd_row_tc_kernel<48, true>) : go(monarch_bwd_row_tc_kernel<48, false>); break;
+            case 64: rc = rp.tiles == 1 ? go(monarch_bwd_row_tc_kernel<64, true>) : go(monarch_bwd_row_tc_kernel<64, false>); break;
             default: return SFM_ERR_UNSUPPORTED;
         }
         if (rc) return rc;
         if (cudaGetLastError() != cudaSuccess) return SFM_ERR_UNSUPPORTED;
     }
-    if (g1 > g0) {
+    if (g1 > g0 && rp.tiles > 1) {
         LaunchScope scope(kClsBackward, s);
         const long long n_sel = (long long)(g1 - g0) * mp.blk.b1 * mp.blk.b2;
         const long long n = n_sel * (kHeadDim / 4) * mp.nbh;
