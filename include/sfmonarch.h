@@ -99,6 +99,8 @@ int sfm_rope_cache_write(const void* q, const void* k, const void* v, void* q_ou
  *   rope, norm_q_weight, norm_k_weight, roll_*   as in sfm_rope_cache_write_roll; each may be NULL / 0
  *   k_cache, v_cache   the cache view [B, n_kv, H, D], batch stride cache_batch_stride; n_kv includes the new tokens
  *   out          [B, n_q, H, D] contiguous;  workspace: sfm_monarch_workspace_bytes(..., 0) bytes (unused when dense)
+ * Every check comes before the first launch: a call refused with an SFM_ERR_* code has not touched the cache (nor moved its
+ * tokens) and may be made again, with more scratch for instance.
  * Replaces: the cache branch of CausalWanSelfAttention.forward between the projections
  * (wan/modules/causal_model.py:900-1103), and monarch_attn_with_kv_cache (wan/modules/monarch_attn.py:1778-1796).
  */

@@ -93,10 +93,25 @@ struct OutShards {
     int world, rank;
 };
 
-int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out, void* ws,
-                size_t ws_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce, int w_reduce,
-                int h, int w, float sm_scale, int num_iters, int causal_groups, size_t budget, cudaStream_t stream,
-                const OutShards* os = nullptr, float* lse = nullptr) {
+// A checked call: its plan, launch parameters and tensor maps.
+struct MonarchCall {
+    Plan pl;
+    MonarchParams p;
+    CUtensorMap maps[5];     // q, K, V, query rows, iteration state
+    int BH, n_s, num_iters, num_sms;
+    bool use_tc, iter_tc;
+    float sm_scale;
+    float* lse;
+    int* status;
+    cudaStream_t stream;
+};
+
+// Every check of a call, and what its launches need.  Launches nothing: a caller that writes a cache first asks here before
+// it does, so that a refused call leaves the cache as it was and can be made again with other arguments.
+int prepare_monarch(MonarchCall* mc, const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out,
+                    void* ws, size_t ws_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce,
+                    int w_reduce, int h, int w, float sm_scale, int num_iters, int causal_groups, size_t budget,
+                    cudaStream_t stream, const OutShards* os = nullptr, float* lse = nullptr) {
     if (!q || !kc || !vc || !ws) return SFM_ERR_NULL_POINTER;
     if (!os && !out) return SFM_ERR_NULL_POINTER;
     if (os) {
@@ -109,7 +124,7 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         }
         out = os->shards[os->rank];
     }
-    Plan pl;
+    Plan& pl = mc->pl;
     int rc = make_plan(&pl, B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, num_iters, budget);
     if (rc) return rc;
     if (ws_bytes < pl.total) return SFM_ERR_WORKSPACE;
@@ -118,7 +133,7 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         return SFM_ERR_ALIGNMENT;
     if (causal_groups < 0 || (causal_groups > 0 && num_iters != 1)) return SFM_ERR_UNSUPPORTED;
 
-    MonarchParams p;
+    MonarchParams& p = mc->p;
     p.q = (const __nv_bfloat16*)q; p.q_bs = q_bs;
     p.kc = (const __nv_bfloat16*)kc; p.vc = (const __nv_bfloat16*)vc; p.c_bs = c_bs;
     p.out = (__nv_bfloat16*)out;
@@ -153,16 +168,14 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
     if (pl.blk.b2 > kB2Max && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
     // only the tensor-core column step knows how to scatter its rows
     if (os && os->world > 1 && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
-    const int num_sms = device_sms();
-    int* status = reinterpret_cast<int*>(base + pl.off_status);
-    CUtensorMap maps[5];     // q, K, V, query rows, iteration state
     const int n_s = (pl.blk.b2 + 15) & ~15;
-    // Every path starts from a clear status word: the workspace may be recycled memory.  The tensor-core path's first
-    // kernel clears it; the mma.sync kernels have no bounded waits and never write it.
-    if (!use_tc) {
-        cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), stream);
-        if (e != cudaSuccess) return (int)e;
-    }
+    mc->BH = B * H; mc->n_s = n_s; mc->num_iters = num_iters; mc->num_sms = device_sms();
+    mc->use_tc = use_tc; mc->iter_tc = iter_tc;
+    mc->sm_scale = sm_scale;
+    mc->lse = lse;
+    mc->status = reinterpret_cast<int*>(base + pl.off_status);
+    mc->stream = stream;
+    CUtensorMap* maps = mc->maps;
     if (use_tc) {
         const uint64_t row = (uint64_t)kHeadDim * 2, tok = (uint64_t)H * row;
         uint64_t dq[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_q, (uint64_t)B};
@@ -180,8 +193,27 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         uint32_t bqr[5] = {64, 1, 1, (uint32_t)pl.blk.b1, 1};
         if (pl.blk.b1 <= 128 && (rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
     }
+    return SFM_OK;
+}
 
-    const int BH = B * H;
+// The launches of a checked call.
+int launch_monarch(MonarchCall& mc) {
+    const Plan& pl = mc.pl;
+    MonarchParams& p = mc.p;
+    CUtensorMap* maps = mc.maps;
+    const bool use_tc = mc.use_tc, iter_tc = mc.iter_tc;
+    const int num_iters = mc.num_iters, num_sms = mc.num_sms, n_s = mc.n_s, BH = mc.BH;
+    const float sm_scale = mc.sm_scale;
+    float* lse = mc.lse;
+    int* status = mc.status;
+    cudaStream_t stream = mc.stream;
+    int rc;
+    // Every path starts from a clear status word: the workspace may be recycled memory.  The tensor-core path's first
+    // kernel clears it; the mma.sync kernels have no bounded waits and never write it.
+    if (!use_tc) {
+        cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), stream);
+        if (e != cudaSuccess) return (int)e;
+    }
     for (int bh0 = 0; bh0 < BH; bh0 += pl.nbh_chunk) {
         p.bh0 = bh0; p.nbh = std::min(pl.nbh_chunk, BH - bh0);
         for (int a0 = 0; a0 < pl.A; a0 += pl.na_chunk) {
@@ -234,6 +266,16 @@ int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int
         }
     }
     return SFM_OK;
+}
+
+int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out, void* ws,
+                size_t ws_bytes, int B, int H, int D, int n_q, int n_kv, int f_tied, int h_reduce, int w_reduce,
+                int h, int w, float sm_scale, int num_iters, size_t budget, cudaStream_t stream,
+                const OutShards* os = nullptr) {
+    MonarchCall mc;
+    int rc = prepare_monarch(&mc, q, q_bs, kc, vc, c_bs, out, ws, ws_bytes, B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce,
+                             h, w, sm_scale, num_iters, 0, budget, stream, os);
+    return rc ? rc : launch_monarch(mc);
 }
 
 }  // namespace
@@ -336,7 +378,7 @@ extern "C" int sfm_monarch_fwd_scatter(const void* q, int64_t q_batch_stride, co
                                        size_t bridge_budget_bytes, void* stream) {
     OutShards os = {out_shards, world, rank};
     return run_monarch(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, nullptr, workspace, workspace_bytes, B, H,
-                       D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, 1, 0, bridge_budget_bytes,
+                       D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, 1, bridge_budget_bytes,
                        (cudaStream_t)stream, &os);
 }
 
@@ -345,7 +387,7 @@ extern "C" int sfm_monarch_fwd(const void* q, int64_t q_batch_stride, const void
                                int H, int D, int n_q, int n_kv, int f_tied, int h_reduce, int w_reduce, int h, int w,
                                float sm_scale, int num_iters, size_t bridge_budget_bytes, void* stream) {
     return run_monarch(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, out, workspace, workspace_bytes, B, H,
-                       D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, 0, bridge_budget_bytes,
+                       D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, bridge_budget_bytes,
                        (cudaStream_t)stream);
 }
 
@@ -384,7 +426,7 @@ extern "C" int sfm_monarch_fwd_static(const void* q, int64_t q_batch_stride, con
     if (rc) return rc;
     if (pl.total > kStaticScratchBytes) return SFM_ERR_STATIC_SCRATCH;
     return run_monarch(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, out, g_static_scratch_ptr[dev],
-                       kStaticScratchBytes, B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, 0,
+                       kStaticScratchBytes, B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters,
                        budget, (cudaStream_t)stream);
 }
 
@@ -404,12 +446,14 @@ extern "C" int sfm_monarch_nocache_fwd(const void* q, const void* k, const void*
                                        int f_tied, int h_reduce, int w_reduce, int h, int w, float sm_scale,
                                        int causal_groups, int num_iters, size_t bridge_budget_bytes, void* stream) {
     if (!k_mon || !v_mon) return SFM_ERR_NULL_POINTER;
-    int rc = sfm_rope_cache_write(nullptr, k, v, nullptr, k_mon, v_mon, (int64_t)N * H * D, nullptr, B, N, H, D, 0,
-                                  f_tied, h_reduce, w_reduce, h, w, 0, 1, stream);
+    MonarchCall mc;
+    int rc = prepare_monarch(&mc, q, (int64_t)N * H * D, k_mon, v_mon, (int64_t)N * H * D, out, workspace, workspace_bytes, B,
+                             H, D, N, N, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, causal_groups,
+                             bridge_budget_bytes, (cudaStream_t)stream);
     if (rc) return rc;
-    return run_monarch(q, (int64_t)N * H * D, k_mon, v_mon, (int64_t)N * H * D, out, workspace, workspace_bytes, B, H,
-                       D, N, N, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, causal_groups,
-                       bridge_budget_bytes, (cudaStream_t)stream);
+    rc = sfm_rope_cache_write(nullptr, k, v, nullptr, k_mon, v_mon, (int64_t)N * H * D, nullptr, B, N, H, D, 0, f_tied,
+                              h_reduce, w_reduce, h, w, 0, 1, stream);
+    return rc ? rc : launch_monarch(mc);
 }
 
 extern "C" int sfm_kv_attention(const void* call) {
@@ -417,24 +461,30 @@ extern "C" int sfm_kv_attention(const void* call) {
     SfmKvCall c;
     memcpy(&c, call, sizeof(c));
     if (!c.k || !c.v || !c.q || (c.q_rot && !c.rope)) return SFM_ERR_NULL_POINTER;
-    const int order = c.dense ? 0 : 1;
-    int rc = c.roll_shift > 0 || c.norm_q_weight || c.norm_k_weight
-                 ? sfm_rope_cache_write_roll(c.q_rot ? c.q : nullptr, c.k, c.v, c.norm_q_weight, c.norm_k_weight, c.eps, c.q_rot,
-                                             c.k_cache, c.v_cache, c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new,
-                                             c.H, c.D, c.start_idx, c.roll_dst, c.roll_shift, c.f_tied, c.h_reduce,
-                                             c.w_reduce, c.h, c.w, c.start_frame, order, c.stream)
-                 : sfm_rope_cache_write(c.q_rot ? c.q : nullptr, c.k, c.v, c.q_rot, c.k_cache, c.v_cache,
-                                        c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new, c.H, c.D, c.start_idx,
-                                        c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.start_frame, order, c.stream);
-    if (rc) return rc;
+    // The attention's checks come before the first launch: the cache write may evict (move cached tokens), which must happen
+    // once, and a caller whose scratch is too small makes the same call again.  The cache write checks its own arguments
+    // before it launches.
     const void* q = c.q_rot ? c.q_rot : c.q;
     const int64_t q_bs = c.q_rot ? (int64_t)c.n_q * c.H * c.D : c.q_batch_stride;
-    if (c.dense)
-        return sfm_dense_fwd(q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.B, c.H, c.D, c.n_q, c.n_kv, c.sm_scale,
-                             c.stream);
-    return run_monarch(q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.workspace, c.workspace_bytes, c.B, c.H, c.D,
-                       c.n_q, c.n_kv, c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.sm_scale, c.num_iters, 0, 0,
-                       (cudaStream_t)c.stream, nullptr, (float*)c.lse);
+    MonarchCall mc;
+    DenseCall dc;
+    int rc = c.dense ? prepare_dense(&dc, q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.B, c.H, c.D, c.n_q, c.n_kv,
+                                     c.sm_scale)
+                     : prepare_monarch(&mc, q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.workspace,
+                                       c.workspace_bytes, c.B, c.H, c.D, c.n_q, c.n_kv, c.f_tied, c.h_reduce, c.w_reduce, c.h,
+                                       c.w, c.sm_scale, c.num_iters, 0, 0, (cudaStream_t)c.stream, nullptr, (float*)c.lse);
+    if (rc) return rc;
+    const int order = c.dense ? 0 : 1;
+    rc = c.roll_shift > 0 || c.norm_q_weight || c.norm_k_weight
+             ? sfm_rope_cache_write_roll(c.q_rot ? c.q : nullptr, c.k, c.v, c.norm_q_weight, c.norm_k_weight, c.eps, c.q_rot,
+                                         c.k_cache, c.v_cache, c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new,
+                                         c.H, c.D, c.start_idx, c.roll_dst, c.roll_shift, c.f_tied, c.h_reduce,
+                                         c.w_reduce, c.h, c.w, c.start_frame, order, c.stream)
+             : sfm_rope_cache_write(c.q_rot ? c.q : nullptr, c.k, c.v, c.q_rot, c.k_cache, c.v_cache,
+                                    c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new, c.H, c.D, c.start_idx,
+                                    c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.start_frame, order, c.stream);
+    if (rc) return rc;
+    return c.dense ? launch_dense(dc, (cudaStream_t)c.stream) : launch_monarch(mc);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -17,13 +17,10 @@ namespace {
 // the last sfm_dense_status call, which reads and clears it.
 __device__ int g_dense_status;
 }  // namespace
-}  // namespace sfm
 
-using namespace sfm;
-
-extern "C" int sfm_dense_fwd(const void* q, int64_t q_batch_stride, const void* k, const void* v,
-                             int64_t kv_batch_stride, void* out, int B, int H, int D, int n_q, int n_kv,
-                             float sm_scale, void* stream) {
+// Every check of a call, and what its launch needs; launches nothing (see prepare_monarch).
+int prepare_dense(DenseCall* c, const void* q, int64_t q_batch_stride, const void* k, const void* v, int64_t kv_batch_stride,
+                  void* out, int B, int H, int D, int n_q, int n_kv, float sm_scale) {
     if (!q || !k || !v || !out) return SFM_ERR_NULL_POINTER;
     if (D != kHeadDim) return SFM_ERR_UNSUPPORTED;
     if (B <= 0 || H <= 0 || n_q <= 0 || n_kv <= 0) return SFM_ERR_BAD_SHAPE;
@@ -48,13 +45,29 @@ extern "C" int sfm_dense_fwd(const void* q, int64_t q_batch_stride, const void* 
     uint64_t dk[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_kv, (uint64_t)B};
     uint64_t sk[3] = {row, tok, (uint64_t)kv_batch_stride * 2};
     uint32_t box[4] = {64, 1, 128, 1};
-    CUtensorMap maps[3];
     int rc;
-    if ((rc = make_tmap_bf16(&maps[0], k, 4, dk, sk, box))) return rc;
-    if ((rc = make_tmap_bf16(&maps[1], v, 4, dk, sk, box))) return rc;
-    if ((rc = make_tmap_bf16(&maps[2], q, 4, dq, sq, box))) return rc;
-    return launch_dense_tc(maps, (__nv_bfloat16*)out, B, H, n_q, n_kv, sm_scale, status, device_sms(),
-                           (cudaStream_t)stream);
+    if ((rc = make_tmap_bf16(&c->maps[0], k, 4, dk, sk, box))) return rc;
+    if ((rc = make_tmap_bf16(&c->maps[1], v, 4, dk, sk, box))) return rc;
+    if ((rc = make_tmap_bf16(&c->maps[2], q, 4, dq, sq, box))) return rc;
+    c->out = out; c->status = status;
+    c->B = B; c->H = H; c->n_q = n_q; c->n_kv = n_kv;
+    c->scale = sm_scale;
+    return SFM_OK;
+}
+
+int launch_dense(const DenseCall& c, cudaStream_t s) {
+    return launch_dense_tc(c.maps, (__nv_bfloat16*)c.out, c.B, c.H, c.n_q, c.n_kv, c.scale, c.status, device_sms(), s);
+}
+}  // namespace sfm
+
+using namespace sfm;
+
+extern "C" int sfm_dense_fwd(const void* q, int64_t q_batch_stride, const void* k, const void* v,
+                             int64_t kv_batch_stride, void* out, int B, int H, int D, int n_q, int n_kv,
+                             float sm_scale, void* stream) {
+    DenseCall c;
+    int rc = prepare_dense(&c, q, q_batch_stride, k, v, kv_batch_stride, out, B, H, D, n_q, n_kv, sm_scale);
+    return rc ? rc : launch_dense(c, (cudaStream_t)stream);
 }
 
 // Waits for `stream`, then reports (and clears) the status word of the dense-attention kernels on the

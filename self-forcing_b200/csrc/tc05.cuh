@@ -303,4 +303,17 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
 // Bridge tensor aL or Y, [group][key][column][128]; one box = 64 channels x box_cols columns x box_keys keys of one group.
 int make_bridge_tmap(CUtensorMap* out, const void* base, int b2, int n_keys, int groups, int box_cols, int box_keys);
 
+// ----------------------------------------------------------------------------- host: dense attention in two steps
+// A checked call.  prepare_dense makes every check and launches nothing; launch_dense launches.
+struct DenseCall {
+    CUtensorMap maps[3];     // K, V, q
+    void* out;
+    int* status;
+    int B, H, n_q, n_kv;
+    float scale;
+};
+int prepare_dense(DenseCall* c, const void* q, int64_t q_batch_stride, const void* k, const void* v, int64_t kv_batch_stride,
+                  void* out, int B, int H, int D, int n_q, int n_kv, float sm_scale);
+int launch_dense(const DenseCall& c, cudaStream_t s);
+
 }  // namespace sfm

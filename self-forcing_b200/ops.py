@@ -238,7 +238,9 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
             eps, sm_scale, B, H, D, n_q, k.shape[1], n_kv, start_idx, roll_dst, roll_shift, start_frame, *blocking, num_iters,
             dense, 0)
         rc = _lib.load().sfm_kv_attention(call)
-        if rc != _ERR_WORKSPACE or attempt:               # the cached scratch may be too small for this call: get more, once
+        # the cached scratch may be too small for this call: get more, once (a refused call has launched nothing, so the
+        # cache write and its eviction still happen once)
+        if rc != _ERR_WORKSPACE or attempt:
             break
     if rc:
         _lib.check(rc, "sfm_kv_attention")

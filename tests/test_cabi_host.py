@@ -150,6 +150,22 @@ def test_entry_points_validate_arguments_without_a_gpu(sfb):
                                        3 * 60 * 52, 3, 1, 1, 60, 52, 1.0, 0, null) == -3
 
 
+@pytest.mark.parametrize("field,value,rc", [("workspace_bytes", 0, -5), ("workspace_bytes", 1, -5), ("n_kv", 1561, -2),
+                                            ("num_iters", 0, -2), ("out", 260, -4), ("k_cache", 0, -1)])
+def test_layer_call_is_refused_before_its_cache_write(sfb, field, value, rc):
+    """sfm_kv_attention makes the attention's checks before it launches the cache write, which may evict: without a GPU a
+    launch would be a CUDA error (a positive code)."""
+    from self_forcing_b200 import _lib, ops
+    need = sfb.workspace_bytes(1, 2, 1560, 3120, 1, 1, 1, 30, 52)
+    names = ("q k v wq wk q_rot k_cache v_cache rope out workspace stream lse q_bs cache_bs workspace_bytes eps sm_scale "
+             "B H D n_q n_new n_kv start_idx roll_dst roll_shift start_frame f_tied h_reduce w_reduce h w num_iters dense "
+             "reserved").split()
+    call = dict(zip(names, [256, 256, 256, 0, 0, 256, 256, 256, 256, 256, 256, 0, 0, 1560 * 256, 3120 * 256, need, 1e-6, 0.088,
+                            1, 2, 128, 1560, 1560, 3120, 1560, 0, 1560, 0, 1, 1, 1, 30, 52, 1, 0, 0]))
+    call[field] = need - 1 if (field, value) == ("workspace_bytes", 1) else value
+    assert _lib.load().sfm_kv_attention(ops._KV_CALL.pack(*call.values())) == rc
+
+
 def test_plan_cache_step_equals_oracle(sfb):
     """The product's cache bookkeeping against the oracle's restatement of causal_model.py:907-938,
     over a random walk of rollouts with and without a sliding window (integers: exact)."""

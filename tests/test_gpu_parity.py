@@ -534,6 +534,7 @@ def test_layer_rollout_matches_oracle(sfb, mode):
     """Several chunks through self_attention_kv (each chunk denoised twice, as the few-step sampler does)
     against the oracle's restatement of the reference layer, including the sliding window with a sink frame,
     the dense first chunk and the all-dense configuration; the caches must agree too."""
+    sfb.ops.release_workspaces()      # scratch grows during the rollout, also in the call that evicts (window of 10 frames)
     rng = np.random.default_rng({"plain": 1, "window_sink": 2, "dense_init": 3, "regular": 4, "window10_sink2": 5,
                                  "window7_dense": 6}[mode])
     B, H, gh, gw = 1, 2, 6, 8
@@ -573,6 +574,38 @@ def test_layer_rollout_matches_oracle(sfb, mode):
             assert dk <= 0.05, dk
             # keep the two caches in lock step (the oracle's keys are fp32, ours bf16)
             state["k"][:, :used] = cache.k[:, :used].cpu().float()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dense", [False, True])
+def test_refused_layer_call_leaves_the_cache_alone(sfb, dense):
+    """sfm_kv_attention with the eviction shift: scratch one byte short (or, dense, a scale that is refused) is an error
+    before anything is launched, and the same call made again with what it asks for evicts once."""
+    from self_forcing_b200 import _lib, ops
+    lib = _lib.load()
+    B, H, h, w, n_kv = 1, 2, 6, 8, 6 * 48
+    n, shift = 3 * 48, 2 * 48
+    torch.manual_seed(3)
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    q, k, v, kc, vc = mk(B, n, H, 128), mk(B, n, H, 128), mk(B, n, H, 128), mk(B, n_kv, H, 128), mk(B, n_kv, H, 128)
+    rope, q_rot, out = ops._rope_table_from_freqs(None, q.device), torch.empty_like(q), torch.empty_like(q)
+    need = lib.sfm_monarch_workspace_bytes(B, H, 128, n, n_kv, 1, 1, 1, h, w, 1, 0)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+    def call(nbytes, scale):
+        return lib.sfm_kv_attention(ops._KV_CALL.pack(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), 0, 0, q_rot.data_ptr(), kc.data_ptr(), vc.data_ptr(), rope.data_ptr(),
+            out.data_ptr(), ws.data_ptr(), ops._stream().value or 0, 0, n * H * 128, n_kv * H * 128, nbytes, 1e-6, scale,
+            B, H, 128, n, n, n_kv, n_kv - n, 48, shift, 0, 1, 1, 1, h, w, 1, dense, 0))
+
+    k0, v0 = kc.clone(), vc.clone()
+    assert call(need, 0.0) == -2 if dense else call(need - 1, 0.088) == -5
+    torch.cuda.synchronize()
+    assert torch.equal(kc, k0) and torch.equal(vc, v0)
+    assert call(need, 0.088) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(vc[:, 48:n_kv - n], v0[:, 48 + shift:n_kv - n + shift])          # moved once
+    assert torch.equal(vc[:, :48], v0[:, :48])
 
 
 @pytest.mark.gpu
