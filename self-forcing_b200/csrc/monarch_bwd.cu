@@ -702,7 +702,11 @@ int make_bwd_plan(BwdPlan* pl, int B, int H, int D, int n_q, int n_kv, int f_tie
     pl->n_keys = pl->F * blk.b1;
     if (budget == 0) budget = kDefaultBwdBudget;
     const size_t per_bh = (size_t)pl->A * blk.b2 * pl->n_keys * (2 * kHeadDim + 2) * sizeof(float);
-    pl->nbh = (int)std::max<size_t>(1, std::min<size_t>((size_t)B * H, budget / per_bh));
+    {
+        const int BH = B * H, most = (int)std::max<size_t>(1, std::min<size_t>((size_t)BH, budget / per_bh));
+        const int slices = (BH + most - 1) / most;
+        pl->nbh = (BH + slices - 1) / slices;                 // slices of one size, the last at most slices - 1 pairs smaller
+    }
     const size_t units = (size_t)pl->nbh * pl->A * blk.b2 * pl->n_keys;
     size_t o = 256;                                   // the status word of the call sits at the start, in both layouts
     pl->off_aL = o; o = up256(o + units * kHeadDim * sizeof(float));
@@ -806,35 +810,39 @@ static int monarch_bwd(bool train, const void* out_fwd, const float* lse_fwd, co
     const int num_sms = device_sms();
     // one status word per call: a kernel that gives up on a bounded wait sets it, nothing clears it before the end
     if (cudaMemsetAsync(ws, 0, sizeof(int), s) != cudaSuccess) return SFM_ERR_UNSUPPORTED;
+    // Workspace of the tensor-core path: status | for the whole call: delta, a scratch output, dq2 | for a slice: aL, Y (bf16
+    // bridge), cL, dcL, lse, then the row kernel's partials.  Every offset is that of a full slice, so that a last slice of
+    // fewer pairs finds what the call has written once (delta) where the first one left it.
+    const int n_keys_c = (pl.n_keys + 3) & ~3;
+    size_t o = 0;
+    auto place = [&](size_t bytes) { unsigned char* at = ws + o; o = up256(o + bytes); return at; };
+    const size_t rows = (size_t)B * n_q * H, slabs = (size_t)pl.nbh * pl.A * blk.b2;
+    int* status = (int*)place(sizeof(int));
+    float* delta = (float*)place(rows * sizeof(float));
+    bf16* out_s = (bf16*)place(rows * kHeadDim * sizeof(bf16));
+    float* dq2 = (float*)place(rows * kHeadDim * sizeof(float));
+    bf16* aLb = (bf16*)place(slabs * pl.n_keys * kHeadDim * sizeof(bf16));
+    bf16* Yb = (bf16*)place(slabs * pl.n_keys * kHeadDim * sizeof(bf16));
+    float* cL = (float*)place(slabs * n_keys_c * sizeof(float));
+    float* dcL = (float*)place(slabs * n_keys_c * sizeof(float));
+    float* lse_s = (float*)place(slabs * blk.b1 * sizeof(float));
+    if (use_tc && o > workspace_bytes) return SFM_ERR_WORKSPACE;
+
     for (int bh0 = 0; bh0 < BH; bh0 += pl.nbh) {
         const int nbh = std::min(pl.nbh, BH - bh0);
         p.bh0 = bh0;
         if (use_tc) {
-            // workspace of this slice: status | aL, Y (bf16 bridge) | cL, dcL | lse | out (scratch) | delta | dq2
-            const size_t slabs = (size_t)nbh * pl.A * blk.b2;
-            const int n_keys_c = (pl.n_keys + 3) & ~3;
-            const size_t rows = (size_t)B * n_q * H;
-            size_t o = 0;
-            int* status = (int*)(ws + o); o = up256(o + sizeof(int));
-            bf16* aLb = (bf16*)(ws + o); o = up256(o + slabs * pl.n_keys * kHeadDim * sizeof(bf16));
-            bf16* Yb = (bf16*)(ws + o); o = up256(o + slabs * pl.n_keys * kHeadDim * sizeof(bf16));
-            float* cL = (float*)(ws + o); o = up256(o + slabs * n_keys_c * sizeof(float));
-            float* dcL = (float*)(ws + o); o = up256(o + slabs * n_keys_c * sizeof(float));
-            float* lse = (float*)(ws + o); o = up256(o + slabs * blk.b1 * sizeof(float));
-            bf16* out_s = (bf16*)(ws + o); o = up256(o + rows * kHeadDim * sizeof(bf16));
-            float* delta = (float*)(ws + o); o = up256(o + rows * sizeof(float));
-            p.dq2 = (float*)(ws + o); o = up256(o + rows * kHeadDim * sizeof(float));
-            if (o > workspace_bytes) return SFM_ERR_WORKSPACE;
+            p.dq2 = dq2;
             if (train) p.dq = p.dq2;                          // the fp32 shares stay in the scratch
             MonarchParams mp;
             CUtensorMap maps[8];
             const bool have_fwd = out_fwd && lse_fwd;
-            if (have_fwd) lse = const_cast<float*>(lse_fwd) + (size_t)bh0 * n_q;
+            float* lse = have_fwd ? const_cast<float*>(lse_fwd) + (size_t)bh0 * n_q : lse_s;
             int rc = forward_tc_slice(q, q_batch_stride, k_cache, v_cache, kv_batch_stride, out_s, aLb, Yb, cL, lse, status,
                                       B, H, n_q, n_kv, blk, sm_scale, bh0, nbh, !have_fwd, &mp, maps, s);
             if (rc) return rc;
-            // delta = dOut . out for every (token, head); the scratch output holds this slice's heads only, the
-            // other heads' products are never read
+            // delta = dOut . out for every (token, head): once for the call from the forward's output, else slice by slice
+            // (the scratch output then holds this slice's heads only, the other heads' products are never read)
             if ((!have_fwd || bh0 == 0) && (rc = launch_bwd_delta(dout, have_fwd ? out_fwd : out_s, delta, (long long)rows, s))) return rc;
             // query rows of q and dOut for the column kernel: (d, head, column, row of the token grid, batch), boxes of
             // 32 consecutive grid rows (fewer when the whole call has fewer)

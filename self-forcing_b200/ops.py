@@ -301,13 +301,14 @@ def _bwd_workspace(q, n_kv, f_tied, h_reduce, w_reduce, h, w, budget_bytes=0):
     return _workspace(q.device, max(int(nbytes), 256), "monarch_bwd")
 
 
-def _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1):
+def _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1, budget_bytes=0):
     """(dq bf16, dk, dv with their tokens in natural order) of the cached groups [g0, g1), or None for shapes the
-    tensor-core backward does not take.  out, lse: what the forward left, or None.  The tensors are those a forward call of this module has accepted."""
+    tensor-core backward does not take.  out, lse: what the forward left, or None.  The tensors are those a forward call of
+    this module has accepted.  budget_bytes as in monarch_attn_with_kv_cache_backward."""
     B, n_q, H, D = q.shape
     n_kv = k_cache.shape[1]
     q, grad_out = _as_token_major(q), grad_out.contiguous()
-    ws = _bwd_workspace(q, n_kv, *blocking)
+    ws = _bwd_workspace(q, n_kv, *blocking, budget_bytes)
     f_tied, h_reduce, w_reduce, h, w = blocking
     dq = torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
     dk = torch.empty((B, (g1 - g0) * (f_tied * h * w) // (h_reduce * w_reduce), H, D), dtype=q.dtype, device=q.device)
@@ -316,7 +317,7 @@ def _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scal
         q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache),
         None if out is None else out.data_ptr(), None if lse is None else lse.data_ptr(), grad_out.data_ptr(), dq.data_ptr(),
         dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w,
-        float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1, 0, _raw_stream(q.get_device()))
+        float(D ** -0.5 if sm_scale is None else sm_scale), g0, g1, budget_bytes, _raw_stream(q.get_device()))
     if rc == _ERR_UNSUPPORTED:
         return None
     _lib.check(rc, "sfm_monarch_bwd_natural")

@@ -183,6 +183,31 @@ def test_natural_order_backward(sfb, blocking, frames_q, cached, change_out):
         assert torch.equal(mon.reshape(leaf.shape), full[:, c["start"]:c["end"]].cpu())
 
 
+@pytest.mark.parametrize("with_forward", [True, False])
+@pytest.mark.parametrize("B,H,pairs", [(1, 3, 2), (1, 13, 5), (2, 5, 4)])
+def test_natural_order_backward_in_uneven_slices(sfb, B, H, pairs, with_forward):
+    """A training backward whose scratch holds `pairs` (batch, head) pairs, the last slice fewer (2 + 1, 5 + 5 + 3, 4 + 4 + 2
+    pairs): bit-equal to the uncut call and, permuted and cast, to the full backward, with the forward's output and
+    log-sum-exps given and without."""
+    blocking = (1, 1, 1, 6, 8)
+    c = make_case(blocking, 2, 4, B=B, H=H, seed=8490)
+    kv, vv = (c[n].cuda().clone()[:, :c["n_kv"]] for n in ("kbuf", "vbuf"))
+    q, g, nk, nv = (c[n].cuda() for n in ("q", "g", "nk", "nv"))
+    lse = torch.empty(q.shape[:-1], dtype=torch.float32, device="cuda")
+    out = sfb.monarch_attn_with_kv_cache(q, kv, vv, nk, nv, c["start"], c["end"], *blocking, _no_grad=True, _lse=lse)
+    one_pair = 2 * 8 * (4 * 6) * (2 * 128 + 2) * 4          # scratch of one pair: A b2 n_keys (2 D + 2) floats
+    args = (q, kv, vv, out if with_forward else None, lse if with_forward else None, g, blocking, None, 2, 4)
+    uncut = sfb.ops._backward_natural(*args)
+    sfb.ops.release_workspaces()
+    cut = sfb.ops._backward_natural(*args, budget_bytes=pairs * one_pair)
+    for x, y in zip(cut, uncut):
+        assert torch.equal(x, y)
+    dq, dk, dv = sfb.monarch_attn_with_kv_cache_backward(q, kv, vv, g, *blocking, kv_groups=(2, 4))
+    assert torch.equal(cut[0], bf(dq))
+    for nat, full in ((cut[1], dk), (cut[2], dv)):
+        assert torch.equal(orc.to_monarch_order(nat.cpu(), *blocking).reshape(full.shape), full.cpu())
+
+
 @pytest.mark.parametrize("only_new", [False, True])
 def test_autograd_function(sfb, only_new):
     """monarch_attn_with_kv_cache under autograd: same forward result and cache content as without it;
