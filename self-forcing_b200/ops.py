@@ -355,15 +355,24 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
         out = monarch_attn_with_kv_cache(q.detach(), k_cache.detach(), v_cache.detach(), new_k.detach(), new_v.detach(),
                                          start_idx, end_idx, f_tied, h_reduce, w_reduce, h, w, sm_scale, 1,
                                          _no_grad=True, _lse=lse)
-        ctx.save_for_backward(q, k_cache, v_cache)
-        # not a saved tensor: the caller may change the output in place, and the backward then does without it
-        ctx.forward_out = (out.detach(), out._version, lse) if lse is not None else None
+        # The output and the log-sum-exps are saved like the inputs, so that saved-tensor hooks (checkpointing, offloading) see
+        # them and they go when the backward has run.  The caller may change the output in place: what is saved is a tensor
+        # on its memory with a version counter of its own (a changed saved tensor is an error otherwise), and an empty
+        # tensor with the output's counter tells the backward whether it has to do without.
+        ctx.out_version = None
+        if lse is None:
+            ctx.save_for_backward(q, k_cache, v_cache)
+        else:
+            ctx.save_for_backward(q, k_cache, v_cache, out.data, lse)
+            counter = out.detach()
+            counter.data = out.new_empty(0)
+            ctx.out_version = (counter, counter._version)
         ctx.args = (int(start_idx), int(end_idx), blocking, sm_scale, bool(grad_only_new_kv))
         return out
 
     @staticmethod
     def backward(ctx, grad_out):
-        q, k_cache, v_cache = ctx.saved_tensors
+        q, k_cache, v_cache, *fwd = ctx.saved_tensors
         start, end, blocking, sm_scale, only_new = ctx.args
         f_tied, h_reduce, w_reduce, h, w = blocking
         group = (f_tied * h * w) // (h_reduce * w_reduce)
@@ -372,9 +381,9 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
         g0, g1 = (0, n_kv // group) if want_cache else (start // group, -(-end // group))
         grad_out = grad_out.to(q.dtype)
         if not want_cache and start % (f_tied * h * w) == 0:
-            out, version, lse = ctx.forward_out or (None, 0, None)
-            if out is not None and out._version != version:
-                out = lse = None
+            out = lse = None
+            if fwd and ctx.out_version[0]._version == ctx.out_version[1]:
+                out, lse = fwd
             grads = _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1)
             if grads is not None:
                 return (*grads, None, None, None, None, None, None, None)

@@ -183,6 +183,45 @@ def test_natural_order_backward(sfb, blocking, frames_q, cached, change_out):
         assert torch.equal(mon.reshape(leaf.shape), full[:, c["start"]:c["end"]].cpu())
 
 
+@pytest.mark.parametrize("change_out", [False, True])
+@pytest.mark.parametrize("how", ["offload", "checkpoint"])
+def test_saved_tensor_hooks_see_what_the_training_call_keeps(sfb, how, change_out):
+    """Under hooks that move saved tensors to the host, and under non-reentrant checkpointing, a training call keeps no device
+    memory for its backward beyond the cache and the inputs, and its gradients are bit-equal to those without hooks, also
+    when the output is changed in place inside the region."""
+    from torch.utils.checkpoint import checkpoint
+    blocking = (1, 1, 1, 6, 8)
+    c = make_case(blocking, 2, 4, B=2, H=2, seed=8495)
+    kv, vv = (c[n].cuda().clone()[:, :c["n_kv"]] for n in ("kbuf", "vbuf"))
+
+    def attend(q, nk, nv):
+        z = sfb.monarch_attn_with_kv_cache(q, kv, vv, nk, nv, c["start"], c["end"], *blocking, grad_only_new_kv=True)
+        return z.mul_(2.0) if change_out else z
+
+    def step(call):
+        leaves = [c[n].cuda().requires_grad_() for n in ("q", "nk", "nv")]
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        loss = call(*leaves).sum()                        # its backward needs no copy of the output
+        held = torch.cuda.memory_allocated() - before
+        loss.backward()
+        return held, [t.grad for t in leaves]
+
+    def hooked(*leaves):
+        if how == "checkpoint":
+            return checkpoint(attend, *leaves, use_reentrant=False)
+        with torch.autograd.graph.save_on_cpu():
+            return attend(*leaves)
+
+    step(attend)                                          # scratch is allocated and kept
+    held, plain = step(attend)
+    held_hooked, grads = step(hooked)
+    out_bytes = c["q"].numel() * 2
+    assert held >= out_bytes and held_hooked < out_bytes, (held, held_hooked, out_bytes)
+    for x, y in zip(grads, plain):
+        assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("with_forward", [True, False])
 @pytest.mark.parametrize("B,H,pairs", [(1, 3, 2), (1, 13, 5), (2, 5, 4)])
 def test_natural_order_backward_in_uneven_slices(sfb, B, H, pairs, with_forward):
