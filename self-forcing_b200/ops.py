@@ -10,6 +10,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 import struct
+import threading
+from collections import OrderedDict
 from typing import Dict, Optional, Tuple
 
 import numpy as np
@@ -17,7 +19,8 @@ import torch
 
 from . import _lib
 
-_workspaces: Dict[Tuple[int, int, str], torch.Tensor] = {}
+_workspaces: "OrderedDict[Tuple[int, int, str], torch.Tensor]" = OrderedDict()      # least recently used first
+_workspaces_lock = threading.RLock()
 _rope_tables: Dict[tuple, torch.Tensor] = {}
 _status_mirror: Dict[int, list] = {}
 
@@ -67,29 +70,43 @@ def _batch_stride(t: torch.Tensor) -> int:
 
 
 _MAX_WORKSPACES = 8
+_MAX_WORKSPACE_BYTES = 8 << 30
+
+
+def _cached_workspace(key) -> Optional[torch.Tensor]:
+    """The buffer of (GPU, stream, kind), now the most recently used one, or None."""
+    with _workspaces_lock:
+        ws = _workspaces.get(key)
+        if ws is not None:
+            _workspaces.move_to_end(key)
+        return ws
 
 
 def _workspace(device: torch.device, nbytes: int, tag: str = "monarch") -> torch.Tensor:
     """Scratch for the row-step results, cached per (GPU, stream, kind): calls queued on one stream run in
     order and may share it, calls on different streams may overlap and must not.  A buffer only grows (up to
-    the bridge budget, 4 GiB by default, plus the call's fixed part); at most _MAX_WORKSPACES buffers are kept,
-    the least recently used one is dropped beyond that (a buffer was allocated on the stream that uses it, so
-    PyTorch's allocator hands its memory out again in that stream's order only), and release_workspaces()
-    drops them all."""
+    the bridge budget, 4 GiB by default, plus the call's fixed part; SFM_BRIDGE_MB lowers it).  At most _MAX_WORKSPACES
+    buffers and _MAX_WORKSPACE_BYTES (or the newest buffer alone) are kept, the least recently used ones are dropped beyond
+    that (a buffer was allocated on the stream that uses it, so PyTorch's allocator hands its memory out again in that
+    stream's order only), and release_workspaces() drops them all."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     key = (index, _raw_stream(index), tag)
-    ws = _workspaces.pop(key, None)
+    ws = _cached_workspace(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=device)
-    _workspaces[key] = ws                          # re-inserted last: dict order is the LRU order
-    while len(_workspaces) > _MAX_WORKSPACES:
-        _workspaces.pop(next(iter(_workspaces)))       # freed in the order of the stream it was allocated on
+        with _workspaces_lock:
+            _workspaces[key] = ws
+            _workspaces.move_to_end(key)
+            kept = sum(w.numel() for w in _workspaces.values())
+            while len(_workspaces) > 1 and (len(_workspaces) > _MAX_WORKSPACES or kept > _MAX_WORKSPACE_BYTES):
+                kept -= _workspaces.popitem(last=False)[1].numel()
     return ws
 
 
 def release_workspaces() -> None:
     """Drops every cached scratch buffer (they come back on demand)."""
-    _workspaces.clear()
+    with _workspaces_lock:
+        _workspaces.clear()
 
 
 _WATCH_EVERY = 32
@@ -226,7 +243,7 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
     stream = _raw_stream(device)
     q_rot = torch.empty_like(q) if rope is not None else None
     out = torch.empty_like(q) if q.is_contiguous() else torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
-    ws = None if dense else _workspaces.get((device, stream, "monarch"))
+    ws = None if dense else _cached_workspace((device, stream, "monarch"))
     for attempt in (0, 1):
         if not dense and (ws is None or attempt):
             nbytes = _lib.load().sfm_monarch_workspace_bytes(B, H, D, n_q, n_kv, *blocking, num_iters, 0)

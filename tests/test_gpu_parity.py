@@ -789,6 +789,39 @@ def test_two_streams_use_separate_workspaces(sfb):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bound", ["count", "bytes"])
+def test_least_recently_used_workspace_is_dropped(sfb, monkeypatch, bound):
+    """Scratch kept for two streams at most, by count or by bytes: a stream that has just been used keeps its buffer, the
+    other one loses it; the newest buffer is kept whatever its size."""
+    from self_forcing_b200 import ops
+    c = small_case(1, 1, H=3)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+
+    def call(i):
+        with torch.cuda.stream(streams[i]):
+            z, _, _ = run_gpu_cache(sfb, c)
+        torch.cuda.synchronize()
+        return z
+
+    def kept():
+        return {i for i, s in enumerate(streams) if (torch.cuda.current_device(), s.cuda_stream, "monarch") in ops._workspaces}
+
+    ops.release_workspaces()
+    call(0)
+    if bound == "count":
+        monkeypatch.setattr(ops, "_MAX_WORKSPACES", 2)
+    else:
+        monkeypatch.setattr(ops, "_MAX_WORKSPACE_BYTES", 2 * next(iter(ops._workspaces.values())).numel())
+    ref = call(1)
+    call(0)                                               # a hit: stream 1 is now the least recently used
+    assert torch.equal(call(2), ref) and kept() == {0, 2}
+    assert torch.equal(call(1), ref) and kept() == {2, 1}
+    monkeypatch.setattr(ops, "_MAX_WORKSPACE_BYTES", 1)
+    assert torch.equal(call(0), ref) and kept() == {0}
+    ops.release_workspaces()
+
+
+@pytest.mark.gpu
 def test_recycled_workspace_does_not_raise_a_false_status(sfb):
     """A workspace that holds garbage (recycled allocator memory) must not read as a failed call: every path,
     the iterative one included, clears the status word before its first launch."""
