@@ -98,7 +98,8 @@ int sfm_rope_cache_write(const void* q, const void* k, const void* v, void* q_ou
  *   q_rot        [B, n_q, H, D]: normalised and rotated q (n_q = n_new); NULL: q is attended as it is
  *   rope, norm_q_weight, norm_k_weight, roll_*   as in sfm_rope_cache_write_roll; each may be NULL / 0
  *   k_cache, v_cache   the cache view [B, n_kv, H, D], batch stride cache_batch_stride; n_kv includes the new tokens
- *   out          [B, n_q, H, D] contiguous;  workspace: sfm_monarch_workspace_bytes(..., 0) bytes (unused when dense)
+ *   out          [B, n_q, H, D] contiguous;  workspace: sfm_monarch_workspace_bytes(..., bridge_budget_mb << 20) bytes (unused
+ *                when dense); bridge_budget_mb 0 = default
  * Every check comes before the first launch: a call refused with an SFM_ERR_* code has not touched the cache (nor moved its
  * tokens) and may be made again, with more scratch for instance.
  * Replaces: the cache branch of CausalWanSelfAttention.forward between the projections
@@ -113,7 +114,7 @@ typedef struct SfmKvCall {
     uint64_t workspace_bytes;
     float eps, sm_scale;
     int32_t B, H, D, n_q, n_new, n_kv, start_idx, roll_dst, roll_shift, start_frame;
-    int32_t f_tied, h_reduce, w_reduce, h, w, num_iters, dense, reserved;
+    int32_t f_tied, h_reduce, w_reduce, h, w, num_iters, dense, bridge_budget_mb;
 } SfmKvCall;
 int sfm_kv_attention(const void* call);
 /* lse (or null; Monarch attention with num_iters 1 and block rows up to 128): fp32 [B * H][n_q], every query's log-sum-exp

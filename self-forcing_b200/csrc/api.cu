@@ -472,7 +472,8 @@ extern "C" int sfm_kv_attention(const void* call) {
                                      c.sm_scale)
                      : prepare_monarch(&mc, q, q_bs, c.k_cache, c.v_cache, c.cache_batch_stride, c.out, c.workspace,
                                        c.workspace_bytes, c.B, c.H, c.D, c.n_q, c.n_kv, c.f_tied, c.h_reduce, c.w_reduce, c.h,
-                                       c.w, c.sm_scale, c.num_iters, 0, 0, (cudaStream_t)c.stream, nullptr, (float*)c.lse);
+                                       c.w, c.sm_scale, c.num_iters, 0, (size_t)std::max(0, c.bridge_budget_mb) << 20,
+                                       (cudaStream_t)c.stream, nullptr, (float*)c.lse);
     if (rc) return rc;
     const int order = c.dense ? 0 : 1;
     rc = c.roll_shift > 0 || c.norm_q_weight || c.norm_k_weight

@@ -103,6 +103,24 @@ def _workspace(device: torch.device, nbytes: int, tag: str = "monarch") -> torch
     return ws
 
 
+_TIGHT_BRIDGE_MB = 1024
+
+
+def _bridge_scratch(device, sizes, num_iters) -> Tuple[torch.Tensor, int]:
+    """(scratch, budget in MiB) of a Monarch forward; sizes = (B, H, D, n_q, n_kv, *blocking).  Budget 0 is the library's
+    default; where the GPU has no memory left for that, the call is cut into chunks of _TIGHT_BRIDGE_MB (same bits)."""
+    lib = _lib.load()
+    # unsupported sizes need 0 bytes: any buffer will do, the entry point names the error
+    nbytes = lib.sfm_monarch_workspace_bytes(*sizes, num_iters, 0) or 256
+    try:
+        return _workspace(device, nbytes), 0
+    except torch.OutOfMemoryError:
+        tight = lib.sfm_monarch_workspace_bytes(*sizes, num_iters, _TIGHT_BRIDGE_MB << 20)
+        if tight >= nbytes:
+            raise
+    return _workspace(device, tight), _TIGHT_BRIDGE_MB
+
+
 def release_workspaces() -> None:
     """Drops every cached scratch buffer (they come back on demand)."""
     with _workspaces_lock:
@@ -207,16 +225,12 @@ def _cache_view_ok(c: torch.Tensor, name: str) -> None:
 def _monarch_fwd(q, k_cache, v_cache, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters):
     B, n_q, H, D = q.shape
     n_kv = k_cache.shape[1]
-    lib = _lib.load()
-    nbytes = lib.sfm_monarch_workspace_bytes(B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, num_iters, 0)
-    if nbytes == 0:
-        # let the entry point produce the precise error
-        nbytes = 256
-    ws = _workspace(q.device, nbytes)
+    ws, budget = _bridge_scratch(q.device, (B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w), num_iters)
     out = torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
-    rc = lib.sfm_monarch_fwd(q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache),
-                             out.data_ptr(), ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w,
-                             float(sm_scale), int(num_iters), 0, _raw_stream(q.get_device()))
+    rc = _lib.load().sfm_monarch_fwd(
+        q.data_ptr(), _batch_stride(q), k_cache.data_ptr(), v_cache.data_ptr(), _batch_stride(k_cache), out.data_ptr(),
+        ws.data_ptr(), ws.numel(), B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, float(sm_scale), int(num_iters),
+        budget << 20, _raw_stream(q.get_device()))
     _lib.check(rc, "sfm_monarch_fwd")
     _after_call(ws)
     return out
@@ -244,16 +258,16 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
     q_rot = torch.empty_like(q) if rope is not None else None
     out = torch.empty_like(q) if q.is_contiguous() else torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
     ws = None if dense else _cached_workspace((device, stream, "monarch"))
+    budget = 0
     for attempt in (0, 1):
         if not dense and (ws is None or attempt):
-            nbytes = _lib.load().sfm_monarch_workspace_bytes(B, H, D, n_q, n_kv, *blocking, num_iters, 0)
-            ws = _workspace(q.device, nbytes or 256)      # unsupported sizes: let the entry point name the error
+            ws, budget = _bridge_scratch(q.device, (B, H, D, n_q, n_kv, *blocking), num_iters)
         call = _KV_CALL.pack(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), 0 if wq is None else wq.data_ptr(), 0 if wk is None else wk.data_ptr(),
             0 if q_rot is None else q_rot.data_ptr(), kc_ptr, vc_ptr, 0 if rope is None else rope.data_ptr(), out.data_ptr(),
             0 if dense else ws.data_ptr(), stream, 0 if lse is None else lse.data_ptr(), q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws.numel(),
             eps, sm_scale, B, H, D, n_q, k.shape[1], n_kv, start_idx, roll_dst, roll_shift, start_frame, *blocking, num_iters,
-            dense, 0)
+            dense, budget)
         rc = _lib.load().sfm_kv_attention(call)
         # the cached scratch may be too small for this call: get more, once (a refused call has launched nothing, so the
         # cache write and its eviction still happen once)
@@ -660,11 +674,10 @@ def rope_monarch_attn_with_kv_cache_sharded(q_shards, k_shards, v_shards, out_sh
     _mark_written(k_cache, v_cache)
     n_kv = end_idx
     kc, vc = k_cache[:, :n_kv], v_cache[:, :n_kv]
-    nbytes = lib.sfm_monarch_workspace_bytes(B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w, 1, 0) or 256
-    ws = _workspace(k_cache.device, nbytes)
+    ws, budget = _bridge_scratch(k_cache.device, (B, H, D, n_q, n_kv, f_tied, h_reduce, w_reduce, h, w), 1)
     rc = lib.sfm_monarch_fwd_scatter(_ptr(q_rot), _batch_stride(q_rot), _ptr(kc), _ptr(vc), _batch_stride(kc),
                                      _ptr_array(out_shards), world, int(rank), _ptr(ws), ws.numel(), B, H, D, n_q,
-                                     n_kv, f_tied, h_reduce, w_reduce, h, w, float(sm_scale), 0, _stream())
+                                     n_kv, f_tied, h_reduce, w_reduce, h, w, float(sm_scale), budget << 20, _stream())
     _lib.check(rc, "sfm_monarch_fwd_scatter")
     if os.environ.get("SFM_CHECK_STATUS") == "1":
         _lib.check(lib.sfm_workspace_status(_ptr(ws), _stream()), "sfm_workspace_status")
@@ -711,14 +724,13 @@ def _monarch_attn_fwd(q, k, v, f_tied, h_reduce, w_reduce, h, w, sm_scale, block
                                       0, 1, _stream())
         _lib.check(rc, "sfm_rope_cache_write")
         return _monarch_fwd(q, k_mon, v_mon, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters), k_mon, v_mon, 0
-    nbytes = lib.sfm_monarch_workspace_bytes(B, H, D, N, N, f_tied, h_reduce, w_reduce, h, w, num_iters, 0) or 256
-    ws = _workspace(q.device, nbytes)
+    ws, budget = _bridge_scratch(q.device, (B, H, D, N, N, f_tied, h_reduce, w_reduce, h, w), num_iters)
     out = torch.empty_like(q)
     k_mon = torch.empty_like(k)
     v_mon = torch.empty_like(v)
     rc = lib.sfm_monarch_nocache_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(k_mon), _ptr(v_mon), _ptr(out), _ptr(ws),
                                      ws.numel(), B, H, D, N, f_tied, h_reduce, w_reduce, h, w, float(sm_scale),
-                                     causal_groups, int(num_iters), 0, _stream())
+                                     causal_groups, int(num_iters), budget << 20, _stream())
     _lib.check(rc, "sfm_monarch_nocache_fwd")
     return out, k_mon, v_mon, causal_groups
 

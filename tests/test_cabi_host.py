@@ -159,7 +159,7 @@ def test_layer_call_is_refused_before_its_cache_write(sfb, field, value, rc):
     need = sfb.workspace_bytes(1, 2, 1560, 3120, 1, 1, 1, 30, 52)
     names = ("q k v wq wk q_rot k_cache v_cache rope out workspace stream lse q_bs cache_bs workspace_bytes eps sm_scale "
              "B H D n_q n_new n_kv start_idx roll_dst roll_shift start_frame f_tied h_reduce w_reduce h w num_iters dense "
-             "reserved").split()
+             "bridge_budget_mb").split()
     call = dict(zip(names, [256, 256, 256, 0, 0, 256, 256, 256, 256, 256, 256, 0, 0, 1560 * 256, 3120 * 256, need, 1e-6, 0.088,
                             1, 2, 128, 1560, 1560, 3120, 1560, 0, 1560, 0, 1, 1, 1, 30, 52, 1, 0, 0]))
     call[field] = need - 1 if (field, value) == ("workspace_bytes", 1) else value

@@ -215,6 +215,39 @@ def test_monarch_chunking_is_invisible(sfb, monkeypatch):
     assert torch.equal(z_a, z_b)
 
 
+@pytest.mark.parametrize("path", ["cache", "on_cache", "iterative", "clip"])
+def test_monarch_in_smaller_chunks_where_memory_is_short(sfb, monkeypatch, path):
+    """Where the default scratch cannot be allocated a call runs in smaller chunks, with the same bits."""
+    from self_forcing_b200 import ops
+    c = small_case(0, 1, B=3, H=5)
+    q, kc, vc = c["q"].cuda(), c["kbuf"].cuda(), c["vbuf"].cuda()
+
+    def call():
+        if path == "cache":
+            return run_gpu_cache(sfb, c)[0]
+        if path == "clip":
+            return sfb.monarch_attn(kc, vc, kc, *c["blocking"], block_causal_size=q.shape[1])
+        return ops.monarch_attention_on_cache(q, kc[:, :c["n_kv"]], vc[:, :c["n_kv"]], *c["blocking"],
+                                              num_iters=3 if path == "iterative" else 1)
+
+    ref = call()
+    ops.release_workspaces()
+    refused = []
+
+    def short_of_memory(device, nbytes, tag="monarch", real=ops._workspace):
+        if nbytes > 3 << 20:
+            refused.append(nbytes)
+            raise torch.OutOfMemoryError("no memory")
+        return real(device, nbytes, tag)
+
+    monkeypatch.setattr(ops, "_workspace", short_of_memory)
+    with pytest.raises(torch.OutOfMemoryError):           # the smaller chunks do not fit either
+        call()
+    monkeypatch.setattr(ops, "_TIGHT_BRIDGE_MB", 1)
+    assert torch.equal(call(), ref) and len(refused) >= 2
+    ops.release_workspaces()
+
+
 def test_monarch_properties_full_size(sfb):
     """Size-independent properties at the full benchmark size (12 heads, 32760 cached tokens):
     (1) bitwise run-to-run determinism, (2) a constant V comes back unchanged (all softmax
