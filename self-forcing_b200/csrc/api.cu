@@ -168,6 +168,8 @@ int prepare_monarch(MonarchCall* mc, const void* q, int64_t q_bs, const void* kc
     if (pl.blk.b2 > kB2Max && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
     // only the tensor-core column step knows how to scatter its rows
     if (os && os->world > 1 && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
+    // its stores are 32 bytes wide (the mma.sync one's 16)
+    if (use_tc && pl.blk.b1 <= 128 && (reinterpret_cast<uintptr_t>(out) & 31)) return SFM_ERR_ALIGNMENT;
     const int n_s = (pl.blk.b2 + 15) & ~15;
     mc->BH = B * H; mc->n_s = n_s; mc->num_iters = num_iters; mc->num_sms = device_sms();
     mc->use_tc = use_tc; mc->iter_tc = iter_tc;
@@ -351,7 +353,7 @@ extern "C" const char* sfm_error_string(int code) {
         case SFM_ERR_NULL_POINTER: return "null pointer argument";
         case SFM_ERR_BAD_SHAPE: return "sizes inconsistent with the blocking";
         case SFM_ERR_UNSUPPORTED: return "unsupported size (head_dim must be 128; block columns <= 128, and <= 64 for the iterative variant or block rows above 128)";
-        case SFM_ERR_ALIGNMENT: return "pointer or stride not 16-byte aligned";
+        case SFM_ERR_ALIGNMENT: return "pointer or stride not 16-byte aligned (attention output: 32-byte)";
         case SFM_ERR_WORKSPACE: return "workspace too small";
         case SFM_ERR_NO_DEVICE: return "no sm_100 device";
         case SFM_ERR_DEVICE_STATUS: return "kernel recorded an internal error status";

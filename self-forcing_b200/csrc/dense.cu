@@ -27,6 +27,7 @@ int prepare_dense(DenseCall* c, const void* q, int64_t q_batch_stride, const voi
     if (!(sm_scale > 0.f)) return SFM_ERR_BAD_SHAPE;       // the row maximum is taken before scaling
     auto mis = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
     if (mis(q) || mis(k) || mis(v) || mis(out) || (q_batch_stride % 8) || (kv_batch_stride % 8)) return SFM_ERR_ALIGNMENT;
+    if (reinterpret_cast<uintptr_t>(out) & 31) return SFM_ERR_ALIGNMENT;       // the kernel's stores are 32 bytes wide
 
     static std::atomic<int*> words[64];                     // the status word's address, looked up once per device
     int dev = 0;

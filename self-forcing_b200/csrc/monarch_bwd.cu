@@ -791,6 +791,8 @@ static int monarch_bwd(bool train, const void* out_fwd, const float* lse_fwd, co
     const char* row_fp32 = getenv("SFM_BWD_ROW_FP32");          // keeps the fp32 row kernel
     if (train && (!use_tc || (row_fp32 && row_fp32[0] == '1') || kv_group_begin % blk.gpt || kv_group_end % blk.gpt))
         return SFM_ERR_UNSUPPORTED;
+    // the recompute's output lies in the workspace, and the column step stores 32 bytes at a time
+    if (use_tc && (reinterpret_cast<uintptr_t>(workspace) & 31)) return SFM_ERR_ALIGNMENT;
 
     const int T = blk.b1 <= 16 ? 2 : (blk.b1 <= 32 ? 4 : (blk.b1 <= 64 ? 8 : 16));
     const int LT = blk.b2 <= 64 ? 16 : 32;

@@ -101,6 +101,13 @@ def test_entry_points_validate_arguments_without_a_gpu(sfb):
                                1.0, 1, 0, null) == -5
     assert lib.sfm_monarch_fwd(one, 0, one, one, 0, one, one, 1 << 30, 1, 1, 128, 1000, 1560, 1, 1, 1, 30, 52,
                                1.0, 1, 0, null) == -2
+    # the attention kernels store 32 bytes at a time
+    for out in (C.c_void_p(272), C.c_void_p(264)):
+        assert lib.sfm_dense_fwd(one, 0, one, one, 0, out, 1, 1, 128, 16, 16, 1.0, null) == -4
+        assert lib.sfm_monarch_fwd(one, 0, one, one, 0, out, one, 1 << 30, 1, 1, 128, 1560, 1560, 1, 1, 1, 30, 52,
+                                   1.0, 1, 0, null) == -4
+    assert lib.sfm_monarch_bwd(one, 0, one, one, 0, one, one, one, one, C.c_void_p(272), 1 << 40, 1, 1, 128, 1560, 3120, 1, 1, 1,
+                               30, 52, 1.0, 0, 2, 0, 0, null) == -4
     assert lib.sfm_rope_cache_write(null, one, one, null, one, one, 0, null, 1, 100, 1, 128, 0, 1, 1, 1, 30, 52,
                                     0, 1, null) == -2
     # fused RMSNorm front end: both weights and q are required
