@@ -21,7 +21,9 @@ from . import _lib
 
 _workspaces: "OrderedDict[Tuple[int, int, str], torch.Tensor]" = OrderedDict()      # least recently used first
 _workspaces_lock = threading.RLock()
-_rope_tables: Dict[tuple, torch.Tensor] = {}
+_lib_rope_tables: Dict[Optional[int], torch.Tensor] = {}         # the library's own table, per GPU
+_rope_tables: Dict[tuple, tuple] = {}
+_MAX_ROPE_TABLES = 8
 _status_mirror: Dict[int, list] = {}
 
 
@@ -172,23 +174,33 @@ def _rope_table_from_freqs(freqs: Optional[torch.Tensor], device: torch.device) 
     """Device table [1024, 64, 2] fp32 = (cos, sin).  Built from the model's complex128
     ``freqs`` buffer when given (causal_model.py:1352-1357), else by the library."""
     if freqs is None:
-        key = ("lib", device.index)
-        tab = _rope_tables.get(key)
+        tab = _lib_rope_tables.get(device.index)
         if tab is None:
             host = np.empty((1024, 64, 2), dtype=np.float32)
             _lib.check(_lib.load().sfm_rope_table(host.ctypes.data_as(C.c_void_p), 128, 1024, 10000.0),
                        "sfm_rope_table")
             tab = torch.from_numpy(host).to(device)
-            _rope_tables[key] = tab
+            _lib_rope_tables[device.index] = tab
         return tab
-    key = (freqs.data_ptr(), tuple(freqs.shape), device)
-    tab = _rope_tables.get(key)
-    if tab is None:
+    # The entry keeps ``freqs`` alive, so that its address cannot come to hold another table, and the version of its content.
+    key = (freqs.data_ptr(), tuple(freqs.shape), freqs.stride(), freqs.dtype, freqs.device, device)
+    entry = _rope_tables.get(key)
+    if entry is None or not entry[1] == _version(freqs) == _version(entry[0]):
         if freqs.dim() != 2 or freqs.shape[1] != 64 or freqs.shape[0] < 1024 or not freqs.is_complex():
             raise ValueError("freqs must be a complex [>=1024, 64] table")
         tab = torch.view_as_real(freqs[:1024].to(torch.complex128)).to(torch.float32).contiguous().to(device)
-        _rope_tables[key] = tab
-    return tab
+        # complete for calls on any stream, and nothing reads a table that is dropped
+        if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.synchronize(device)
+        _rope_tables.pop(key, None)
+        while len(_rope_tables) >= _MAX_ROPE_TABLES:
+            _rope_tables.pop(next(iter(_rope_tables)))
+        entry = _rope_tables[key] = (freqs, _version(freqs), tab)
+    return entry[2]
+
+
+def _version(t: torch.Tensor) -> int:
+    return 0 if t.is_inference() else t._version           # inference tensors carry no version counter
 
 
 def _mark_written(*tensors) -> None:

@@ -64,6 +64,27 @@ def test_rope_table_matches_oracle(sfb):
     assert np.array_equal(host[..., 1], sin.numpy().astype(np.float32))
 
 
+def test_rope_table_follows_its_freqs(sfb):
+    """The device table built from a model's freqs is kept while they stay as they are: not past a change in place, and not
+    for another table at the same address (a transposed view of the same memory here)."""
+    import torch
+    from self_forcing_b200 import ops
+    cpu = torch.device("cpu")
+    base = torch.randn(2048, 64, dtype=torch.complex128)
+    want = lambda f: torch.view_as_real(f[:1024]).float()
+    freqs = base[:1024]
+    tab = ops._rope_table_from_freqs(freqs, cpu)
+    assert torch.equal(tab, want(freqs)) and ops._rope_table_from_freqs(freqs, cpu) is tab
+    other = base.as_strided((1024, 64), (1, 1024))
+    assert torch.equal(ops._rope_table_from_freqs(other, cpu), want(other))
+    with torch.no_grad():
+        freqs.mul_(2.0)
+    assert torch.equal(ops._rope_table_from_freqs(freqs, cpu), want(freqs))
+    for _ in range(2 * ops._MAX_ROPE_TABLES):              # the kept tables are bounded
+        ops._rope_table_from_freqs(torch.randn(1024, 64, dtype=torch.complex64), cpu)
+    assert len(ops._rope_tables) <= ops._MAX_ROPE_TABLES
+
+
 def test_workspace_planning(sfb):
     # framewise, 7 chunks cached: the bridge of one head is 3*52 columns x 630 keys x 516 bytes
     per_head = 3 * 52 * 630 * (2 * 128 * 2 + 4)
