@@ -822,6 +822,41 @@ def test_two_streams_use_separate_workspaces(sfb):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("entry", ["with_cache", "on_cache", "clip", "dense", "layer", "backward"])
+def test_first_gpu_work_of_a_thread(sfb, entry):
+    """A thread whose first work on the GPU is a call of this package: the thread has no CUDA context yet when the tensor
+    maps are made."""
+    import threading
+    c = small_case(0, 1, B=1)
+    q, nk, nv = c["q"].cuda(), c["nk"].cuda(), c["nv"].cuda()
+    kc, vc = c["kbuf"].cuda()[:, :c["n_kv"]].contiguous(), c["vbuf"].cuda()[:, :c["n_kv"]].contiguous()
+    _, _, _, h, w = c["blocking"]
+    cfg = sfb.LayerConfig(max_attention_size=c["n_kv"])
+    call = {
+        "with_cache": lambda: sfb.monarch_attn_with_kv_cache(q, kc, vc, nk, nv, c["start"], c["end"], *c["blocking"]),
+        "on_cache": lambda: sfb.ops.monarch_attention_on_cache(q, kc, vc, *c["blocking"]),
+        "clip": lambda: sfb.monarch_attn(q, nk, nv, *c["blocking"]),
+        "dense": lambda: sfb.attention(q, kc, vc),
+        "layer": lambda: sfb.self_attention_kv(q, nk, nv, sfb.KVCache(kc, vc, c["start"], c["start"]), c["start"], (3, h, w), cfg),
+        "backward": lambda: sfb.monarch_attn_with_kv_cache_backward(q, kc, vc, q, *c["blocking"])[0],
+    }[entry]
+    ref, got = call(), []
+    torch.cuda.synchronize()
+
+    def first():
+        try:
+            got.append(call())
+        except Exception as e:
+            got.append(e)
+
+    t = threading.Thread(target=first)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert isinstance(got[0], torch.Tensor) and torch.equal(got[0], ref), got[0]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bound", ["count", "bytes"])
 def test_least_recently_used_workspace_is_dropped(sfb, monkeypatch, bound):
     """Scratch kept for two streams at most, by count or by bytes: a stream that has just been used keeps its buffer, the
