@@ -209,6 +209,7 @@ int launch_monarch(MonarchCall& mc) {
     float* lse = mc.lse;
     int* status = mc.status;
     cudaStream_t stream = mc.stream;
+    std::lock_guard<std::mutex> lock(launch_mutex(status));       // the workspace's first word
     int rc;
     // Every path starts from a clear status word: the workspace may be recycled memory.  The tensor-core path's first
     // kernel clears it; the mma.sync kernels have no bounded waits and never write it.

@@ -808,6 +808,7 @@ static int monarch_bwd(bool train, const void* out_fwd, const float* lse_fwd, co
     if (bad) return SFM_ERR_UNSUPPORTED;
 
     cudaStream_t s = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> lock(launch_mutex(workspace));
     const int BH = B * H;
     const int num_sms = device_sms();
     // one status word per call: a kernel that gives up on a bounded wait sets it, nothing clears it before the end

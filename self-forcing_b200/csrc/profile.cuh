@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 namespace sfm {
 
 enum KernelClass { kClsLayout = 0, kClsRStep = 1, kClsLStep = 2, kClsLIter = 3, kClsDense = 4, kClsBackward = 5, kNumClasses = 6 };
@@ -19,6 +21,9 @@ struct LaunchScope {
 // and a kernel's opt-in to `bytes` of dynamic shared memory.
 int device_sms();
 int opt_in_smem(const void* kernel, int bytes);
+// Held while a call's kernels are launched: they pass their results through its workspace, so the launches of two threads
+// that share one (and a stream) must not mix.  A few mutexes serve all workspaces.
+std::mutex& launch_mutex(const void* workspace);
 
 // Launch as a programmatic dependent of the kernel before it in the stream: the grid may be set up while that one
 // finishes, and every thread waits (pdl_wait) for its completion before it touches global memory.  Every kernel launched

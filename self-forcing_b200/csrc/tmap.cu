@@ -42,6 +42,11 @@ int opt_in_smem(const void* kernel, int bytes) {
     return (int)e;
 }
 
+std::mutex& launch_mutex(const void* workspace) {
+    static std::mutex mutexes[64];
+    return mutexes[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
+}
+
 EncodeTiledFn get_encode_tiled() {
     static EncodeTiledFn fn = nullptr;
     if (fn) return fn;

@@ -3,7 +3,7 @@
 Every function here launches hand-written sm_100a kernels through the C ABI on the current
 CUDA stream.  Inputs must be CUDA bf16 tensors with head_dim 128; anything else raises (there
 is no eager / CPU fallback).  Scratch memory is a buffer per (GPU, stream) that grows on demand, is
-reused by later calls queued on that stream and can be dropped with release_workspaces().
+reused by later calls queued on that stream, from whichever thread, and can be dropped with release_workspaces().
 """
 from __future__ import annotations
 

@@ -857,6 +857,41 @@ def test_first_gpu_work_of_a_thread(sfb, entry):
 
 
 @pytest.mark.gpu
+def test_threads_may_share_a_stream(sfb):
+    """Calls from three threads on one stream use the same scratch one after the other: every result is bit-equal to the
+    one that the same inputs gave alone."""
+    import threading
+    from self_forcing_b200 import ops
+    work = []
+    for seed in (11, 12, 13):
+        c = small_case(0, 1, B=1, seed=seed)
+        args = (c["q"].cuda(), c["kbuf"].cuda()[:, :c["n_kv"]].contiguous(), c["vbuf"].cuda()[:, :c["n_kv"]].contiguous(),
+                c["nk"].cuda(), c["nv"].cuda(), c["start"], c["end"], *c["blocking"])
+        out = sfb.monarch_attn_with_kv_cache(*args)
+        bwd = (*args[:3], out, *c["blocking"])
+        work.append((args, bwd, out, sfb.monarch_attn_with_kv_cache_backward(*bwd)[0]))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def repeat(args, bwd, out, dq):
+        try:
+            for i in range(400):
+                if not torch.equal(sfb.monarch_attn_with_kv_cache(*args), out):
+                    wrong.append("out")
+                if i % 4 == 0 and not torch.equal(ops.monarch_attn_with_kv_cache_backward(*bwd)[0], dq):
+                    wrong.append("dq")
+        except Exception as e:
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=repeat, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, (len(wrong), set(wrong))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bound", ["count", "bytes"])
 def test_least_recently_used_workspace_is_dropped(sfb, monkeypatch, bound):
     """Scratch kept for two streams at most, by count or by bytes: a stream that has just been used keeps its buffer, the
