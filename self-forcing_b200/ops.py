@@ -375,8 +375,9 @@ _nat2mon_index: Dict[tuple, torch.Tensor] = {}
 
 
 def _nat2mon_on_device(n_tokens, blocking, device):
-    """The permutation as an index tensor on the GPU; the last few are kept (a copy from the host waits for the GPU)."""
-    key = (n_tokens, blocking, device.index)
+    """The permutation as an index tensor on the GPU; the last few are kept (a copy from the host waits for the GPU), each for
+    the stream that it was made on, so that its memory is not handed out while another stream reads it."""
+    key = (n_tokens, blocking, device.index, _raw_stream(device.index))
     idx = _nat2mon_index.get(key)
     if idx is None:
         idx = torch.from_numpy(build_maps(n_tokens, *blocking)[0].astype(np.int64)).to(device)

@@ -857,6 +857,19 @@ def test_first_gpu_work_of_a_thread(sfb, entry):
 
 
 @pytest.mark.gpu
+def test_kept_permutations_stay_on_their_stream(sfb):
+    """The index tensors that the backward keeps are allocated on the stream that uses them: one of another stream could be
+    dropped, and its memory reused there, while it is read here."""
+    from self_forcing_b200 import ops
+    made = []
+    for s in (torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(s):
+            made.append(ops._nat2mon_on_device(96, (1, 2, 2, 6, 8), torch.device("cuda", torch.cuda.current_device())))
+    torch.cuda.synchronize()
+    assert made[0].data_ptr() != made[1].data_ptr() and torch.equal(*made)
+
+
+@pytest.mark.gpu
 def test_threads_may_share_a_stream(sfb):
     """Calls from three threads on one stream use the same scratch one after the other: every result is bit-equal to the
     one that the same inputs gave alone."""
