@@ -439,28 +439,6 @@ def run_model(args, rank, world, device, barrier):
                           "gpu_launches": int(launches), "clocks": clocks}), flush=True)
 
 
-def run_probe_dsmem(device):
-    """Store bandwidth between the CTAs of a cluster through distributed shared memory (sfm_probe_dsmem_store):
-    the ceiling of an on-chip hand-off between the row step and the column step."""
-    import ctypes as C
-    from self_forcing_b200 import _lib
-    lib = _lib.load()
-    rows = []
-    for cluster in (1, 2, 4, 8, 16):
-        for remote in ((0,) if cluster == 1 else (0, 1)):
-            for pattern in (0, 1):
-                ms, ctas, nbytes = C.c_float(), C.c_int(), C.c_double()
-                rc = lib.sfm_probe_dsmem_store(cluster, pattern, remote, 2000, C.byref(ms), C.byref(ctas), C.byref(nbytes))
-                row = {"cluster": cluster, "remote": bool(remote), "pattern": "row-per-lane 32 B" if pattern == 0 else "coalesced 16 B"}
-                if rc:
-                    row["error"] = lib.sfm_error_string(rc).decode()
-                else:
-                    row.update(ctas=ctas.value, ms=ms.value, tb_per_s=nbytes.value / ms.value * 1e-9,
-                               bytes_per_clk_per_sm=nbytes.value / (ms.value * 1e-3) / ctas.value / 1.965e9)
-                rows.append(row)
-    print(json.dumps({"probe": "dsmem_store", "sm_clock_assumed_mhz": 1965, "rows": rows}, indent=1))
-
-
 def run_incumbent(args, device):
     """The reference's own Triton Monarch path (monarch_attn_with_kv_cache, num_iters=1: _al_cl_y_fwd + _z_fwd
     in 3x3 group chunks, monarch_attn.py:1227-1323), imported unmodified from the staged checkout and timed on
@@ -716,8 +694,6 @@ def main():
     ap.add_argument("--p2p", action="store_true",
                     help="with --ulysses or --model --sp: the kernels gather / scatter over peer memory instead of the two "
                          "NCCL all-to-alls")
-    ap.add_argument("--probe-dsmem", action="store_true",
-                    help="measure store bandwidth between the CTAs of a cluster (distributed shared memory) and exit")
     ap.add_argument("--incumbent", action="store_true",
                     help="time the reference's own Triton Monarch op beside this package's on the same tensors "
                          "(needs the staged reference sources) and exit")
@@ -757,9 +733,9 @@ def main():
     else:
         barrier = lambda: None
 
-    if args.probe_dsmem or args.incumbent:
+    if args.incumbent:
         if rank == 0:
-            run_probe_dsmem(device) if args.probe_dsmem else run_incumbent(args, device)
+            run_incumbent(args, device)
         if use_dist:
             dist.destroy_process_group()
         return

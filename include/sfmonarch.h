@@ -401,16 +401,6 @@ int sfm_profile_enable(int on);
 int sfm_profile_read(float* ms, long long* launches, int n_classes);
 
 /*
- * Diagnostic (no counterpart in the reference): store bandwidth between the CTAs of a thread-block
- * cluster through distributed shared memory, the traffic pattern of an on-chip hand-off between the row
- * step and the column step.  `cluster` CTAs per cluster (1, 2, 4, 8, 16), one CTA per SM, `iters` passes of
- * 64 KB per CTA; pattern 0 = one 256-byte row per lane written in 32-byte pieces, 1 = coalesced 16-byte
- * stores; remote 0 = own shared memory, 1 = the peers'.  Plain stores to cluster-mapped addresses only.
- * Returns elapsed milliseconds, CTAs launched and bytes stored.
- */
-int sfm_probe_dsmem_store(int cluster, int pattern, int remote, int iters, float* ms, int* ctas, double* bytes);
-
-/*
  * Self-test of the failure path (no counterpart in the reference, whose kernels have no device-side waits): one
  * small CTA allocates tensor memory as the attention kernels do and waits, for `polls` polls (1 .. 65536), on an
  * mbarrier nothing arrives at.  The wait runs out, the kernel stores `code` (1 .. 255) in the status word at the
