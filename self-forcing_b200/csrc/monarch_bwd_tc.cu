@@ -62,7 +62,6 @@ struct BwdColParams {
     float* dq;                     // natural order [B, n_q, H, 128] fp32
     int H, n_q, A, n_keys, n_keys_c, bh0, nbh;
     int n_units;                   // nbh * A * b2
-    int q_rows_tma;
     int q_box_rows;                // rows per box of the q / dOut row maps (32, or all the grid rows there are)
     float scale;
     Blocking blk;
@@ -466,7 +465,8 @@ int launch_bwd_delta(const void* dout, const void* out, float* delta, long long 
 // Column-step backward for one slice of (batch, head) pairs.  maps = {q rows, dOut rows}, 5-D (d, head, column, row of the token grid, batch) with boxes of 32 rows.
 int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const float* delta, float* dcL, float* dq,
                       int* status, int num_sms, cudaStream_t s) {
-    if (mp.blk.b1 > kMaxNC * kNI) return SFM_ERR_UNSUPPORTED;
+    // query rows come by TMA: they must be consecutive rows of the token grid
+    if (mp.blk.b1 > kMaxNC * kNI || (mp.blk.f_tied != 1 && mp.blk.h_reduce != 1)) return SFM_ERR_UNSUPPORTED;
     LaunchScope scope(kClsBackward, s);
     BwdColParams p;
     p.delta = delta; p.lse = mp.lse;
@@ -475,8 +475,6 @@ int launch_bwd_col_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
     p.bh0 = mp.bh0; p.nbh = mp.nbh;
     p.n_units = mp.nbh * mp.na * mp.blk.b2;
     p.q_box_rows = std::min(32, mp.n_q / mp.blk.w);
-    p.q_rows_tma = (mp.blk.f_tied == 1 || mp.blk.h_reduce == 1) ? 1 : 0;
-    if (!p.q_rows_tma) return SFM_ERR_UNSUPPORTED;
     p.scale = mp.scale;
     p.blk = mp.blk;
     p.status = status;

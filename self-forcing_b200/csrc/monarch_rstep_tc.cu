@@ -41,7 +41,7 @@ using namespace tc;
 
 namespace {
 
-constexpr int kStages = 10;           // K/V tile ring, at most
+constexpr int kStages = 8;            // K/V tile ring, at most
 constexpr int kThreads = 608;          // 19 warps: one more would lower the register ceiling from 104 to 96
 constexpr int kTileRows = 128;
 constexpr int kMaxSBufs = 4;

@@ -32,7 +32,7 @@ def _stream() -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else None
+_raw_stream = torch._C._cuda_getCurrentRawStream
 
 
 def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
@@ -814,13 +814,6 @@ def full_attention_with_kv_cache(q, k_cache, v_cache, new_k, new_v, start_idx, e
     _lib.check(rc, "sfm_rope_cache_write")
     _mark_written(k_cache, v_cache)
     return attention(q, k_cache, v_cache, softmax_scale=sm_scale)
-
-
-def dense_attention_on_cache(q, k_view, v_view, sm_scale=None):
-    """Dense attention of already rotated q against a cache view that already holds the new tokens."""
-    _cache_view_ok(k_view, "k_cache")
-    _cache_view_ok(v_view, "v_cache")
-    return attention(q, k_view, v_view, softmax_scale=sm_scale)
 
 
 def monarch_attention_on_cache(q, k_view, v_view, f_tied, h_reduce, w_reduce, h, w, sm_scale=None, num_iters=1):
