@@ -2,7 +2,7 @@
 
 The harness imports ``wan/modules/causal_model.py``, ``utils/wan_wrapper.py`` and
 ``pipeline/causal_inference.py`` from a staged checkout (``baseline/_ref/``, see
-``baseline/stage_reference.py``, or ``SF_REFERENCE_ROOT``) and builds what BASELINE's full-model
+``baseline/stage_reference.py``, or ``SF_REFERENCE_ROOT``) and builds what the full-model
 configurations describe: a random-init causal Wan DiT, a 21-frame latent generated in 7 chunks of 3
 frames with 4 denoising steps per chunk, a random 512x4096 text context through cross-attention.
 

@@ -42,21 +42,18 @@ CHUNK = CHUNK_FRAMES * H_GRID * W_GRID          # 4680 tokens
 N_LAYER_CACHES = 4                              # rotated so K/V (201 MB per layer at k=7) is never L2 resident
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of each kernel at the bench
-# workload, from the ncu capture summarised in profiles/monarch_framewise_k7_ncu.md.
-# dram__bytes_read.sum + dram__bytes_write.sum per launch from ncu captures of this bench at k = 7 (averaged over a
-# step's launches where the bridge budget cuts the step into several); profiles/monarch_framewise_k7_ncu.md,
-# profiles/sweep_blockings_k1_7.md and profiles/dense_k7_ncu.md give the commands
+# DRAM bytes of each kernel in one step of this bench at k = 7 (dram__bytes_read.sum + dram__bytes_write.sum, ncu, one pass,
+# summed over the step's launches: two row and two column steps for reduce4xw2xh, one of each elsewhere)
 NCU_TRAFFIC = {
-    ("framewise", 7): {"monarch_row_step": 261.1e6 + 561.3e6, "monarch_col_step": 624.0e6 + 9.4e6,
-                       "layout_rope_cache_write": 43.2e6 + 2.5e6},
-    ("tied3frame", 7): {"monarch_row_step": 216.4e6 + 157.1e6, "monarch_col_step": 217.5e6 + 6.0e6,
-                        "layout_rope_cache_write": 43.2e6 + 2.5e6},
-    ("reduce2xh", 7): {"monarch_row_step": (347.5e6 + 1123.6e6) / 2, "monarch_col_step": (1233.6e6 + 9.7e6) / 2,
-                       "layout_rope_cache_write": 43.2e6 + 3.0e6},
-    ("reduce4xw2xh", 7): {"monarch_row_step": (564.7e6 + 4543.0e6) / 6, "monarch_col_step": (4884.8e6 + 2.2e6) / 6,
-                          "layout_rope_cache_write": 43.2e6 + 2.5e6},
-    ("dense", 7): {"dense": 215.9e6 + 13.0e6},
+    ("framewise", 7): {"monarch_row_step": 256.6e6 + 554.4e6, "monarch_col_step": 623.4e6 + 9.3e6,
+                       "layout_rope_cache_write": 43.2e6 + 2.9e6},
+    ("tied3frame", 7): {"monarch_row_step": 216.0e6 + 151.6e6, "monarch_col_step": 217.4e6 + 5.4e6,
+                        "layout_rope_cache_write": 43.2e6 + 2.6e6},
+    ("reduce2xh", 7): {"monarch_row_step": 357.2e6 + 1170.6e6, "monarch_col_step": 1232.6e6 + 9.3e6,
+                       "layout_rope_cache_write": 43.2e6 + 2.7e6},
+    ("reduce4xw2xh", 7): {"monarch_row_step": 586.3e6 + 4788.4e6, "monarch_col_step": 4885.0e6 + 10.3e6,
+                          "layout_rope_cache_write": 43.2e6 + 2.7e6},
+    ("dense", 7): {"dense": 215.8e6 + 7.9e6},
 }
 
 
@@ -365,7 +362,7 @@ def run_rollout(args, sfb, rank, world, device, barrier):
 
 
 def run_model(args, rank, world, device, barrier):
-    """BASELINE's full-model configurations: the reference's own CausalWanModel, WanDiffusionWrapper and
+    """The full-model configurations: the reference's own CausalWanModel, WanDiffusionWrapper and
     CausalInferencePipeline, imported unmodified from a staged checkout (baseline/stage_reference.py), with
     random-init bf16 weights, a random 512x4096 text context and seeded latent noise; 21 frames in 7 chunks
     of 3, 4 denoising steps plus the clean-context pass per chunk.  --attention selects what the model's
@@ -888,7 +885,7 @@ def main():
         dom_ms = kernels[dom]["ms_per_step"]
         dom_flops = {"monarch_row_step": r_flops, "monarch_col_step": l_flops, "dense": flops}.get(dom, 0.0)
         ach = dom_flops / (dom_ms * 1e-3) / 1e12 if dom_ms > 0 else 0.0
-        traffic = NCU_TRAFFIC.get((args.blocking, args.k), {}).get(dom)
+        traffic = NCU_TRAFFIC.get((args.blocking, args.k), {}).get(dom) if args.num_iters == 1 else None
         roofline = {"kernel": dom, "bound": "tensor", "achieved": ach, "peak": tf_peak, "unit": "TFLOP/s",
                     "frac": ach / tf_peak, "peak_kind": f"of {peak_kind}", "traffic": traffic,
                     "launch_ms_per_step": dom_ms,

@@ -132,7 +132,7 @@ int sfm_rope_apply(const void* x, void* out, const float* rope, int B, int L, in
 /*
  * Scratch bytes sfm_monarch_fwd needs for these sizes.  The row-step results (aL, Y,
  * cL) of one chunk of (batch, head, query-group) live there between the two kernels;
- * bridge_budget_bytes bounds one chunk so that it stays L2 resident (0 = default).
+ * bridge_budget_bytes bounds one chunk (0 = default, 4 GiB).
  * Replaces: the aL / y / cL scratch tensors of _attention_with_cache.forward
  * (wan/modules/monarch_attn.py:1246-1259).
  */

@@ -14,8 +14,10 @@
 //
 // What bounds it: per 128 x 128 tile the S halves take 768 tensor-pipe cycles (an N = 64 instruction reads as much shared
 // memory for its A operand as an N = 128 one: 48 cycles instead of 32), PV 512, the exponentials 1024 on the
-// transcendental pipe, and the softmax chain overlaps the two.  4680 queries x 18720 keys x 12 heads: 0.567 ms with
-// the MMAs issued from one-lane code, 0.440 ms as it is (0.72 of the bf16 GEMM rate).  One N = 128 S GEMM per tile
+// transcendental pipe, and the softmax chain overlaps the two.  4680 queries x 18720 keys x 12 heads, in
+// runs of 20 calls: 0.567 ms with the MMAs issued from one-lane code, 0.440 ms as it is (0.73 of the bf16 GEMM burst rate).
+// In long runs the power cap holds the SMs at 1.7 GHz and the kernel takes 0.51 ms: the call with its cache write 0.642 ms
+// before, 0.528 ms as it is.  One N = 128 S GEMM per tile
 // instead of two halves: 0.488 ms, the halves' overlap is worth more than its 256 cycles.
 //
 // Arithmetic: softmax(q k^T * scale) v (wan/modules/attention.py:177-187).

@@ -42,7 +42,7 @@ using namespace tc;
 namespace {
 
 constexpr int kStages = 8;            // K/V tile ring, at most
-constexpr int kThreads = 608;          // 19 warps: one more would lower the register ceiling from 104 to 96
+constexpr int kThreads = 608;          // 19 warps, 96 registers a thread
 constexpr int kTileRows = 128;
 constexpr int kMaxSBufs = 4;
 constexpr uint32_t kTmemCols = 512;
@@ -136,7 +136,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     static_assert(kStg >= 2 && kStg <= kStages, "K / V ring");
     unsigned char* q_s = base;
     unsigned char* kv_s = q_s + kQBufs * kQBytes;
-    unsigned char* o_s = kv_s + kStg * kStgBytes;            // one 4 KB staging buffer per epilogue warp
+    unsigned char* o_s = kv_s + kStg * kStgBytes;            // two 4 KB staging buffers per epilogue warp
     Barriers* bars = reinterpret_cast<Barriers*>(base + kSmemData);
 
     if (warp == 2 && lane == 0) { prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tal); prefetch_tmap(&ty); }
@@ -280,7 +280,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         }
     } else if (warp >= 3 && warp < 11) {
         // ------------------------------------------------------------------ softmax warpgroups
-        const int wg = (warp - 3) >> 2;                 // 0: even steps / buffer 0, 1: odd steps / buffer 1
+        const int wg = (warp - 3) >> 2;                 // 0: even steps, 1: odd steps; the S / P buffers rotate over all steps
         const int quad = warp & 3;                      // TMEM lane quadrant this warp may access
         const int row = quad * 32 + lane;               // tile row == TMEM lane
         const int gl = row / RG, j = row - gl * RG;
@@ -569,7 +569,6 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     rp.status = status;
     rp.clear_status = clear_status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
-    // wide blocks: two 64 KB K / V stages instead of five 32 KB ones
     const bool iter = p.use_aR != 0;
     if (iter && (n_s > 64 || p.causal_groups > 0)) return SFM_ERR_UNSUPPORTED;
     const int smem_bytes = kSmemBytes;

@@ -86,7 +86,7 @@ def real_case():
 
 
 def c1_case():
-    """B=1, 12 heads, D=128, one 3-frame chunk, empty cache."""
+    """The CPU-runnable case: B=1, 12 heads, D=128, one 3-frame chunk, empty cache."""
     rng = np.random.default_rng(0)
     B, H, D, h, w = 1, 12, 128, 30, 52
     chunk = 3 * h * w

@@ -161,7 +161,7 @@ def main():
         out[f"real_{name}_z_sample"] = z[0, ::37, 0, :].numpy()
         out[f"real_{name}_z_sum"] = np.array([z.double().sum().item(), z.double().abs().sum().item()])
 
-    # ---- 6. 12 heads, first chunk, empty cache ----------
+    # ---- 6. the CPU-runnable case: 12 heads, first chunk, empty cache ----------
     c = cases.c1_case()
     n = c["chunk"]
     for iters in (1, 20):
