@@ -164,6 +164,7 @@ int prepare_monarch(MonarchCall* mc, const void* q, int64_t q_bs, const void* kc
     const bool iter_tc = num_iters > 1 && pl.blk.b1 <= 128 && pl.blk.b2 <= kB2Max;
     const bool use_tc = (num_iters == 1 && (causal_groups == 0 || pl.blk.b1 <= 128)) || iter_tc;
     if (lse && (num_iters != 1 || pl.blk.b1 > 128)) return SFM_ERR_UNSUPPORTED;
+    if (reinterpret_cast<uintptr_t>(lse) & 3) return SFM_ERR_ALIGNMENT;
     // block columns above 64 exist on the tensor-core kernels only (single pass, block rows up to 128)
     if (pl.blk.b2 > kB2Max && !(use_tc && pl.blk.b1 <= 128)) return SFM_ERR_UNSUPPORTED;
     // only the tensor-core column step knows how to scatter its rows

@@ -765,6 +765,7 @@ static int monarch_bwd(bool train, const void* out_fwd, const float* lse_fwd, co
                             (const void*)workspace})
         if (reinterpret_cast<uintptr_t>(ptr) & 15) return SFM_ERR_ALIGNMENT;
     if ((q_batch_stride & 7) || (kv_batch_stride & 7)) return SFM_ERR_ALIGNMENT;
+    if ((reinterpret_cast<uintptr_t>(out_fwd) & 15) || (reinterpret_cast<uintptr_t>(lse_fwd) & 3)) return SFM_ERR_ALIGNMENT;
 
     const Blocking& blk = pl.blk;
     BwdParams p{};

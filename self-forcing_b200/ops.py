@@ -430,7 +430,7 @@ class _MonarchWithKVCacheFn(torch.autograd.Function):
         if not want_cache and start % (f_tied * h * w) == 0:
             out = lse = None
             if fwd and ctx.out_version[0]._version == ctx.out_version[1]:
-                out, lse = fwd
+                out, lse = (t.contiguous() for t in fwd)           # a saved-tensor hook may hand back another layout
             grads = _backward_natural(q, k_cache, v_cache, out, lse, grad_out, blocking, sm_scale, g0, g1)
             if grads is not None:
                 return (*grads, None, None, None, None, None, None, None)

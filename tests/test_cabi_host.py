@@ -127,6 +127,9 @@ def test_entry_points_validate_arguments_without_a_gpu(sfb):
         assert lib.sfm_dense_fwd(one, 0, one, one, 0, out, 1, 1, 128, 16, 16, 1.0, null) == -4
         assert lib.sfm_monarch_fwd(one, 0, one, one, 0, out, one, 1 << 30, 1, 1, 128, 1560, 1560, 1, 1, 1, 30, 52,
                                    1.0, 1, 0, null) == -4
+    for out, lse in ((264, 256), (256, 258)):
+        assert lib.sfm_monarch_bwd_natural(one, 0, one, one, 0, C.c_void_p(out), C.c_void_p(lse), one, one, one, one, one, 1 << 40,
+                                           1, 1, 128, 1560, 3120, 1, 1, 1, 30, 52, 1.0, 1, 2, 0, null) == -4
     assert lib.sfm_monarch_bwd(one, 0, one, one, 0, one, one, one, one, C.c_void_p(272), 1 << 40, 1, 1, 128, 1560, 3120, 1, 1, 1,
                                30, 52, 1.0, 0, 2, 0, 0, null) == -4
     assert lib.sfm_rope_cache_write(null, one, one, null, one, one, 0, null, 1, 100, 1, 128, 0, 1, 1, 1, 30, 52,
@@ -179,7 +182,7 @@ def test_entry_points_validate_arguments_without_a_gpu(sfb):
 
 
 @pytest.mark.parametrize("field,value,rc", [("workspace_bytes", 0, -5), ("workspace_bytes", 1, -5), ("n_kv", 1561, -2),
-                                            ("num_iters", 0, -2), ("out", 260, -4), ("k_cache", 0, -1)])
+                                            ("num_iters", 0, -2), ("out", 260, -4), ("lse", 258, -4), ("k_cache", 0, -1)])
 def test_layer_call_is_refused_before_its_cache_write(sfb, field, value, rc):
     """sfm_kv_attention makes the attention's checks before it launches the cache write, which may evict: without a GPU a
     launch would be a CUDA error (a positive code)."""
