@@ -27,7 +27,7 @@ extern "C" {
 #define SFM_OK                    0
 #define SFM_ERR_NULL_POINTER     -1
 #define SFM_ERR_BAD_SHAPE        -2   /* sizes inconsistent with the blocking            */
-#define SFM_ERR_UNSUPPORTED      -3   /* head_dim != 128, b2 > 64, ...                   */
+#define SFM_ERR_UNSUPPORTED      -3   /* head_dim != 128, b2 > 128, ...                  */
 #define SFM_ERR_ALIGNMENT        -4   /* pointers / strides must be 16-byte aligned (attention outputs and the backward's workspace 32, the forward's workspace 256) */
 #define SFM_ERR_WORKSPACE        -5   /* workspace too small                             */
 #define SFM_ERR_NO_DEVICE        -6   /* not an sm_100 device                            */
