@@ -186,7 +186,7 @@ int prepare_monarch(MonarchCall* mc, const void* q, int64_t q_bs, const void* kc
         uint32_t bq[4] = {64, 1, (uint32_t)pl.blk.b2, 1};
         uint64_t dk[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_kv, (uint64_t)B};
         uint64_t sk[3] = {row, tok, (uint64_t)c_bs * 2};
-        uint32_t bk[4] = {64, 1, (uint32_t)n_s, 1};
+        uint32_t bk[4] = {64, 1, (uint32_t)pl.blk.b2, 1};
         if ((rc = make_tmap_bf16(&maps[0], q, 4, dq, sq, bq))) return rc;
         if ((rc = make_tmap_bf16(&maps[1], kc, 4, dk, sk, bk))) return rc;
         if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
@@ -322,7 +322,7 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
     uint32_t bq[4] = {64, 1, (uint32_t)blk.b2, 1};
     uint64_t dk[4] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)n_kv, (uint64_t)B};
     uint64_t sk[3] = {row, tok, (uint64_t)c_bs * 2};
-    uint32_t bk[4] = {64, 1, (uint32_t)n_s, 1};
+    uint32_t bk[4] = {64, 1, (uint32_t)blk.b2, 1};
     uint64_t dqr[5] = {(uint64_t)kHeadDim, (uint64_t)H, (uint64_t)blk.w, (uint64_t)(n_q / blk.w), (uint64_t)B};
     uint64_t sqr[4] = {row, tok, (uint64_t)blk.w * tok, (uint64_t)q_bs * 2};
     uint32_t bqr[5] = {64, 1, 1, (uint32_t)blk.b1, 1};

@@ -13,6 +13,36 @@ constexpr int kLds = kHeadDim + 8;       // padded shared-memory row (bf16 eleme
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kMaxPeers = 8;             // GPUs of one box that may share a head-sharded call
 
+// Division by a number that the host knows, for 0 <= n < 2^31: the kernels' roles decode their unit once per unit or tile, one
+// warp wide, and the compiler's division of two run-time integers is a chain of some hundred cycles there.
+// With d <= 2^l and m = floor(2^(31+l) / d) + 1 (fits 32 bits), m d exceeds 2^(31+l) by at most d <= 2^l, so n m / 2^(31+l) is
+// less than 1 / d above n / d, and its floor is the quotient.
+struct FastDiv {
+    uint32_t d, mul, shift;
+    constexpr __host__ __device__ static FastDiv of(uint32_t d) {
+        uint32_t l = 0;
+        while ((1u << l) < d) ++l;
+        return {d, (uint32_t)(((uint64_t)1 << (31 + l)) / d + 1), 31 + l};
+    }
+    constexpr __host__ __device__ int div(int n) const { return (int)(((uint64_t)(uint32_t)n * mul) >> shift); }
+    constexpr __host__ __device__ int divmod(int n, int& rem) const {
+        const int q = div(n);
+        rem = n - q * (int)d;
+        return q;
+    }
+};
+constexpr bool fast_div_exact() {
+    for (uint32_t d = 1; d <= 131; ++d)
+        for (uint32_t k : {0u, 1u, 2u, 1000u, 0x7fffffffu / d - 1, 0x7fffffffu / d})
+            for (uint32_t n : {k * d, k * d + d - 1 > 0x7fffffffu ? k * d : k * d + d - 1})
+                if (FastDiv::of(d).div((int)n) != (int)(n / d)) return false;
+    for (uint32_t d : {1000u, 65536u, 1000003u, 0x3fffffffu, 0x40000000u, 0x40000001u})
+        for (uint32_t n : {0u, d - 1, d, 2 * d - 1, 0x7fffffffu})
+            if (FastDiv::of(d).div((int)n) != (int)(n / d)) return false;
+    return true;
+}
+static_assert(fast_div_exact(), "quotients at multiples, one below them and the ends of the range");
+
 // Monarch blocking of an h x w token grid (see sfmonarch.h).
 struct Blocking {
     int f_tied, h_reduce, w_reduce, h, w;

@@ -187,14 +187,14 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 const int tok = (f * b1 + un.k) * b2;
                 unsigned char* kt = kv_s + s * kKVTile;
                 unsigned char* vt = kv_s + 2 * kKVTile;
-                mbar_arrive_expect_tx_e(el, &bars->k_full[s], (uint32_t)(2 * kHalf));
+                mbar_arrive_expect_tx_e(el, &bars->k_full[s], (uint32_t)(2 * b2 * 128));
                 tma_load_4d_e(el, kt, &tk, &bars->k_full[s], 0, hd, tok, b);
                 tma_load_4d_e(el, kt + kHalf, &tk, &bars->k_full[s], 64, hd, tok, b);
                 const int key = f * b1 + un.k;
                 for (int which = 0; which < 2; ++which) {
                     if (which) {
                         if (g >= 1 && !mbar_wait_u(&bars->v_empty, (g - 1) & 1)) { fail(13); ok = false; break; }
-                        mbar_arrive_expect_tx_e(el, &bars->v_full, (uint32_t)(2 * kHalf));
+                        mbar_arrive_expect_tx_e(el, &bars->v_full, (uint32_t)(2 * b2 * 128));
                         tma_load_4d_e(el, vt, &tv, &bars->v_full, 0, hd, tok, b);
                         tma_load_4d_e(el, vt + kHalf, &tv, &bars->v_full, 64, hd, tok, b);
                     }

@@ -7,27 +7,28 @@
 // computes per query row a complete softmax over the b2 keys of K[f,k,:]:
 //   S  = Q_tile K[f,k]^T                 tcgen05.mma, both operands from shared memory (K-major)
 //   P  = softmax rows of S (scaled)      one thread per row: tcgen05.ld, registers, tcgen05.st (bf16)
-//   [aL | Y] = P [K[f,k] | V[f,k]]       one N=256 tcgen05.mma per 16 keys, A = P from TMEM,
-//                                        B = the K and V tiles side by side (MN-major)
+//   aL = P K[f,k], Y = P V[f,k]          one N=128 tcgen05.mma each per 16 keys, A = P from TMEM, B = the tile (MN-major)
 //   cL = sum_l P ln P                    from the softmax registers
 // and streams aL, Y (bf16) and cL to the chunk's bridge.
 //
-// Warp roles (19 warps): 0 = TMA producer, 1 = issuer of the [aL | Y] GEMMs (owns the TMEM allocation), 2 = issuer of the S
-// GEMMs (all three run as whole warps with an elected issuing lane), 3..6 and 7..10 = two softmax warpgroups that take even
-// / odd steps (a warp reaches TMEM lane quadrant warp % 4, and four consecutive warps cover all four), 11..14 and 15..18 =
-// two epilogue warpgroups (aL half / Y half of the accumulator).  All roles run the same unit loop and meet only through
-// mbarriers whose phases follow running step counters, so the pipeline keeps flowing across unit boundaries.  Every wait
-// is bounded; on a timeout the CTA records a status code and unwinds.
+// Warp roles (20 warps): 0 = K and query tiles, 3 = V tiles, 1 = issuer of the aL and Y GEMMs (owns the TMEM allocation), 2 =
+// issuer of the S GEMMs (all four run as whole warps with an elected issuing lane), 4..7 and 8..11 = two softmax warpgroups
+// that take even / odd steps (a warp reaches TMEM lane quadrant warp % 4), 12..15 and 16..19 = two epilogue warpgroups (aL /
+// Y).  All roles run the same unit loop and meet only through mbarriers whose phases follow running step counters, so the
+// pipeline keeps flowing across unit boundaries.  Every wait is bounded; on a timeout the CTA records a status code and
+// unwinds.
 //
-// What bounds it: the bridge rows it writes, 512 bytes per (query row, cached group, block row).  Written by the epilogue
-// threads themselves (one 256-byte row per lane in 32-byte pieces) they go out at 25-27 KB per us and SM, 3.8 TB/s in all,
-// into L2 or DRAM alike; without the stores the same kernel takes a third to a half of the time.  So each epilogue warp packs
-// 32 rows x 64 columns to bf16 into a swizzled 4 KB staging buffer (two, in turn) and one lane hands it to the TMA store
-// engine.  With four S / P buffers in TMEM (the S GEMMs then run ahead of the softmax instead of waiting for the last P to
-// be consumed), one query tile and four 32 KB K / V stages: framewise, 21 cached frames, 12 heads 0.188 -> 0.167 ms;
-// reduce2xh, 9 frames, 4 videos 0.563 -> 0.500 ms; reduce4xw2xh, 21 frames 1.237 -> 1.135 ms (4.6 TB/s of DRAM traffic).
-// Tried and slower: 16 epilogue warps with a register split by setmaxnreg, separate accumulator hand-overs for the two
-// halves, one K / V tile for two query tiles, L2 prefetch of the K / V tiles.
+// What bounds it: the bridge rows it writes, 512 bytes per (query row, cached group, block row).  An SM's TMA engine stores 29
+// bytes a cycle at most (loads 82 with all SMs at it, 125 alone) and does one thing at a time, so a step of 104 rows takes 1840
+// cycles for its stores and 210 for its K and V; at long caches DRAM takes them at 5.5 TB/s beside what is read (a bare stream
+// of the same boxes 6.4).  Written by the epilogue threads themselves, a row a lane or four rows an instruction, they go out
+// slower (first chunk 33 -> 39 us), and K / V by cp.async instead do not help (31 -> 35).
+// The epilogue's hand-over of an accumulator comes before its stores, aL and Y each have their own, and the working
+// warpgroups have 104 registers instead of 96 (a few dozen spilled bytes a thread go through an L1 that is all shared memory:
+// 160 -> 190 us).  framewise, 21 cached frames, 12 heads 0.167 -> 0.158 ms; reduce2xh, 9 frames, 4 videos 0.527 -> 0.490;
+// reduce4xw2xh, 21 frames 1.15 -> 1.09; a pass of the iterative variant, first chunk, 31.7 -> 25.4 us.
+// Tried and slower: results to TMA as 5-D boxes of both halves (158 -> 179 us), three staging buffers a warp (same), all
+// columns to registers before the first is stored, two tiles' queries against one K / V tile, L2 prefetch of the K / V tiles.
 //
 // Arithmetic follows monarch_attn_ref_op (wan/modules/monarch_attn.py:1813-1823, 1828); the sqrt(s)
 // scaling of q and k is folded into the softmax scale, so aL here is the reference's aL / sqrt(s).
@@ -41,12 +42,14 @@ using namespace tc;
 
 namespace {
 
-constexpr int kStages = 8;            // K/V tile ring, at most
-constexpr int kThreads = 608;          // 19 warps, 96 registers a thread
+constexpr int kKStages = 4, kVStages = 2;    // K and V tiles held, at most
+constexpr int kThreads = 640;          // 20 warps, 96 registers a thread when launched
+constexpr int kRegsIssue = 56, kRegsWork = 104;     // of the issuing warpgroup and of the four others, from there on
 constexpr int kTileRows = 128;
 constexpr int kMaxSBufs = 4;
+constexpr int kMaxQBufs = 3;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColO = 256;        // O = [aL | Y], 256 columns; the S/P buffers lie below it
+constexpr uint32_t kColO = 256;        // two accumulators of 128 columns; the S/P buffers lie below them
 
 struct RTcParams {
     MonarchParams mp;
@@ -55,6 +58,7 @@ struct RTcParams {
     int tiles;             // tiles per (batch*head) of the chunk
     int fsplit, f_per;     // split of the F loop over units
     int n_units;           // nbh * tiles * b1 * fsplit
+    FastDiv by_fsplit, by_b1, by_tiles, by_H;
     int col_kt;            // keys per tile of the column step (block-causal: it reads whole tiles)
     int* status;           // device status word (0 = ok)
     int clear_status;      // the call's first launch starts it from zero
@@ -70,10 +74,10 @@ template <bool kCausal>
 __device__ __forceinline__ RUnit decode_unit(const RTcParams& rp, int u) {
     const MonarchParams& p = rp.mp;
     RUnit r;
-    int fs = u % rp.fsplit; u /= rp.fsplit;
-    r.k = u % p.blk.b1; u /= p.blk.b1;
-    r.tile = u % rp.tiles;
-    r.bhl = u / rp.tiles;
+    int fs;
+    u = rp.by_fsplit.divmod(u, fs);
+    u = rp.by_b1.divmod(u, r.k);
+    r.bhl = rp.by_tiles.divmod(u, r.tile);
     r.f_begin = fs * rp.f_per;
     int f_end = min(p.F, r.f_begin + rp.f_per);
     if (kCausal) {
@@ -87,35 +91,36 @@ __device__ __forceinline__ RUnit decode_unit(const RTcParams& rp, int u) {
 }
 
 struct __align__(8) Barriers {
-    uint64_t q_full[2], q_empty[2];   // single pass: buffer 0, once per unit; iterative variant: one per step, alternating
-    uint64_t kv_full[kStages];
-    uint64_t kv_empty[kStages];
+    uint64_t q_full[kMaxQBufs], q_empty[kMaxQBufs];   // query tiles in turn: one per unit, iterative variant: one per step
+    uint64_t k_full[kKStages], k_empty[kKStages];
+    uint64_t v_full[kVStages], v_empty[kVStages];
     uint64_t s_full[kMaxSBufs];
     uint64_t p_full[kMaxSBufs];
     uint64_t sp_free[kMaxSBufs];   // PV GEMM has consumed the P operand held in this S/P buffer
-    uint64_t o_full;
-    uint64_t o_free;
+    uint64_t o_full[2], o_free[2];    // accumulator: aL / Y, or of the even / odd steps
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
 // shared memory carve-up (bytes from a 1024-aligned base)
 constexpr int kQBytes = 2 * kTileRows * 128;               // two 64-column halves
-constexpr int kOutBytes = 8 * 2 * 32 * 128;                    // result staging: 32 rows x 64 columns per epilogue warp
+constexpr int kOutBytes = 8 * 2 * 32 * 128;                        // result staging: 32 rows x 64 columns per epilogue warp
 constexpr int kSmemData = 224 << 10;                       // query tiles | K / V ring | staging
 constexpr int kSmemBytes = 1024 + kSmemData + 512;
 static_assert(sizeof(Barriers) <= 512, "barriers follow the tiles");
 
 // kIter: a pass of the iterative variant after the first one.  The query operand is no longer the chunk's q
 // (one tile per unit) but the state aR[a,f,k,j,:] of the previous pass, which differs for every cached group f:
-// one tile per STEP, loaded through `tq` = a 3-D map of aR ([bh*F*b1][na*b2][128]) into two alternating
-// buffers, and every row's logits are divided by its cR (monarch_attn.py:1716-1719).
-template <int N_S, bool kCausal, bool kIter>
+// one tile per STEP, loaded through `tq` = a 3-D map of aR ([bh*F*b1][na*b2][128]) into two or three buffers in
+// turn, and every row's logits are divided by its cR (monarch_attn.py:1716-1719).
+// kY: Y is wanted.  The passes of the iterative variant before the last need aL and cL only: their stages hold K alone, and
+// the two epilogue warpgroups take whole steps in turn, each with a 128-column accumulator of its own.
+template <int N_S, bool kCausal, bool kIter, bool kY>
 __global__ void __launch_bounds__(kThreads, 1)
 monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tal,
                     const __grid_constant__ CUtensorMap ty, RTcParams rp) {
-    static_assert(!kIter || (N_S <= 64 && !kCausal), "the iterative variant exists for block columns up to 64, no mask");
+    static_assert(!(kIter || !kY) || (N_S <= 64 && !kCausal), "the iterative variant exists for block columns up to 64, no mask");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const MonarchParams& p = rp.mp;
@@ -124,31 +129,42 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     const int b1 = blk.b1, b2 = blk.b2;
     const int RG = rp.rows_per_group;
     constexpr int kHalf = N_S * 128;                    // bytes of one 64-column half of a K or V tile
-    // Block columns above 64 (wide grids): 128-row K / V stages (two of them fit), S/P buffers and the
-    // accumulator move up in TMEM, and the softmax walks its row in 32-column chunks (see below).
+    // Block columns above 64 (wide grids): two S/P buffers, and the softmax walks its row in 32-column chunks (see below).
     constexpr bool kWide = N_S > 64;
-    // a stage holds K lo, K hi, V lo, V hi of N_S rows each: 16 KB up to 32 block columns, 32 KB up to 64, 64 KB beyond
-    constexpr int kStgBytes = kWide ? 65536 : (N_S <= 32 ? 16384 : 32768);
+    constexpr int kTile = 2 * kHalf;                     // a K or V tile: two halves
     constexpr int kSBufs = kWide ? 2 : 4;
     constexpr uint32_t kSCols = kColO / kSBufs;          // TMEM columns per S/P buffer
-    constexpr int kQBufs = kIter ? 2 : 1;               // a query tile per unit, or per step
-    constexpr int kStg = (kSmemData - kQBufs * kQBytes - kOutBytes) / kStgBytes;
-    static_assert(kStg >= 2 && kStg <= kStages, "K / V ring");
+    // A query tile per unit, or per step.
+    constexpr int kQBufs = kWide ? 1 : (kIter && !kY ? 3 : 2);
+    // A K tile stays from its S GEMM to its PV GEMM, two to three steps later, a V tile for its PV GEMM only.  21 frames, 12 heads,
+    // 52 columns, K / V slots of 16 KB: 3 / 1 195 us, 3 / 2 162, 4 / 2 159, 4 / 4 162, 5 / 3 171: copies share the TMA engine
+    // with the result stores, and those asked for earlier than needed hold them up.
+    constexpr int kSlots = (kSmemData - kQBufs * kQBytes - kOutBytes) / kTile;
+    constexpr int kVStg = kY ? kVStages : 0, kKStg = kSlots - kVStg < kKStages ? kSlots - kVStg : kKStages;
+    static_assert(kKStg >= 2 && kQBufs <= kMaxQBufs, "K ring, query tiles");
     unsigned char* q_s = base;
-    unsigned char* kv_s = q_s + kQBufs * kQBytes;
-    unsigned char* o_s = kv_s + kStg * kStgBytes;            // two 4 KB staging buffers per epilogue warp
+    unsigned char* k_s = q_s + kQBufs * kQBytes;
+    unsigned char* v_s = k_s + kKStg * kTile;
+    unsigned char* o_s = v_s + kVStg * kTile;                // staging of the epilogue warps
     Barriers* bars = reinterpret_cast<Barriers*>(base + kSmemData);
 
     if (warp == 2 && lane == 0) { prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
-        for (int s = 0; s < kStg; ++s) { mbar_init(&bars->kv_full[s], 1); mbar_init(&bars->kv_empty[s], 1); }
+        for (int s = 0; s < kQBufs; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
+        for (int s = 0; s < kKStg; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1); }
+        for (int s = 0; s < kVStg; ++s) { mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], 1); }
         for (int s = 0; s < kSBufs; ++s) { mbar_init(&bars->s_full[s], 1); mbar_init(&bars->p_full[s], 128); mbar_init(&bars->sp_free[s], 1); }
-        mbar_init(&bars->o_full, 1);
-        mbar_init(&bars->o_free, 256);
+        for (int w = 0; w < 2; ++w) { mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128); }
         bars->abort_flag = 0;
         mbar_init_fence();
     }
+    // The copies bring the b2 rows of a block and no more (64 of every 52 rows were 20 % of what the kernel read); the GEMMs
+    // read N_S, with weight zero past b2: those rows must hold finite numbers.
+    for (int i = tid; i < (kKStg + kVStg) * 2 * (N_S - b2) * 8; i += kThreads) {
+        const int r = i >> 3, h = r / (N_S - b2);
+        reinterpret_cast<uint4*>(k_s + h * kHalf + (b2 + r - h * (N_S - b2)) * 128)[i & 7] = make_uint4(0, 0, 0, 0);
+    }
+    fence_async_smem();
     if (warp == 1) { tmem_alloc(&bars->tmem_base, kTmemCols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
@@ -165,27 +181,29 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     if (rp.clear_status && blockIdx.x == 0 && tid == 0) *rp.status = 0;
     const int u_first = blockIdx.x, u_stride = gridDim.x;
 
+    // Each branch of a role takes its registers itself: where branches of both counts meet, the compiler has the smaller one.
+    if (warp < 4) {
+    reg_dec<kRegsIssue>();
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
+        // ------------------------------------------------------------------ K and query tiles
         {
             const uint32_t el = elect_one();
             int g = 0, uc = 0;
             for (int u = u_first; u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
                 if (kCausal && un.n_it == 0) continue;
-                const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+                int hd;
+                const int b = rp.by_H.divmod(p.bh0 + un.bhl, hd);
                 const int g_first = un.tile * rp.groups_per_tile;
                 const int ng = min(rp.groups_per_tile, p.na - g_first);
                 for (int i = 0; i < un.n_it; ++i, ++g) {
-                    const int s = g % kStg;
-                    if (g >= kStg && !mbar_wait_u(&bars->kv_empty[s], ((g / kStg) - 1) & 1)) { fail(11); break; }
+                    const int s = g % kKStg;
+                    if (g >= kKStg && !mbar_wait_u(&bars->k_empty[s], ((g / kKStg) - 1) & 1)) { fail(11); break; }
                     const int tok = ((un.f_begin + i) * b1 + un.k) * b2;
-                    unsigned char* st = kv_s + s * kStgBytes;
-                    mbar_arrive_expect_tx_e(el, &bars->kv_full[s], (uint32_t)(4 * kHalf));
-                    tma_load_4d_e(el, st, &tk, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + kHalf, &tk, &bars->kv_full[s], 64, hd, tok, b);
-                    tma_load_4d_e(el, st + 2 * kHalf, &tv, &bars->kv_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + 3 * kHalf, &tv, &bars->kv_full[s], 64, hd, tok, b);
+                    unsigned char* st = k_s + s * kTile;
+                    mbar_arrive_expect_tx_e(el, &bars->k_full[s], (uint32_t)(2 * b2 * 128));
+                    tma_load_4d_e(el, st, &tk, &bars->k_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + kHalf, &tk, &bars->k_full[s], 64, hd, tok, b);
                     if (!kIter && i > 0) continue;
                     // the query tile: the unit's rows of q, or this step's state rows (a, j) of (f, k), group by group
                     const int qc = kIter ? g : uc, qb = qc % kQBufs;
@@ -207,6 +225,27 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                 ++uc;
             }
         }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ V tiles
+        if constexpr (kY) {
+            const uint32_t el = elect_one();
+            int g = 0;
+            bool ok = true;
+            for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
+                const RUnit un = decode_unit<kCausal>(rp, u);
+                int hd;
+                const int b = rp.by_H.divmod(p.bh0 + un.bhl, hd);
+                for (int i = 0; i < un.n_it; ++i, ++g) {
+                    const int s = g % kVStages;
+                    if (g >= kVStages && !mbar_wait_u(&bars->v_empty[s], ((g / kVStages) - 1) & 1)) { fail(12); ok = false; break; }
+                    const int tok = ((un.f_begin + i) * b1 + un.k) * b2;
+                    unsigned char* st = v_s + s * kTile;
+                    mbar_arrive_expect_tx_e(el, &bars->v_full[s], (uint32_t)(2 * b2 * 128));
+                    tma_load_4d_e(el, st, &tv, &bars->v_full[s], 0, hd, tok, b);
+                    tma_load_4d_e(el, st + kHalf, &tv, &bars->v_full[s], 64, hd, tok, b);
+                }
+            }
+        }
     } else if (warp == 2) {
         // ------------------------------------------------------------------ S-GEMM issuer
         {
@@ -215,37 +254,34 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             // Descriptors differ from step to step only in the start-address field (16-byte units
             // in the low word), so they are built once and advanced with integer adds.
             const uint64_t q_desc = smem_desc_sw128(smem_addr(q_s), 16, 1024);
-            const uint64_t k_desc0 = smem_desc_sw128(smem_addr(kv_s), 16, 1024);
+            const uint64_t k_desc0 = smem_desc_sw128(smem_addr(k_s), 16, 1024);
             int g = 0, uc = 0;
             bool ok = true;
             for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
                 if (kCausal && un.n_it == 0) continue;
                 if constexpr (!kIter) {
-                    if (!mbar_wait_u(&bars->q_full[0], uc & 1)) { fail(20); break; }
+                    if (!mbar_wait_u(&bars->q_full[uc % kQBufs], (uc / kQBufs) & 1)) { fail(20); break; }
                 }
                 for (int i = 0; i < un.n_it; ++i, ++g) {
-                    const int s = g % kStg;
+                    const int s = g % kKStg, qb = (kIter ? g : uc) % kQBufs;
                     if constexpr (kIter) {
-                        if (!mbar_wait_u(&bars->q_full[g & 1], (g >> 1) & 1)) { fail(20); ok = false; break; }
+                        if (!mbar_wait_u(&bars->q_full[qb], (g / kQBufs) & 1)) { fail(20); ok = false; break; }
                     }
-                    if (!mbar_wait_u(&bars->kv_full[s], (g / kStg) & 1)) { fail(21); ok = false; break; }
+                    if (!mbar_wait_u(&bars->k_full[s], (g / kKStg) & 1)) { fail(21); ok = false; break; }
                     if (g >= kSBufs && !mbar_wait_u(&bars->sp_free[g % kSBufs], ((g / kSBufs) - 1) & 1)) { fail(25); ok = false; break; }
                     tc_fence_after();
-                    const uint64_t kd = k_desc0 + (uint64_t)((s * kStgBytes) >> 4);
+                    const uint64_t kd = k_desc0 + (uint64_t)((s * kTile) >> 4);
+                    const uint64_t qd = q_desc + (uint64_t)((qb * kQBytes) >> 4);
                     const uint32_t d = tmem + (g % kSBufs) * kSCols;
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t q_off = ((ks >> 2) * (kTileRows * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t k_off = ((ks >> 2) * kHalf + (ks & 3) * 32) >> 4;
-                        mma_ss_e(el, d, q_desc + (uint32_t)(((kIter ? g & 1 : 0) * kQBytes) >> 4) + q_off, kd + k_off, idesc_s, ks > 0);
+                        mma_ss_e(el, d, qd + q_off, kd + k_off, idesc_s, ks > 0);
                     }
                     mma_commit_e(el, &bars->s_full[g % kSBufs]);
-                    if constexpr (kIter) {
-                        mma_commit_e(el, &bars->q_empty[g & 1]);                 // this step's query tile has been read
-                    } else {
-                        if (i + 1 == un.n_it) mma_commit_e(el, &bars->q_empty[0]);   // last read of this unit's Q tile
-                    }
+                    if (kIter || i + 1 == un.n_it) mma_commit_e(el, &bars->q_empty[qb]);   // last read of the query tile
                 }
                 ++uc;
             }
@@ -254,33 +290,48 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         // ------------------------------------------------------------------ PV-GEMM issuer
         {
             const uint32_t el = elect_one();
-            // [aL | Y] in one N = 256 GEMM; the passes of the iterative variant that only need aL and cL stop at N = 128
-            const uint32_t idesc_o = p.write_Y ? idesc_bf16(kTileRows, 2 * kHeadDim, 0, 1) : idesc_bf16(kTileRows, kHeadDim, 0, 1);
+            constexpr uint32_t idesc_o = idesc_bf16(kTileRows, kHeadDim, 0, 1);
             constexpr int ksteps_pv = N_S / 16;
-            const uint64_t kv_desc_mn0 = smem_desc_sw128(smem_addr(kv_s), kHalf, 1024);   // 4 column blocks: K lo, K hi, V lo, V hi
+            const uint64_t k_desc_mn0 = smem_desc_sw128(smem_addr(k_s), kHalf, 1024);     // column blocks: lo, hi
+            const uint64_t v_desc_mn0 = smem_desc_sw128(smem_addr(v_s), kHalf, 1024);
             int g = 0;
             bool ok = true;
             for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
                 for (int i = 0; i < un.n_it; ++i, ++g) {
                     if (!mbar_wait_u(&bars->p_full[g % kSBufs], (g / kSBufs) & 1)) { fail(22); ok = false; break; }
-                    if (g > 0 && !mbar_wait_u(&bars->o_free, (g - 1) & 1)) { fail(23); ok = false; break; }
+                    const int ob = kY ? 0 : g & 1, og = kY ? g : g >> 1;         // accumulator, its uses before this one
+                    if (og > 0 && !mbar_wait_u(&bars->o_free[ob], (og - 1) & 1)) { fail(23); ok = false; break; }
                     tc_fence_after();
-                    const int s = g % kStg;
-                    const uint64_t bd = kv_desc_mn0 + (uint64_t)((s * kStgBytes) >> 4);
+                    const int s = g % kKStg;
+                    const uint64_t kd = k_desc_mn0 + (uint64_t)((s * kTile) >> 4);
                     const uint32_t p_t = tmem + (g % kSBufs) * kSCols;
 #pragma unroll
                     for (int kk = 0; kk < ksteps_pv; ++kk)
-                        mma_ts_e(el, tmem + kColO, p_t + kk * 8, bd + ((kk * 2048) >> 4), idesc_o, kk > 0);
-                    mma_commit_e(el, &bars->o_full);
-                    mma_commit_e(el, &bars->kv_empty[s]);
+                        mma_ts_e(el, tmem + kColO + ob * kHeadDim, p_t + kk * 8, kd + ((kk * 2048) >> 4), idesc_o, kk > 0);
+                    mma_commit_e(el, &bars->o_full[ob]);
+                    mma_commit_e(el, &bars->k_empty[s]);
+                    if constexpr (kY) {
+                        const int sv = g % kVStages;
+                        const uint64_t vd = v_desc_mn0 + (uint64_t)((sv * kTile) >> 4);
+                        if (!mbar_wait_u(&bars->v_full[sv], (g / kVStages) & 1)) { fail(24); ok = false; break; }
+                        if (g > 0 && !mbar_wait_u(&bars->o_free[1], (g - 1) & 1)) { fail(26); ok = false; break; }
+                        tc_fence_after();
+#pragma unroll
+                        for (int kk = 0; kk < ksteps_pv; ++kk)
+                            mma_ts_e(el, tmem + kColO + kHeadDim, p_t + kk * 8, vd + ((kk * 2048) >> 4), idesc_o, kk > 0);
+                        mma_commit_e(el, &bars->o_full[1]);
+                        mma_commit_e(el, &bars->v_empty[sv]);
+                    }
                     mma_commit_e(el, &bars->sp_free[g % kSBufs]);
                 }
             }
         }
-    } else if (warp >= 3 && warp < 11) {
+    }
+    } else if (warp < 12) {
+        reg_inc<kRegsWork>();
         // ------------------------------------------------------------------ softmax warpgroups
-        const int wg = (warp - 3) >> 2;                 // 0: even steps, 1: odd steps; the S / P buffers rotate over all steps
+        const int wg = (warp - 4) >> 2;                 // 0: even steps, 1: odd steps; the S / P buffers rotate over all steps
         const int quad = warp & 3;                      // TMEM lane quadrant this warp may access
         const int row = quad * 32 + lane;               // tile row == TMEM lane
         const int gl = row / RG, j = row - gl * RG;
@@ -455,18 +506,24 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                 mbar_arrive(&bars->p_full[sb]);
             }
         }
-    } else if (warp >= 11) {
+    } else {
+        reg_inc<kRegsWork>();
         // ------------------------------------------------------------------ epilogue warpgroups
-        const int which = (warp - 11) >> 2;              // 0: aL (columns 0..127 of O), 1: Y (columns 128..255)
+        // with Y: 0 takes aL (columns 0..127 of the accumulator), 1 takes Y (128..255); without: even, odd steps
+        const int which = (warp - 12) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const uint32_t o_t = tmem + ((uint32_t)(quad * 32) << 16) + kColO + which * kHeadDim;
         const uint32_t el = elect_one();
-        // this warp's staging: 32 tile rows x 64 columns, 128-byte swizzle; its rows of a group start at column j0
-        unsigned char* const st = o_s + (warp - 11) * 8192;
-        unsigned char* const st_row = st + lane * 128;
+        // This warp's staging, 128-byte swizzle: 32 tile rows x 64 columns, twice; with 16 rows a group, 16 x 64 twice for each of
+        // its two groups.  Its rows of a group start at column j0.
+        unsigned char* const st = o_s + (warp - 12) * 8192;
+        const int half_bytes = RG == 16 ? 2048 : 4096;
+        unsigned char* const st_row = st + (RG == 16 ? (lane >> 4) * 4096 + (lane & 15) * 128 : lane * 128);
         const int gl0 = quad * 32 / RG, j0 = quad * 32 - gl0 * RG, n_box = RG == 16 ? 2 : 1;
-        const CUtensorMap* const om = which ? &ty : &tal;
+        const CUtensorMap* const om = kY && which ? &ty : &tal;
+        uint64_t* const o_full = &bars->o_full[which];
+        uint64_t* const o_free = &bars->o_free[which];
         int g = 0;
         bool ok = true;
         for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
@@ -475,20 +532,18 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             const int ng = min(rp.groups_per_tile, p.na - g_first);
             const bool warp_active = quad * 32 < ng * RG;
             for (int i = 0; ok && i < un.n_it; ++i, ++g) {
-                if (!mbar_wait(&bars->o_full, g & 1)) { fail(41); ok = false; break; }
+                if (!kY && (g & 1) != which) continue;
+                if (!mbar_wait(o_full, (kY ? g : g >> 1) & 1)) { fail(41); ok = false; break; }
                 tc_fence_after();
                 const int key = (un.f_begin + i) * b1 + un.k;
-                const bool work = warp_active && (which == 0 || p.write_Y);
-                if (!work) {
+                if (!warp_active) {
                     tc_fence_before();
-                    mbar_arrive(&bars->o_free);
+                    mbar_arrive(o_free);
                     continue;
                 }
                 uint32_t ra[32], rb[32];
-                // 64 columns from registers to this warp's staging rows, and on to the bridge
+                // 64 columns from registers to this warp's staging rows
                 auto put = [&](int h) {
-                    tma_store_wait_read();                     // the previous box has been read
-                    __syncwarp();
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const uint32_t (&r)[32] = c < 4 ? ra : rb;
@@ -496,25 +551,29 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 #pragma unroll
                         for (int e = 0; e < 4; ++e)
                             w[e] = pack_bf16(__uint_as_float(r[(c & 3) * 8 + 2 * e]), __uint_as_float(r[(c & 3) * 8 + 2 * e + 1]));
-                        *reinterpret_cast<uint4*>(st_row + h * 4096 + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *reinterpret_cast<uint4*>(st_row + h * half_bytes + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                    fence_async_smem();
-                    __syncwarp();
-                    for (int x = 0; x < n_box; ++x)
-                        if (gl0 + x < ng)
-                            tma_store_4d_e(el, om, st + h * 4096 + x * 2048, h * 64, j0, key, un.bhl * p.na + g_first + gl0 + x);
-                    tma_store_commit();
                 };
                 tmem_ld32(o_t, ra);
                 tmem_ld32(o_t + 32, rb);
+                tma_store_wait_read_all();                     // the rows of the step before have been read
+                __syncwarp();
                 tmem_wait_ld();
                 put(0);
                 tmem_ld32(o_t + 64, ra);
                 tmem_ld32(o_t + 96, rb);
                 tmem_wait_ld();
                 tc_fence_before();
-                mbar_arrive(&bars->o_free);                    // accumulator may be overwritten from here on
+                mbar_arrive(o_free);                           // accumulator may be overwritten from here on
                 put(1);
+                fence_async_smem();
+                __syncwarp();
+                for (int x = 0; x < n_box; ++x)
+                    if (gl0 + x < ng) {
+                        tma_store_4d_e(el, om, st + x * 4096, 0, j0, key, un.bhl * p.na + g_first + gl0 + x);
+                        tma_store_4d_e(el, om, st + x * 4096 + half_bytes, 64, j0, key, un.bhl * p.na + g_first + gl0 + x);
+                    }
+                tma_store_commit();
             }
             if (kCausal && which == 1 && warp_active && un.n_it > 0 && un.f_begin + un.n_it == un.f_limit) {
                 // The column step reads whole tiles of col_kt keys and gives the keys past the limit weight zero: their Y
@@ -566,13 +625,14 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
         }
     }
     rp.n_units = p.nbh * rp.tiles * p.blk.b1 * rp.fsplit;
+    rp.by_fsplit = FastDiv::of(rp.fsplit); rp.by_b1 = FastDiv::of(p.blk.b1); rp.by_tiles = FastDiv::of(rp.tiles); rp.by_H = FastDiv::of(p.H);
     rp.status = status;
     rp.clear_status = clear_status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
     const bool iter = p.use_aR != 0;
     if (iter && (n_s > 64 || p.causal_groups > 0)) return SFM_ERR_UNSUPPORTED;
     const int smem_bytes = kSmemBytes;
-    // result stores: one box = 64 channels of up to 32 columns of one key
+    // result stores: one box = the 128 channels of up to 32 columns of one key
     CUtensorMap out_maps[2];
     for (int i = 0; i < 2; ++i)
         if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, rp.rows_per_group < 32 ? rp.rows_per_group : 32, 1)) return rc;
@@ -582,23 +642,32 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     };
     int rc;
     const bool causal = p.causal_groups > 0;
-    if (iter) {
+    if (iter || !p.write_Y) {
         switch (n_s) {
-            case 16: rc = go(monarch_r_tc_kernel<16, false, true>); break;
-            case 32: rc = go(monarch_r_tc_kernel<32, false, true>); break;
-            case 48: rc = go(monarch_r_tc_kernel<48, false, true>); break;
-            case 64: rc = go(monarch_r_tc_kernel<64, false, true>); break;
+#define SFM_R_CASE(n)                                                                                                            \
+    case n:                                                                                                                      \
+        rc = iter ? (p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true>) : go(monarch_r_tc_kernel<n, false, true, false>)) \
+                  : go(monarch_r_tc_kernel<n, false, false, false>);                                                             \
+        break;
+            SFM_R_CASE(16)
+            SFM_R_CASE(32)
+            SFM_R_CASE(48)
+            SFM_R_CASE(64)
+#undef SFM_R_CASE
             default: return SFM_ERR_UNSUPPORTED;
         }
     } else switch (n_s) {
-        case 16: rc = causal ? go(monarch_r_tc_kernel<16, true, false>) : go(monarch_r_tc_kernel<16, false, false>); break;
-        case 32: rc = causal ? go(monarch_r_tc_kernel<32, true, false>) : go(monarch_r_tc_kernel<32, false, false>); break;
-        case 48: rc = causal ? go(monarch_r_tc_kernel<48, true, false>) : go(monarch_r_tc_kernel<48, false, false>); break;
-        case 64: rc = causal ? go(monarch_r_tc_kernel<64, true, false>) : go(monarch_r_tc_kernel<64, false, false>); break;
-        case 80: rc = causal ? go(monarch_r_tc_kernel<80, true, false>) : go(monarch_r_tc_kernel<80, false, false>); break;
-        case 96: rc = causal ? go(monarch_r_tc_kernel<96, true, false>) : go(monarch_r_tc_kernel<96, false, false>); break;
-        case 112: rc = causal ? go(monarch_r_tc_kernel<112, true, false>) : go(monarch_r_tc_kernel<112, false, false>); break;
-        case 128: rc = causal ? go(monarch_r_tc_kernel<128, true, false>) : go(monarch_r_tc_kernel<128, false, false>); break;
+#define SFM_R_CASE(n) \
+    case n: rc = causal ? go(monarch_r_tc_kernel<n, true, false, true>) : go(monarch_r_tc_kernel<n, false, false, true>); break;
+        SFM_R_CASE(16)
+        SFM_R_CASE(32)
+        SFM_R_CASE(48)
+        SFM_R_CASE(64)
+        SFM_R_CASE(80)
+        SFM_R_CASE(96)
+        SFM_R_CASE(112)
+        SFM_R_CASE(128)
+#undef SFM_R_CASE
         default: return SFM_ERR_UNSUPPORTED;
     }
     if (rc) return rc;

@@ -51,6 +51,14 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
 // Make generic-proxy writes to shared memory visible to the async proxy (TMA / tcgen05.mma reads).
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ----------------------------------------------------------------------------- registers
+// Registers a thread from here on, for all four warps of a warpgroup.  The warpgroups' shares may not exceed what the block
+// was launched with.
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ----------------------------------------------------------------------------- TMEM
 // Allocation is warp-wide (.sync.aligned); ncols is a power of two >= 32.  The base address
 // (lane 0, first column) is written to *smem_dst.
