@@ -13,17 +13,19 @@
 //   aR_tile [128 x 128]   = P^T * Q_j                                      tcgen05.mma, A from TMEM, B = Q_j MN-major
 // N_I = block rows padded to 16.  The log-sum-exp of a query comes from a column step run before this kernel, or, when all
 // keys fit one tile, from the tile itself: every warp has 32 keys on its lanes and takes each query's maximum and sum over
-// them, and the four warps of a tile exchange them.
-// Warp roles (16 warps): 0 = aL tiles, 1 = S^T GEMMs (owns TMEM), 2 = query rows and log-sum-exps, 3 = aR GEMMs, all with an
-// elected issuing lane, 4-7 and 8-11 = two warpgroups that take even / odd tiles for the softmax-like pass, 12-15 = drain
-// warpgroup: accumulator -> bf16 -> swizzled staging (two 4 KB buffers per warp) -> TMA store of 32 keys x 64 channels.
+// them, and the four warps of a tile exchange them.  Up to 32 queries the exponentials against the warp's maximum stay in
+// registers meanwhile, and a factor per query makes them weights.
+// Warp roles (20 warps, 16 above 32 queries): 0 = aL tiles, 1 = S^T GEMMs (owns TMEM), 2 = query rows and log-sum-exps, 3 = aR
+// GEMMs, all with an elected issuing lane, then three (two) warpgroups that take the tiles in turn for the softmax-like pass,
+// and the drain warpgroup: accumulator -> bf16 -> swizzled staging (8 KB per warp) -> TMA store of 32 keys x 64 channels twice.
 // Persistent CTAs take contiguous shares of the unit list; all roles walk the same (unit, tile) sequence and meet through
 // mbarriers with bounded waits.
 //
-// What bounds it: with one tile per unit, the chain of a unit and its loads; with longer caches the aR rows, 256 bytes per
-// key a whole (query group, column) set apart.  With one loading warp (each unit's rows waited for its predecessor's
-// log-sum-exps to arrive from memory), one issuer, two query tiles and the log-sum-exps from a pass of the column step, 20
-// passes over a 4680-token chunk, 12 heads, took 1711 us, now 1005 (update 40 -> 27 us each, the pass, 27 us, gone).
+// What bounds it: with one tile per unit, its start (7000 cycles until the first tile is through) and then some 1500 cycles a
+// tile, of which the TMA engine stores for 800; with longer caches the aR rows, 256 bytes per key a whole (query group,
+// column) set apart.  20 passes over a 4680-token chunk, 12 heads: the update took 40 us with one loading warp, one issuer
+// and the log-sum-exps from a pass of the column step, 27 with those taken from the tile in two sweeps over it (892 us in
+// all), 23 now (810).  A second drain warpgroup: nothing.
 #include "monarch_params.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -34,16 +36,21 @@ using namespace tc;
 
 namespace {
 
-constexpr int kThreadsIt = 512;
+// Working warpgroups, each with an S / P buffer.  Up to 32 queries three of them fit 96 registers a thread (20 passes over a
+// 4680-token chunk, 12 heads: 810 us with three, 820 with two, 816 with four at 80 registers).
+__host__ __device__ constexpr int it_nw(int n_i) { return n_i <= 32 ? 3 : 2; }
+__host__ __device__ constexpr int it_threads(int n_i) { return (8 + 4 * it_nw(n_i)) * 32; }
 constexpr int kKTile = 128;               // keys per tile
 constexpr uint32_t kTmemColsIt = 512;
-__host__ __device__ constexpr uint32_t it_col_s(int w) { return (uint32_t)w * 128u; }
+template <int N_I>
+__host__ __device__ constexpr uint32_t it_col_s(int w) { return (uint32_t)w * (it_nw(N_I) > 2 ? 64u : 128u); }
 __host__ __device__ constexpr uint32_t it_col_o(int w) { return 256u + (uint32_t)w * 128u; }
 
 struct ItParams {
     MonarchParams mp;
     int n_units;       // nbh * na * b2
     int q_rows_tma;    // query rows of a unit are consecutive rows of the token grid
+    FastDiv by_tiles;  // tiles per unit
     int own_lse;       // one tile per unit: the queries' log-sum-exps are taken from it
     int* status;
 };
@@ -55,11 +62,11 @@ __host__ __device__ constexpr int it_na(int n_i) { return n_i <= 32 ? 4 : 3; }
 template <int N_I>
 struct __align__(16) ItBarriers {
     float lse2[it_nq(N_I)][N_I];            // per query tile (log-sum-exps that come from memory)
-    float2 part[2][4][N_I];                 // [warpgroup][lane quadrant][query]: maximum, sum over the quadrant's keys
-    float lse2_own[8][N_I];                 // [working warp]: log-sum-exps of its tile's queries
+    float2 part[it_nw(N_I)][4][N_I];        // [warpgroup][lane quadrant][query]: maximum, sum over the quadrant's keys
+    alignas(16) float own[4 * it_nw(N_I)][N_I];         // [working warp]: its tile's log-sum-exps, or the factors of its weights
     uint64_t q_full[it_nq(N_I)], q_empty[it_nq(N_I)];
     uint64_t a_full[it_na(N_I)], a_empty[it_na(N_I)];
-    uint64_t s_full[2], p_full[2], sp_free[2], x_full[2];
+    uint64_t s_full[it_nw(N_I)], p_full[it_nw(N_I)], sp_free[it_nw(N_I)], x_full[it_nw(N_I)];
     uint64_t o_full[2], o_free[2];          // accumulator w
     uint32_t tmem_base;
     volatile int abort_flag;
@@ -94,21 +101,20 @@ __device__ __forceinline__ float warp_max(float v) {
 struct ItUnit { int bhl, al, j; };
 __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
     ItUnit r;
-    r.j = u % p.blk.b2; u /= p.blk.b2;
-    r.al = u % p.na;
-    r.bhl = u / p.na;
+    u = p.by_b2.divmod(u, r.j);
+    r.bhl = p.by_na.divmod(u, r.al);
     return r;
 }
 
 // tal = bridge aL map (box 64 x 1 column x 128 keys), tqr = query rows (5-D, box of b1 rows), tar = state aR
 // [bh][key][query group, column][128] (box 64 x 1 x 32 keys).
 template <int N_I>
-__global__ void __launch_bounds__(kThreadsIt, 1)
+__global__ void __launch_bounds__(it_threads(N_I), 1)
 monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap tqr,
                        const __grid_constant__ CUtensorMap tar, ItParams ip) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr int NQ = it_nq(N_I), NA = it_na(N_I);
+    constexpr int NQ = it_nq(N_I), NA = it_na(N_I), NW = it_nw(N_I), kThreadsIt = it_threads(N_I);
     constexpr int kQHalf = N_I * 128, kQTile = 2 * kQHalf;       // a query tile: two 64-column halves
     unsigned char* q_s = base;
     unsigned char* a_s = q_s + NQ * kQTile;
@@ -128,10 +134,11 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
     if (tid == 0) {
         for (int s = 0; s < NQ; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
         for (int s = 0; s < NA; ++s) { mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1); }
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 0; w < NW; ++w) {
             mbar_init(&bars->s_full[w], 1); mbar_init(&bars->p_full[w], 128); mbar_init(&bars->sp_free[w], 1);
-            mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128); mbar_init(&bars->x_full[w], 128);
+            mbar_init(&bars->x_full[w], 128);
         }
+        for (int w = 0; w < 2; ++w) { mbar_init(&bars->o_full[w], 1); mbar_init(&bars->o_free[w], 128); }
         bars->abort_flag = 0;
         mbar_init_fence();
     }
@@ -175,7 +182,8 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
         int qb = 0, ph = 1;
         for (int u = u_begin; u < u_end && !bars->abort_flag; ++u) {
             const ItUnit un = it_decode(p, u);
-            const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+            int hd;
+            const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
             unsigned char* qd_s = q_s + qb * kQTile;
             constexpr int kL = (N_I + 31) / 32;
             float l2[kL];
@@ -193,8 +201,8 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             }
             if (ip.q_rows_tma) {
                 mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(b1 * 256));
-                const int tok0 = blk.row_token(p.a0 + un.al, 0);
-                const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
+                int col;
+                const int frow0 = p.first_row(un.al, un.j, col);
                 tma_load_5d_e(el, qd_s, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
                 tma_load_5d_e(el, qd_s + kQHalf, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
             } else {
@@ -222,9 +230,9 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
         for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
             if (!mbar_wait_u(&bars->q_full[qb], qp)) { fail(20); break; }
             for (int t = 0; t < n_tiles; ++t, ++g) {
-                const int w = g & 1;
+                const int w = g % NW;
                 if (!mbar_wait_u(&bars->a_full[s], ph)) { fail(21); ok = false; break; }
-                if (g >= 2 && !mbar_wait_u(&bars->sp_free[w], ((g >> 1) - 1) & 1)) { fail(22); ok = false; break; }
+                if (g >= NW && !mbar_wait_u(&bars->sp_free[w], ((g / NW) - 1) & 1)) { fail(22); ok = false; break; }
                 tc_fence_after();
                 const uint64_t ad = a_desc0 + (uint64_t)((s * kItTileBytes) >> 4);
                 const uint64_t qd = q_desc0 + (uint64_t)((qb * kQTile) >> 4);
@@ -232,7 +240,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint32_t ao = ((ks >> 2) * (kKTile * 128) + (ks & 3) * 32) >> 4;
                     const uint32_t qo = ((ks >> 2) * kQHalf + (ks & 3) * 32) >> 4;
-                    mma_ss_e(el, tmem + it_col_s(w), ad + ao, qd + qo, idesc_s, ks > 0);
+                    mma_ss_e(el, tmem + it_col_s<N_I>(w), ad + ao, qd + qo, idesc_s, ks > 0);
                 }
                 mma_commit_e(el, &bars->s_full[w]);
                 mma_commit_e(el, &bars->a_empty[s]);
@@ -249,89 +257,122 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
         bool ok = true;
         for (int u = u_begin; ok && u < u_end && !bars->abort_flag; ++u) {
             for (int t = 0; t < n_tiles; ++t, ++g) {
-                const int w = g & 1;
-                if (!mbar_wait_u(&bars->p_full[w], (g >> 1) & 1)) { fail(23); ok = false; break; }
-                if (g >= 2 && !mbar_wait_u(&bars->o_free[w], ((g >> 1) - 1) & 1)) { fail(24); ok = false; break; }
+                const int w = g % NW, ob = g & 1;
+                if (!mbar_wait_u(&bars->p_full[w], (g / NW) & 1)) { fail(23); ok = false; break; }
+                if (g >= 2 && !mbar_wait_u(&bars->o_free[ob], ((g >> 1) - 1) & 1)) { fail(24); ok = false; break; }
                 tc_fence_after();
                 const uint64_t qd = q_desc0 + (uint64_t)((qb * kQTile) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < N_I / 16; ++kk)
-                    mma_ts_e(el, tmem + it_col_o(w), tmem + it_col_s(w) + kk * 8, qd + ((kk * 2048) >> 4), idesc_o, kk > 0);
-                mma_commit_e(el, &bars->o_full[w]);
+                    mma_ts_e(el, tmem + it_col_o(ob), tmem + it_col_s<N_I>(w) + kk * 8, qd + ((kk * 2048) >> 4), idesc_o, kk > 0);
+                mma_commit_e(el, &bars->o_full[ob]);
                 mma_commit_e(el, &bars->sp_free[w]);
                 if (t + 1 == n_tiles) mma_commit_e(el, &bars->q_empty[qb]);       // last read of this unit's query tile
             }
             if (++qb == NQ) qb = 0;
         }
-    } else if (warp >= 4 && warp < 12) {
-        // ------------------------------------------------------------------ the two working warpgroups
+    } else if (warp >= 4 && warp < 4 + 4 * NW) {
+        // ------------------------------------------------------------------ the working warpgroups
         const int w = (warp - 4) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                       // TMEM lane == key within the tile
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-        const uint32_t s_t = tmem + lane_sel + it_col_s(w);
+        const uint32_t s_t = tmem + lane_sel + it_col_s<N_I>(w);
         const float scale_l2 = p.scale * kLog2e;
         const int total = (u_end - u_begin) * n_tiles;
+        float* const own = bars->own[warp - 4];
         // bias of tile g's key on this lane, in log2 units; a key past the end gets weight zero
         auto load_cl = [&](int g) -> float {
-            const int uc = g / n_tiles, key = (g - uc * n_tiles) * kKTile + row;
+            const int uc = ip.by_tiles.div(g), key = (g - uc * n_tiles) * kKTile + row;
             return g < total && key < n_keys ? kLog2e * p.cL[(long long)(u_begin + uc) * p.n_keys_c + key] : INFINITY;
         };
+        // Maximum and sum over the 32 keys of this warp for the 16 queries from c0 on, for the tile's other warps, and the
+        // exponentials e against that maximum
+        auto chunk_stats = [&](int c0, float cl2, float (&e)[16]) {
+            uint32_t r[16];
+            tmem_ld16(s_t + c0, r);
+            tmem_wait_ld();
+            float m = 0.f, v[16];                               // m: of query c0 + (lane & 15)
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                const float x = fmaf(__uint_as_float(r[c]), scale_l2, -cl2);
+                const float mc = fmaxf(warp_max(x), -1e30f);    // finite also if none of these keys exists
+                if ((lane & 15) == c) m = mc;
+                v[c] = e[c] = exp2f(x - mc);
+            }
+            const float sum = column_sums(v, lane);
+            if (lane < 16) bars->part[w][quad][c0 + lane] = make_float2(m, sum);
+        };
+        constexpr bool kKeep = N_I <= 32;                       // the exponentials stay in registers meanwhile
         float cl_next = load_cl(w);
-        for (int g = w; g < total && !bars->abort_flag; g += 2) {
-            const int uc = g / n_tiles, t = g - uc * n_tiles;
+        for (int g = w; g < total && !bars->abort_flag; g += NW) {
+            const int uc = ip.by_tiles.div(g), t = g - uc * n_tiles;
             const int u = u_begin + uc;
             const int key = t * kKTile + row;
             const bool valid = key < n_keys;
             const float cl2 = cl_next;
-            cl_next = load_cl(g + 2);
-            if (!mbar_wait_u(&bars->s_full[w], (g >> 1) & 1)) { fail(31); break; }
+            cl_next = load_cl(g + NW);
+            if (!mbar_wait_u(&bars->s_full[w], (g / NW) & 1)) { fail(31); break; }
             tc_fence_after();
             const float* lse2 = bars->lse2[uc % NQ];
+            float csum = 0.f;
+            bool done = false;
             if (ip.own_lse) {
-#pragma unroll 1
-                for (int c0 = 0; c0 < N_I; c0 += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(s_t + c0, r);
-                    tmem_wait_ld();
-                    float e[16], m = 0.f;                       // m: of query c0 + (lane & 15)
+                float e[kKeep ? N_I / 16 : 1][16];
+                if constexpr (kKeep) {
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        const float x = fmaf(__uint_as_float(r[c]), scale_l2, -cl2);
-                        const float mc = fmaxf(warp_max(x), -1e30f);        // finite also if none of these keys exists
-                        if ((lane & 15) == c) m = mc;
-                        e[c] = exp2f(x - mc);
-                    }
-                    const float sum = column_sums(e, lane);
-                    if (lane < 16) bars->part[w][quad][c0 + lane] = make_float2(m, sum);
+                    for (int c0 = 0; c0 < N_I; c0 += 16) chunk_stats(c0, cl2, e[c0 / 16]);
+                } else {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < N_I; c0 += 16) chunk_stats(c0, cl2, e[0]);
                 }
                 mbar_arrive(&bars->x_full[w]);
-                if (!mbar_wait_u(&bars->x_full[w], (g >> 1) & 1)) { fail(32); break; }
-                float* own = bars->lse2_own[warp - 4];
+                if (!mbar_wait_u(&bars->x_full[w], (g / NW) & 1)) { fail(32); break; }
 #pragma unroll
                 for (int c = lane; c < N_I; c += 32) {
-                    const float2 a = bars->part[w][0][c], b = bars->part[w][1][c], d = bars->part[w][2][c], e = bars->part[w][3][c];
-                    const float m = fmaxf(fmaxf(a.x, b.x), fmaxf(d.x, e.x));
-                    const float z = a.y * exp2f(a.x - m) + b.y * exp2f(b.x - m) + d.y * exp2f(d.x - m) + e.y * exp2f(e.x - m);
-                    own[c] = c < b1 ? m + __log2f(z) : INFINITY;
+                    const float2 a = bars->part[w][0][c], b = bars->part[w][1][c], d = bars->part[w][2][c], f = bars->part[w][3][c];
+                    const float m = fmaxf(fmaxf(a.x, b.x), fmaxf(d.x, f.x));
+                    const float z = a.y * exp2f(a.x - m) + b.y * exp2f(b.x - m) + d.y * exp2f(d.x - m) + f.y * exp2f(f.x - m);
+                    if constexpr (kKeep) own[c] = c < b1 ? exp2f(bars->part[w][quad][c].x - m) / z : 0.f;
+                    else own[c] = c < b1 ? m + __log2f(z) : INFINITY;
                 }
                 __syncwarp();
-                lse2 = own;
-            }
-            float csum = 0.f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < N_I; c0 += 16) {
-                uint32_t r[16], pk[8];
-                tmem_ld16(s_t + c0, r);
-                tmem_wait_ld();
+                if constexpr (kKeep) {
+                    // weight = exponential against the warp's maximum x what that maximum is worth against all keys
 #pragma unroll
-                for (int c = 0; c < 16; c += 2) {
-                    const float e0 = exp2f(fmaf(__uint_as_float(r[c]), scale_l2, -(cl2 + lse2[c0 + c])));
-                    const float e1 = exp2f(fmaf(__uint_as_float(r[c + 1]), scale_l2, -(cl2 + lse2[c0 + c + 1])));
-                    csum += e0 + e1;
-                    pk[c >> 1] = pack_bf16(e0, e1);
+                    for (int c0 = 0; c0 < N_I; c0 += 16) {
+                        uint32_t pk[8];
+#pragma unroll
+                        for (int c = 0; c < 16; c += 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(&own[c0 + c]);
+                            const float (&ec)[16] = e[c0 / 16];
+                            const float p0 = ec[c] * f.x, p1 = ec[c + 1] * f.y, p2 = ec[c + 2] * f.z, p3 = ec[c + 3] * f.w;
+                            csum += (p0 + p1) + (p2 + p3);
+                            pk[c >> 1] = pack_bf16(p0, p1);
+                            pk[(c >> 1) + 1] = pack_bf16(p2, p3);
+                        }
+                        tmem_st8(s_t + (c0 >> 1), pk);
+                    }
+                    done = true;
+                } else {
+                    lse2 = own;
                 }
-                tmem_st8(s_t + (c0 >> 1), pk);
+            }
+            if (!done) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < N_I; c0 += 16) {
+                    uint32_t r[16], pk[8];
+                    tmem_ld16(s_t + c0, r);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 16; c += 2) {
+                        const float e0 = exp2f(fmaf(__uint_as_float(r[c]), scale_l2, -(cl2 + lse2[c0 + c])));
+                        const float e1 = exp2f(fmaf(__uint_as_float(r[c + 1]), scale_l2, -(cl2 + lse2[c0 + c + 1])));
+                        csum += e0 + e1;
+                        pk[c >> 1] = pack_bf16(e0, e1);
+                    }
+                    tmem_st8(s_t + (c0 >> 1), pk);
+                }
             }
             tmem_wait_st();
             tc_fence_before();
@@ -342,7 +383,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                 p.cR[(((long long)un.bhl * n_keys + key) * p.na + un.al) * b2 + un.j] = csum;
             }
         }
-    } else if (warp >= 12) {
+    } else {
         // ------------------------------------------------------------------ drain warpgroup
         const uint32_t el = elect_one();
         const int quad = warp & 3;
@@ -351,25 +392,19 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
         unsigned char* const st_row = st + lane * 128;
         const int total = (u_end - u_begin) * n_tiles;
         for (int g = 0; g < total && !bars->abort_flag; ++g) {
-            const int uc = g / n_tiles, t = g - uc * n_tiles, w = g & 1;
+            const int uc = ip.by_tiles.div(g), t = g - uc * n_tiles, w = g & 1;
             const ItUnit un = it_decode(p, u_begin + uc);
             const uint32_t o_t = tmem + lane_sel + it_col_o(w);
             const int key0 = t * kKTile + quad * 32;
             if (!mbar_wait_u(&bars->o_full[w], (g >> 1) & 1)) { fail(41); break; }
             tc_fence_after();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {                       // 64 columns at a time
-                uint32_t ra[32], rb[32];
-                tmem_ld32(o_t + h * 64, ra);
-                tmem_ld32(o_t + h * 64 + 32, rb);
-                tmem_wait_ld();
-                if (h == 1) {
-                    tc_fence_before();
-                    mbar_arrive(&bars->o_free[w]);
-                }
-                if (key0 >= n_keys) continue;                   // keys past the end of the last tile
-                tma_store_wait_read();
-                __syncwarp();
+            if (key0 >= n_keys) {                               // keys past the end of the last tile
+                tc_fence_before();
+                mbar_arrive(&bars->o_free[w]);
+                continue;
+            }
+            uint32_t ra[32], rb[32];
+            auto put = [&](int h) {                             // 64 columns to the staging rows
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const uint32_t (&r)[32] = c < 4 ? ra : rb;
@@ -379,11 +414,24 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                         wv[e] = pack_bf16(__uint_as_float(r[(c & 3) * 8 + 2 * e]), __uint_as_float(r[(c & 3) * 8 + 2 * e + 1]));
                     *reinterpret_cast<uint4*>(st_row + h * 4096 + ((c ^ (lane & 7)) << 4)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
                 }
-                fence_async_smem();
-                __syncwarp();
-                tma_store_4d_e(el, &tar, st + h * 4096, h * 64, un.al * b2 + un.j, key0, un.bhl);
-                tma_store_commit();
-            }
+            };
+            tmem_ld32(o_t, ra);
+            tmem_ld32(o_t + 32, rb);
+            tma_store_wait_read_all();                          // the rows of the tile before have been read
+            __syncwarp();
+            tmem_wait_ld();
+            put(0);
+            tmem_ld32(o_t + 64, ra);
+            tmem_ld32(o_t + 96, rb);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(&bars->o_free[w]);
+            put(1);
+            fence_async_smem();
+            __syncwarp();
+            tma_store_4d_e(el, &tar, st, 0, un.al * b2 + un.j, key0, un.bhl);
+            tma_store_4d_e(el, &tar, st + 4096, 64, un.al * b2 + un.j, key0, un.bhl);
+            tma_store_commit();
         }
         tma_store_wait_all();
     }
@@ -405,6 +453,8 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     LaunchScope scope(kClsLIter, s);
     ItParams ip;
     ip.mp = p;
+    ip.mp.set_divs();
+    ip.by_tiles = FastDiv::of((p.n_keys + kKTile - 1) / kKTile);
     ip.n_units = p.nbh * p.na * p.blk.b2;
     CUtensorMap map_al;
     if (int rc = make_bridge_tmap(&map_al, p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, 1, kKTile)) return rc;
@@ -414,20 +464,20 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     ip.own_lse = l_iter_own_lse(p);
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
-    auto go = [&](auto kernel, int smem) -> int {
+    auto go = [&](auto kernel, int threads, int smem) -> int {
         if (int rc = opt_in_smem((const void*)kernel, smem)) return rc;
-        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, kThreadsIt, smem, s, map_al, *map_qrows, map_ar, ip);
+        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, threads, smem, s, map_al, *map_qrows, map_ar, ip);
     };
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {
-        case 16: rc = go(monarch_iter_tc_kernel<16>, it_smem_bytes<16>()); break;
-        case 32: rc = go(monarch_iter_tc_kernel<32>, it_smem_bytes<32>()); break;
-        case 48: rc = go(monarch_iter_tc_kernel<48>, it_smem_bytes<48>()); break;
-        case 64: rc = go(monarch_iter_tc_kernel<64>, it_smem_bytes<64>()); break;
-        case 80: rc = go(monarch_iter_tc_kernel<80>, it_smem_bytes<80>()); break;
-        case 96: rc = go(monarch_iter_tc_kernel<96>, it_smem_bytes<96>()); break;
-        case 112: rc = go(monarch_iter_tc_kernel<112>, it_smem_bytes<112>()); break;
-        case 128: rc = go(monarch_iter_tc_kernel<128>, it_smem_bytes<128>()); break;
+        case 16: rc = go(monarch_iter_tc_kernel<16>, it_threads(16), it_smem_bytes<16>()); break;
+        case 32: rc = go(monarch_iter_tc_kernel<32>, it_threads(32), it_smem_bytes<32>()); break;
+        case 48: rc = go(monarch_iter_tc_kernel<48>, it_threads(48), it_smem_bytes<48>()); break;
+        case 64: rc = go(monarch_iter_tc_kernel<64>, it_threads(64), it_smem_bytes<64>()); break;
+        case 80: rc = go(monarch_iter_tc_kernel<80>, it_threads(80), it_smem_bytes<80>()); break;
+        case 96: rc = go(monarch_iter_tc_kernel<96>, it_threads(96), it_smem_bytes<96>()); break;
+        case 112: rc = go(monarch_iter_tc_kernel<112>, it_threads(112), it_smem_bytes<112>()); break;
+        case 128: rc = go(monarch_iter_tc_kernel<128>, it_threads(128), it_smem_bytes<128>()); break;
         default: return SFM_ERR_UNSUPPORTED;
     }
     if (rc) return rc;

@@ -39,12 +39,25 @@ struct MonarchParams {
     float mult0;                   // row-step multiplier when the operand is q itself (scale, or
                                    // scale/(1+1e-6) on the first pass of the iterative path)
     Blocking blk;
+    FastDiv by_b2, by_na, by_H, by_gpt, by_wr;       // set_divs
     // Where the column step puts its result.  Unsharded: one [B, n_q, H, 128] tensor (out_peers[0] = out,
     // out_tokens = n_q, out_heads = H, out_head0 = 0).  Head-sharded call: the output is sharded by token
     // over the GPUs of the box, shard t / out_tokens being a [B, out_tokens, out_heads, 128] tensor on that
     // GPU, of which this GPU writes heads [out_head0, out_head0 + H) with plain stores over NVLink.
     __nv_bfloat16* out_peers[kMaxPeers];
     int out_tokens, out_heads, out_head0;
+
+    void set_divs() {
+        by_b2 = FastDiv::of(blk.b2); by_na = FastDiv::of(na); by_H = FastDiv::of(H);
+        by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce);
+    }
+    // Row of the token grid, and column there, of the first token of (query group a0 + al, column j).
+    __device__ __forceinline__ int first_row(int al, int j, int& col) const {
+        int ce, e;
+        const int a = by_gpt.divmod(a0 + al, ce), c = by_wr.divmod(ce, e);
+        col = e * blk.ww + j;
+        return (a * blk.f_tied * blk.h_reduce + c) * blk.hh;
+    }
 
     __device__ __forceinline__ __nv_bfloat16* out_row(int b, long long tok, int hd) const {
         const int peer = (int)(tok / out_tokens);

@@ -284,6 +284,24 @@ def test_monarch_iterative_small(sfb, ci, iters):
     check_close(z, z_ref, f"{c['name']} T={iters}")
 
 
+# (h, w, frames cached): block columns on both sides of every width the row step is built for, block rows on both sides of
+# 32 queries, where the update keeps its exponentials in registers (one tile of keys) or goes over them twice
+@pytest.mark.gpu
+@pytest.mark.parametrize("edge", [(16, 16, 4), (30, 17, 3), (32, 32, 4), (33, 33, 3), (31, 48, 4), (5, 49, 3), (32, 64, 3), (1, 5, 3)],
+                         ids=lambda e: "h{}w{}_F{}".format(*e))
+def test_monarch_iterative_widths(sfb, edge):
+    h, w, cached = edge
+    rng = np.random.default_rng(77 + h * w)
+    frame, H, T = h * w, 3, 3
+    n_q, n_kv = 3 * frame, cached * frame
+    mk = lambda *s: bf(cases.randn(rng, *s))
+    c = dict(blocking=(1, 1, 1, h, w), q=mk(2, n_q, H, 128), nk=mk(2, n_q, H, 128), nv=mk(2, n_q, H, 128), kbuf=mk(2, n_kv + frame, H, 128),
+             vbuf=mk(2, n_kv + frame, H, 128), start=n_kv - n_q, end=n_kv, n_kv=n_kv, sm_scale=128 ** -0.5)
+    ref, _, _ = run_oracle_cache(c, T)
+    got, _, _ = run_gpu_cache(sfb, c, T)
+    check_close(got, ref, str(edge))
+
+
 # (h, w, f_tied, h_reduce, w_reduce, frames cached): 128 and 129 keys (one tile, two tiles), block rows of 16 to 120, query
 # rows that are gathered
 @pytest.mark.parametrize("edge", [(32, 8, 1, 1, 1, 4), (43, 8, 1, 1, 1, 3), (16, 16, 1, 1, 1, 8), (40, 6, 3, 1, 1, 3), (20, 8, 3, 2, 1, 3),
