@@ -93,9 +93,8 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) 
 struct LUnit { int bhl, al, j; };
 __device__ __forceinline__ LUnit decode_unit(const MonarchParams& p, int u) {
     LUnit r;
-    r.j = u % p.blk.b2; u /= p.blk.b2;
-    r.al = u % p.na;
-    r.bhl = u / p.na;
+    u = p.by_b2.divmod(u, r.j);
+    r.bhl = p.by_na.divmod(u, r.al);
     return r;
 }
 
@@ -129,7 +128,9 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     struct GroupKeys { int first, second, split; __device__ __forceinline__ int of(int us) const { return us < split ? first : second; } };
     auto keys_of = [&](int u0) -> GroupKeys {
         if (!kCausal) return {p.n_keys, p.n_keys, kMaxU};
-        const int slab = u0 / b2, al = slab % p.na;
+        int al;
+        const int slab = p.by_b2.div(u0);
+        p.by_na.divmod(slab, al);
         return {group_keys(al), group_keys(al + 1 == p.na ? 0 : al + 1), b2 - (u0 - slab * b2)};
     };
     auto group_tiles = [&](const GroupKeys& gk, int nu) -> int {
@@ -261,9 +262,10 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                 mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(nu * b1 * 256));
                 for (int us = 0; us < nu; ++us) {
                     const LUnit un = decode_unit(p, u0 + us);
-                    const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-                    const int tok0 = blk.row_token(p.a0 + un.al, 0);
-                    const int frow0 = tok0 / blk.w, col = tok0 - frow0 * blk.w + un.j;
+                    int hd;
+                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
+                    int col;
+                    const int frow0 = p.first_row(un.al, un.j, col);
                     unsigned char* dst = q_s + us * R * 128;
                     tma_load_5d_e(el, dst, &tqr, &bars->q_full, 0, hd, col, frow0, b);
                     tma_load_5d_e(el, dst + 128 * 128, &tqr, &bars->q_full, 64, hd, col, frow0, b);
@@ -272,7 +274,8 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                 // query rows that are not consecutive rows of the token grid are gathered with plain loads
                 for (int us = 0; us < nu; ++us) {
                     const LUnit un = decode_unit(p, u0 + us);
-                    const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
+                    int hd;
+                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
                     const __nv_bfloat16* qb = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
                     for (int idx = lane; idx < b1 * 16; idx += 32) {
                         const int i = idx >> 4, ch = idx & 15;
@@ -526,9 +529,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
             __nv_bfloat16* out_row = nullptr;
             if (row_ok) {
                 const LUnit un = decode_unit(p, u0 + us);
-                const int bh = p.bh0 + un.bhl, b = bh / p.H, hd = bh - b * p.H;
-                const long long tok = blk.row_token(p.a0 + un.al, i_row) + un.j;
-                out_row = p.out_row(b, tok, hd);
+                int hd;
+                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
+                int col;
+                const int frow = p.first_row(un.al, un.j, col) + p.row_ahead(i_row);
+                out_row = p.out_row(b, frow * blk.w + col, hd);
                 // iterative variant, backward: the softmax's log-sum-exp (natural log)
                 if (lp.write_lse) p.lse[(long long)(u0 + us) * b1 + i_row] = (ms + log2f(den)) * 0.6931471805599453f;
             }
@@ -597,6 +602,7 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     LaunchScope scope(kClsLStep, s);
     LTcParams lp;
     lp.mp = p;
+    lp.mp.set_divs();
     lp.n_units = p.nbh * p.na * p.blk.b2;
     // as many units per group as the tile holds, but no more than it takes to give every SM one: the units of a group
     // follow one another through the MMA pipe and the rings (two heads on a 6 x 8 grid: 18 -> 11 us)

@@ -39,7 +39,7 @@ struct MonarchParams {
     float mult0;                   // row-step multiplier when the operand is q itself (scale, or
                                    // scale/(1+1e-6) on the first pass of the iterative path)
     Blocking blk;
-    FastDiv by_b2, by_na, by_H, by_gpt, by_wr;       // set_divs
+    FastDiv by_b2, by_na, by_H, by_gpt, by_wr, by_hh, by_out;       // set_divs
     // Where the column step puts its result.  Unsharded: one [B, n_q, H, 128] tensor (out_peers[0] = out,
     // out_tokens = n_q, out_heads = H, out_head0 = 0).  Head-sharded call: the output is sharded by token
     // over the GPUs of the box, shard t / out_tokens being a [B, out_tokens, out_heads, 128] tensor on that
@@ -49,7 +49,7 @@ struct MonarchParams {
 
     void set_divs() {
         by_b2 = FastDiv::of(blk.b2); by_na = FastDiv::of(na); by_H = FastDiv::of(H);
-        by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce);
+        by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce); by_hh = FastDiv::of(blk.hh); by_out = FastDiv::of(out_tokens);
     }
     // Row of the token grid, and column there, of the first token of (query group a0 + al, column j).
     __device__ __forceinline__ int first_row(int al, int j, int& col) const {
@@ -58,10 +58,12 @@ struct MonarchParams {
         col = e * blk.ww + j;
         return (a * blk.f_tied * blk.h_reduce + c) * blk.hh;
     }
+    // How many rows of the token grid further query i of that column is.
+    __device__ __forceinline__ int row_ahead(int i) const { return i + by_hh.div(i) * (blk.h - blk.hh); }
 
-    __device__ __forceinline__ __nv_bfloat16* out_row(int b, long long tok, int hd) const {
-        const int peer = (int)(tok / out_tokens);
-        const long long t = tok - (long long)peer * out_tokens;
+    __device__ __forceinline__ __nv_bfloat16* out_row(int b, int tok, int hd) const {
+        int t;
+        const int peer = by_out.divmod(tok, t);
         return out_peers[peer] + (((long long)b * out_tokens + t) * out_heads + out_head0 + hd) * kHeadDim;
     }
 };
