@@ -17,9 +17,10 @@
 //
 // Warp roles (16 warps): 0 = bias slices and aL tiles, 3 = Y tiles, 1 = PV-GEMM issuer (owns the TMEM allocation), 2 = the
 // groups' query rows and the S GEMMs, 4..7 / 8..11 = softmax warpgroups, 12..15 = epilogue warpgroup.  Roles 0 to 3 run as
-// whole warps with an elected issuing lane.  The query rows have one buffer: warp 2 reloads it as soon as its last S GEMM
+// whole warps with an elected issuing lane.  With one buffer of query rows, warp 2 reloads it as soon as its last S GEMM
 // of a group has completed, which the softmax and PV GEMMs of that group cover, while warp 0 is already loading the next
-// group's keys.  All roles meet only through mbarriers with bounded waits; a timeout records a status code and the CTA
+// group's keys; groups of few tiles have two.  The code is kept small: a short launch fetches it from L2 or DRAM as it goes (a
+// second copy of the query load cost the first chunk 2 us).  All roles meet only through mbarriers with bounded waits; a timeout records a status code and the CTA
 // unwinds.
 //
 // What bounds it: reading the bridge (604 MB in 0.114 ms at framewise, 21 cached frames, 12 heads: 5.4 TB/s with the start-up
@@ -58,7 +59,7 @@ struct LTcParams {
     int U;           // units per group
     int R;           // tile rows per unit slot (128 / U, rounded down)
     int kt;          // keys per tile (multiple of 16, <= 128)
-    int n_a, n_y;    // tiles in the aL and Y rings
+    int n_q, n_a, n_y;    // query tiles, tiles in the aL and Y rings
     int q_rows_tma;  // the query rows of a unit are consecutive rows of the token grid: load them with TMA
     int write_lse;   // also store the log-sum-exp of every query row (iterative variant, backward)
     int lse_only;    // nothing but that (no value tiles, no PV GEMMs, no output rows)
@@ -68,7 +69,7 @@ struct LTcParams {
 struct __align__(16) Barriers {
     alignas(16) float cl[4][kMaxU][kBiasPitch];   // bias slices, per unit slot: a ring of four tiles
     float stats[2][2][128];                // [warpgroup][m | l][tile row]
-    uint64_t q_full, q_empty;
+    uint64_t q_full[2], q_empty[2];
     uint64_t a_full[kMaxStages], a_empty[kMaxStages];
     uint64_t y_full[kMaxStages], y_empty[kMaxStages];
     uint64_t cl_full[4], cl_empty[4];
@@ -81,8 +82,8 @@ struct __align__(16) Barriers {
 };
 
 constexpr int kQBytes = 2 * 128 * 128;     // query tile, two 64-column halves
-constexpr int kRing = 172 << 10;           // aL tiles, then Y tiles
-constexpr int kSmemBytes = 1024 + kQBytes + kRing + (int)sizeof(Barriers) + 64;
+constexpr int kTiles = 204 << 10;          // query tiles, aL tiles, Y tiles
+constexpr int kSmemBytes = 1024 + kTiles + (int)sizeof(Barriers) + 64;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) {
@@ -106,9 +107,9 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = base;
-    unsigned char* a_s = q_s + kQBytes;
+    unsigned char* a_s = q_s + lp.n_q * kQBytes;
     unsigned char* y_s = a_s + lp.n_a * lp.kt * 256;
-    Barriers* bars = reinterpret_cast<Barriers*>(a_s + kRing);
+    Barriers* bars = reinterpret_cast<Barriers*>(base + kTiles);
 
     const MonarchParams& p = lp.mp;
     const Blocking& blk = p.blk;
@@ -151,8 +152,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
 
     if (warp == 2 && lane == 0) { prefetch_tmap(&tqr); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
-        mbar_init(&bars->q_full, 1);
-        mbar_init(&bars->q_empty, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1);
             mbar_init(&bars->y_full[s], 1); mbar_init(&bars->y_empty[s], 1);
@@ -166,7 +166,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         mbar_init_fence();
     }
     // rows of the query tile that no unit writes must still hold finite numbers
-    for (int i = tid; i < kQBytes / 16; i += kThreads) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < lp.n_q * kQBytes / 16; i += kThreads) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 1) { tmem_alloc(&bars->tmem_base, kTmemCols); tmem_relinquish(); }
     fence_async_smem();
     tc_fence_before();
@@ -194,10 +194,47 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         atomicCAS(lp.status, 0, code);
     };
 
+    // query rows of a group
+    auto load_q = [&](uint32_t el, int qb, int u0, int nu) {
+        unsigned char* const qt = q_s + qb * kQBytes;
+        if (lp.q_rows_tma) {
+            // the 128-byte swizzle is a function of the shared-memory address, so a box may land on any tile row
+            mbar_arrive_expect_tx_e(el, &bars->q_full[qb], (uint32_t)(nu * b1 * 256));
+            for (int us = 0; us < nu; ++us) {
+                const LUnit un = decode_unit(p, u0 + us);
+                int hd;
+                const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
+                int col;
+                const int frow0 = p.first_row(un.al, un.j, col);
+                unsigned char* dst = qt + us * R * 128;
+                tma_load_5d_e(el, dst, &tqr, &bars->q_full[qb], 0, hd, col, frow0, b);
+                tma_load_5d_e(el, dst + 128 * 128, &tqr, &bars->q_full[qb], 64, hd, col, frow0, b);
+            }
+        } else {
+            // query rows that are not consecutive rows of the token grid are gathered with plain loads
+            for (int us = 0; us < nu; ++us) {
+                const LUnit un = decode_unit(p, u0 + us);
+                int hd;
+                const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
+                const __nv_bfloat16* src = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
+                for (int idx = lane; idx < b1 * 16; idx += 32) {
+                    const int i = idx >> 4, ch = idx & 15;
+                    const uint4 val = *reinterpret_cast<const uint4*>(
+                        src + (long long)(blk.row_token(p.a0 + un.al, i) + un.j) * p.H * kHeadDim + ch * 8);
+                    const int r = us * R + i;
+                    *reinterpret_cast<uint4*>(qt + (ch >> 3) * (128 * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = val;
+                }
+            }
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->q_full[qb]);
+        }
+    };
+
     if (warp == 0) {
         // ------------------------------------------------------------------ bias slices and key tiles
         const uint32_t el = elect_one();
-        int sa = 0, pa = 1, gt = 0;              // ring slot and its phase, tiles of all groups so far
+        int sa = 0, pa = 1, gt = 0;       // ring slots and their phases, tiles of all groups so far
         bool ok = true;
         for (int gi = 0; ok && gi < n_my; ++gi) {
             int nu;
@@ -254,51 +291,24 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         const uint32_t idesc_s = idesc_bf16(128, 0, 0, 0) | ((uint32_t)(kt >> 3) << 17);
         const uint64_t q_desc = smem_desc_sw128(smem_addr(q_s), 16, 1024);
         const uint64_t a_desc0 = smem_desc_sw128(smem_addr(a_s), 16, 1024);
-        auto load_q = [&](int gi) {
-            int nu;
-            const int u0 = group_at(gi, nu);
-            if (lp.q_rows_tma) {
-                // the 128-byte swizzle is a function of the shared-memory address, so a box may land on any tile row
-                mbar_arrive_expect_tx_e(el, &bars->q_full, (uint32_t)(nu * b1 * 256));
-                for (int us = 0; us < nu; ++us) {
-                    const LUnit un = decode_unit(p, u0 + us);
-                    int hd;
-                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
-                    int col;
-                    const int frow0 = p.first_row(un.al, un.j, col);
-                    unsigned char* dst = q_s + us * R * 128;
-                    tma_load_5d_e(el, dst, &tqr, &bars->q_full, 0, hd, col, frow0, b);
-                    tma_load_5d_e(el, dst + 128 * 128, &tqr, &bars->q_full, 64, hd, col, frow0, b);
-                }
-            } else {
-                // query rows that are not consecutive rows of the token grid are gathered with plain loads
-                for (int us = 0; us < nu; ++us) {
-                    const LUnit un = decode_unit(p, u0 + us);
-                    int hd;
-                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
-                    const __nv_bfloat16* qb = p.q + (long long)b * p.q_bs + (long long)hd * kHeadDim;
-                    for (int idx = lane; idx < b1 * 16; idx += 32) {
-                        const int i = idx >> 4, ch = idx & 15;
-                        const uint4 val = *reinterpret_cast<const uint4*>(
-                            qb + (long long)(blk.row_token(p.a0 + un.al, i) + un.j) * p.H * kHeadDim + ch * 8);
-                        const int r = us * R + i;
-                        *reinterpret_cast<uint4*>(q_s + (ch >> 3) * (128 * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = val;
-                    }
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->q_full);
-            }
-        };
-        int sa = 0, pa = 0, gc = 0, gt = 0;
+        int sa = 0, pa = 0, gt = 0;
         bool ok = true;
-        if (n_my > 0) load_q(0);
-        for (int gi = 0; ok && gi < n_my; ++gi, ++gc) {
+        // with two query tiles a group's rows are asked for before the GEMMs of the group before it, else after them
+        const int lead = lp.n_q - 1;
+        for (int x = 0; ok && x < n_my + lead; ++x) {
             int nu;
-            const int u0 = group_at(gi, nu);
+            if (x < n_my) {
+                const int qb = x & lead, u0 = group_at(x, nu);
+                if (!mbar_wait_u(&bars->q_empty[qb], ((x >> lead) & 1) ^ 1)) { fail(10); break; }
+                load_q(el, qb, u0, nu);
+            }
+            const int gi = x - lead;
+            if (gi < 0) continue;
+            const int qb = gi & lead, u0 = group_at(gi, nu);
             const GroupKeys gk = keys_of(u0);
             const int n_tiles = group_tiles(gk, nu);
-            if (!mbar_wait_u(&bars->q_full, gc & 1)) { fail(20); break; }
+            if (!mbar_wait_u(&bars->q_full[qb], (gi >> lead) & 1)) { fail(20); break; }
+            const uint64_t qd = q_desc + (uint64_t)((qb * kQBytes) >> 4);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;
                 if (!mbar_wait_u(&bars->sp_free[w], ((gt >> 1) & 1) ^ 1)) { fail(25); ok = false; break; }
@@ -312,7 +322,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                     for (int ks = 0; ks < 8; ++ks) {
                         const uint32_t qo = ((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t ao = ((ks >> 2) * half + (ks & 3) * 32) >> 4;
-                        mma_ss_masked_e(el, tmem + col_s(w), q_desc + qo, ad + ao, idesc_s, ks > 0, m);
+                        mma_ss_masked_e(el, tmem + col_s(w), qd + qo, ad + ao, idesc_s, ks > 0, m);
                     }
                     mma_commit_e(el, &bars->a_empty[sa]);
                     if (++sa == lp.n_a) { sa = 0; pa ^= 1; }
@@ -321,11 +331,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                 mma_commit_e(el, &bars->s_full[w]);
             }
             if (!ok) break;
-            if (gi + 1 < n_my) {
-                mma_commit_e(el, &bars->q_empty);
-                if (!mbar_wait_u(&bars->q_empty, gc & 1)) { fail(10); break; }
-                load_q(gi + 1);
-            }
+            mma_commit_e(el, &bars->q_empty[qb]);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ PV-GEMM issuer
@@ -613,7 +619,11 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     lp.R = 128 / lp.U;
     lp.kt = l_tile_keys(p);
     // A value tile stays until its softmax and GEMM are done, a key tile only until its GEMM: two slots of five for keys
-    const int slots = kRing / (lp.kt * 256);
+    // Two query tiles where a group has few tiles: its rows take 2000 to 4000 cycles to arrive, which the GEMMs and softmax of a
+    // longer group cover, whose rings need the room (first chunk 73.2 -> 71.8 us a call, tied3frame 106.3 -> 101.1 with one tile of
+    // four units, three of one; with 24 of eight units the column step went from 350 to 367).
+    lp.n_q = lp.U * ((p.n_keys + lp.kt - 1) / lp.kt) <= 4 ? 2 : 1;
+    const int slots = (kTiles - lp.n_q * kQBytes) / (lp.kt * 256);
     lp.n_a = (slots * 2 + 4) / 5 < kMaxStages ? (slots * 2 + 4) / 5 : kMaxStages;
     lp.n_y = slots - lp.n_a < kMaxStages ? slots - lp.n_a : kMaxStages;
     lp.status = status;
