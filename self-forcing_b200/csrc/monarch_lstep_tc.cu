@@ -100,7 +100,8 @@ __device__ __forceinline__ LUnit decode_unit(const MonarchParams& p, int u) {
 }
 
 // tal / ty = bridge aL / Y maps [group][key][column][128] (box 64 x 1 column x kt keys), tqr = query rows (5-D, box b1 rows).
-template <bool kCausal>
+// kLarge: the bridge is much larger than L2 (MonarchParams::large_bridge).
+template <bool kCausal, bool kLarge>
 __global__ void __launch_bounds__(kThreads, 1)
 monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap ty,
                     const __grid_constant__ CUtensorMap tqr, LTcParams lp) {
@@ -234,6 +235,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     if (warp == 0) {
         // ------------------------------------------------------------------ bias slices and key tiles
         const uint32_t el = elect_one();
+        const uint64_t policy = kLarge ? l2_evict_first() : 0;
         int sa = 0, pa = 1, gt = 0;       // ring slots and their phases, tiles of all groups so far
         bool ok = true;
         for (int gi = 0; ok && gi < n_my; ++gi) {
@@ -255,8 +257,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                     const LUnit un = decode_unit(p, u0 + us);
                     unsigned char* at = a_s + sa * tile_bytes;
                     mbar_arrive_expect_tx_e(el, &bars->a_full[sa], (uint32_t)tile_bytes);
-                    tma_load_4d_e(el, at, &tal, &bars->a_full[sa], 0, un.j, t * kt, un.bhl * p.na + un.al);
-                    tma_load_4d_e(el, at + half, &tal, &bars->a_full[sa], 64, un.j, t * kt, un.bhl * p.na + un.al);
+                    tma_load_halves_e<kLarge>(el, at, half, &tal, &bars->a_full[sa], un.j, t * kt, un.bhl * p.na + un.al, policy);
                     if (++sa == lp.n_a) { sa = 0; pa ^= 1; }
                 }
             }
@@ -265,6 +266,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
         // ------------------------------------------------------------------ value tiles
         if (!lp.lse_only) {
             const uint32_t el = elect_one();
+            const uint64_t policy = kLarge ? l2_evict_first() : 0;
             int sy = 0, py = 1;
             bool ok = true;
             for (int gi = 0; ok && gi < n_my; ++gi) {
@@ -279,8 +281,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                         const LUnit un = decode_unit(p, u0 + us);
                         unsigned char* yt = y_s + sy * tile_bytes;
                         mbar_arrive_expect_tx_e(el, &bars->y_full[sy], (uint32_t)tile_bytes);
-                        tma_load_4d_e(el, yt, &ty, &bars->y_full[sy], 0, un.j, t * kt, un.bhl * p.na + un.al);
-                        tma_load_4d_e(el, yt + half, &ty, &bars->y_full[sy], 64, un.j, t * kt, un.bhl * p.na + un.al);
+                        tma_load_halves_e<kLarge>(el, yt, half, &ty, &bars->y_full[sy], un.j, t * kt, un.bhl * p.na + un.al, policy);
                         if (++sy == lp.n_y) { sy = 0; py ^= 1; }
                     }
             }
@@ -636,7 +637,9 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     if (int rc = make_bridge_tmap(&maps[1], p.Y, p.blk.b2, p.n_keys, p.nbh * p.na, 1, lp.kt)) return rc;
     const int n_groups = (lp.n_units + lp.U - 1) / lp.U;
     dim3 grid(n_groups < num_sms ? n_groups : num_sms);
-    auto kernel = p.causal_groups > 0 ? monarch_l_tc_kernel<true> : monarch_l_tc_kernel<false>;
+    const bool large = p.large_bridge();
+    auto kernel = p.causal_groups > 0 ? (large ? monarch_l_tc_kernel<true, true> : monarch_l_tc_kernel<true, false>)
+                                      : (large ? monarch_l_tc_kernel<false, true> : monarch_l_tc_kernel<false, false>);
     if (int rc = opt_in_smem((const void*)kernel, kSmemBytes)) return rc;
     const bool is_short = (long long)n_groups * ((p.n_keys + lp.kt - 1) / lp.kt) <= 16ll * num_sms;
     return launch_pdl(is_short, kernel, grid, kThreads, kSmemBytes, s, maps[0], maps[1], *map_qrows, lp);

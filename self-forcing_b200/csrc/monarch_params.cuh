@@ -47,6 +47,11 @@ struct MonarchParams {
     __nv_bfloat16* out_peers[kMaxPeers];
     int out_tokens, out_heads, out_head0;
 
+    // The chunk's bridge is more than twice what L2 holds: the column step then reads most of it from DRAM, and what it has read
+    // should leave L2 before what it has not; K and V, which a tile of query groups reads a few microseconds after the other,
+    // should stay.  12 heads, 21 frames (604 MB) 317 -> 310 us a call, 12 frames 214 -> 210, reduce4xw2xh (4.8 GB) 1854 -> 1823,
+    // reduce2xh, 4 videos 883 -> 878.  Bridges of 86 and 151 MB: 71.2 -> 71.6 and 105.9 -> 107.5, hence the line.
+    bool large_bridge() const { return (long long)nbh * na * blk.b2 * n_keys * (2 * kHeadDim * 2) > (252ll << 20); }
     void set_divs() {
         by_b2 = FastDiv::of(blk.b2); by_na = FastDiv::of(na); by_H = FastDiv::of(H);
         by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce); by_hh = FastDiv::of(blk.hh); by_out = FastDiv::of(out_tokens);

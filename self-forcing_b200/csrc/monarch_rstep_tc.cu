@@ -115,7 +115,8 @@ static_assert(sizeof(Barriers) <= 512, "barriers follow the tiles");
 // turn, and every row's logits are divided by its cR (monarch_attn.py:1716-1719).
 // kY: Y is wanted.  The passes of the iterative variant before the last need aL and cL only: their stages hold K alone, and
 // the two epilogue warpgroups take whole steps in turn, each with a 128-column accumulator of its own.
-template <int N_S, bool kCausal, bool kIter, bool kY>
+// kLarge: the bridge is much larger than L2 (MonarchParams::large_bridge).
+template <int N_S, bool kCausal, bool kIter, bool kY, bool kLarge>
 __global__ void __launch_bounds__(kThreads, 1)
 monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tal,
@@ -188,6 +189,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         // ------------------------------------------------------------------ K and query tiles
         {
             const uint32_t el = elect_one();
+            const uint64_t policy = kLarge ? l2_evict_last() : 0;
             int g = 0, uc = 0;
             for (int u = u_first; u < rp.n_units && !bars->abort_flag; u += u_stride) {
                 const RUnit un = decode_unit<kCausal>(rp, u);
@@ -202,8 +204,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                     const int tok = ((un.f_begin + i) * b1 + un.k) * b2;
                     unsigned char* st = k_s + s * kTile;
                     mbar_arrive_expect_tx_e(el, &bars->k_full[s], (uint32_t)(2 * b2 * 128));
-                    tma_load_4d_e(el, st, &tk, &bars->k_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + kHalf, &tk, &bars->k_full[s], 64, hd, tok, b);
+                    tma_load_halves_e<kLarge>(el, st, kHalf, &tk, &bars->k_full[s], hd, tok, b, policy);
                     if (!kIter && i > 0) continue;
                     // the query tile: the unit's rows of q, or this step's state rows (a, j) of (f, k), group by group
                     const int qc = kIter ? g : uc, qb = qc % kQBufs;
@@ -229,6 +230,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         // ------------------------------------------------------------------ V tiles
         if constexpr (kY) {
             const uint32_t el = elect_one();
+            const uint64_t policy = kLarge ? l2_evict_last() : 0;
             int g = 0;
             bool ok = true;
             for (int u = u_first; ok && u < rp.n_units && !bars->abort_flag; u += u_stride) {
@@ -241,8 +243,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                     const int tok = ((un.f_begin + i) * b1 + un.k) * b2;
                     unsigned char* st = v_s + s * kTile;
                     mbar_arrive_expect_tx_e(el, &bars->v_full[s], (uint32_t)(2 * b2 * 128));
-                    tma_load_4d_e(el, st, &tv, &bars->v_full[s], 0, hd, tok, b);
-                    tma_load_4d_e(el, st + kHalf, &tv, &bars->v_full[s], 64, hd, tok, b);
+                    tma_load_halves_e<kLarge>(el, st, kHalf, &tv, &bars->v_full[s], hd, tok, b, policy);
                 }
             }
         }
@@ -641,13 +642,13 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
         return launch_pdl(rp.n_units * rp.f_per <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
     };
     int rc;
-    const bool causal = p.causal_groups > 0;
+    const bool causal = p.causal_groups > 0, large = p.large_bridge();
     if (iter || !p.write_Y) {
         switch (n_s) {
-#define SFM_R_CASE(n)                                                                                                            \
-    case n:                                                                                                                      \
-        rc = iter ? (p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true>) : go(monarch_r_tc_kernel<n, false, true, false>)) \
-                  : go(monarch_r_tc_kernel<n, false, false, false>);                                                             \
+#define SFM_R_CASE(n)                                                                                                    \
+    case n:                                                                                                              \
+        rc = !iter ? go(monarch_r_tc_kernel<n, false, false, false, false>)                                              \
+             : p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true, false>) : go(monarch_r_tc_kernel<n, false, true, false, false>); \
         break;
             SFM_R_CASE(16)
             SFM_R_CASE(32)
@@ -657,8 +658,11 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
             default: return SFM_ERR_UNSUPPORTED;
         }
     } else switch (n_s) {
-#define SFM_R_CASE(n) \
-    case n: rc = causal ? go(monarch_r_tc_kernel<n, true, false, true>) : go(monarch_r_tc_kernel<n, false, false, true>); break;
+#define SFM_R_CASE(n)                                                                                                                    \
+    case n:                                                                                                                              \
+        rc = causal ? (large ? go(monarch_r_tc_kernel<n, true, false, true, true>) : go(monarch_r_tc_kernel<n, true, false, true, false>)) \
+                    : (large ? go(monarch_r_tc_kernel<n, false, false, true, true>) : go(monarch_r_tc_kernel<n, false, false, true, false>)); \
+        break;
         SFM_R_CASE(16)
         SFM_R_CASE(32)
         SFM_R_CASE(48)

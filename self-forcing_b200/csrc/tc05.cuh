@@ -216,6 +216,38 @@ __device__ __forceinline__ void tma_load_4d_e(uint32_t el, void* smem_dst, const
         ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
         "r"(el) : "memory");
 }
+// Cache policies for the copies that take one.
+__device__ __forceinline__ uint64_t l2_evict_first() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_evict_last() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tma_load_4d_hint_e(uint32_t el, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
+                                                   int c2, int c3, uint64_t policy) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.b32 e, %7, 0;\n"
+        "@e cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %8;\n}"
+        ::"r"(smem_addr(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+        "r"(el), "l"(policy) : "memory");
+}
+// Both 64-channel halves of a tile, `half` bytes apart in shared memory; with a policy or without.  (The choice is the
+// compiler's: made by the loading warps at run time it cost short launches 0.4 us.)
+template <bool kHint>
+__device__ __forceinline__ void tma_load_halves_e(uint32_t el, unsigned char* smem_dst, int half, const CUtensorMap* m, uint64_t* bar, int c1,
+                                                  int c2, int c3, uint64_t policy) {
+    if constexpr (kHint) {
+        tma_load_4d_hint_e(el, smem_dst, m, bar, 0, c1, c2, c3, policy);
+        tma_load_4d_hint_e(el, smem_dst + half, m, bar, 64, c1, c2, c3, policy);
+    } else {
+        tma_load_4d_e(el, smem_dst, m, bar, 0, c1, c2, c3);
+        tma_load_4d_e(el, smem_dst + half, m, bar, 64, c1, c2, c3);
+    }
+}
 __device__ __forceinline__ void tma_load_5d_e(uint32_t el, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
                                               int c2, int c3, int c4) {
     asm volatile(
