@@ -416,6 +416,18 @@ def test_dense_attention(sfb, n_q, n_kv):
     check_close(got, ref, f"dense {n_q}x{n_kv}")
 
 
+# keys around the 64-key halves (the second may hold none), several units per CTA, whose queries follow one another in TMEM
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_q, n_kv, H", [(1, 1, 1), (129, 63, 2), (128, 64, 1), (64, 65, 3), (257, 127, 2), (100, 128, 1), (128, 129, 2),
+                                          (128 * 20, 200, 16), (128 * 20 + 5, 385, 16)])
+def test_dense_attention_half_tiles(sfb, n_q, n_kv, H):
+    rng = np.random.default_rng(n_q * 7 + n_kv)
+    q, k, v = (bf(cases.randn(rng, 1, n, H, 128)) for n in (n_q, n_kv, n_kv))
+    got = sfb.attention(q.cuda(), k.cuda(), v.cuda())
+    sfb.ops.check_device_status()
+    check_close(got, orc.dense_attention(q.float(), k.float(), v.float()), f"{n_q} x {n_kv} x {H}")
+
+
 @pytest.mark.parametrize("i", range(len(cases.DENSE_CASES)))
 def test_dense_attention_vs_reference_fixture(sfb, i):
     """Against the reference's own attention() run through its SDPA branch in fp32 (pins_golden.npz)."""
