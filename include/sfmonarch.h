@@ -95,13 +95,16 @@ int sfm_rope_cache_write(const void* q, const void* k, const void* v, void* q_ou
  * arguments in one struct so that a binding passes a single pointer.
  *   q, k, v      [B, n_q | n_new, H, D] natural order; k, v contiguous, q too when q_rot is given, else batch stride
  *                q_batch_stride
- *   q_rot        [B, n_q, H, D]: normalised and rotated q (n_q = n_new); NULL: q is attended as it is
+ *   q_rot        [B, n_q, H, D]: normalised and rotated q (n_q = n_new), needed during the call only; NULL: q is attended as
+ *                it is.  It may lie in the same allocation as the workspace, outside the workspace_bytes given: calls that
+ *                share a workspace address launch all their kernels one call after the other
  *   rope, norm_q_weight, norm_k_weight, roll_*   as in sfm_rope_cache_write_roll; each may be NULL / 0
  *   k_cache, v_cache   the cache view [B, n_kv, H, D], batch stride cache_batch_stride; n_kv includes the new tokens
  *   out          [B, n_q, H, D] contiguous;  workspace: sfm_monarch_workspace_bytes(..., bridge_budget_mb << 20) bytes (unused
  *                when dense); bridge_budget_mb 0 = default
  * Every check comes before the first launch: a call refused with an SFM_ERR_* code has not touched the cache (nor moved its
- * tokens) and may be made again, with more scratch for instance.
+ * tokens) and may be made again, with more scratch for instance.  With SFM_CHECK_STATUS=1 in the environment the call waits
+ * for its kernels and returns SFM_ERR_DEVICE_STATUS if one gave up.
  * Replaces: the cache branch of CausalWanSelfAttention.forward between the projections
  * (wan/modules/causal_model.py:900-1103), and monarch_attn_with_kv_cache (wan/modules/monarch_attn.py:1778-1796).
  */

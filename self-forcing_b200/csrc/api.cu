@@ -199,8 +199,8 @@ int prepare_monarch(MonarchCall* mc, const void* q, int64_t q_bs, const void* kc
     return SFM_OK;
 }
 
-// The launches of a checked call.
-int launch_monarch(MonarchCall& mc) {
+// The launches of a checked call; the caller holds launch_mutex(mc.status).
+int launch_monarch_held(MonarchCall& mc) {
     const Plan& pl = mc.pl;
     MonarchParams& p = mc.p;
     CUtensorMap* maps = mc.maps;
@@ -210,7 +210,6 @@ int launch_monarch(MonarchCall& mc) {
     float* lse = mc.lse;
     int* status = mc.status;
     cudaStream_t stream = mc.stream;
-    std::lock_guard<std::mutex> lock(launch_mutex(status));       // the workspace's first word
     int rc;
     // Every path starts from a clear status word: the workspace may be recycled memory.  The tensor-core path's first
     // kernel clears it; the mma.sync kernels have no bounded waits and never write it.
@@ -270,6 +269,11 @@ int launch_monarch(MonarchCall& mc) {
         }
     }
     return SFM_OK;
+}
+
+int launch_monarch(MonarchCall& mc) {
+    std::lock_guard<std::mutex> lock(launch_mutex(mc.status));       // the workspace's first word
+    return launch_monarch_held(mc);
 }
 
 int run_monarch(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out, void* ws,
@@ -480,6 +484,9 @@ extern "C" int sfm_kv_attention(const void* call) {
                                        (cudaStream_t)c.stream, nullptr, (float*)c.lse);
     if (rc) return rc;
     const int order = c.dense ? 0 : 1;
+    // q_rot may lie in the workspace too: from the kernel that writes it on, no other call may come between
+    std::unique_lock<std::mutex> lock;
+    if (!c.dense) lock = std::unique_lock<std::mutex>(launch_mutex(mc.status));
     rc = c.roll_shift > 0 || c.norm_q_weight || c.norm_k_weight
              ? sfm_rope_cache_write_roll(c.q_rot ? c.q : nullptr, c.k, c.v, c.norm_q_weight, c.norm_k_weight, c.eps, c.q_rot,
                                          c.k_cache, c.v_cache, c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new,
@@ -488,8 +495,13 @@ extern "C" int sfm_kv_attention(const void* call) {
              : sfm_rope_cache_write(c.q_rot ? c.q : nullptr, c.k, c.v, c.q_rot, c.k_cache, c.v_cache,
                                     c.cache_batch_stride, (const float*)c.rope, c.B, c.n_new, c.H, c.D, c.start_idx,
                                     c.f_tied, c.h_reduce, c.w_reduce, c.h, c.w, c.start_frame, order, c.stream);
+    if (!rc) rc = c.dense ? launch_dense(dc, (cudaStream_t)c.stream) : launch_monarch_held(mc);
+    if (lock) lock.unlock();
     if (rc) return rc;
-    return c.dense ? launch_dense(dc, (cudaStream_t)c.stream) : launch_monarch(mc);
+    // debugging aid: waits for the call and reports what its kernels recorded
+    const char* strict = getenv("SFM_CHECK_STATUS");
+    if (!strict || strcmp(strict, "1")) return SFM_OK;
+    return c.dense ? sfm_dense_status(c.stream) : sfm_workspace_status(c.workspace, c.stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -111,16 +111,18 @@ def _workspace(device: torch.device, nbytes: int, tag: str = "monarch") -> torch
 _TIGHT_BRIDGE_MB = 1024
 
 
-def _bridge_scratch(device, sizes, num_iters) -> Tuple[torch.Tensor, int]:
-    """(scratch, budget in MiB) of a Monarch forward; sizes = (B, H, D, n_q, n_kv, *blocking).  Budget 0 is the library's
-    default; where the GPU has no memory left for that, the call is cut into chunks of _TIGHT_BRIDGE_MB (same bits)."""
+def _bridge_scratch(device, sizes, num_iters, tail=0) -> Tuple[torch.Tensor, int]:
+    """(scratch, budget in MiB) of a Monarch forward; sizes = (B, H, D, n_q, n_kv, *blocking), tail = bytes the caller wants
+    behind what the library asks for.  Budget 0 is the library's default; where the GPU has no memory left for that, the call is
+    cut into chunks of _TIGHT_BRIDGE_MB (same bits)."""
     lib = _lib.load()
     # unsupported sizes need 0 bytes: any buffer will do, the entry point names the error
-    nbytes = lib.sfm_monarch_workspace_bytes(*sizes, num_iters, 0) or 256
+    tail = tail and tail + 255                     # the library's part may be any number of bytes
+    nbytes = (lib.sfm_monarch_workspace_bytes(*sizes, num_iters, 0) or 256) + tail
     try:
         return _workspace(device, nbytes), 0
     except torch.OutOfMemoryError:
-        tight = lib.sfm_monarch_workspace_bytes(*sizes, num_iters, _TIGHT_BRIDGE_MB << 20)
+        tight = lib.sfm_monarch_workspace_bytes(*sizes, num_iters, _TIGHT_BRIDGE_MB << 20) + tail
         if tight >= nbytes:
             raise
     return _workspace(device, tight), _TIGHT_BRIDGE_MB
@@ -210,6 +212,9 @@ def _mark_written(*tensors) -> None:
     """The kernels write the caches through raw pointers, which autograd cannot see.  Bumping the version
     counters makes a later backward that saved one of these tensors fail loudly, as it does after the
     reference's slice assignment (monarch_attn.py:1230-1231), instead of using overwritten keys."""
+    if not any(t.is_inference() for t in tensors):
+        torch.autograd.graph.increment_version(tensors)
+        return
     for t in tensors:
         if not t.is_inference():                   # inference tensors carry no version counter
             torch.autograd.graph.increment_version(t)
@@ -270,17 +275,29 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
     B, n_q, H, D = q.shape
     device = q.get_device()
     stream = _raw_stream(device)
-    q_rot = torch.empty_like(q) if rope is not None else None
+    # The rotated queries live for this call only: they take the end of the scratch (a tensor of their own cost 1.3 us of host
+    # time); dense calls have no scratch.
+    q_rot, tail = 0, 0
+    if rope is not None:
+        if dense:
+            q_tmp = torch.empty_like(q)
+            q_rot = q_tmp.data_ptr()
+        else:
+            tail = -(-B * n_q * H * D * 2 // 256) * 256
     out = torch.empty_like(q) if q.is_contiguous() else torch.empty((B, n_q, H, D), dtype=q.dtype, device=q.device)
     ws = None if dense else _cached_workspace((device, stream, "monarch"))
     budget = 0
     for attempt in (0, 1):
-        if not dense and (ws is None or attempt):
-            ws, budget = _bridge_scratch(q.device, (B, H, D, n_q, n_kv, *blocking), num_iters)
+        if not dense:
+            if attempt or ws is None or ws.numel() < tail:
+                ws, budget = _bridge_scratch(q.device, (B, H, D, n_q, n_kv, *blocking), num_iters, tail)
+            ws_ptr, ws_bytes = ws.data_ptr(), (ws.numel() & -256) - tail
+            if tail:
+                q_rot = ws_ptr + ws_bytes
         call = _KV_CALL.pack(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), 0 if wq is None else wq.data_ptr(), 0 if wk is None else wk.data_ptr(),
-            0 if q_rot is None else q_rot.data_ptr(), kc_ptr, vc_ptr, 0 if rope is None else rope.data_ptr(), out.data_ptr(),
-            0 if dense else ws.data_ptr(), stream, 0 if lse is None else lse.data_ptr(), q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws.numel(),
+            q_rot, kc_ptr, vc_ptr, 0 if rope is None else rope.data_ptr(), out.data_ptr(), 0 if dense else ws_ptr, stream,
+            0 if lse is None else lse.data_ptr(), q.stride(0) if B > 1 else n_q * H * D, cache_bs, 0 if dense else ws_bytes,
             eps, sm_scale, B, H, D, n_q, k.shape[1], n_kv, start_idx, roll_dst, roll_shift, start_frame, *blocking, num_iters,
             dense, budget)
         rc = _lib.load().sfm_kv_attention(call)
@@ -291,9 +308,7 @@ def _kv_attention(q, k, v, kc_ptr, vc_ptr, cache_bs, n_kv, start_idx, blocking, 
     if rc:
         _lib.check(rc, "sfm_kv_attention")
     if not dense:
-        _after_call(ws)
-    elif os.environ.get("SFM_CHECK_STATUS") == "1":
-        _lib.check(_lib.load().sfm_dense_status(stream), "sfm_dense_status")
+        _watch_status(ws)              # SFM_CHECK_STATUS=1 is the library's to see: os.environ takes a microsecond
     return out
 
 
@@ -572,28 +587,36 @@ def layer_attention(q, k, v, k_full, v_full, cache_start, n_kv, start_idx, start
     """norm_rope_cache_write followed by attention (Monarch, or dense with the cache in natural order) over the view
     [cache_start, cache_start + n_kv) of the cache tensors ``k_full`` / ``v_full``, in one call of the library.
     ``start_idx`` and ``roll`` are relative to the view."""
-    if not (_good(q) and _good(k) and _good(v)):
+    # what _good says of each, asked with as few attribute reads as it takes (a shape is 0.2 us): equal shapes are asked once
+    if not all(isinstance(t, torch.Tensor) and t.dtype is _BF16 and t.is_cuda for t in (q, k, v, k_full, v_full)):
+        for t, name in ((q, "q"), (k, "k"), (v, "v"), (k_full, "k_cache"), (v_full, "v_cache")):
+            _require(t, name)
+    shape, cache_shape = q.shape, k_full.shape
+    same = k.shape == shape and v.shape == shape
+    if len(shape) != 4 or shape[3] != 128 or not same:
         for t, name in ((q, "q"), (k, "k"), (v, "v")):
             _require(t, name)
-    if not (_good(k_full) and _good(v_full) and k_full.is_contiguous() and v_full.is_contiguous()):
+    same_cache = v_full.shape == cache_shape
+    dense_caches = len(cache_shape) == 4 and cache_shape[3] == 128 and same_cache and k_full.is_contiguous() and v_full.is_contiguous()
+    if not dense_caches:
         _cache_view_ok(k_full, "k_cache")
         _cache_view_ok(v_full, "v_cache")
-    shape, cache_shape = q.shape, k_full.shape
     B, n, H, D = shape
-    if k.shape != shape or v.shape != shape or start_idx < 0 or start_idx + n > n_kv or cache_start + n_kv > cache_shape[1]:
+    if not same or start_idx < 0 or start_idx + n > n_kv or cache_start + n_kv > cache_shape[1]:
         raise ValueError("q, k, v shapes or the cache extent do not match")
-    cache_bs = _batch_stride(k_full)
-    if v_full.shape != cache_shape or _batch_stride(v_full) != cache_bs or cache_shape[0] != B or cache_shape[2] != H:
+    cache_bs = cache_shape[1] * cache_shape[2] * 128 if dense_caches else _batch_stride(k_full)
+    if not same_cache or not (dense_caches or _batch_stride(v_full) == cache_bs) or cache_shape[0] != B or cache_shape[2] != H:
         raise ValueError("k_cache and v_cache must share shape and strides")
     if (norm_q_weight is None) != (norm_k_weight is None):
         raise ValueError("give both norm weights or neither")
     wq = wk = None
+    device = q.device
     if norm_q_weight is not None:
-        wq, wk = _norm_weight(norm_q_weight, H * D, q.device), _norm_weight(norm_k_weight, H * D, q.device)
+        wq, wk = _norm_weight(norm_q_weight, H * D, device), _norm_weight(norm_k_weight, H * D, device)
     dst, shift = (0, 0) if roll is None else (int(roll[0]), int(roll[1]))
     if start_idx + shift > n_kv:
         raise ValueError("the eviction shift reads past the cache view")
-    tab = _rope_table_from_freqs(freqs, q.device)
+    tab = _rope_table_from_freqs(freqs, device)
     offset = cache_start * (H * D * 2)
     _mark_written(k_full, v_full)
     return _kv_attention(q.contiguous(), k.contiguous(), v.contiguous(), k_full.data_ptr() + offset, v_full.data_ptr() + offset,

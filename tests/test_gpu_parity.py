@@ -935,6 +935,37 @@ def test_threads_may_share_a_stream(sfb):
 
 
 @pytest.mark.gpu
+def test_layer_calls_of_threads_that_share_a_stream(sfb):
+    """The rotated queries of a layer call lie at the end of the stream's scratch: calls of different sizes from two threads
+    do not come between each other's cache write and attention."""
+    import threading
+    from self_forcing_b200 import ops
+    work = []
+    for seed, H in ((21, 1), (22, 3)):
+        c = small_case(0, 1, B=1, H=H, seed=seed)
+        h, w = c["blocking"][3:]
+        args = (c["q"].cuda(), c["nk"].cuda(), c["nv"].cuda(), c["kbuf"].cuda(), c["vbuf"].cuda(), 0, c["n_kv"], c["start"], 6, 1, 1, 1, h, w)
+        work.append((args, ops.layer_attention(*args)))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def repeat(args, out):
+        try:
+            for _ in range(300):
+                if not torch.equal(ops.layer_attention(*args), out):
+                    wrong.append("out")
+        except Exception as e:
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=repeat, args=x) for x in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, (len(wrong), set(wrong))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bound", ["count", "bytes"])
 def test_least_recently_used_workspace_is_dropped(sfb, monkeypatch, bound):
     """Scratch kept for two streams at most, by count or by bytes: a stream that has just been used keeps its buffer, the
