@@ -159,7 +159,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         bars->abort_flag = 0;
         mbar_init_fence();
     }
-    // The copies bring the b2 rows of a block and no more (64 of every 52 rows were 20 % of what the kernel read); the GEMMs
+    // The copies bring the b2 rows of a block and no more (64 for every 52 were 20 % of what the TMA engine loaded); the GEMMs
     // read N_S, with weight zero past b2: those rows must hold finite numbers.
     for (int i = tid; i < (kKStg + kVStg) * 2 * (N_S - b2) * 8; i += kThreads) {
         const int r = i >> 3, h = r / (N_S - b2);
