@@ -284,8 +284,6 @@ __device__ __forceinline__ void tma_store_4d_e(uint32_t el, const CUtensorMap* m
 }
 // Bulk-group bookkeeping is per thread: lanes that issued nothing have nothing to commit or wait for.
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// At most one store's staging is still unread: with two buffers in turn, the next one to be filled is free.
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // No store's staging is still unread.
 __device__ __forceinline__ void tma_store_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
