@@ -1,6 +1,7 @@
 // Launch accounting and optional per-kernel timing (CUDA events on the launching stream).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <mutex>
 
@@ -23,6 +24,14 @@ int device_sms();
 int opt_in_smem(const void* kernel, int bytes);
 // Held while a call's kernels are launched: they pass their results through its workspace, so the launches of two threads
 // that share one (and a stream) must not mix.  A few mutexes serve all workspaces.
+constexpr int kLaunchMutexes = 64;
+// Which of them an address has.  Large buffers start on 2 MiB boundaries, and those of several streams or GPUs lie a multiple
+// of that apart: the bits that tell them from one another, 21 and up, all have to count (multiplicative hashing, Knuth,
+// vol. 3, 6.4), or threads that share nothing would wait for one another.
+constexpr int launch_slot(uint64_t address) {
+    const uint64_t x = address >> 8;                   // workspaces are aligned to 256 bytes
+    return (int)(((x ^ (x >> 32)) * 0x9E3779B97F4A7C15ull) >> 58);
+}
 std::mutex& launch_mutex(const void* workspace);
 
 // Launch as a programmatic dependent of the kernel before it in the stream: the grid may be set up while that one

@@ -43,8 +43,8 @@ int opt_in_smem(const void* kernel, int bytes) {
 }
 
 std::mutex& launch_mutex(const void* workspace) {
-    static std::mutex mutexes[64];
-    return mutexes[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
+    static std::mutex mutexes[kLaunchMutexes];
+    return mutexes[launch_slot(reinterpret_cast<uintptr_t>(workspace))];
 }
 
 EncodeTiledFn get_encode_tiled() {

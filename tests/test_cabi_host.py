@@ -197,6 +197,24 @@ def test_layer_call_is_refused_before_its_cache_write(sfb, field, value, rc):
     assert _lib.load().sfm_kv_attention(ops._KV_CALL.pack(*call.values())) == rc
 
 
+def test_workspaces_take_different_launch_mutexes(tmp_path):
+    """Eight workspaces, as many as the Python layer keeps, on the boundaries that large allocations have, any usual distance
+    apart: at most two pairs of them share a launch mutex."""
+    import subprocess
+    from self_forcing_b200 import build
+    strides = [512, 2 << 20, 20 << 20, 64 << 20, 606 << 20, 1 << 30, 2 << 30, 4 << 30, 32 << 30]
+    src = tmp_path / "slots.cu"
+    src.write_text('#include "profile.cuh"\n#include <cstdio>\nint main() {\n    unsigned long long a;\n'
+                   '    while (scanf("%llu", &a) == 1) printf("%d\\n", sfm::launch_slot(a));\n}\n')
+    exe = tmp_path / "slots"
+    subprocess.check_call([build.nvcc_path(), "-std=c++17", f"-I{build.CSRC}", "-o", str(exe), str(src)])
+    starts = [base + i * stride for stride in strides for base in (0x7f0000000000, 0x7fd2e0000000, 0x302000000) for i in range(8)]
+    out = subprocess.run([str(exe)], input="\n".join(map(str, starts)), capture_output=True, text=True, check=True).stdout
+    slots = np.array(out.split(), dtype=int).reshape(-1, 8)
+    assert slots.min() >= 0 and slots.max() < 64
+    assert min(len(set(row)) for row in slots.tolist()) >= 6, slots
+
+
 def test_plan_cache_step_equals_oracle(sfb):
     """The product's cache bookkeeping against the oracle's restatement of causal_model.py:907-938,
     over a random walk of rollouts with and without a sliding window (integers: exact)."""
