@@ -302,10 +302,12 @@ def test_monarch_iterative_widths(sfb, edge):
     check_close(got, ref, str(edge))
 
 
-# (h, w, f_tied, h_reduce, w_reduce, frames cached): 128 and 129 keys (one tile, two tiles), block rows of 16 to 120, query
-# rows that are gathered
+# (h, w, f_tied, h_reduce, w_reduce, frames cached): 128 and 129 keys (one tile, two tiles), block rows at both edges of every
+# width that the state update is built for (16, 32, ... 128), query rows that are gathered
 @pytest.mark.parametrize("edge", [(32, 8, 1, 1, 1, 4), (43, 8, 1, 1, 1, 3), (16, 16, 1, 1, 1, 8), (40, 6, 3, 1, 1, 3), (20, 8, 3, 2, 1, 3),
-                                  (3, 8, 1, 1, 1, 3)], ids=lambda e: "h{}w{}_ft{}hr{}wr{}_F{}".format(*e))
+                                  (3, 8, 1, 1, 1, 3), (49, 5, 1, 1, 1, 3), (64, 4, 1, 1, 1, 3), (65, 4, 1, 1, 1, 3), (80, 4, 1, 1, 1, 3),
+                                  (81, 4, 1, 1, 1, 3), (96, 4, 1, 1, 1, 3), (97, 4, 1, 1, 1, 3), (112, 4, 1, 1, 1, 3),
+                                  (17, 6, 3, 1, 1, 3), (22, 6, 3, 1, 1, 3), (31, 4, 3, 1, 1, 3), (37, 4, 3, 1, 1, 3)], ids=lambda e: "h{}w{}_ft{}hr{}wr{}_F{}".format(*e))
 def test_monarch_iterative_tile_edges(sfb, edge):
     h, w, ft, hr, wr, frames = edge
     rng = np.random.default_rng(h * 1000 + w)
@@ -385,6 +387,32 @@ def test_block_causal_unit_groups(sfb, grid):
     q, k, v = (bf(cases.randn(rng, 2, frames * h * w, 3, 128)) for _ in range(3))
     got = sfb.monarch_attn(q.cuda(), k.cuda(), v.cuda(), 1, 1, 1, h, w, block_causal_size=3 * h * w)
     check_close(got, orc.monarch_attn(q.float(), k.float(), v.float(), 1, 1, 1, h, w, block_causal_size=3 * h * w), str(grid))
+
+
+# block columns at both edges of every width that the row step is built for (16, 32, ... 128), its tiles filled or not
+@pytest.mark.parametrize("w", [17, 32, 33, 48, 49, 52, 64, 65, 80, 81, 96, 97, 112, 113, 128])
+def test_block_causal_widths(sfb, w):
+    rng = np.random.default_rng(9000 + w)
+    h, frames = 7, 9
+    q, k, v = (bf(cases.randn(rng, 1, frames * h * w, 2, 128)) for _ in range(3))
+    got = sfb.monarch_attn(q.cuda(), k.cuda(), v.cuda(), 1, 1, 1, h, w, block_causal_size=3 * h * w)
+    check_close(got, orc.monarch_attn(q.float(), k.float(), v.float(), 1, 1, 1, h, w, block_causal_size=3 * h * w), f"w{w}")
+
+
+# As many heads as it takes for a bridge just above 252 MiB, where both steps give cache hints; heads do not see each other, so the
+# first and the last are compared
+@pytest.mark.parametrize("causal", [False, True], ids=["all", "causal"])
+@pytest.mark.parametrize("w", [13, 32, 44, 52, 76, 96, 104, 128])
+def test_bridges_larger_than_l2(sfb, w, causal):
+    h, frames = 12, 12
+    H = (252 << 20) // (frames * frames * h * w * 512) + 1
+    g = torch.Generator(device="cuda").manual_seed(w)
+    q, k, v = (torch.randn(1, frames * h * w, H, 128, device="cuda", generator=g).bfloat16() for _ in range(3))
+    size = 3 * h * w if causal else None
+    got = sfb.monarch_attn(q, k, v, 1, 1, 1, h, w, block_causal_size=size)
+    hs = [0, H - 1]
+    ref = orc.monarch_attn(*(t[:, :, hs].float().cpu() for t in (q, k, v)), 1, 1, 1, h, w, block_causal_size=size)
+    check_close(got[:, :, hs], ref, f"w{w} H{H}")
 
 
 @pytest.mark.parametrize("ci", range(4))
@@ -935,24 +963,36 @@ def test_threads_may_share_a_stream(sfb):
 
 
 @pytest.mark.gpu
-def test_layer_calls_of_threads_that_share_a_stream(sfb):
-    """The rotated queries of a layer call lie at the end of the stream's scratch: calls of different sizes from two threads
-    do not come between each other's cache write and attention."""
+@pytest.mark.parametrize("other", ["layer", "clip", "with_cache", "on_cache", "iterative", "backward"])
+def test_layer_calls_of_threads_that_share_a_stream(sfb, other):
+    """The rotated queries of a layer call lie at the end of the stream's scratch, where calls of other threads may keep what
+    passes between their kernels: nothing comes between a call's launches."""
     import threading
     from self_forcing_b200 import ops
-    work = []
-    for seed, H in ((21, 1), (22, 3)):
-        c = small_case(0, 1, B=1, H=H, seed=seed)
-        h, w = c["blocking"][3:]
-        args = (c["q"].cuda(), c["nk"].cuda(), c["nv"].cuda(), c["kbuf"].cuda(), c["vbuf"].cuda(), 0, c["n_kv"], c["start"], 6, 1, 1, 1, h, w)
-        work.append((args, ops.layer_attention(*args)))
+    c = small_case(0, 1, B=1, H=1, seed=21)
+    h, w = c["blocking"][3:]
+    layer = lambda c: (c["q"].cuda(), c["nk"].cuda(), c["nv"].cuda(), c["kbuf"].cuda(), c["vbuf"].cuda(), 0, c["n_kv"], c["start"], 6,
+                       1, 1, 1, h, w)
+    args, d = layer(c), small_case(0, 1, B=1, H=3, seed=22)
+    q, nk, nv = d["q"].cuda(), d["nk"].cuda(), d["nv"].cuda()
+    kc, vc = (d[n].cuda()[:, :d["n_kv"]].contiguous() for n in ("kbuf", "vbuf"))
+    d_args = layer(d)
+    beside = {
+        "layer": lambda: ops.layer_attention(*d_args),
+        "clip": lambda: sfb.monarch_attn(kc, vc, kc, *d["blocking"], block_causal_size=q.shape[1]),
+        "with_cache": lambda: sfb.monarch_attn_with_kv_cache(q, kc, vc, nk, nv, d["start"], d["end"], *d["blocking"]),
+        "on_cache": lambda: ops.monarch_attention_on_cache(q, kc, vc, *d["blocking"]),
+        "iterative": lambda: ops.monarch_attention_on_cache(q, kc, vc, *d["blocking"], num_iters=3),
+        "backward": lambda: ops.monarch_attn_with_kv_cache_backward(q, kc, vc, q, *d["blocking"])[0],
+    }[other]
+    work = [(call, call()) for call in (lambda: ops.layer_attention(*args), beside)]
     torch.cuda.synchronize()
     wrong = []
 
-    def repeat(args, out):
+    def repeat(call, out):
         try:
             for _ in range(300):
-                if not torch.equal(ops.layer_attention(*args), out):
+                if not torch.equal(call(), out):
                     wrong.append("out")
         except Exception as e:
             wrong.append(repr(e))
