@@ -292,8 +292,8 @@ namespace sfm {
 // Single-pass forward on the tensor-core kernels for the (batch, head) pairs [bh0, bh0 + nbh) with all query
 // groups at once, into caller-given bridge buffers (aL, Y: bf16 [bh_local * A + a][n_keys][b2][128], cL: fp32 [slab][n_keys_c],
 // slab = (bh_local * A + a) * b2 + j) and, optionally, the column step's log-sum-exp per query row
-// (lse: fp32 [slab][b1]); without `column` the row step only.  The backward uses it to recompute what the forward did not keep.  Returns the launch
-// parameters and the tensor maps of q, K, V and the query rows for the kernels that follow.
+// (lse: fp32 [slab][b1]); without `column` the row step only.  The backward uses it to recompute what the forward did not
+// keep.  Returns the launch parameters and the tensor maps of q, K, V and the query rows for the kernels that follow.
 int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc, int64_t c_bs, void* out,
                      __nv_bfloat16* aL, __nv_bfloat16* Y, float* cL, float* lse, int* status, int B, int H, int n_q,
                      int n_kv, const Blocking& blk, float scale, int bh0, int nbh, bool column, MonarchParams* p_out,

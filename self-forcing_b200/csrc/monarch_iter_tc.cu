@@ -25,7 +25,10 @@
 // tile, of which the TMA engine stores for 800; with longer caches the aR rows, 256 bytes per key a whole (query group,
 // column) set apart.  20 passes over a 4680-token chunk, 12 heads: the update took 40 us with one loading warp, one issuer
 // and the log-sum-exps from a pass of the column step, 27 with those taken from the tile in two sweeps over it (892 us in
-// all), 23 now (810).  A second drain warpgroup: nothing.
+// all), 23 now (810; by events, which keep launches apart: in the call an update takes some 18).  Calls of 8 passes, with two
+// working warpgroups and run-time divisions and now: 16 rows 271 -> 229 us, 30 rows 414 -> 341; above 32 queries, where 8 bytes a
+// thread spill, 40 rows 435 -> 380, 64 rows 301 -> 252, 96 rows 227 -> 199, 128 rows 281 -> 242; several tiles, 64 rows, 4 passes
+// 764 -> 682 (the row step's part of it included).  A second drain warpgroup: nothing.
 #include "monarch_params.cuh"
 #include "profile.cuh"
 #include "tc05.cuh"
@@ -466,7 +469,8 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel, int threads, int smem) -> int {
         if (int rc = opt_in_smem((const void*)kernel, smem)) return rc;
-        return launch_pdl((long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms, kernel, grid, threads, smem, s, map_al, *map_qrows, map_ar, ip);
+        const bool is_short = (long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms;
+        return launch_pdl(is_short, kernel, grid, threads, smem, s, map_al, *map_qrows, map_ar, ip);
     };
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {

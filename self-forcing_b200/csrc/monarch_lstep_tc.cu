@@ -20,10 +20,10 @@
 // whole warps with an elected issuing lane.  With one buffer of query rows, warp 2 reloads it as soon as its last S GEMM
 // of a group has completed, which the softmax and PV GEMMs of that group cover, while warp 0 is already loading the next
 // group's keys; groups of few tiles have two.  The code is kept small: a short launch fetches it from L2 or DRAM as it goes (a
-// second copy of the query load cost the first chunk 2 us).  All roles meet only through mbarriers with bounded waits; a timeout records a status code and the CTA
-// unwinds.
+// second copy of the query load cost the first chunk 2 us).  All roles meet only through mbarriers with bounded waits; a timeout
+// records a status code and the CTA unwinds.
 //
-// What bounds it: reading the bridge (604 MB in 0.114 ms at framewise, 21 cached frames, 12 heads: 5.4 TB/s with the start-up
+// What bounds it: reading the bridge (604 MB in 0.111 ms at framewise, 21 cached frames, 12 heads: 5.4 TB/s with the start-up
 // and the uneven last round, 6.3 in between; a bare TMA stream of the same tiles reaches 6.5), and at short caches, whose
 // bridge is in L2, the chain of a group (90 keys: 43 -> 29 us).  Against the form with queries spread over the four lane
 // quadrants, MMAs issued from one-lane code, two softmax passes and a warpgroup chosen by tile parity within the group:
@@ -537,7 +537,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
             if (row_ok) {
                 const LUnit un = decode_unit(p, u0 + us);
                 int hd;
-                    const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
+                const int b = p.by_H.divmod(p.bh0 + un.bhl, hd);
                 int col;
                 const int frow = p.first_row(un.al, un.j, col) + p.row_ahead(i_row);
                 out_row = p.out_row(b, frow * blk.w + col, hd);
@@ -621,8 +621,10 @@ int launch_l_step_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     lp.kt = l_tile_keys(p);
     // A value tile stays until its softmax and GEMM are done, a key tile only until its GEMM: two slots of five for keys
     // Two query tiles where a group has few tiles: its rows take 2000 to 4000 cycles to arrive, which the GEMMs and softmax of a
-    // longer group cover, whose rings need the room (first chunk 73.2 -> 71.8 us a call, tied3frame 106.3 -> 101.1 with one tile of
-    // four units, three of one; with 24 of eight units the column step went from 350 to 367).
+    // longer group cover, whose rings need the room.  Calls with one and with two, by tiles times units a group: 4 (first chunk)
+    // 72.6 -> 71.0 us, 3 (tied3frame, 9 and 12 frames) 89.3 -> 85.8 and 109.5 -> 104.5; 8 (two tiles, 6 frames, 5 and 12 heads) 58.7
+    // -> 60.0 and 110.2 -> 112.5; 24 (reduce2xh, 9 frames, 4 videos) 858 -> 873.  Groups of one or two units would gain up to six
+    // tiles: tied3frame, 21 frames 162.5 -> 158.7, 45 x 80 tokens, 6 frames 314.5 -> 312.8.
     lp.n_q = lp.U * ((p.n_keys + lp.kt - 1) / lp.kt) <= 4 ? 2 : 1;
     const int slots = (kTiles - lp.n_q * kQBytes) / (lp.kt * 256);
     lp.n_a = (slots * 2 + 4) / 5 < kMaxStages ? (slots * 2 + 4) / 5 : kMaxStages;

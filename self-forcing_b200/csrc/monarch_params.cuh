@@ -49,12 +49,19 @@ struct MonarchParams {
 
     // The chunk's bridge is more than twice what L2 holds: the column step then reads most of it from DRAM, and what it has read
     // should leave L2 before what it has not; K and V, which a tile of query groups reads a few microseconds after the other,
-    // should stay.  12 heads, 21 frames (604 MB) 317 -> 310 us a call, 12 frames 214 -> 210, reduce4xw2xh (4.8 GB) 1854 -> 1823,
-    // reduce2xh, 4 videos 883 -> 878.  Bridges of 86 and 151 MB: 71.2 -> 71.6 and 105.9 -> 107.5, hence the line.
+    // should stay.  Calls without and with the hints, framewise: 604 MB (12 heads, 21 frames) 317.1 -> 304.9 us, 345 MB 197.2 ->
+    // 191.7, 302 MB 184.3 -> 179.0, 288 MB 174.4 -> 167.7 (all the column step's); reduce4xw2xh (4.8 GB) 1856 -> 1822, reduce2xh, 4
+    // videos (2 GB) 889 -> 871 (all the row step's); block-causal clips and block columns above 64: 1.2 % slower to 3 % faster.
+    // Below the line it depends on more than the size: 86, 201 and 230 MB framewise the same, tied3frame 115 and 201 MB 104.6 ->
+    // 106.5 and 162.5 -> 165.2, 45 x 80 tokens 199 MB 170.5 -> 173.3, but few heads with long caches faster (5 heads, 21 frames,
+    // 252 MB 146.4 -> 136.7; 6 heads, 12 frames, 173 MB 105.2 -> 99.7): the line is where hardly a call gets slower.  With the
+    // model's own GEMMs between the calls (8 layers' weights and caches in turn) the hints keep their gain: 717 -> 710 us a layer at
+    // 21 frames, 594 -> 585 at 12, 40 heads the same.
     bool large_bridge() const { return (long long)nbh * na * blk.b2 * n_keys * (2 * kHeadDim * 2) > (252ll << 20); }
     void set_divs() {
         by_b2 = FastDiv::of(blk.b2); by_na = FastDiv::of(na); by_H = FastDiv::of(H);
-        by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce); by_hh = FastDiv::of(blk.hh); by_out = FastDiv::of(out_tokens);
+        by_gpt = FastDiv::of(blk.gpt); by_wr = FastDiv::of(blk.w_reduce); by_hh = FastDiv::of(blk.hh);
+        by_out = FastDiv::of(out_tokens);
     }
     // Row of the token grid, and column there, of the first token of (query group a0 + al, column j).
     __device__ __forceinline__ int first_row(int al, int j, int& col) const {

@@ -20,12 +20,13 @@
 //
 // What bounds it: the bridge rows it writes, 512 bytes per (query row, cached group, block row).  An SM's TMA engine stores 29
 // bytes a cycle at most (loads 82 with all SMs at it, 125 alone) and does one thing at a time, so a step of 104 rows takes 1840
-// cycles for its stores and 210 for its K and V; at long caches DRAM takes them at 5.5 TB/s beside what is read (a bare stream
-// of the same boxes 6.4).  Written by the epilogue threads themselves, a row a lane or four rows an instruction, they go out
+// cycles for its stores and 210 for its K and V; at long caches DRAM takes 5.1 TB/s of stores and what is read beside them (a bare
+// stream of the same boxes 6.4).  Written by the epilogue threads themselves, a row a lane or four rows an instruction, they go out
 // slower (first chunk 33 -> 39 us), and K / V by cp.async instead do not help (31 -> 35).
 // The epilogue's hand-over of an accumulator comes before its stores, aL and Y each have their own, and the working
 // warpgroups have 104 registers instead of 96 (a few dozen spilled bytes a thread go through an L1 that is all shared memory:
-// 160 -> 190 us).  framewise, 21 cached frames, 12 heads 0.167 -> 0.158 ms; reduce2xh, 9 frames, 4 videos 0.527 -> 0.490;
+// 160 -> 190 us; the block-causal instance for 49 to 64 columns still spills 48 bytes, those for 80 and 112 columns 68).  framewise,
+// 21 cached frames, 12 heads 0.167 -> 0.158 ms; reduce2xh, 9 frames, 4 videos 0.527 -> 0.490;
 // reduce4xw2xh, 21 frames 1.15 -> 1.09; a pass of the iterative variant, first chunk, 31.7 -> 25.4 us.
 // Tried and slower: results to TMA as 5-D boxes of both halves (158 -> 179 us), three staging buffers a warp (same), all
 // columns to registers before the first is stored, two tiles' queries against one K / V tile, L2 prefetch of the K / V tiles.
@@ -63,7 +64,6 @@ struct RTcParams {
     int* status;           // device status word (0 = ok)
     int clear_status;      // the call's first launch starts it from zero
 };
-
 
 struct RUnit {
     int bhl, tile, k, f_begin, n_it;
@@ -139,7 +139,10 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     constexpr int kQBufs = kWide ? 1 : (kIter && !kY ? 3 : 2);
     // A K tile stays from its S GEMM to its PV GEMM, two to three steps later, a V tile for its PV GEMM only.  21 frames, 12 heads,
     // 52 columns, K / V slots of 16 KB: 3 / 1 195 us, 3 / 2 162, 4 / 2 159, 4 / 4 162, 5 / 3 171: copies share the TMA engine
-    // with the result stores, and those asked for earlier than needed hold them up.
+    // with the result stores, and those asked for earlier than needed hold them up.  Other slot sizes, whole calls with 3 / 2,
+    // 4 / 2, 4 / 3 slots: 30 columns (8 KB), 3 frames 41, 38, 38 us; 32 columns, 21 frames 168, 168, 171; 46 columns (12 KB), 12
+    // frames 165, 161, 158; 16 columns (4 KB), 40 heads, 3 frames 71, 64, 64, 21 frames 308, 305, 292.  Above 64 columns room for
+    // two or three K slots is all there is (3 / 3 instead of 4 / 2 at 52: first chunk 62 -> 65, block-causal clip 470 -> 487).
     constexpr int kSlots = (kSmemData - kQBufs * kQBytes - kOutBytes) / kTile;
     constexpr int kVStg = kY ? kVStages : 0, kKStg = kSlots - kVStg < kKStages ? kSlots - kVStg : kKStages;
     static_assert(kKStg >= 2 && kQBufs <= kMaxQBufs, "K ring, query tiles");
@@ -598,7 +601,6 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 
 }  // namespace
 
-
 // Launches the tensor-core row step for one chunk as a persistent grid.  `status` is a device int the
 // kernel sets on an internal timeout.
 int l_tile_keys(const MonarchParams& p);
@@ -626,7 +628,8 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
         }
     }
     rp.n_units = p.nbh * rp.tiles * p.blk.b1 * rp.fsplit;
-    rp.by_fsplit = FastDiv::of(rp.fsplit); rp.by_b1 = FastDiv::of(p.blk.b1); rp.by_tiles = FastDiv::of(rp.tiles); rp.by_H = FastDiv::of(p.H);
+    rp.by_fsplit = FastDiv::of(rp.fsplit); rp.by_b1 = FastDiv::of(p.blk.b1);
+    rp.by_tiles = FastDiv::of(rp.tiles); rp.by_H = FastDiv::of(p.H);
     rp.status = status;
     rp.clear_status = clear_status;
     dim3 grid(rp.n_units < num_sms ? rp.n_units : num_sms);
@@ -635,20 +638,23 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
     const int smem_bytes = kSmemBytes;
     // result stores: one box = the 128 channels of up to 32 columns of one key
     CUtensorMap out_maps[2];
+    const int box_cols = rp.rows_per_group < 32 ? rp.rows_per_group : 32;
     for (int i = 0; i < 2; ++i)
-        if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, rp.rows_per_group < 32 ? rp.rows_per_group : 32, 1)) return rc;
+        if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, box_cols, 1)) return rc;
     auto go = [&](auto kernel) -> int {
         if (int rc = opt_in_smem((const void*)kernel, smem_bytes)) return rc;
-        return launch_pdl(rp.n_units * rp.f_per <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, maps[0], maps[1], maps[2], out_maps[0], out_maps[1], rp);
+        return launch_pdl(rp.n_units * rp.f_per <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, maps[0], maps[1], maps[2],
+                          out_maps[0], out_maps[1], rp);
     };
     int rc;
     const bool causal = p.causal_groups > 0, large = p.large_bridge();
     if (iter || !p.write_Y) {
         switch (n_s) {
-#define SFM_R_CASE(n)                                                                                                    \
-    case n:                                                                                                              \
-        rc = !iter ? go(monarch_r_tc_kernel<n, false, false, false, false>)                                              \
-             : p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true, false>) : go(monarch_r_tc_kernel<n, false, true, false, false>); \
+#define SFM_R_CASE(n)                                                                           \
+    case n:                                                                                     \
+        rc = !iter       ? go(monarch_r_tc_kernel<n, false, false, false, false>)               \
+             : p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true, false>)                 \
+                         : go(monarch_r_tc_kernel<n, false, true, false, false>);               \
         break;
             SFM_R_CASE(16)
             SFM_R_CASE(32)
@@ -657,22 +663,26 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (or th
 #undef SFM_R_CASE
             default: return SFM_ERR_UNSUPPORTED;
         }
-    } else switch (n_s) {
-#define SFM_R_CASE(n)                                                                                                                    \
-    case n:                                                                                                                              \
-        rc = causal ? (large ? go(monarch_r_tc_kernel<n, true, false, true, true>) : go(monarch_r_tc_kernel<n, true, false, true, false>)) \
-                    : (large ? go(monarch_r_tc_kernel<n, false, false, true, true>) : go(monarch_r_tc_kernel<n, false, false, true, false>)); \
+    } else {
+        switch (n_s) {
+#define SFM_R_CASE(n)                                                                           \
+    case n:                                                                                     \
+        rc = causal ? (large ? go(monarch_r_tc_kernel<n, true, false, true, true>)              \
+                             : go(monarch_r_tc_kernel<n, true, false, true, false>))            \
+                    : (large ? go(monarch_r_tc_kernel<n, false, false, true, true>)             \
+                             : go(monarch_r_tc_kernel<n, false, false, true, false>));          \
         break;
-        SFM_R_CASE(16)
-        SFM_R_CASE(32)
-        SFM_R_CASE(48)
-        SFM_R_CASE(64)
-        SFM_R_CASE(80)
-        SFM_R_CASE(96)
-        SFM_R_CASE(112)
-        SFM_R_CASE(128)
+            SFM_R_CASE(16)
+            SFM_R_CASE(32)
+            SFM_R_CASE(48)
+            SFM_R_CASE(64)
+            SFM_R_CASE(80)
+            SFM_R_CASE(96)
+            SFM_R_CASE(112)
+            SFM_R_CASE(128)
 #undef SFM_R_CASE
-        default: return SFM_ERR_UNSUPPORTED;
+            default: return SFM_ERR_UNSUPPORTED;
+        }
     }
     if (rc) return rc;
     return (int)cudaGetLastError();
