@@ -54,7 +54,6 @@ struct ItParams {
     int n_units;       // nbh * na * b2
     int q_rows_tma;    // query rows of a unit are consecutive rows of the token grid
     FastDiv by_tiles;  // tiles per unit
-    int own_lse;       // one tile per unit: the queries' log-sum-exps are taken from it
     int* status;
 };
 
@@ -111,7 +110,10 @@ __device__ __forceinline__ ItUnit it_decode(const MonarchParams& p, int u) {
 
 // tal = bridge aL map (box 64 x 1 column x 128 keys), tqr = query rows (5-D, box of b1 rows), tar = state aR
 // [bh][key][query group, column][128] (box 64 x 1 x 32 keys).
-template <int N_I>
+// kOwnLse: one tile per unit, the queries' log-sum-exps are taken from it.  An instance for each: with the choice at run time the
+// tiles of longer caches paid for the kept exponentials (24 bytes a thread spilled; 30 rows, 6 / 12 / 21 frames 34.2 / 71.1 / 122
+// -> 33.0 / 68.6 / 120 us an update).
+template <int N_I, bool kOwnLse>
 __global__ void __launch_bounds__(it_threads(N_I), 1)
 monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_constant__ CUtensorMap tqr,
                        const __grid_constant__ CUtensorMap tar, ItParams ip) {
@@ -190,13 +192,13 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             unsigned char* qd_s = q_s + qb * kQTile;
             constexpr int kL = (N_I + 31) / 32;
             float l2[kL];
-            if (!ip.own_lse) {
+            if constexpr (!kOwnLse) {
 #pragma unroll
                 for (int c = 0; c < kL; ++c)
                     l2[c] = c * 32 + lane < b1 ? kLog2e * p.lse[(long long)u * b1 + c * 32 + lane] : INFINITY;
             }
             if (!mbar_wait_u(&bars->q_empty[qb], ph)) { fail(10); break; }
-            if (!ip.own_lse) {
+            if constexpr (!kOwnLse) {
 #pragma unroll
                 for (int c = 0; c < kL; ++c)
                     if (c * 32 + lane < N_I) bars->lse2[qb][c * 32 + lane] = l2[c];
@@ -306,7 +308,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             const float sum = column_sums(v, lane);
             if (lane < 16) bars->part[w][quad][c0 + lane] = make_float2(m, sum);
         };
-        constexpr bool kKeep = N_I <= 32;                       // the exponentials stay in registers meanwhile
+        constexpr bool kKeep = kOwnLse && N_I <= 32;            // the exponentials stay in registers meanwhile
         float cl_next = load_cl(w);
         for (int g = w; g < total && !bars->abort_flag; g += NW) {
             const int uc = ip.by_tiles.div(g), t = g - uc * n_tiles;
@@ -319,8 +321,7 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
             tc_fence_after();
             const float* lse2 = bars->lse2[uc % NQ];
             float csum = 0.f;
-            bool done = false;
-            if (ip.own_lse) {
+            if constexpr (kOwnLse) {
                 float e[kKeep ? N_I / 16 : 1][16];
                 if constexpr (kKeep) {
 #pragma unroll
@@ -356,12 +357,11 @@ monarch_iter_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_con
                         }
                         tmem_st8(s_t + (c0 >> 1), pk);
                     }
-                    done = true;
                 } else {
                     lse2 = own;
                 }
             }
-            if (!done) {
+            if constexpr (!kKeep) {
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_I; c0 += 16) {
                     uint32_t r[16], pk[8];
@@ -464,7 +464,6 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
     CUtensorMap map_ar;
     if (int rc = make_bridge_tmap(&map_ar, p.aR, p.na * p.blk.b2, p.n_keys, p.nbh, 1, 32)) return rc;
     ip.q_rows_tma = (p.blk.f_tied == 1 || p.blk.h_reduce == 1) ? 1 : 0;
-    ip.own_lse = l_iter_own_lse(p);
     ip.status = status;
     dim3 grid(ip.n_units < num_sms ? ip.n_units : num_sms);
     auto go = [&](auto kernel, int threads, int smem) -> int {
@@ -472,16 +471,23 @@ int launch_l_iter_tc(const MonarchParams& p, const CUtensorMap* map_qrows, int* 
         const bool is_short = (long long)ip.n_units * p.n_keys <= 64ll * kKTile * num_sms;
         return launch_pdl(is_short, kernel, grid, threads, smem, s, map_al, *map_qrows, map_ar, ip);
     };
+    const bool own = l_iter_own_lse(p);
     int rc;
     switch ((p.blk.b1 + 15) & ~15) {
-        case 16: rc = go(monarch_iter_tc_kernel<16>, it_threads(16), it_smem_bytes<16>()); break;
-        case 32: rc = go(monarch_iter_tc_kernel<32>, it_threads(32), it_smem_bytes<32>()); break;
-        case 48: rc = go(monarch_iter_tc_kernel<48>, it_threads(48), it_smem_bytes<48>()); break;
-        case 64: rc = go(monarch_iter_tc_kernel<64>, it_threads(64), it_smem_bytes<64>()); break;
-        case 80: rc = go(monarch_iter_tc_kernel<80>, it_threads(80), it_smem_bytes<80>()); break;
-        case 96: rc = go(monarch_iter_tc_kernel<96>, it_threads(96), it_smem_bytes<96>()); break;
-        case 112: rc = go(monarch_iter_tc_kernel<112>, it_threads(112), it_smem_bytes<112>()); break;
-        case 128: rc = go(monarch_iter_tc_kernel<128>, it_threads(128), it_smem_bytes<128>()); break;
+#define SFM_IT_CASE(n)                                                                              \
+    case n:                                                                                         \
+        rc = own ? go(monarch_iter_tc_kernel<n, true>, it_threads(n), it_smem_bytes<n>())           \
+                 : go(monarch_iter_tc_kernel<n, false>, it_threads(n), it_smem_bytes<n>());         \
+        break;
+        SFM_IT_CASE(16)
+        SFM_IT_CASE(32)
+        SFM_IT_CASE(48)
+        SFM_IT_CASE(64)
+        SFM_IT_CASE(80)
+        SFM_IT_CASE(96)
+        SFM_IT_CASE(112)
+        SFM_IT_CASE(128)
+#undef SFM_IT_CASE
         default: return SFM_ERR_UNSUPPORTED;
     }
     if (rc) return rc;

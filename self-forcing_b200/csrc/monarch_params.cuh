@@ -56,7 +56,8 @@ struct MonarchParams {
     // 106.5 and 162.5 -> 165.2, 45 x 80 tokens 199 MB 170.5 -> 173.3, but few heads with long caches faster (5 heads, 21 frames,
     // 252 MB 146.4 -> 136.7; 6 heads, 12 frames, 173 MB 105.2 -> 99.7): the line is where hardly a call gets slower.  With the
     // model's own GEMMs between the calls (8 layers' weights and caches in turn) the hints keep their gain: 717 -> 710 us a layer at
-    // 21 frames, 594 -> 585 at 12, 40 heads the same.
+    // 21 frames, 594 -> 585 at 12, 40 heads the same.  In the iterative variant with longer caches what the column step's pass gains
+    // the update that reads aL after it loses (12 frames 59 + 65 -> 53 + 70 us).
     bool large_bridge() const { return (long long)nbh * na * blk.b2 * n_keys * (2 * kHeadDim * 2) > (252ll << 20); }
     void set_divs() {
         by_b2 = FastDiv::of(blk.b2); by_na = FastDiv::of(na); by_H = FastDiv::of(H);
