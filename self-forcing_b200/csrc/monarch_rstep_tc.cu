@@ -141,7 +141,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     // 52 columns, K / V slots of 16 KB: 3 / 1 195 us, 3 / 2 162, 4 / 2 159, 4 / 4 162, 5 / 3 171: copies share the TMA engine
     // with the result stores, and those asked for earlier than needed hold them up.  Other slot sizes, whole calls with 3 / 2,
     // 4 / 2, 4 / 3 slots: 30 columns (8 KB), 3 frames 41, 38, 38 us; 32 columns, 21 frames 168, 168, 171; 46 columns (12 KB), 12
-    // frames 165, 161, 158; 16 columns (4 KB), 40 heads, 3 frames 71, 64, 64, 21 frames 308, 305, 292.  Above 64 columns room for
+    // frames 165, 161, 158; 16 columns (4 KB), 40 heads, 3 frames 71, 64, 64, 21 frames 308, 305, 292.  Above 80 columns room for
     // two or three K slots is all there is (3 / 3 instead of 4 / 2 at 52: first chunk 62 -> 65, block-causal clip 470 -> 487).
     constexpr int kSlots = (kSmemData - kQBufs * kQBytes - kOutBytes) / kTile;
     constexpr int kVStg = kY ? kVStages : 0, kKStg = kSlots - kVStg < kKStages ? kSlots - kVStg : kKStages;
