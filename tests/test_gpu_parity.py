@@ -557,8 +557,9 @@ def test_gather_scatter_shards_match_unsharded(sfb):
 
 
 # ------------------------------------------------------------------------------- layer level
+# 12 heads are the most that one warp holds in registers, 48 the most that four do
 @pytest.mark.gpu
-@pytest.mark.parametrize("H", [2, 12])
+@pytest.mark.parametrize("H", [2, 12, 13, 40, 49])
 def test_norm_rope_cache_write_vs_oracle(sfb, H):
     """Full-width RMSNorm of q and k + RoPE + Monarch-order cache write in one kernel against the oracle
     chain rms_norm (reference WanRMSNorm) -> fp64 rotation -> permutation.  bf16 results may differ by one
@@ -583,9 +584,33 @@ def test_norm_rope_cache_write_vs_oracle(sfb, H):
     perm = torch.from_numpy(mon2nat)
     for got, ref in ((q_rot.cpu(), ref_q), (kc[:, n:].cpu(), ref_k[:, perm])):
         n_diff, max_ulp = ulp_mismatch(got, ref)
-        assert max_ulp <= 2 and n_diff <= 0.01 * ref.numel(), (n_diff, max_ulp)
+        assert (max_ulp <= 2 or H > 12) and n_diff <= 0.01 * ref.numel(), (n_diff, max_ulp)
+        # Among millions of values some have a neighbour in bf16 after each of the norm's two roundings (2^-7 each at most), and
+        # the rotation may leave a small difference of two such values: bounded by the length of the pair that is rotated
+        # (and the result's own rounding), not by the result.
+        pair = ref.float().unflatten(-1, (64, 2)).norm(dim=-1).repeat_interleave(2, dim=-1)
+        assert ((got.float() - ref.float()).abs() <= (2 ** -6 + 2 ** -8) * pair).all()
     assert torch.equal(vc[:, n:].cpu(), v[:, perm])
     assert not kc[:, :n].any() and not vc[:, :n].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("monarch_order", [True, False])
+@pytest.mark.parametrize("H", [1, 13, 26, 49])
+def test_eviction_inside_the_cache_write(sfb, H, monarch_order):
+    """A full window of 12 frames that keeps 2: the shift by 3 frames inside the write of the new ones leaves the bytes that
+    copies before it leave, with one, two and four warps a token and a token wider than their registers."""
+    h, w = 6, 8
+    f = h * w
+    g = torch.Generator(device="cuda").manual_seed(H)
+    q, k, v = (torch.randn(2, 3 * f, H, 128, device="cuda", generator=g).bfloat16() for _ in range(3))
+    k1, v1 = (torch.randn(2, 12 * f, H, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k2, v2 = k1.clone(), v1.clone()
+    args = (9 * f, 9, 1, 1, 1, h, w)
+    q1 = sfb.norm_rope_cache_write(q, k, v, k1, v1, *args, monarch_order=monarch_order, roll=(2 * f, 3 * f))
+    sfb.KVCache(k2, v2)._roll((2 * f, 5 * f, 7 * f))
+    q2 = sfb.norm_rope_cache_write(q, k, v, k2, v2, *args, monarch_order=monarch_order)
+    assert torch.equal(q1, q2) and torch.equal(k1, k2) and torch.equal(v1, v2)
 
 
 def _oracle_layer_call(state, q, k, v, current_start, grid, cfg, wq, wk):
