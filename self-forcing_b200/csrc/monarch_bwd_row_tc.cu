@@ -77,14 +77,16 @@ struct BwdRowParams {
     int* status;
 };
 
-// At most: a kv step's two tiles stay until its GEMMs, and with five more slots a later step's dR could be ready before them.
+// At most.  With four, dR of the step after a kv step can be complete before the gradient warp has looked at the kv step's, behind its
+// R copy: dr_full has a barrier for even and one for odd steps.  The parity it looks at would turn back two steps on: that dR waits for
+// dr_read of the step between, which the element-wise warps give behind rz_free of the kv step, and that the gradient warp commits last.
 constexpr int kRowSlots = 4;
 constexpr int kKSlots = 3;                                 // at most
 struct __align__(16) RBBarriers {
     uint64_t q_full, q_empty;
     uint64_t k_full[kKSlots], k_empty[kKSlots], v_full, v_empty;
     uint64_t rt_full[kRowSlots], rt_empty[kRowSlots];      // daL and dY tiles in turn
-    uint64_t s_full, dr_full, s_read, dr_read;             // S, dR: written, in registers
+    uint64_t s_full, dr_full[2], s_read, dr_read;          // S, dR (even, odd steps): written; S, dR: in registers
     uint64_t r_full, p_full, rz_free;                      // R copy (kv steps), dz copy: written; both free
     uint64_t dkv_full, dkv_free, dq_full[2], dq_free[2];
     uint32_t tmem_base;
@@ -185,10 +187,10 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
         for (int s = 0; s < kKSlots; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1); }
         mbar_init(&bars->v_full, 1); mbar_init(&bars->v_empty, 1);
         for (int s = 0; s < kRowSlots; ++s) { mbar_init(&bars->rt_full[s], 1); mbar_init(&bars->rt_empty[s], 1); }
-        mbar_init(&bars->s_full, 1); mbar_init(&bars->dr_full, 1); mbar_init(&bars->s_read, 256); mbar_init(&bars->dr_read, 256);
+        mbar_init(&bars->s_full, 1); mbar_init(&bars->s_read, 256); mbar_init(&bars->dr_read, 256);
         mbar_init(&bars->r_full, 256); mbar_init(&bars->p_full, 256); mbar_init(&bars->rz_free, 1);
         mbar_init(&bars->dkv_full, 1); mbar_init(&bars->dkv_free, 128);
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars->dq_full[s], 1); mbar_init(&bars->dq_free[s], 128); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars->dr_full[s], 1); mbar_init(&bars->dq_full[s], 1); mbar_init(&bars->dq_free[s], 128); }
         bars->abort_flag = 0;
         mbar_init_fence();
     }
@@ -318,7 +320,7 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                     if (++sr == n_rt) { sr = 0; pr ^= 1; }
                 }
                 if (!ok) break;
-                mma_commit_e(el, &bars->dr_full);
+                mma_commit_e(el, &bars->dr_full[g & 1]);
                 mma_commit_e(el, &bars->v_empty);
             }
         }
@@ -350,7 +352,7 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 if (kvw) {
                     // R is there long before dz: the row tiles leave as soon as dR has been taken from them
                     if (!mbar_wait_u(&bars->r_full, gd & 1)) { fail(29); ok = false; break; }
-                    if (!mbar_wait_u(&bars->dr_full, g & 1)) { fail(30); ok = false; break; }
+                    if (!mbar_wait_u(&bars->dr_full[g & 1], (g >> 1) & 1)) { fail(30); ok = false; break; }
                     if (gd >= 1 && !mbar_wait_u(&bars->dkv_free, (gd - 1) & 1)) { fail(26); ok = false; break; }
                     tc_fence_after();
                     const uint64_t da_mn = rt_mn0 + (uint64_t)((da * q_tile) >> 4), dy_mn = rt_mn0 + (uint64_t)((dy * q_tile) >> 4);
@@ -497,7 +499,7 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                     fence_async_smem();
                     mbar_arrive(&bars->r_full);
                 }
-                if (!mbar_wait_u(&bars->dr_full, g & 1)) { fail(32); ok = false; break; }
+                if (!mbar_wait_u(&bars->dr_full[g & 1], (g >> 1) & 1)) { fail(32); ok = false; break; }
                 tc_fence_after();
                 {
                     uint32_t r[N_S / 2];
