@@ -70,6 +70,7 @@ struct __align__(16) Barriers {
     alignas(16) float cl[4][kMaxU][kBiasPitch];   // bias slices, per unit slot: a ring of four tiles
     float stats[2][2][128];                // [warpgroup][m | l][tile row]
     uint64_t q_full[2], q_empty[2];
+    uint64_t q_first;                      // the first group's query rows are there: once a launch
     uint64_t a_full[kMaxStages], a_empty[kMaxStages];
     uint64_t y_full[kMaxStages], y_empty[kMaxStages];
     uint64_t cl_full[4], cl_empty[4];
@@ -154,6 +155,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
     if (warp == 2 && lane == 0) { prefetch_tmap(&tqr); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
+        mbar_init(&bars->q_first, 1);
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(&bars->a_full[s], 1); mbar_init(&bars->a_empty[s], 1);
             mbar_init(&bars->y_full[s], 1); mbar_init(&bars->y_empty[s], 1);
@@ -289,10 +291,11 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
                         const LUnit un = decode_unit(p, u0 + us);
                         unsigned char* yt = y_s + sy * tile_bytes;
                         if (waiting) {
-                            // a launch's first value tiles go out behind its queries and keys, which are needed first
+                            // a launch's first value tiles go out behind its queries and keys, which are needed first (not by
+                            // q_full: groups of one or two tiles fill it again without a value tile)
                             keep(un.j + un.al + un.bhl);
                             pdl_wait();
-                            if (!mbar_wait_u(&bars->q_full[0], 0)) { fail(14); ok = false; break; }
+                            if (!mbar_wait_u(&bars->q_first, 0)) { fail(14); ok = false; break; }
                             waiting = false;
                         }
                         mbar_arrive_expect_tx_e(el, &bars->y_full[sy], (uint32_t)tile_bytes);
@@ -324,6 +327,7 @@ monarch_l_tc_kernel(const __grid_constant__ CUtensorMap tal, const __grid_consta
             const GroupKeys gk = keys_of(u0);
             const int n_tiles = group_tiles(gk, nu);
             if (!mbar_wait_u(&bars->q_full[qb], (gi >> lead) & 1)) { fail(20); break; }
+            if (gi == 0 && lane == 0) mbar_arrive(&bars->q_first);
             const uint64_t qd = q_desc + (uint64_t)((qb * kQBytes) >> 4);
             for (int t = 0; ok && t < n_tiles; ++t, ++gt) {
                 const int w = gt & 1;

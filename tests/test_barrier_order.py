@@ -172,3 +172,104 @@ def test_row_backward(wants_kv):
     for n_rt in range(3, slots + 1):
         for n_k in (2, 3):
             never_stuck(lambda: row_backward(len(kv), kv, n_rt, n_k, n_dr))
+
+
+def column_step(groups, tiles, units, n_q, n_a, n_y, first):
+    """monarch_l_tc_kernel: groups of `units` units with tiles[group] key tiles, n_q query tiles, n_a / n_y slots for key and
+    value tiles; the warp of the value tiles waits for the barrier `first` before its first load."""
+    one = lambda n: [Barrier() for _ in range(n)]
+    q_full, q_empty, cl_full, cl_empty = one(n_q), one(n_q), one(4), one(4)
+    a_full, a_empty, y_full, y_empty = one(n_a), one(n_a), one(n_y), one(n_y)
+    s_full, p_full, sp_free, o_full, o_free = one(2), one(2), one(2), one(2), one(2)
+    named = {"q_full[0]": q_full[0], "q_first": Barrier()}
+    eng = {n: deque() for n in ("keys", "values", "queries", "s", "pv")}
+    order = [(gi, t) for gi in range(groups) for t in range(tiles[gi])]
+
+    def load_keys():
+        x = 0
+        for gt in range(len(order)):
+            for _ in range(units):
+                yield a_empty[x % n_a], x // n_a - 1
+                eng["keys"].append(a_full[x % n_a].arrive)
+                x += 1
+            yield cl_empty[gt & 3], (gt >> 2) - 1
+            eng["keys"].append(cl_full[gt & 3].arrive)
+
+    def load_values():
+        for x in range(len(order) * units):
+            yield y_empty[x % n_y], x // n_y - 1
+            if x == 0 and first:
+                yield named[first], 0
+            eng["values"].append(y_full[x % n_y].arrive)
+
+    def issue_s():
+        x = gt = 0
+        for step in range(groups + n_q - 1):
+            if step < groups:
+                yield q_empty[step % n_q], step // n_q - 1
+                eng["queries"].append(q_full[step % n_q].arrive)
+            gi = step - (n_q - 1)
+            if gi < 0:
+                continue
+            yield q_full[gi % n_q], gi // n_q
+            if gi == 0:
+                named["q_first"].arrive()
+            for _ in range(tiles[gi]):
+                yield sp_free[gt & 1], (gt >> 1) - 1
+                for _ in range(units):
+                    yield a_full[x % n_a], x // n_a
+                    eng["s"].append(a_empty[x % n_a].arrive)
+                    x += 1
+                eng["s"].append(s_full[gt & 1].arrive)
+                gt += 1
+            eng["s"].append(q_empty[gi % n_q].arrive)
+
+    def issue_pv():
+        x, used = 0, [0, 0]
+        for gt, (gi, t) in enumerate(order):
+            w = gt & 1
+            yield p_full[w], gt >> 1
+            if t < 2:
+                yield o_free[w], used[w] - 1
+                used[w] += 1
+            for _ in range(units):
+                yield y_full[x % n_y], x // n_y
+                eng["pv"].append(y_empty[x % n_y].arrive)
+                x += 1
+            eng["pv"].append(sp_free[w].arrive)
+            if t + 1 == tiles[gi]:
+                eng["pv"].append(o_full[gi & 1].arrive)
+
+    def softmax(w):
+        used = 0
+        for gt, (gi, t) in enumerate(order):
+            if gt & 1 != w:
+                continue
+            yield s_full[w], gt >> 1
+            yield cl_full[gt & 3], gt >> 2
+            cl_empty[gt & 3].arrive()
+            if t + 2 >= tiles[gi]:
+                yield o_free[w], used - 1
+                used += 1
+            p_full[w].arrive()
+
+    def epilogue():
+        gt = 0
+        for gi in range(groups):
+            yield o_full[gi & 1], gi >> 1
+            o_free[gt & 1].arrive()
+            if tiles[gi] > 1:
+                o_free[gt & 1 ^ 1].arrive()
+            gt += tiles[gi]
+
+    return {"load_keys": load_keys(), "load_values": load_values(), "issue_s": issue_s(), "issue_pv": issue_pv(),
+            "softmax0": softmax(0), "softmax1": softmax(1), "epilogue": epilogue()}, eng
+
+
+@pytest.mark.parametrize("tiles", [[1], [2], [3], [5], [1, 2, 3]], ids=str)
+@pytest.mark.parametrize("units,n_q", [(1, 2), (2, 2), (4, 1), (4, 2)])
+def test_column_step(units, n_q, tiles):
+    text = (CSRC / "monarch_lstep_tc.cu").read_text()
+    first = re.search(r"mbar_wait_u\(&bars->(q_\w+(?:\[0\])?), 0\)\)", text)
+    for n_a, n_y in ((2, 3), (3, 5)):
+        never_stuck(lambda: column_step(6, (tiles * 6)[:6], units, n_q, n_a, n_y, first and first.group(1)))
