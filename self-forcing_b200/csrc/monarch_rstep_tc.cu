@@ -56,6 +56,7 @@ struct RTcParams {
     MonarchParams mp;
     int spg;               // slots per query group, 0: two groups in a slot
     int n_slots, tiles;    // slots and tiles per (batch*head) of the chunk
+    int per_tile, more;    // tiles that cut groups: slots of each, tiles from the first on that have one more
     int n_whole;           // units that take all cached groups; of the others each is cut into
     int fsplit, f_per;     // fsplit units of f_per cached groups
     int n_units;           // of both kinds
@@ -97,8 +98,8 @@ __device__ __forceinline__ RUnit decode_unit(const RTcParams& rp, int u) {
     // of its rows stood empty (clip of 12 frames, 24 x 70 tokens, 6 heads 388 -> 317 us, this and the spills).  Tiles of fours
     // otherwise: even ones (3 + 3 for three groups of two slots) load their queries in more boxes (20 passes 805 -> 831 us).
     if constexpr (kCut) {
-        r.slot0 = rp.by_tiles.div(tile * rp.n_slots);
-        r.ns = rp.by_tiles.div((tile + 1) * rp.n_slots) - r.slot0;
+        r.slot0 = tile * rp.per_tile + min(tile, rp.more);
+        r.ns = rp.per_tile + (tile < rp.more ? 1 : 0);
     } else {
         r.slot0 = 4 * tile;
         r.ns = min(4, rp.n_slots - r.slot0);
@@ -684,6 +685,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box o
     rp.col_kt = l_tile_keys(p);
     rp.n_slots = b2 <= 16 ? (p.na + 1) / 2 : p.na * rp.spg;
     rp.tiles = (rp.n_slots + 3) / 4;
+    rp.per_tile = rp.n_slots / rp.tiles; rp.more = rp.n_slots % rp.tiles;
     const long long whole = (long long)p.nbh * rp.tiles * p.blk.b1;       // units, not cut
     {
         // Persistent CTAs take units round-robin, so a launch lasts as long as its fullest CTA.  Either all units are cut in the same
