@@ -229,13 +229,24 @@ int launch_monarch_held(MonarchCall& mc) {
                 p.f_per = (pl.F + fsplit - 1) / fsplit;
                 p.fsplit = (pl.F + p.f_per - 1) / p.f_per;
             }
+            CUtensorMap state_maps[3];       // for the later passes of the iterative variant: state, K, V
+            if (iter_tc) {
+                // iteration state aR of this chunk as [nbh * F * b1][na * b2][128]: one (f, k) block of (query group, column) rows
+                // per index of the slowest dimension
+                const uint64_t row = (uint64_t)kHeadDim * 2, rows = (uint64_t)p.na * pl.blk.b2;
+                const uint64_t dims[3] = {(uint64_t)kHeadDim, rows, (uint64_t)p.nbh * pl.F * pl.blk.b1};
+                const uint64_t strides[2] = {row, rows * row};
+                const uint32_t box[3] = {64, (uint32_t)pl.blk.b2, 1};
+                if ((rc = make_tmap_bf16(&state_maps[0], p.aR, 3, dims, strides, box))) return rc;
+                state_maps[1] = maps[1]; state_maps[2] = maps[2];
+            }
             for (int it = 0; it < num_iters; ++it) {
                 const bool last = it == num_iters - 1;
                 p.use_aR = it > 0;
                 p.write_Y = last;
                 p.mult0 = num_iters > 1 ? sm_scale * (1.0f / (1.0f + 1e-6f)) : sm_scale;
                 if (use_tc) {
-                    if ((rc = launch_r_step_tc(p, maps, n_s, status, bh0 == 0 && a0 == 0 && it == 0, num_sms, stream))) return rc;
+                    if ((rc = launch_r_step_tc(p, p.use_aR ? state_maps : maps, n_s, status, bh0 == 0 && a0 == 0 && it == 0, num_sms, stream))) return rc;
                 } else {
                     if ((rc = launch_r_step(p, stream))) return rc;
                 }
@@ -287,7 +298,8 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
                      __nv_bfloat16* aL, __nv_bfloat16* Y, float* cL, float* lse, int* status, int B, int H, int n_q,
                      int n_kv, const Blocking& blk, float scale, int bh0, int nbh, bool column, bool clear_status, MonarchParams* p_out,
                      CUtensorMap* maps, cudaStream_t stream) {
-    if (blk.b1 > 128 || blk.b2 > kB2MaxTc) return SFM_ERR_UNSUPPORTED;
+    // one box brings a block row's queries, here and in the row step's backward (r_load_columns)
+    if (blk.b1 > 128 || blk.b2 > kB2Max) return SFM_ERR_UNSUPPORTED;
     const int group = blk.b1 * blk.b2;
     MonarchParams p;
     p.q = (const __nv_bfloat16*)q; p.q_bs = q_bs;
@@ -323,10 +335,7 @@ int forward_tc_slice(const void* q, int64_t q_bs, const void* kc, const void* vc
     if ((rc = make_tmap_bf16(&maps[1], kc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[2], vc, 4, dk, sk, bk))) return rc;
     if ((rc = make_tmap_bf16(&maps[3], q, 5, dqr, sqr, bqr))) return rc;
-    const uint32_t bs[4] = {64, 1, (uint32_t)r_load_columns(blk.b2, false), 1};
-    CUtensorMap rmaps[3] = {{}, maps[1], maps[2]};
-    if ((rc = make_tmap_bf16(&rmaps[0], q, 4, dq, sq, bs))) return rc;
-    if ((rc = launch_r_step_tc(p, rmaps, n_s, status, clear_status, num_sms, stream))) return rc;
+    if ((rc = launch_r_step_tc(p, maps, n_s, status, clear_status, num_sms, stream))) return rc;
     if (column && (rc = launch_l_step_tc(p, &maps[3], status, num_sms, stream, lse ? 1 : 0))) return rc;
     *p_out = p;
     return SFM_OK;

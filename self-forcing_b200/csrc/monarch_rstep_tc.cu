@@ -52,6 +52,13 @@ constexpr int kMaxQBufs = 3;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 256;        // two accumulators of 128 columns; the S/P buffers lie below them
 
+// A query group of 65 to 96 columns takes three slots, so that tiles cut groups.
+__host__ __device__ constexpr bool cuts_groups(int n_s) { return n_s == 80 || n_s == 96; }
+
+// What loads of query rows bring: a group's rows, or a slot's and, in the second map, those of a group's last slot.
+template <bool kCut>
+struct QueryMaps { CUtensorMap m[kCut ? 2 : 1]; };
+
 struct RTcParams {
     MonarchParams mp;
     int spg;               // slots per query group, 0: two groups in a slot
@@ -143,7 +150,7 @@ static_assert(sizeof(Barriers) <= 512, "barriers follow the tiles");
 // kLarge: the bridge is much larger than L2 (MonarchParams::large_bridge).
 template <int N_S, bool kCausal, bool kIter, bool kY, bool kLarge>
 __global__ void __launch_bounds__(kThreads, 1)
-monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tq_last, const __grid_constant__ CUtensorMap tk,
+monarch_r_tc_kernel(const __grid_constant__ QueryMaps<cuts_groups(N_S)> tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tal,
                     const __grid_constant__ CUtensorMap ty, RTcParams rp) {
     static_assert(!(kIter || !kY) || (N_S <= 64 && !kCausal), "the iterative variant exists for block columns up to 64, no mask");
@@ -156,7 +163,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     constexpr int kHalf = N_S * 128;                    // bytes of one 64-column half of a K or V tile
     // Block columns above 64 (wide grids): two S/P buffers, and the softmax walks its row in 32-column chunks (see below).
     constexpr bool kWide = N_S > 64;
-    constexpr bool kCut = N_S == 80 || N_S == 96;       // a group takes three slots, so that tiles cut groups
+    constexpr bool kCut = cuts_groups(N_S);
     constexpr int kTile = 2 * kHalf;                     // a K or V tile: two halves
     constexpr int kSBufs = kWide ? 2 : 4;
     constexpr uint32_t kSCols = kColO / kSBufs;          // TMEM columns per S/P buffer
@@ -177,7 +184,7 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     unsigned char* o_s = v_s + kVStg * kTile;                // staging of the epilogue warps
     Barriers* bars = reinterpret_cast<Barriers*>(base + kSmemData);
 
-    if (warp == 2 && lane == 0) { prefetch_tmap(&tq); prefetch_tmap(&tq_last); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tal); prefetch_tmap(&ty); }
+    if (warp == 2 && lane == 0) { prefetch_tmap(tq.m); prefetch_tmap(&tq.m[kCut]); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tal); prefetch_tmap(&ty); }
     if (tid == 0) {
         for (int s = 0; s < kQBufs; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
         for (int s = 0; s < kKStg; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1); }
@@ -263,12 +270,12 @@ monarch_r_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
                             }
                         }
                         for (int x = 0; x < n_q; ++x, qd += kCut ? 32 * 128 : q_pitch) {
-                            const CUtensorMap* m = &tq;
+                            const CUtensorMap* m = tq.m;
                             int gr = g_first + x;
                             j0 = 0;
                             if constexpr (kCut) {
                                 gr = slot_group(rp, un.slot0 + x, j0);
-                                if (j0 == 64) m = &tq_last;
+                                if (j0 == 64) m = &tq.m[1];
                             }
                             if (x == 0) {
                                 if (g == 0) {
@@ -674,7 +681,7 @@ int r_load_columns(int b2, bool last) { return b2 <= 64 || b2 > 96 ? b2 : (last 
 // kernel sets on an internal timeout.
 int l_tile_keys(const MonarchParams& p);
 
-int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box of r_load_columns tokens), K, V */, int n_s, int* status,
+int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box of r_load_columns tokens) or the aR state, K, V */, int n_s, int* status,
                      int clear_status, int num_sms, cudaStream_t s) {
     LaunchScope scope(kClsRStep, s);
     RTcParams rp;
@@ -712,36 +719,23 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box o
     const bool iter = p.use_aR != 0;
     if (iter && (n_s > 64 || p.causal_groups > 0)) return SFM_ERR_UNSUPPORTED;
     const int smem_bytes = kSmemBytes;
-    // query rows: those that one load brings, and those of a group's last slot
-    CUtensorMap q_maps[2] = {maps[0], maps[0]};
-    for (int i = 0; i < 2; ++i) {
-        const uint32_t cols = r_load_columns(b2, i);
-        const uint64_t row = (uint64_t)kHeadDim * 2;
-        int rc = 0;
-        if (iter) {
-            // iteration state aR of the chunk as [nbh * F * b1][na * b2][128]: one (f, k) block of (query group, column) rows
-            // per index of the slowest dimension
-            const uint64_t dims[3] = {(uint64_t)kHeadDim, (uint64_t)p.na * b2, (uint64_t)p.nbh * p.F * p.blk.b1};
-            const uint64_t strides[2] = {row, (uint64_t)p.na * b2 * row};
-            const uint32_t box[3] = {64, cols, 1};
-            rc = make_tmap_bf16(&q_maps[i], p.aR, 3, dims, strides, box);
-        } else if (i && rp.spg == 3) {
-            const uint64_t dims[4] = {(uint64_t)kHeadDim, (uint64_t)p.H, (uint64_t)p.n_q, (uint64_t)((p.bh0 + p.nbh - 1) / p.H + 1)};
-            const uint64_t strides[3] = {row, row * p.H, (uint64_t)p.q_bs * 2};
-            const uint32_t box[4] = {64, 1, cols, 1};
-            rc = make_tmap_bf16(&q_maps[i], p.q, 4, dims, strides, box);
-        }
-        if (rc) return rc;
-    }
     // result stores: one box = the 128 channels of up to 32 columns of one key
     CUtensorMap out_maps[2];
     const int box_cols = b2 <= 16 ? 16 : 32;
     for (int i = 0; i < 2; ++i)
         if (int rc = make_bridge_tmap(&out_maps[i], i ? p.Y : p.aL, p.blk.b2, p.n_keys, p.nbh * p.na, box_cols, 1)) return rc;
-    auto go = [&](auto kernel) -> int {
+    auto go = [&](auto kernel, auto q_maps) -> int {
+        q_maps.m[0] = maps[0];
+        if constexpr (sizeof(q_maps) > sizeof(CUtensorMap)) {
+            const uint64_t row = (uint64_t)kHeadDim * 2;
+            const uint64_t dims[4] = {(uint64_t)kHeadDim, (uint64_t)p.H, (uint64_t)p.n_q, (uint64_t)((p.bh0 + p.nbh - 1) / p.H + 1)};
+            const uint64_t strides[3] = {row, row * p.H, (uint64_t)p.q_bs * 2};
+            const uint32_t box[4] = {64, 1, (uint32_t)r_load_columns(b2, true), 1};
+            if (int rc = make_tmap_bf16(&q_maps.m[1], p.q, 4, dims, strides, box)) return rc;
+        }
         if (int rc = opt_in_smem((const void*)kernel, smem_bytes)) return rc;
-        return launch_pdl(whole * p.F <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, q_maps[0], q_maps[1], maps[1], maps[2],
-                          out_maps[0], out_maps[1], rp);
+        return launch_pdl(whole * p.F <= 32 * num_sms, kernel, grid, kThreads, smem_bytes, s, q_maps, maps[1], maps[2], out_maps[0],
+                          out_maps[1], rp);
     };
     int rc;
     // Unmasked clips whose keys are in natural order take the block-causal instances, with one block: 3 videos, 12 heads, 3 frames in
@@ -749,14 +743,17 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box o
     // heads, 6 x 8 tokens 32 -> 26.
     const bool causal = p.causal_groups > 0 || p.kv_natural, large = p.large_bridge();
     if (causal && p.causal_groups == 0) rp.mp.causal_groups = p.A > p.F ? p.A : p.F;
+#define SFM_R_GO(...) go(monarch_r_tc_kernel<__VA_ARGS__>, QueryMaps<cuts_groups(N)>())
     if (iter || !p.write_Y) {
         switch (n_s) {
-#define SFM_R_CASE(n)                                                                           \
-    case n:                                                                                     \
-        rc = !iter       ? go(monarch_r_tc_kernel<n, false, false, false, false>)               \
-             : p.write_Y ? go(monarch_r_tc_kernel<n, false, true, true, false>)                 \
-                         : go(monarch_r_tc_kernel<n, false, true, false, false>);               \
-        break;
+#define SFM_R_CASE(n)                                                     \
+    case n: {                                                             \
+        constexpr int N = n;                                              \
+        rc = !iter       ? SFM_R_GO(N, false, false, false, false)        \
+             : p.write_Y ? SFM_R_GO(N, false, true, true, false)          \
+                         : SFM_R_GO(N, false, true, false, false);        \
+        break;                                                            \
+    }
             SFM_R_CASE(16)
             SFM_R_CASE(32)
             SFM_R_CASE(48)
@@ -766,13 +763,13 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box o
         }
     } else {
         switch (n_s) {
-#define SFM_R_CASE(n)                                                                           \
-    case n:                                                                                     \
-        rc = causal ? (large ? go(monarch_r_tc_kernel<n, true, false, true, true>)              \
-                             : go(monarch_r_tc_kernel<n, true, false, true, false>))            \
-                    : (large ? go(monarch_r_tc_kernel<n, false, false, true, true>)             \
-                             : go(monarch_r_tc_kernel<n, false, false, true, false>));          \
-        break;
+#define SFM_R_CASE(n)                                                                                       \
+    case n: {                                                                                               \
+        constexpr int N = n;                                                                                \
+        rc = causal ? (large ? SFM_R_GO(N, true, false, true, true) : SFM_R_GO(N, true, false, true, false))    \
+                    : (large ? SFM_R_GO(N, false, false, true, true) : SFM_R_GO(N, false, false, true, false)); \
+        break;                                                                                              \
+    }
             SFM_R_CASE(16)
             SFM_R_CASE(32)
             SFM_R_CASE(48)
@@ -785,6 +782,7 @@ int launch_r_step_tc(const MonarchParams& p, const CUtensorMap* maps /* q (box o
             default: return SFM_ERR_UNSUPPORTED;
         }
     }
+#undef SFM_R_GO
     if (rc) return rc;
     return (int)cudaGetLastError();
 }
