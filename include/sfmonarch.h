@@ -216,7 +216,8 @@ int sfm_dense_status(void* stream);
  * contiguous.  Query groups of causal block c attend the key groups of blocks 0..c;
  * causal_groups = groups per causal block (0 = no mask).  k_mon / v_mon are scratch
  * [B, N, H, D] that receive k, v in Monarch order; they may be k and v themselves, which are then read
- * in place, for h_reduce = w_reduce = 1 (one order) and for one pass with block rows up to 128.
+ * in place, for h_reduce = w_reduce = 1 (one order) and for one pass with block rows up to 128.  Any other
+ * overlap with k or v is refused (SFM_ERR_UNSUPPORTED), but for a copy of one order on its own source.
  * Replaces: monarch_attn / _attention_no_cache.forward
  * (wan/modules/monarch_attn.py:1753-1776, 1472-1563).
  */

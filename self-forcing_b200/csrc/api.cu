@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 
 #include "monarch_params.cuh"
 #include "profile.cuh"
@@ -455,6 +456,17 @@ extern "C" int sfm_monarch_nocache_fwd(const void* q, const void* k, const void*
                                        int f_tied, int h_reduce, int w_reduce, int h, int w, float sm_scale,
                                        int causal_groups, int num_iters, size_t bridge_budget_bytes, void* stream) {
     if (!k_mon || !v_mon) return SFM_ERR_NULL_POINTER;
+    const bool in_place = k_mon == k && v_mon == v, one_order = h_reduce == 1 && w_reduce == 1;
+    if (!in_place && B > 0 && H > 0 && D > 0 && N > 0) {
+        // A copy must not write what it still has to read; one that stays as it is may lie on itself.
+        const size_t bytes = (size_t)B * N * H * D * 2;
+        auto overlap = [&](const void* a, const void* b) {
+            const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+            return x < y + bytes && y < x + bytes;
+        };
+        for (auto [copy, source] : {std::pair<const void*, const void*>(k_mon, k), {v_mon, v}})
+            if ((overlap(copy, k) || overlap(copy, v)) && !(one_order && copy == source)) return SFM_ERR_UNSUPPORTED;
+    }
     MonarchCall mc;
     int rc = prepare_monarch(&mc, q, (int64_t)N * H * D, k_mon, v_mon, (int64_t)N * H * D, out, workspace, workspace_bytes, B,
                              H, D, N, N, f_tied, h_reduce, w_reduce, h, w, sm_scale, num_iters, causal_groups,
@@ -463,9 +475,9 @@ extern "C" int sfm_monarch_nocache_fwd(const void* q, const void* k, const void*
     // A caller that names k and v themselves as the scratch has them read where they are (12 frames, 12 heads, block-causal: 462 ->
     // 421 us with the copies left out): the row step on the tensor cores finds a block row's tokens in either order, and frames that
     // are not cut into bands have only one.
-    if (k_mon == k && v_mon == v) {
-        if (h_reduce != 1 || w_reduce != 1) {
-            if (!mc.use_tc || num_iters != 1) return SFM_ERR_UNSUPPORTED;
+    if (in_place) {
+        if (!one_order) {
+            if (!mc.use_tc || num_iters != 1 || mc.pl.blk.b1 > 128) return SFM_ERR_UNSUPPORTED;
             mc.p.kv_natural = 1;
         }
     } else

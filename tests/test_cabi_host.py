@@ -181,6 +181,21 @@ def test_entry_points_validate_arguments_without_a_gpu(sfb):
                                        3 * 60 * 52, 3, 1, 1, 60, 52, 1.0, 0, null) == -3
 
 
+# The copies of k and v in Monarch order (k, v at 1 and 2 MiB, 0.4 MB each): read in place, beside their sources, or refused
+@pytest.mark.parametrize("bands", [(1, 1), (2, 1), (1, 4)])
+@pytest.mark.parametrize("k_mon,v_mon,one_order,several", [
+    (4 << 20, 5 << 20, True, True), (1 << 20, 2 << 20, True, True), (1 << 20, 5 << 20, True, False), (4 << 20, 2 << 20, True, False),
+    (2 << 20, 1 << 20, False, False), ((1 << 20) + 4096, 5 << 20, False, False), (4 << 20, (2 << 20) - 4096, False, False),
+    (2 << 20, 5 << 20, False, False), (4 << 20, 1 << 20, False, False)])
+def test_nocache_copies_that_overlap_their_sources(sfb, bands, k_mon, v_mon, one_order, several):
+    from self_forcing_b200 import _lib
+    p = C.c_void_p
+    rc = _lib.load().sfm_monarch_nocache_fwd(p(8 << 20), p(1 << 20), p(2 << 20), p(k_mon), p(v_mon), p(9 << 20), p(256), 0, 1, 1, 128,
+                                             1560, 1, *bands, 30, 52, 1.0, 0, 1, 0, p(0))
+    taken = one_order if bands == (1, 1) else several
+    assert rc == (-5 if taken else -3)                     # what is taken ends at its workspace of no bytes
+
+
 @pytest.mark.parametrize("field,value,rc", [("workspace_bytes", 0, -5), ("workspace_bytes", 1, -5), ("n_kv", 1561, -2),
                                             ("num_iters", 0, -2), ("out", 260, -4), ("lse", 258, -4), ("k_cache", 0, -1)])
 def test_layer_call_is_refused_before_its_cache_write(sfb, field, value, rc):
