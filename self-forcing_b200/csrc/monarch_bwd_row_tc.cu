@@ -680,16 +680,17 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
 }
 
 // dk / dv [B, n_sel, H, 128] bf16 (Monarch order, or the tokens in natural order) = sum over the tiles' fp32 partials, in tile order.
-// A thread has eight channels of a token of pair blockIdx.y.  Bound by the partials' trip from memory (144 MB with the results for
+// A thread has eight channels of a token, a block 16 tokens of a (batch, head) pair.  Bound by the partials' trip from memory (144 MB with the results for
 // 4680 tokens, 12 heads, two tiles: 30 us).
 __global__ void __launch_bounds__(256) bwd_merge_kv_kernel(const float* __restrict__ part_k, const float* __restrict__ part_v,
                                                            __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                                           int tiles, int n_sel, MonarchParams mp, FastDiv by_group, int natural) {
+                                                           int tiles, int n_sel, MonarchParams mp, FastDiv by_blocks, FastDiv by_group, int natural) {
     pdl_trigger();
     pdl_wait();
-    const int idx = (int)(blockIdx.x * 256 + threadIdx.x), tok = idx >> 4, c8 = (idx & 15) * 8;
+    int block;
+    const int bhl = by_blocks.divmod((int)blockIdx.x, block);
+    const int tok = block * 16 + (int)(threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
     if (tok >= n_sel) return;
-    const int bhl = blockIdx.y;
     const long long tile_step = (long long)mp.nbh * n_sel * kHeadDim;
     long long o = ((long long)bhl * n_sel + tok) * kHeadDim + c8;
     float k[8] = {}, v[8] = {};
@@ -778,8 +779,9 @@ int launch_bwd_row_tc(const MonarchParams& mp, const CUtensorMap* maps, const fl
         const int n_sel = (g1 - g0) * mp.blk.b1 * mp.blk.b2;
         MonarchParams m = mp;
         m.set_divs();
-        if (int e = launch_pdl(true, bwd_merge_kv_kernel, dim3((n_sel + 15) / 16, mp.nbh), 256, 0, s, (const float*)part_k, (const float*)part_v, dk, dv,
-                               rp.tiles, n_sel, m, FastDiv::of(mp.blk.b1 * mp.blk.b2), natural))
+        const int blocks = (n_sel + 15) / 16;                        // of a pair
+        if (int e = launch_pdl(true, bwd_merge_kv_kernel, dim3((unsigned)blocks * mp.nbh), 256, 0, s, (const float*)part_k, (const float*)part_v, dk, dv,
+                               rp.tiles, n_sel, m, FastDiv::of(blocks), FastDiv::of(mp.blk.b1 * mp.blk.b2), natural))
             return e;
     }
     return SFM_OK;

@@ -140,6 +140,22 @@ def test_backward_several_units_per_cta(sfb, h, w, frames_q, cached, H):
         assert torch.equal(dq, dq2) and torch.equal(dk[:, sl], dk2) and torch.equal(dv[:, sl], dv2)
 
 
+def test_backward_more_pairs_than_a_grid_dimension(sfb):
+    """66000 (batch, head) pairs in one slice, two tiles of query groups each, whose dK / dV are merged: heads do not see each other, so
+    the first, the last and those about 65535 are compared."""
+    h, w, frames, H = 2, 2, 17, 66000
+    gen = torch.Generator(device="cuda").manual_seed(8280)
+    q, g = (torch.randn(1, frames * h * w, H, 128, device="cuda", generator=gen, dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(1, h * w, H, 128, device="cuda", generator=gen, dtype=torch.bfloat16) for _ in range(2))
+    got = sfb.monarch_attn_with_kv_cache_backward(q, k, v, g, 1, 1, 1, h, w, budget_bytes=16 << 30)
+    hs = [0, 65534, 65535, 65536, H - 1]
+    ref = [t[:, :, hs].float().cpu().requires_grad_() for t in (q, k, v)]
+    (orc.monarch_attn(*ref, 1, 1, 1, h, w) * g[:, :, hs].float().cpu()).sum().backward()
+    for x, r, name in zip(got, ref, ("dq", "dk", "dv")):
+        grad_close(x[:, :, hs], r.grad, 1e-2, name)
+    sfb.ops.release_workspaces()
+
+
 def test_backward_row_kernels_agree(sfb, monkeypatch):
     """The tensor-core row-step backward against the fp32 one on the same intermediate gradients (the fp32 kernel
     rounds nothing but its inputs): both must sit within bf16 rounding of each other."""
