@@ -582,7 +582,8 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
                 if (!mbar_wait_u(&bars->dkv_full, gd & 1)) { fail(41); ok = false; break; }
                 tc_fence_after();
                 // The keys of the block, at most 64, are on two warps' lanes each for dK and for dV.  16 rows at a time as fragments: a
-                // quad's eight channels of a row are a sector, and the GEMMs have the accumulator back after four loads.
+                // quad's eight channels of a row are a sector of the fp32 partials (half a one of bf16 results), and the GEMMs have
+                // the accumulator back after four loads.
                 const int key0 = (quad & 1) * 32;
                 if (key0 < b2) {
                     const long long row0 = ((long long)un.tile * p.nbh + un.bhl) * n_sel + ((long long)(group_of(i) - rp.g0) * b1 + un.k) * b2;
@@ -680,8 +681,8 @@ monarch_bwd_row_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
 }
 
 // dk / dv [B, n_sel, H, 128] bf16 (Monarch order, or the tokens in natural order) = sum over the tiles' fp32 partials, in tile order.
-// A thread has eight channels of a token, a block 16 tokens of a (batch, head) pair.  Bound by the partials' trip from memory (144 MB with the results for
-// 4680 tokens, 12 heads, two tiles: 30 us).
+// A thread has eight channels of a token, a block 16 tokens of a (batch, head) pair.  Bound by the partials' trip from memory
+// (144 MB with the results for 4680 tokens, 12 heads, two tiles: 20 us).
 __global__ void __launch_bounds__(256) bwd_merge_kv_kernel(const float* __restrict__ part_k, const float* __restrict__ part_v,
                                                            __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
                                                            int tiles, int n_sel, MonarchParams mp, FastDiv by_blocks, FastDiv by_group, int natural) {

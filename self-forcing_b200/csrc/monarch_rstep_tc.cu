@@ -25,7 +25,7 @@
 // slower (first chunk 33 -> 39 us), and K / V by cp.async instead do not help (31 -> 35).
 // The epilogue's hand-over of an accumulator comes before its stores, aL and Y each have their own, and the working
 // warpgroups have 104 registers instead of 96 (a few dozen spilled bytes a thread go through an L1 that is all shared memory:
-// 160 -> 190 us), none of which is spilled in any instance.  framewise,
+// 160 -> 190 us), none of which is spilled in any instance (the loading warps of 18 instances spill one word).  framewise,
 // 21 cached frames, 12 heads 0.167 -> 0.158 ms; reduce2xh, 9 frames, 4 videos 0.527 -> 0.490;
 // reduce4xw2xh, 21 frames 1.15 -> 1.09; a pass of the iterative variant, first chunk, 31.7 -> 25.4 us.
 // Tried and slower: results to TMA as 5-D boxes of both halves (158 -> 179 us), three staging buffers a warp (same), all
